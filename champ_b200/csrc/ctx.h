@@ -92,6 +92,9 @@ struct champ_ctx {
   int el_wpb[3] = {4, 4, 4};
   size_t el_smem[3] = {0, 0, 0};
   int el_nscr = 0;
+  // its Jastrow part on the tensor cores (eltile.cu): warps per walker (0: k_el_jas) and shared memory
+  int jas_wpw = 0;
+  size_t jas_smem = 0;
   // device staging for per-call host arrays
   double *d_in = nullptr, *d_out = nullptr;
   uint8_t *d_mask = nullptr;
@@ -205,6 +208,10 @@ struct OpArgs {
   bool dmc = false;
 };
 
+
+// the staged evaluation's tensor-core parts (eltile.cu)
+int el_tile_setup(champ_ctx *c);
+int el_tile_jas(champ_ctx *c, const State<double> &st, bool vo);
 
 // kernel launchers per (compute type, e-e-n order), one translation unit each (inst_*.cu)
 #define CHAMP_DECL(TAG, NORD)                                    \

@@ -757,7 +757,7 @@ static int setup_el_staged(champ_ctx *c) {
   st.el_rt = dalloc<double>(c, W * 2 * c->C * N);
   if (!st.el_vj || !st.el_sc || !st.el_rt) return fail(CHAMP_ENOMEM, "allocation of the staged-evaluation scratch failed");
   c->el_staged = 1;
-  return CHAMP_OK;
+  return el_tile_setup(c);
 }
 
 // Delayed inverse updates of the moves (struct Delay) for a walker state in HBM: room for up to

@@ -138,8 +138,11 @@ static int run_el_staged(champ_ctx *c, const State<T> &st, bool outputs, bool st
     const int W = st.W, sm = c->num_sms > 0 ? c->num_sms : 148;
     const int w0 = c->el_wpb[0], w1 = c->el_wpb[1], w2 = c->el_wpb[2];
     const bool vo = rebuild && !outputs && !stats;  // the moves' state only: no velocities, no E_L
-    if (vo) k_el_jas<T, NORD, true><<<(W + w0 - 1) / w0, 32 * w0, c->el_smem[0], c->stream>>>(s, st);
+    int rc = CHAMP_OK;
+    if (c->jas_wpw) rc = el_tile_jas(c, st, vo);
+    else if (vo) k_el_jas<T, NORD, true><<<(W + w0 - 1) / w0, 32 * w0, c->el_smem[0], c->stream>>>(s, st);
     else k_el_jas<T, NORD><<<(W + w0 - 1) / w0, 32 * w0, c->el_smem[0], c->stream>>>(s, st);
+    if (rc) return rc;
     CK(cudaGetLastError());
     const long long items = (long long)W * c->N;
     const long long g1 = std::min<long long>((items + w1 - 1) / w1, (long long)sm * 64);

@@ -1,0 +1,49 @@
+"""The staged evaluation's tensor-core parts at the edges of their tiles, against the CPU oracle:
+electrons around multiples of 8 and 32, one centre to more than a tile of them, both e-e-n orders, spins
+of unequal size.  Every sum is FP64 in both, so the tolerance is the parity tests' 1e-9 relative."""
+import dataclasses
+
+import numpy as np
+import pytest
+
+from champ_b200 import system as S
+
+pytestmark = pytest.mark.gpu
+
+CASES = [  # electrons, up electrons, centres, e-e-n order
+    (13, 7, 1, 4), (16, 8, 2, 5), (17, 9, 3, 4), (31, 16, 5, 5), (32, 16, 4, 4), (33, 17, 9, 4), (40, 24, 7, 5),
+    (51, 26, 13, 5), (64, 32, 33, 4), (65, 33, 17, 4), (72, 40, 12, 0), (127, 64, 32, 4), (128, 64, 40, 5),
+]
+
+
+def cluster(n, nup, ncent, nordc):
+    s = S.cluster128(ncent=ncent, box=14.0 * (max(ncent, 4) / 32) ** (1 / 3), norb=max(nup, n - nup))
+    j = S._jastrow(np.random.default_rng(3), 1, 5, 5, nordc)
+    return dataclasses.replace(s, nelec=n, nup=nup, nordc=nordc, een_cusp=j["een_cusp"], c=j["c"],
+                               det_orb=np.array([list(range(nup)) + list(range(n - nup))], np.int32))
+
+
+@pytest.mark.parametrize("n,nup,ncent,nordc", CASES)
+def test_evaluation_matches_oracle(oracle_mod, n, nup, ncent, nordc):
+    from champ_b200.engine import Engine
+    s = cluster(n, nup, ncent, nordc)
+    nw = 3
+    x = S.initial_walkers(s, nw, seed=n)
+    orc = oracle_mod.Oracle(s)
+    for prec in ("fp64", "mixed"):
+        eng = Engine(s, nw, prec)
+        eng.set_walkers(x)
+        r = eng.eval_full()
+        for w in range(nw):
+            o = orc.eval(x[w])
+            scale = max(1.0, abs(o["energy"]), abs(o["d2lnpsi"]))
+            assert abs(r["lnpsi"][w] - o["lnpsi"]) <= 1e-9 * max(1.0, abs(o["lnpsi"]))
+            assert abs(r["psij"][w] - o["psij"]) <= 1e-9 * max(1.0, abs(o["psij"]))
+            assert r["sign"][w] == o["sign"]
+            assert abs(r["pe_nonloc"][w] - o["pe_nonloc"]) <= 1e-9 * scale
+            assert abs(r["energy"][w] - o["energy"]) <= 1e-9 * scale
+            assert abs(r["d2lnpsi"][w] - o["d2lnpsi"]) <= 1e-9 * scale
+            vs = np.abs(o["vel"]).max()
+            assert np.abs(r["velocity"][w] - o["vel"]).max() <= 1e-9 * vs
+            assert np.abs(r["div_v"][w] - o["div_v"]).max() <= 1e-9 * max(scale, np.abs(o["div_v"]).max())
+        eng.close()
