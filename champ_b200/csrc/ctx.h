@@ -92,9 +92,13 @@ struct champ_ctx {
   int el_wpb[3] = {4, 4, 4};
   size_t el_smem[3] = {0, 0, 0};
   int el_nscr = 0;
-  // its Jastrow part on the tensor cores (eltile.cu): warps per walker (0: k_el_jas) and shared memory
+  // its tensor-core parts (eltile.cu): warps per walker and shared memory of the Jastrow part (0:
+  // k_el_jas), orbital tiles of 16 per block and chunks of shells (0: k_el_orb), rows of the inversion
   int jas_wpw = 0;
   size_t jas_smem = 0;
+  int orb_nt = 0, orb_nchunk = 0;
+  int4 *orb_chunk = nullptr;
+  int inv_nm = 64;
   // device staging for per-call host arrays
   double *d_in = nullptr, *d_out = nullptr;
   uint8_t *d_mask = nullptr;
@@ -212,6 +216,8 @@ struct OpArgs {
 // the staged evaluation's tensor-core parts (eltile.cu)
 int el_tile_setup(champ_ctx *c);
 int el_tile_jas(champ_ctx *c, const State<double> &st, bool vo);
+int el_tile_orb(champ_ctx *c, const State<double> &st);
+int el_tile_inv(champ_ctx *c, const State<double> &st);
 
 // kernel launchers per (compute type, e-e-n order), one translation unit each (inst_*.cu)
 #define CHAMP_DECL(TAG, NORD)                                    \

@@ -4,8 +4,8 @@
 //             divergence of its velocity, pair table, Coulomb energies;
 //   k_el_orb  warp per (walker, electron): basis functions and orbitals with their gradients and
 //             Laplacians, and the Slater-matrix row;
-//   k_el_inv  block per (walker, spin): Gauss-Jordan inversion of the Slater matrix in shared
-//             memory, log-determinant and sign;
+//   k_inv_reg (orbtile.cuh) block per (walker, spin): Gauss-Jordan inversion of the Slater matrix
+//             in registers, log-determinant and sign;
 //   k_el_fin  warp per walker: multi-determinant tables, velocities, pseudopotential, E_L, and
 //             the FP32 move tables of a mixed-precision state.
 // The parts exchange per-walker intermediates through HBM (State::el_vj, el_sc, el_rt).  Each
@@ -100,97 +100,6 @@ __global__ void __launch_bounds__(128, 4) k_el_orb(Sys<T> s, State<T> st, int co
     for (int k = lane; k < n; k += 32) A[eo * n + k] = (double)oe[k];
     __syncwarp();
   }
-}
-
-// Gauss-Jordan inversion with partial pivoting of one walker's Slater matrix of one spin by a
-// block, in shared memory; the same steps, pivot choice and element updates as warp_gj (matinv,
-// qmc/vmc/matinv.f90).  Writes the inverse ([orbital][electron]) back, and ln|D| and sign(D)
-// (0 for a singular matrix) to sc[4 + 2 sp], sc[5 + 2 sp].
-static __global__ void __launch_bounds__(128) k_el_inv(double *ainv, int astride, int nup, int ndn, int W, double *scr) {
-  extern __shared__ __align__(16) double A[];
-  __shared__ int perm[CHAMP_MAX_SPIN];
-  __shared__ int s_piv, s_fail;
-  const int w = blockIdx.x >> 1, sp = blockIdx.x & 1;
-  if (w >= W) return;
-  const int n = sp ? ndn : nup, tid = threadIdx.x, nt = blockDim.x;
-  double *out = scr + (size_t)w * 8 + 4 + 2 * sp;
-  if (n == 0) {
-    if (tid == 0) { out[0] = 0.0; out[1] = 1.0; }
-    return;
-  }
-  double *g = ainv + (size_t)w * astride + (sp ? nup * nup : 0);
-  const int nn = n * n;
-  for (int i = tid; i < nn; i += nt) A[i] = g[i];
-  __syncthreads();
-  // this thread's first element of the elimination and its step through the matrix
-  const int i0 = tid / n, j0 = tid - i0 * n, di = nt / n, dj = nt - di * n;
-  double lnd = 0, sg = 1;
-  for (int k = 0; k < n; k++) {
-    if (tid < 32) {
-      double best = -1.0;
-      int bi = k;
-      for (int i = k + tid; i < n; i += 32) {
-        const double v = fabs(A[i * n + k]);
-        if (v > best) { best = v; bi = i; }
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-      }
-      if (tid == 0) {
-        s_piv = bi;
-        s_fail = !(best > 0.0);
-        perm[k] = bi;
-      }
-    }
-    __syncthreads();
-    if (s_fail) break;
-    const int bi = s_piv;
-    if (bi != k) {
-      for (int j = tid; j < n; j += nt) {
-        const double t = A[k * n + j];
-        A[k * n + j] = A[bi * n + j];
-        A[bi * n + j] = t;
-      }
-      sg = -sg;
-    }
-    __syncthreads();
-    const double piv = A[k * n + k];
-    lnd += log(fabs(piv));
-    if (piv < 0) sg = -sg;
-    const double pinv = 1.0 / piv;
-    __syncthreads();
-    for (int j = tid; j < n; j += nt) A[k * n + j] = (j == k) ? pinv : A[k * n + j] * pinv;
-    __syncthreads();
-    for (int idx = tid, i = i0, j = j0; idx < nn; idx += nt) {
-      if (i != k && j != k) A[idx] -= A[i * n + k] * A[k * n + j];
-      i += di;
-      j += dj;
-      if (j >= n) { j -= n; i++; }
-    }
-    __syncthreads();
-    for (int i = tid; i < n; i += nt)
-      if (i != k) A[i * n + k] = -A[i * n + k] * pinv;
-    __syncthreads();
-  }
-  if (s_fail) {
-    if (tid == 0) { out[0] = 0.0; out[1] = 0.0; }
-    return;
-  }
-  for (int k = n - 1; k >= 0; k--) {
-    const int p = perm[k];
-    if (p != k)
-      for (int i = tid; i < n; i += nt) {
-        const double t = A[i * n + k];
-        A[i * n + k] = A[i * n + p];
-        A[i * n + p] = t;
-      }
-    __syncthreads();
-  }
-  for (int i = tid; i < nn; i += nt) g[i] = A[i];
-  if (tid == 0) { out[0] = lnd; out[1] = sg; }
 }
 
 // Rotation of the quadrature grid: per walker and sweep (VMC) or one for all walkers.

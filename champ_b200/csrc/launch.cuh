@@ -42,7 +42,6 @@ static int set_smem_attrs(champ_ctx *c) {
     if (!rc) rc = set_attrs(c, k_el_jas<T, NORD, true>, c->el_smem[0]);
     if (!rc) rc = set_attrs(c, k_el_orb<T>, c->el_smem[1]);
     if (!rc) rc = set_attrs(c, k_el_fin<T, NORD, MD>, c->el_smem[2]);
-    if (!rc) rc = set_attrs(c, k_el_inv, sizeof(double) * CHAMP_MAX_SPIN * CHAMP_MAX_SPIN);
   }
   if (!rc && c->smem_pg > 0) {
     for (auto kern : {k_pgrad<T, NORD, MD, 1>, k_pgrad<T, NORD, MD, 2>, k_pgrad<T, NORD, MD, 3>, k_pgrad<T, NORD, MD, 4>}) {
@@ -144,14 +143,17 @@ static int run_el_staged(champ_ctx *c, const State<T> &st, bool outputs, bool st
     else k_el_jas<T, NORD><<<(W + w0 - 1) / w0, 32 * w0, c->el_smem[0], c->stream>>>(s, st);
     if (rc) return rc;
     CK(cudaGetLastError());
-    const long long items = (long long)W * c->N;
-    const long long g1 = std::min<long long>((items + w1 - 1) / w1, (long long)sm * 64);
-    k_el_orb<T><<<(unsigned)std::max<long long>(g1, 1), 32 * w1, c->el_smem[1], c->stream>>>(
-        s, st, c->orb_coop && c->orb_coop_ok, c->orb_stage);
-    CK(cudaGetLastError());
-    const int nmax = std::max(c->nup, c->ndn);
-    k_el_inv<<<2 * W, 128, sizeof(double) * nmax * nmax, c->stream>>>(st.ainv, st.astride, c->nup, c->ndn, W, st.el_sc);
-    CK(cudaGetLastError());
+    if (c->orb_nt) {
+      rc = el_tile_orb(c, st);
+    } else {
+      const long long items = (long long)W * c->N;
+      const long long g1 = std::min<long long>((items + w1 - 1) / w1, (long long)sm * 64);
+      k_el_orb<T><<<(unsigned)std::max<long long>(g1, 1), 32 * w1, c->el_smem[1], c->stream>>>(
+          s, st, c->orb_coop && c->orb_coop_ok, c->orb_stage);
+      CK(cudaGetLastError());
+    }
+    if (!rc) rc = el_tile_inv(c, st);
+    if (rc) return rc;
     k_el_fin<T, NORD, MD><<<(W + w2 - 1) / w2, 32 * w2, c->el_smem[2], c->stream>>>(
         s, st, c->el_nscr, outputs ? 1 : 0, stats ? 1 : 0, rot, vo ? 1 : 0);
     CK(cudaGetLastError());

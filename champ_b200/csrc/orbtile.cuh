@@ -1,0 +1,267 @@
+// orbtile.cuh -- basis functions and orbitals of every electron (value, gradient, Laplacian) for the
+// staged evaluation, as FP64 tensor-core products, and the Slater-matrix inversion in registers.
+#pragma once
+#include "kernels.cuh"
+
+namespace ot {
+
+constexpr int EB = 32;      // electrons of a block (one per lane while the basis is formed)
+constexpr int ROWS = 5 * EB;
+constexpr int LDA = ROWS + 4;  // = 4 mod 16 doubles: the fragment loads hit different banks
+constexpr int KB = 32;      // basis functions of a chunk (whole shells, padded to a multiple of 4)
+constexpr int THREADS = 256;
+
+template <int NT>
+__host__ __device__ constexpr int ldb() { return 16 * NT + 4; }
+template <int NT>
+__host__ __device__ constexpr size_t smem_bytes() { return sizeof(double) * (size_t)KB * (LDA + ldb<NT>()); }
+
+// A Gaussian shell with n = l + 1, l <= 2: S_lm(d) g(r^2), g = sum_p w e^(-z r^2); no square root or division.
+// grad = grad S g + 2 d S g', lap = S (4 r^2 g'' + (4l + 6) g').
+template <int l, class Put>
+__device__ __forceinline__ void gauss_shell5(const Sys<double> &s, int2 pr, double d0, double d1, double d2, Put put) {
+  const double r2 = d0 * d0 + d1 * d1 + d2 * d2;
+  double g = 0, gp = 0, gpp = 0;
+  for (int p = pr.x; p < pr.x + pr.y; p++) {
+    const double z = s.pz[p], e = s.pc[p] * exp(-z * r2);
+    g += e;
+    gp -= z * e;
+    gpp += z * z * e;
+  }
+  const double lp = 4 * r2 * gpp + (4 * l + 6) * gp, t = 2 * gp;
+  double S[9], G[9][3];
+  solid_all<double, true>(l, d0, d1, d2, S, G);
+  const int nm = 2 * l + 1;
+#pragma unroll
+  for (int sl = 0; sl < 9; sl++)
+    if (sl < nm) {
+      const double st = S[sl] * t;
+      put(sl, 0, S[sl] * g);
+      put(sl, 1, G[sl][0] * g + st * d0);
+      put(sl, 2, G[sl][1] * g + st * d1);
+      put(sl, 3, G[sl][2] * g + st * d2);
+      put(sl, 4, S[sl] * lp);
+    }
+}
+
+// Any other shell (kept out of line: its registers are not those of the contraction).
+static __device__ __noinline__ void general_shell5(const Sys<double> &s, int ish, double x, double y, double z, double *o) {
+  const double pt[3] = {x, y, z};
+  shell_eval_put<double, 5>(s, ish, pt, [o](int sl, int c, double v) { o[sl * LDA + c * EB] = v; });
+}
+
+// Orbitals of 32 electrons of one spin (grid.y) per block: chunks of basis functions are formed in
+// shared memory (lane = electron, a warp per shell, so that every lane runs the same shell) and
+// contracted with the spin's coefficients by mma m8n8k4: 160 rows (5 channels x 32 electrons) by
+// 16 NT orbitals, 8 warps as 4 (rows) x 2 (orbitals), 5 x NT tiles each.  The coefficients of a
+// chunk arrive by cp.async while its basis functions are formed and are shared by the 32
+// electrons (the warp-per-electron contraction streamed them from L2 once per 4 electrons).
+// What bounds it: the FP64 pipe (about a fifth of it the basis functions).  Measured (B200): 4096
+// walkers of 128 electrons, 416 basis functions, 15.6 -> 7.1 ms; 3001 of 20 electrons, 65 functions,
+// 0.32 -> 0.08 ms.  k_el_orb stays for more than 64 orbitals of a spin.
+// chunk[k]: first shell, shells, first basis function, basis functions.
+template <int NT>
+__global__ void __launch_bounds__(THREADS, 2) k_orb_tile(const __grid_constant__ Sys<double> s, State<double> st, const int4 *chunk, int nchunk) {
+  extern __shared__ __align__(16) double sm[];
+  double *phi = sm, *cf = sm + KB * LDA;
+  constexpr int LDB = ldb<NT>();
+  const int sp = blockIdx.y, n = sp ? s.ndn : s.nup, no = s.nocc[sp], e0 = sp ? s.nup : 0;
+  const long long items = (long long)st.W * n, i0 = (long long)blockIdx.x * EB;
+  if (i0 >= items) return;
+  const int tid = threadIdx.x, lane = tid & 31, wib = tid >> 5, rr = lane >> 2, kq = lane & 3;
+  const int wm = wib >> 1, wn = wib & 1;
+  const double *coef = s.cocc[sp];
+  double px[3] = {0, 0, 0};
+  {
+    long long it = i0 + lane;
+    if (it >= items) it = items - 1;  // the last block's spare lanes repeat its last electron
+    const int w = (int)(it / n), e = e0 + (int)(it - (long long)w * n);
+    const double *x = st.x + ((size_t)w * s.N + e) * 3;
+    px[0] = x[0]; px[1] = x[1]; px[2] = x[2];
+  }
+  const bool vec = no % 2 == 0 && (reinterpret_cast<uintptr_t>(coef) & 15) == 0;
+  double acc[5][NT][2];
+#pragma unroll
+  for (int i = 0; i < 5; i++)
+#pragma unroll
+    for (int j = 0; j < NT; j++) acc[i][j][0] = acc[i][j][1] = 0;
+  for (int k = 0; k < nchunk; k++) {
+    const int4 ch = chunk[k];
+    const int nk4 = (ch.w + 3) & ~3;
+    // coefficients of the chunk: rows [k][16 NT], zero past the orbitals and the basis functions
+    if (vec) {
+      constexpr int V = 8 * NT;
+      for (int i = tid; i < nk4 * V; i += THREADS) {
+        const int r = i / V, c = 2 * (i - r * V);
+        double *dst = cf + r * LDB + c;
+        if (r < ch.w && c < no) cp_async16(dst, coef + (size_t)(ch.z + r) * no + c);
+        else dst[0] = dst[1] = 0.0;
+      }
+    } else {
+      for (int i = tid; i < nk4 * 16 * NT; i += THREADS) {
+        const int r = i / (16 * NT), c = i - r * (16 * NT);
+        cf[r * LDB + c] = (r < ch.w && c < no) ? coef[(size_t)(ch.z + r) * no + c] : 0.0;
+      }
+    }
+    cp_async_commit();
+    for (int r = ch.w + wib; r < nk4; r += 8)
+#pragma unroll
+      for (int c = 0; c < 5; c++) phi[r * LDA + c * EB + lane] = 0.0;
+    for (int q = wib; q < ch.y; q += 8) {
+      const int ish = ch.x + q;
+      const int4 sh = s.shell[ish];
+      double *o = phi + (s.shb0[ish] - ch.z) * LDA + lane;
+      auto put = [o](int sl, int c, double v) { o[sl * LDA + c * EB] = v; };
+      if (sh.w == 1 && sh.y == sh.z + 1) {
+        const double *cc = s.cent + 3 * sh.x;
+        const double d0 = px[0] - cc[0], d1 = px[1] - cc[1], d2 = px[2] - cc[2];
+        const int2 pr = s.shprim[ish];
+        switch (sh.z) {
+        case 0: gauss_shell5<0>(s, pr, d0, d1, d2, put); break;
+        case 1: gauss_shell5<1>(s, pr, d0, d1, d2, put); break;
+        case 2: gauss_shell5<2>(s, pr, d0, d1, d2, put); break;
+        default: general_shell5(s, ish, px[0], px[1], px[2], o);
+        }
+      } else {
+        general_shell5(s, ish, px[0], px[1], px[2], o);
+      }
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    const double *ap = phi + kq * LDA + wm * 40 + rr, *bp = cf + kq * LDB + wn * 8 * NT + rr;
+    for (int ks = 0; ks < nk4; ks += 4) {
+      double a[5], b[NT];
+#pragma unroll
+      for (int i = 0; i < 5; i++) a[i] = ap[ks * LDA + 8 * i];
+#pragma unroll
+      for (int j = 0; j < NT; j++) b[j] = bp[ks * LDB + 8 * j];
+#pragma unroll
+      for (int i = 0; i < 5; i++)
+#pragma unroll
+        for (int j = 0; j < NT; j++) dmma_884(acc[i][j][0], acc[i][j][1], a[i], b[j]);
+    }
+    __syncthreads();
+  }
+  const int nomax = s.nomax;
+#pragma unroll
+  for (int i = 0; i < 5; i++) {
+    const int row = wm * 40 + 8 * i + rr, ch = row / EB;
+    const long long it = i0 + (row - ch * EB);
+    if (it >= items) continue;
+    const int w = (int)(it / n), eo = (int)(it - (long long)w * n);
+    double *o = st.orb5 + (((size_t)w * s.N + e0 + eo) * 5 + ch) * nomax;
+    double *A = st.ainv + (size_t)w * st.astride + (sp ? s.nup * s.nup : 0) + (size_t)eo * n;
+#pragma unroll
+    for (int j = 0; j < NT; j++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int c = wn * 8 * NT + 8 * j + 2 * kq + h;
+        if (c < no) o[c] = acc[i][j][h];
+        if (ch == 0 && c < n) A[c] = acc[i][j][h];
+      }
+  }
+}
+
+// Inversion of the Slater matrices (matinv, qmc/vmc/matinv.f90) in registers: a block of NM threads
+// per (walker, spin), a thread per row, Gauss-Jordan with partial pivoting.  Step k eliminates the
+// column that sits at register 0 and every row then shifts left by one with the new column of the
+// inverse entering on the right, so no register is indexed at run time; rows are not exchanged (the
+// pivot row of step k ends as row k of the inverse, its electron as that row's column).  The
+// pivot row goes through shared memory once per step.  Rows and columns past n are those of the
+// identity.  Replaces the elimination in shared memory, which read and wrote the whole matrix there
+// in each of the n steps: 3.4 -> 1.0 ms for 4096 walkers with 64 x 64 matrices (now the latency of the
+// n pivot steps), 0.087 -> 0.037 ms for 3001 with 10 x 10.
+template <int NM>
+__global__ void __launch_bounds__(NM) k_inv_reg(double *ainv, int astride, int nup, int ndn, int W, double *scr) {
+  constexpr int NW = NM / 32;
+  __shared__ __align__(16) double prow[2][NM];
+  __shared__ double s_best[2][NW], s_ln[NW];
+  __shared__ int s_bi[2][NW], s_piv[NM];
+  const int w = blockIdx.x >> 1, sp = blockIdx.x & 1;
+  if (w >= W) return;
+  const int n = sp ? ndn : nup, t = threadIdx.x, lane = t & 31, wib = t >> 5;
+  double *out = scr + (size_t)w * 8 + 4 + 2 * sp;
+  if (n == 0) {
+    if (t == 0) { out[0] = 0.0; out[1] = 1.0; }
+    return;
+  }
+  double *g = ainv + (size_t)w * astride + (sp ? nup * nup : 0);
+  double a[NM];
+#pragma unroll
+  for (int j = 0; j < NM; j++) a[j] = (t < n && j < n) ? g[t * n + j] : 0.0;
+  bool used = t >= n;
+  double mypiv = 1.0;
+  int mycol = -1;
+  for (int k = 0; k < n; k++) {
+    const int b = k & 1;
+    double best = used ? -1.0 : fabs(a[0]);
+    if (!(best > -1.0)) best = -1.0;  // a NaN is no pivot
+    int bi = t;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+      if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
+    }
+    if (NW > 1) {
+      if (lane == 0) { s_best[b][wib] = best; s_bi[b][wib] = bi; }
+      __syncthreads();
+#pragma unroll
+      for (int q = 0; q < NW; q++)
+        if (s_best[b][q] > best || (s_best[b][q] == best && s_bi[b][q] < bi)) { best = s_best[b][q]; bi = s_bi[b][q]; }
+    }
+    if (!(best > 0.0)) {  // singular (every thread sees the same): the matrix stays as it is
+      if (t == 0) { out[0] = 0.0; out[1] = 0.0; }
+      return;
+    }
+    if (t == bi) {
+      used = true;
+      mypiv = a[0];
+      mycol = k;
+      s_piv[k] = t;
+      const double pinv = 1.0 / a[0];
+#pragma unroll
+      for (int j = 1; j < NM; j++) a[j - 1] = a[j] * pinv;
+      a[NM - 1] = pinv;
+#pragma unroll
+      for (int j = 0; j < NM; j += 2) *(double2 *)&prow[b][j] = make_double2(a[j], a[j + 1]);
+    }
+    __syncthreads();
+    if (t != bi) {
+      const double f = a[0];
+#pragma unroll
+      for (int j = 0; j < NM; j += 2) {
+        const double2 p = *(const double2 *)&prow[b][j];
+        a[j] = (j + 1 < NM ? a[j + 1] : 0.0) - f * p.x;
+        a[j + 1] = (j + 2 < NM ? a[j + 2] : 0.0) - f * p.y;
+      }
+    }
+  }
+  __syncthreads();
+  // row of step mycol: inverse[mycol][electron of step m] = a[NM - n + m]
+  if (t < n) {
+#pragma unroll
+    for (int j = 0; j < NM; j++) {
+      const int m = j - (NM - n);
+      if (m >= 0) g[mycol * n + s_piv[m]] = a[j];
+    }
+  }
+  // ln|D| = sum ln|pivot|; sign: pivots below zero and the parity of the row order
+  double ln = t < n ? log(fabs(mypiv)) : 0.0;
+  int neg = (t < n && mypiv < 0) ? 1 : 0;
+  if (t < n)
+    for (int m = 0; m < mycol; m++) neg += s_piv[m] > t;  // inversions of the permutation
+  ln = warp_sum(ln);
+  neg = warp_sum(neg);
+  if (lane == 0) { s_ln[wib] = ln; s_bi[0][wib] = neg; }
+  __syncthreads();
+  if (t == 0) {
+    double l = 0;
+    int q = 0;
+    for (int i = 0; i < NW; i++) { l += s_ln[i]; q += s_bi[0][i]; }
+    out[0] = l;
+    out[1] = (q & 1) ? -1.0 : 1.0;
+  }
+}
+
+}  // namespace ot
