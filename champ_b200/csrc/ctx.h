@@ -99,6 +99,7 @@ struct champ_ctx {
   int orb_nt = 0, orb_nchunk = 0;
   int4 *orb_chunk = nullptr;
   int inv_nm = 64;
+  int move_batch = 0;  // the Gaussian sweeps run as batched moves
   // device staging for per-call host arrays
   double *d_in = nullptr, *d_out = nullptr;
   uint8_t *d_mask = nullptr;
@@ -218,6 +219,9 @@ int el_tile_setup(champ_ctx *c);
 int el_tile_jas(champ_ctx *c, const State<double> &st, bool vo);
 int el_tile_orb(champ_ctx *c, const State<double> &st);
 int el_tile_inv(champ_ctx *c, const State<double> &st);
+// batched Gaussian single-electron moves (movebatch.cu); setup sets champ_ctx::move_batch where they apply
+int move_batch_setup(champ_ctx *c);
+int move_batch_sweep(champ_ctx *c, uint64_t seed, uint64_t isweep, double step);
 
 // kernel launchers per (compute type, e-e-n order), one translation unit each (inst_*.cu)
 #define CHAMP_DECL(TAG, NORD)                                    \

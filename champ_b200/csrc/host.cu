@@ -1506,6 +1506,7 @@ int champ_create(const champ_system *d, int32_t w_max, int32_t precision, void *
       else m = KCfg{};
     }
   }
+  if (use64 && !rc) rc = move_batch_setup(c);
   if (rc) { champ_destroy(c); return rc; }
   c->nfree = c->ncsfp + c->norbp + c->nparm_jas;
   {

@@ -239,6 +239,8 @@ static int launch_t(champ_ctx *c, Op op, const OpArgs &a) {
     }
     if (a.phase >= 0) {
       const bool acc6 = c->mover.kind == 6;
+      if (a.phase == 1 && !acc6 && c->move_batch && c->el_staged && !a.st_override)
+        return move_batch_sweep(c, a.seed, a.sweep0, a.step);  // every phase-1 launch is one sweep
       auto kern = a.phase == 1 ? (acc6 ? k_vmc<T, NORD, MD, 1, 6> : k_vmc<T, NORD, MD, 1>)
                 : a.phase == 2 ? k_vmc<T, NORD, MD, 2>
                 : a.phase == 3 ? k_vmc<T, NORD, MD, 3> : (acc6 ? k_vmc<T, NORD, MD, 0, 6> : k_vmc<T, NORD, MD, 0>);

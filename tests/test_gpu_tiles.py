@@ -47,3 +47,31 @@ def test_evaluation_matches_oracle(oracle_mod, n, nup, ncent, nordc):
             assert np.abs(r["velocity"][w] - o["vel"]).max() <= 1e-9 * vs
             assert np.abs(r["div_v"][w] - o["div_v"]).max() <= 1e-9 * max(scale, np.abs(o["div_v"]).max())
         eng.close()
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("n,nup,ncent,nordc", [c for c in CASES if c[0] > 16])
+def test_batched_moves_walk_as_single_moves(n, nup, ncent, nordc, prec):
+    """Two sweeps of batched moves against the same sweeps move by move (staged evaluation off): the
+    same decisions, so the same positions.  The two differ in the order of FP64 sums (and with it now
+    and then in an FP32 table's last bit), 1e-7 of a decision's probability at most: of 64 walkers and
+    256 decisions each, one walker may differ."""
+    from champ_b200.engine import Engine
+    s = cluster(n, nup, ncent, nordc)
+    x = S.initial_walkers(s, 64, seed=n + 1)
+    out = []
+    for staged in (1, 0):
+        eng = Engine(s, 64, prec)
+        eng.set_walkers(x)
+        if not eng.get_option("staged_eval"):
+            pytest.skip("walker state of this system is resident in shared memory")
+        if not staged:
+            eng.set_option("staged_eval", 0)
+            eng.set_option("reinvert_every", 1)
+        st = eng.vmc_sweeps(2, seed=5, sweep0=3, step=s.step)
+        out.append((eng.get_walkers(), st["accept"]))
+        eng.close()
+    same = np.abs(out[0][0] - out[1][0]).max(axis=(1, 2)) <= 1e-12
+    assert same.sum() >= 63, same.sum()
+    assert np.array_equal(out[0][1][same], out[1][1][same])
+    assert 0 < out[0][1].sum() < 64 * 2 * n
