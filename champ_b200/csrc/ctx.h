@@ -99,6 +99,11 @@ struct champ_ctx {
   int orb_nt = 0, orb_nchunk = 0;
   int4 *orb_chunk = nullptr;
   int inv_nm = 64;
+  // last part (0: k_el_fin): warps per walker, shared memory, radial values of tasks kept there, and
+  // every shell's smallest exponent
+  int fin_wpw = 0, fin_nrow = 0;
+  size_t fin_smem = 0;
+  double *shell_zmin = nullptr;
   int move_batch = 0;  // the Gaussian sweeps run as batched moves
   // device staging for per-call host arrays
   double *d_in = nullptr, *d_out = nullptr;
@@ -219,6 +224,7 @@ int el_tile_setup(champ_ctx *c);
 int el_tile_jas(champ_ctx *c, const State<double> &st, bool vo);
 int el_tile_orb(champ_ctx *c, const State<double> &st);
 int el_tile_inv(champ_ctx *c, const State<double> &st);
+int el_tile_fin(champ_ctx *c, const State<double> &st, bool outputs, bool stats, const ElRot &rot, bool tables_only);
 // batched Gaussian single-electron moves (movebatch.cu); setup sets champ_ctx::move_batch where they apply
 int move_batch_setup(champ_ctx *c);
 int move_batch_sweep(champ_ctx *c, uint64_t seed, uint64_t isweep, double step);

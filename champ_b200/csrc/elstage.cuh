@@ -1,16 +1,16 @@
-// elstage.cuh -- the full evaluation (hpsi) of walkers whose state lives in HBM, as four kernels
-// that each run at the occupancy their own part allows:
-//   k_el_jas  warp per walker: distances to the centres, Jastrow factor, its gradient and the
-//             divergence of its velocity, pair table, Coulomb energies;
-//   k_el_orb  warp per (walker, electron): basis functions and orbitals with their gradients and
-//             Laplacians, and the Slater-matrix row;
-//   k_inv_reg (orbtile.cuh) block per (walker, spin): Gauss-Jordan inversion of the Slater matrix
-//             in registers, log-determinant and sign;
-//   k_el_fin  warp per walker: multi-determinant tables, velocities, pseudopotential, E_L, and
-//             the FP32 move tables of a mixed-precision state.
-// The parts exchange per-walker intermediates through HBM (State::el_vj, el_sc, el_rt).  Each
-// part runs the same device code as the single-kernel evaluation (full_eval), so both give the
-// same results up to the order of floating-point sums.
+// elstage.cuh -- the full evaluation (hpsi) of walkers whose state lives in HBM, as kernels that each
+// run at the occupancy their own part allows:
+//   Jastrow   distances to the centres, Jastrow factor, its gradient and the divergence of its
+//             velocity, pair table, Coulomb energies: k_jas_tile (jastile.cuh; one centre type with e-e-n
+//             terms), else k_el_jas, a warp per walker;
+//   orbitals  basis functions and orbitals with their gradients and Laplacians, and the Slater
+//             matrices: k_orb_tile (orbtile.cuh; up to 64 orbitals of a spin), else k_el_orb;
+//   inverse   k_inv_reg (orbtile.cuh): Gauss-Jordan in registers, log-determinant and sign;
+//   the rest  multi-determinant tables, velocities, pseudopotential, E_L, and the FP32 move tables of
+//             a mixed-precision state: k_gproj and k_fin_points (nlpoints.cuh), else (several centre
+//             types with e-e-n terms) k_el_fin, a warp per walker.
+// The parts exchange per-walker intermediates through HBM (State::el_vj, el_sc, el_rt) and give the
+// single-kernel evaluation's (full_eval) results up to the order of floating-point sums.
 #pragma once
 
 // Per-warp dynamic shared memory of the parts (bytes).
@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(128, 4) k_el_jas(Sys<T> s, State<T> st) {
     for (int i = lane; i < 3 * N; i += 32) vj[i] = v.vacc[i];
     for (int i = lane; i < N; i += 32) vj[3 * N + i] = v.divj[i];
     if (lane == 0) {
-      double *sc = st.el_sc + (size_t)w * 8;
+      double *sc = st.el_sc + (size_t)w * EL_SC;
       sc[0] = fsum;
       sc[1] = d2j;
       sc[2] = pe_ee;
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(128, 4) k_el_fin(Sys<T> s, State<T> st, int ns
     v.wdet = st.wdet + (size_t)w * st.wstride;
     for (int i = lane; i < 3 * N; i += 32) v.xs[i] = st.x[(size_t)w * 3 * N + i];
     __syncwarp();
-    const double *sc = st.el_sc + (size_t)w * 8;
+    const double *sc = st.el_sc + (size_t)w * EL_SC;
     const double fsum = sc[0], d2j = sc[1], pe_ee = sc[2], pe_en = sc[3];
     double lnd = sc[4] + sc[6], sgn = sc[5] * sc[7];
     const bool ok = sc[5] != 0.0 && sc[7] != 0.0;
@@ -161,8 +161,7 @@ __global__ void __launch_bounds__(128, 4) k_el_fin(Sys<T> s, State<T> st, int ns
       if (rot.random) random_rotation(rot.seed, (uint32_t)w, rot.sweep, R);
       else
         for (int i = 0; i < 9; i++) R[i] = rot.R[i];
-      nlpp_energy<T, NORD, MD, false, true>(s, J, E, v, R, lane, nullptr, scr, nscr, st.el_rt + (size_t)w * 2 * C * N, vloc,
-                                      vnl, ntask);
+      nlpp_energy<T, NORD, MD, false>(s, J, E, v, R, lane, nullptr, scr, nscr, vloc, vnl, ntask);
     }
     EvalRes res;
     finish_eval(s, st, w, v, lane, outputs != 0, ok, lnd, sgn, fsum, d2j, pe_ee, pe_en, d2lnd, v2, vloc, vnl, ntask,

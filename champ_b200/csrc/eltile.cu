@@ -4,12 +4,28 @@
 #include "ctx.h"
 #include "jastile.cuh"
 #include "orbtile.cuh"
+#include "nlpoints.cuh"
 
 template <class K>
 static int big_smem(K kern, size_t bytes) {
   CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
   CK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
   return CHAMP_OK;
+}
+
+template <int NORD>
+static int fin_attrs_n() {
+  int rc = big_smem(pt::k_fin_points<NORD, false, 1>, 200 * 1024);
+  if (!rc) rc = big_smem(pt::k_fin_points<NORD, false, 4>, 200 * 1024);
+  if (!rc) rc = big_smem(pt::k_fin_points<NORD, true, 1>, 200 * 1024);
+  if (!rc) rc = big_smem(pt::k_fin_points<NORD, true, 4>, 200 * 1024);
+  return rc;
+}
+static int fin_attrs(champ_ctx *c) {
+  int rc = c->nordc == 4 ? fin_attrs_n<4>() : c->nordc == 5 ? fin_attrs_n<5>() : fin_attrs_n<0>();
+  if (!rc) rc = big_smem(pt::k_gproj<false>, 200 * 1024);
+  if (!rc) rc = big_smem(pt::k_gproj<true>, 200 * 1024);
+  return rc;
 }
 
 // Which parts serve the context's system, their shared memory, and the chunks of whole shells that
@@ -45,7 +61,36 @@ int el_tile_setup(champ_ctx *c) {
     c->orb_nchunk = (int)ch.size();
     c->orb_nt = nomax <= 16 ? 1 : nomax <= 32 ? 2 : 4;
   }
-  int rc = CHAMP_OK;
+  if (c->nordc <= 1 || c->nct == 1) {
+    // every shell's smallest exponent among the primitives that weigh in it
+    std::vector<int2> pr(c->nshell);
+    CK(cudaMemcpy(pr.data(), c->sd.shprim, sizeof(int2) * c->nshell, cudaMemcpyDeviceToHost));
+    int np = 0;
+    for (const int2 &p : pr) np = std::max(np, p.x + p.y);
+    std::vector<double> z(np), wt(np), zm(c->nshell, 0.0);
+    CK(cudaMemcpy(z.data(), c->sd.pz, sizeof(double) * np, cudaMemcpyDeviceToHost));
+    CK(cudaMemcpy(wt.data(), c->sd.pc, sizeof(double) * np, cudaMemcpyDeviceToHost));
+    for (int i = 0; i < c->nshell; i++) {
+      double wmax = 0, m = 1e300;
+      for (int p = pr[i].x; p < pr[i].x + pr[i].y; p++) wmax = std::max(wmax, std::fabs(wt[p]));
+      for (int p = pr[i].x; p < pr[i].x + pr[i].y; p++)
+        if (std::fabs(wt[p]) >= 1e-8 * wmax) m = std::min(m, z[p]);
+      zm[i] = m < 1e300 ? m : 0.0;
+    }
+    double *d = nullptr;
+    CK(cudaMalloc(&d, sizeof(double) * c->nshell));
+    c->allocs.push_back(d);
+    CK(cudaMemcpy(d, zm.data(), sizeof(double) * c->nshell, cudaMemcpyHostToDevice));
+    c->shell_zmin = d;
+    const int wpw = c->N <= 32 ? 1 : 4;
+    c->fin_nrow = std::min(c->N * c->C * std::max(c->sd.nshc, 1), wpw == 1 ? 256 : 768);
+    const size_t b = pt::Dims(c->N, c->C, c->nordc, c->fin_nrow).bytes() * (wpw == 1 ? 4 : 1);
+    if (b <= 200 * 1024) {
+      c->fin_wpw = wpw;
+      c->fin_smem = b;
+    }
+  }
+  int rc = fin_attrs(c);
   for (auto k : {jt::k_jas_tile<4, 1, false>, jt::k_jas_tile<4, 1, true>, jt::k_jas_tile<4, jt::WARPS, false>,
                  jt::k_jas_tile<4, jt::WARPS, true>, jt::k_jas_tile<5, 1, false>, jt::k_jas_tile<5, 1, true>,
                  jt::k_jas_tile<5, jt::WARPS, false>, jt::k_jas_tile<5, jt::WARPS, true>})
@@ -93,4 +138,33 @@ int el_tile_inv(champ_ctx *c, const State<double> &st) {
   else ot::k_inv_reg<64><<<g, 64, 0, c->stream>>>(st.ainv, st.astride, c->nup, c->ndn, st.W, st.el_sc);
   CK(cudaGetLastError());
   return CHAMP_OK;
+}
+
+template <int NORD, bool MD>
+static int fin(champ_ctx *c, const State<double> &st, bool outputs, bool stats, const ElRot &rot, bool tables_only) {
+  const int W = st.W;
+  if (MD) {
+    pt::k_md_tables<<<(W + 3) / 4, 128, 0, c->stream>>>(c->sd, st);
+    CK(cudaGetLastError());
+  }
+  if (c->nloc > 0 && !tables_only) {
+    const size_t sm = sizeof(double) * pt::GP_LD * (size_t)((c->nomax + 3) & ~3);
+    pt::k_gproj<MD><<<2 * W, 128, sm, c->stream>>>(c->sd, st);
+    CK(cudaGetLastError());
+  }
+  if (c->fin_wpw == 1)
+    pt::k_fin_points<NORD, MD, 1><<<(W + 3) / 4, 128, c->fin_smem, c->stream>>>(c->sd, st, c->shell_zmin, c->fin_nrow, outputs, stats, rot, tables_only);
+  else
+    pt::k_fin_points<NORD, MD, 4><<<W, 128, c->fin_smem, c->stream>>>(c->sd, st, c->shell_zmin, c->fin_nrow, outputs, stats, rot, tables_only);
+  CK(cudaGetLastError());
+  return CHAMP_OK;
+}
+template <int NORD>
+static int fin_n(champ_ctx *c, const State<double> &st, bool outputs, bool stats, const ElRot &rot, bool tables_only) {
+  return c->md.multidet ? fin<NORD, true>(c, st, outputs, stats, rot, tables_only)
+                        : fin<NORD, false>(c, st, outputs, stats, rot, tables_only);
+}
+int el_tile_fin(champ_ctx *c, const State<double> &st, bool outputs, bool stats, const ElRot &rot, bool tables_only) {
+  return c->nordc == 4 ? fin_n<4>(c, st, outputs, stats, rot, tables_only)
+       : c->nordc == 5 ? fin_n<5>(c, st, outputs, stats, rot, tables_only) : fin_n<0>(c, st, outputs, stats, rot, tables_only);
 }

@@ -753,7 +753,7 @@ static int setup_el_staged(champ_ctx *c) {
   const size_t W = c->wmax, N = c->N;
   State<double> &st = c->std_;
   st.el_vj = dalloc<double>(c, W * 4 * N);
-  st.el_sc = dalloc<double>(c, W * 8);
+  st.el_sc = dalloc<double>(c, W * EL_SC);
   st.el_rt = dalloc<double>(c, W * 2 * c->C * N);
   if (!st.el_vj || !st.el_sc || !st.el_rt) return fail(CHAMP_ENOMEM, "allocation of the staged-evaluation scratch failed");
   c->el_staged = 1;

@@ -459,7 +459,7 @@ __global__ void __launch_bounds__(128, NORD > 4 ? 2 : 3) k_jas_tile(Sys<double> 
     if (tid < 4) {
       double a = 0;
       for (int k = 0; k < WPW; k++) a += red[4 * k + tid];
-      st.el_sc[(size_t)w * 8 + tid] = a;
+      st.el_sc[(size_t)w * EL_SC + tid] = a;
     }
     walker_sync<WPW>();
   }

@@ -154,8 +154,10 @@ static int run_el_staged(champ_ctx *c, const State<T> &st, bool outputs, bool st
     }
     if (!rc) rc = el_tile_inv(c, st);
     if (rc) return rc;
-    k_el_fin<T, NORD, MD><<<(W + w2 - 1) / w2, 32 * w2, c->el_smem[2], c->stream>>>(
+    if (c->fin_wpw) rc = el_tile_fin(c, st, outputs, stats, rot, vo);
+    else k_el_fin<T, NORD, MD><<<(W + w2 - 1) / w2, 32 * w2, c->el_smem[2], c->stream>>>(
         s, st, c->el_nscr, outputs ? 1 : 0, stats ? 1 : 0, rot, vo ? 1 : 0);
+    if (rc) return rc;
     CK(cudaGetLastError());
     c->orb5_valid = st.orb5 == c->std_.orb5;  // k_el_orb wrote every electron's row
     return CHAMP_OK;

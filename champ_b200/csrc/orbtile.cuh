@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(NM) k_inv_reg(double *ainv, int astride, int n
   const int w = blockIdx.x >> 1, sp = blockIdx.x & 1;
   if (w >= W) return;
   const int n = sp ? ndn : nup, t = threadIdx.x, lane = t & 31, wib = t >> 5;
-  double *out = scr + (size_t)w * 8 + 4 + 2 * sp;
+  double *out = scr + (size_t)w * EL_SC + 4 + 2 * sp;
   if (n == 0) {
     if (t == 0) { out[0] = 0.0; out[1] = 1.0; }
     return;
