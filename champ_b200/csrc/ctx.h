@@ -62,7 +62,7 @@ struct champ_ctx {
   // value index, 0), 10 parameters (r0, h, log h, c0..c4, a0, ak), values and spline second
   // derivatives of all tables one after another; shell -> table
   std::vector<int4> rad_tab;
-  std::vector<double> rad_par, rad_y, rad_y2;
+  std::vector<double> rad_par, rad_y, rad_y2, rad_cub;
   std::vector<int> rad_shell;
   // opt-in device timing of the VMC sweep kernels (option "phase_timing"): event pairs per
   // launch, summed per phase by champ_phase_times

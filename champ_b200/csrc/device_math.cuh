@@ -67,6 +67,7 @@ struct Sys {
   const int4 *rtab;     // [nrad]
   const double *rpar;   // [nrad][10]
   const T *ry, *ry2;    // [sum nr]
+  const double *rcub;   // [sum nr][6]: grid point, the spline's cubic from there (c0..c3), 0
   // occupied orbitals of each spin: det-0 (reference) orbitals in column order, then the
   // other orbitals any determinant of that spin uses ("virtuals"), ascending
   int nocc[2], nvirt[2], nomax, nvmax;
@@ -517,10 +518,52 @@ __device__ __forceinline__ void solid_all(int l, T x, T y, T z, T *S, T (*G)[3])
 // Numerical radial function f, f', f'' of table t at r (splfit_bas, qmc/vmc/splfit.f90): the
 // grid interval from the grid's closed form, cubic-spline interpolation inside the grid, the
 // small-r polynomial below its first point and the exponential beyond its last.
+// FP64 takes the interval's grid point and cubic from a table (rcub) and finds the interval from an FP32
+// logarithm corrected against the grid, instead of a logarithm, two powers and three divisions per
+// value: the radial functions were most of the numerical-basis kernels.
 template <class T, bool DERIV>
 __device__ __forceinline__ void table_radial(const Sys<T> &s, int t, T r, T *R) {
   const int4 tb = s.rtab[t];
   const double *p = s.rpar + 10 * t;
+  if constexpr (sizeof(T) == 8) {
+    const double *g = s.rcub + 6 * (size_t)tb.z;
+    const double r0 = p[0];
+    // the last grid point at or below r (1-based), 0 below the first
+    int jx;
+    if (tb.x == 1) jx = (int)fmin((r - r0) / p[1] + 1.0, (double)tb.y);
+    else {
+      const float q = (float)r / (float)r0 + (tb.x == 2 ? 0.f : 1.f);
+      jx = q > 0.f ? (int)fminf(__log2f(q) * (0.6931472f / (float)p[2]) + 1.f, (float)tb.y) : 0;
+    }
+    jx = jx < 0 ? 0 : (jx > tb.y ? tb.y : jx);
+    while (jx > 0 && r < g[6 * (jx - 1)]) jx--;
+    while (jx < tb.y && r >= g[6 * jx]) jx++;
+    if (jx >= 1 && jx < tb.y) {
+      const double2 *q = (const double2 *)(g + 6 * (jx - 1));
+      const double2 a = q[0], b = q[1], c = q[2];
+      const double x = r - a.x;
+      R[0] = ((c.x * x + b.y) * x + b.x) * x + a.y;
+      if (DERIV) {
+        R[1] = (3.0 * c.x * x + 2.0 * b.y) * x + b.x;
+        R[2] = 6.0 * c.x * x + 2.0 * b.y;
+      }
+    } else if (jx < 1) {
+      const double *c = p + 3;
+      R[0] = (((c[4] * r + c[3]) * r + c[2]) * r + c[1]) * r + c[0];
+      if (DERIV) {
+        R[1] = ((4.0 * c[4] * r + 3.0 * c[3]) * r + 2.0 * c[2]) * r + c[1];
+        R[2] = (12.0 * c[4] * r + 6.0 * c[3]) * r + 2.0 * c[2];
+      }
+    } else {
+      const double ak = p[9];
+      R[0] = p[8] * exp(-ak * r);
+      if (DERIV) {
+        R[1] = -ak * R[0];
+        R[2] = -ak * R[1];
+      }
+    }
+    return;
+  }
   const T r0 = (T)p[0], h = (T)p[1], lh = (T)p[2];
   int jx;
   T ref0, ref1;

@@ -173,7 +173,7 @@ static double host_anorm(int kind, int n, int l, double z) {
 // matched at the last points (its slope is the right end condition), and the spline's second
 // derivatives.  Grid 3 reads the last point as r0 and derives r0 = r_last / (h^(nr-1) - 1).
 static int build_radial_tables(const champ_system *d, champ_ctx *c) {
-  c->rad_tab.clear(); c->rad_par.clear(); c->rad_y.clear(); c->rad_y2.clear();
+  c->rad_tab.clear(); c->rad_par.clear(); c->rad_y.clear(); c->rad_y2.clear(); c->rad_cub.clear();
   c->rad_shell.assign(d->nshell, -1);
   bool any = false;
   for (int i = 0; i < d->nshell; i++)
@@ -244,6 +244,18 @@ static int build_radial_tables(const champ_system *d, champ_ctx *c) {
     c->rad_tab.push_back(make_int4(g, nr, (int)c->rad_y.size(), 0));
     const double par[10] = {r0, h, std::log(h), ce[0], ce[1], ce[2], ce[3], ce[4], ae1, ae2};
     c->rad_par.insert(c->rad_par.end(), par, par + 10);
+    // every interval's grid point (the closed form the interpolation uses) and cubic
+    auto grid = [&](int i) { return g == 1 ? r0 + h * i : g == 2 ? r0 * std::pow(h, i) : r0 * std::pow(h, i) - r0; };
+    for (int i = 0; i < nr; i++) {
+      const double a = grid(i), dl = grid(i + 1) - a;
+      double cb[6] = {a, y[i], 0, 0, 0, 0};
+      if (i + 1 < nr) {
+        cb[2] = (y[i + 1] - y[i]) / dl - dl * (2 * y2[i] + y2[i + 1]) / 6;
+        cb[3] = 0.5 * y2[i];
+        cb[4] = (y2[i + 1] - y2[i]) / (6 * dl);
+      }
+      c->rad_cub.insert(c->rad_cub.end(), cb, cb + 6);
+    }
     c->rad_y.insert(c->rad_y.end(), y, y + nr);
     c->rad_y2.insert(c->rad_y2.end(), y2.begin(), y2.end());
     off += nr;
@@ -679,7 +691,10 @@ static int build_sys(champ_ctx *c, const champ_system *d, const std::vector<doub
       CK(cudaMemcpy(ry, yv.data(), sizeof(T) * ny, cudaMemcpyHostToDevice));
       CK(cudaMemcpy(ry2, y2v.data(), sizeof(T) * ny, cudaMemcpyHostToDevice));
     }
-    s.shrad = shr; s.rtab = rt; s.rpar = rp; s.ry = ry; s.ry2 = ry2;
+    double *rc = dalloc<double>(c, std::max<size_t>(6 * ny, 1));
+    if (!rc) return fail(CHAMP_ENOMEM, "device allocation of the radial tables failed");
+    if (ny) CK(cudaMemcpy(rc, c->rad_cub.data(), sizeof(double) * 6 * ny, cudaMemcpyHostToDevice));
+    s.shrad = shr; s.rtab = rt; s.rpar = rp; s.ry = ry; s.ry2 = ry2; s.rcub = rc;
   }
   return CHAMP_OK;
 }
