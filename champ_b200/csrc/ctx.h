@@ -49,6 +49,9 @@ struct KCfg {
   int wpb = 4;
 };
 
+// Bytes of a context's page-locked staging; calls that move more than this copy their arrays directly.
+constexpr size_t HSTAGE_BYTES = 256 * 1024;
+
 struct champ_ctx {
   int prec = 0;
   cudaStream_t stream = nullptr;
@@ -108,6 +111,9 @@ struct champ_ctx {
   // device staging for per-call host arrays
   double *d_in = nullptr, *d_out = nullptr;
   uint8_t *d_mask = nullptr;
+  // page-locked host memory that kernels can address, for the transfers of small calls (HSTAGE_BYTES): a
+  // call's arrays are copied here by the host instead of by a pageable cudaMemcpy each
+  char *h_stage = nullptr, *h_stage_dev = nullptr;
   int nparm_jas = 0;
   // parameter derivatives and O/H accumulation
   int np_raw = 0;          // raw Jastrow parameters on the device (a, b, all c terms)

@@ -731,8 +731,9 @@ static int build_state(champ_ctx *c, State<T> &st) {
   st.o_vel = dalloc<double>(c, W * N * 3); st.o_divv = dalloc<double>(c, W * N); st.o_d2 = dalloc<double>(c, W);
   st.o_pe = dalloc<double>(c, W); st.o_peee = dalloc<double>(c, W); st.o_penl = dalloc<double>(c, W);
   st.o_eloc = dalloc<double>(c, W);
-  st.s_esum = dalloc<double>(c, W); st.s_e2sum = dalloc<double>(c, W); st.s_acc = dalloc<double>(c, W);
-  st.s_elast = dalloc<double>(c, W);
+  st.s_esum = dalloc<double>(c, 4 * W);  // one block: zeroed and copied together
+  if (!st.s_esum) return fail(CHAMP_ENOMEM, "device allocation of the walker state failed");
+  st.s_e2sum = st.s_esum + W; st.s_acc = st.s_e2sum + W; st.s_elast = st.s_acc + W;
   if (!st.x || !st.ainv || !st.fso || !st.ren || !st.zq || !st.orb5 || !st.s_elast || (c->nloc > 0 && (!st.gproj || !st.nlt)))
     return fail(CHAMP_ENOMEM, "device allocation of the walker state failed");
   return CHAMP_OK;
@@ -854,9 +855,7 @@ static int launch(champ_ctx *c, Op op, const OpArgs &a = OpArgs()) {
   if (op == Op::Vmc && a.phase < 0 && c->prec == CHAMP_PREC_FP64 && c->el_staged) {
     // moves, then the staged E_L, per sweep (the E_L re-inverts the Slater matrices every sweep)
     const State<double> &st = c->std_;
-    CK(cudaMemsetAsync(st.s_esum, 0, sizeof(double) * c->W, c->stream));
-    CK(cudaMemsetAsync(st.s_e2sum, 0, sizeof(double) * c->W, c->stream));
-    CK(cudaMemsetAsync(st.s_acc, 0, sizeof(double) * c->W, c->stream));
+    CK(cudaMemsetAsync(st.s_esum, 0, sizeof(double) * 3 * (size_t)c->wmax, c->stream));  // esum, e2sum, acc
     OpArgs b = a;
     b.nsweep = 1;
     for (int isw = 0; isw < a.nsweep; isw++) {
@@ -907,9 +906,7 @@ static int launch(champ_ctx *c, Op op, const OpArgs &a = OpArgs()) {
   case Op::Vmc: {
     if (a.phase >= 0) return fail(CHAMP_EINVAL, "internal: explicit VMC phase on a mixed context");
     const State<double> &st = c->std_;
-    CK(cudaMemsetAsync(st.s_esum, 0, sizeof(double) * c->W, c->stream));
-    CK(cudaMemsetAsync(st.s_e2sum, 0, sizeof(double) * c->W, c->stream));
-    CK(cudaMemsetAsync(st.s_acc, 0, sizeof(double) * c->W, c->stream));
+    CK(cudaMemsetAsync(st.s_esum, 0, sizeof(double) * 3 * (size_t)c->wmax, c->stream));  // esum, e2sum, acc
     OpArgs b = a;
     b.nsweep = 1;
     for (int isw = 0; isw < a.nsweep; isw++) {
@@ -950,6 +947,16 @@ template <class T>
 static int copy_stats(champ_ctx *c, const champ_vmc_stats *s) {
   State<T> &st = stof<T>(c);
   size_t W = c->W;
+  double *const to[4] = {s->esum, s->e2sum, s->accept, s->elast};
+  const size_t wm = c->wmax, span = sizeof(double) * (3 * wm + W);
+  if (c->h_stage && span <= HSTAGE_BYTES) {
+    // one copy of the block through the page-locked buffer instead of a pageable copy per array
+    CK(cudaMemcpyAsync(c->h_stage, st.s_esum, span, cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    for (int k = 0; k < 4; k++)
+      if (to[k]) memcpy(to[k], c->h_stage + sizeof(double) * wm * k, sizeof(double) * W);
+    return CHAMP_OK;
+  }
   if (s->esum) CK(cudaMemcpyAsync(s->esum, st.s_esum, sizeof(double) * W, cudaMemcpyDeviceToHost, c->stream));
   if (s->e2sum) CK(cudaMemcpyAsync(s->e2sum, st.s_e2sum, sizeof(double) * W, cudaMemcpyDeviceToHost, c->stream));
   if (s->accept) CK(cudaMemcpyAsync(s->accept, st.s_acc, sizeof(double) * W, cudaMemcpyDeviceToHost, c->stream));
@@ -1546,6 +1553,13 @@ int champ_create(const champ_system *d, int32_t w_max, int32_t precision, void *
   c->d_in = dalloc<double>(c, (size_t)w_max * 3 * c->N);
   c->d_out = dalloc<double>(c, (size_t)w_max * 4 * c->N);
   c->d_mask = dalloc<uint8_t>(c, w_max);
+  // without it (no page-locked memory to be had) the calls copy their arrays directly
+  if (cudaHostAlloc((void **)&c->h_stage, HSTAGE_BYTES, cudaHostAllocMapped) != cudaSuccess ||
+      cudaHostGetDevicePointer((void **)&c->h_stage_dev, c->h_stage, 0) != cudaSuccess) {
+    if (c->h_stage) cudaFreeHost(c->h_stage);
+    c->h_stage = nullptr;
+    cudaGetLastError();
+  }
   if (!c->d_in || !c->d_out || !c->d_mask) { champ_destroy(c); return fail(CHAMP_ENOMEM, "staging allocation failed"); }
   {
     size_t W = w_max, P = c->nfree, P1 = P + 1;
@@ -1592,6 +1606,7 @@ int champ_destroy(champ_ctx *c) {
   for (void *e : c->ev_pool) cudaEventDestroy((cudaEvent_t)e);
   if (c->cap_stream) cudaStreamDestroy(c->cap_stream);
   for (void *p : c->allocs) cudaFree(p);
+  if (c->h_stage) cudaFreeHost(c->h_stage);
   if (c->cublas) cublasDestroy((cublasHandle_t)c->cublas);
   delete c;
   return CHAMP_OK;
@@ -2002,8 +2017,11 @@ int champ_set_walkers(champ_ctx *c, int32_t nw, const double *x) {
 int champ_get_walkers(champ_ctx *c, double *x) {
   if (!c || !x) return fail(CHAMP_EINVAL, "null argument");
   if (!c->have_walkers) return fail(CHAMP_ESTATE, "no walkers set");
-  CK(cudaMemcpyAsync(x, state_x(c), sizeof(double) * c->W * 3 * c->N, cudaMemcpyDeviceToHost, c->stream));
+  const size_t bytes = sizeof(double) * c->W * 3 * c->N;
+  const bool staged = c->h_stage && bytes <= HSTAGE_BYTES;
+  CK(cudaMemcpyAsync(staged ? (void *)c->h_stage : x, state_x(c), bytes, cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
+  if (staged) memcpy(x, c->h_stage, bytes);
   return CHAMP_OK;
 }
 
@@ -2036,6 +2054,21 @@ int champ_propose_1e(champ_ctx *c, int32_t iel, const double *xnew, double *rati
   CK(cudaMemcpyAsync(c->d_in, xnew, sizeof(double) * 3 * W, cudaMemcpyHostToDevice, c->stream));
   OpArgs a;
   a.e = iel;
+  if (c->h_stage && sizeof(double) * 7 * W <= HSTAGE_BYTES) {
+    // small calls: the kernel reads the proposals from, and writes its results to, page-locked host memory
+    double *h = (double *)c->h_stage, *d = (double *)c->h_stage_dev;
+    memcpy(h, xnew, sizeof(double) * 3 * W);
+    a.xnew = d;
+    a.ratio = d + 3 * W;
+    a.grad = d + 4 * W;
+    int rc = launch(c, grad_new ? Op::ProposeGrad : Op::Propose, a);
+    if (rc) return rc;
+    CK(cudaStreamSynchronize(c->stream));
+    memcpy(ratio, h + 3 * W, sizeof(double) * W);
+    if (grad_new) memcpy(grad_new, h + 4 * W, sizeof(double) * 3 * W);
+    return CHAMP_OK;
+  }
+  CK(cudaMemcpyAsync(c->d_in, xnew, sizeof(double) * 3 * W, cudaMemcpyHostToDevice, c->stream));
   a.xnew = c->d_in;
   a.ratio = c->d_out;
   a.grad = c->d_out + W;
@@ -2055,6 +2088,12 @@ int champ_accept_1e(champ_ctx *c, int32_t iel, const uint8_t *accept) {
   OpArgs a;
   a.e = iel;
   a.mask = c->d_mask;
+  if (c->h_stage && (size_t)c->W <= HSTAGE_BYTES) {
+    memcpy(c->h_stage, accept, c->W);
+    a.mask = (const uint8_t *)c->h_stage_dev;
+  } else {
+    CK(cudaMemcpyAsync(c->d_mask, accept, c->W, cudaMemcpyHostToDevice, c->stream));
+  }
   int rc = launch(c, Op::Accept, a);
   if (rc) return rc;
   CK(cudaStreamSynchronize(c->stream));
