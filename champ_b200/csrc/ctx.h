@@ -1,6 +1,7 @@
 // ctx.h -- host-side context of the engine, shared by the C-ABI translation unit and
 // the per-precision kernel instantiation units.
 #pragma once
+#include <algorithm>
 #include <string>
 #include <vector>
 
@@ -81,6 +82,7 @@ struct champ_ctx {
   bool have_walkers = false;
   KCfg kf, kd;  // FP32 and FP64 kernels (a mixed-precision context uses both)
   KCfg kfm;     // FP32 Gaussian moves of a state in HBM sharing the coefficient stream (kfm.lay.coop)
+  KCfg kdm;     // FP64 multi-determinant Gaussian moves with the state in shared memory (kdm.lay.resident)
   int move_coop = 0;  // option "move_coop": 1 runs those moves with kfm
   int orb_coop_ok = 0, orb_coop = 0;  // k_el_orb's warps share the coefficient stream (option "orb_coop")
   size_t orb_stage = 0;               // offset of its double buffer in the block's shared memory
@@ -99,14 +101,16 @@ struct champ_ctx {
   // k_el_jas), orbital tiles of 16 per block and chunks of shells (0: k_el_orb), rows of the inversion
   int jas_wpw = 0;
   size_t jas_smem = 0;
-  int orb_nt = 0, orb_nchunk = 0;
+  int orb_nt = 0, orb_nchunk = 0, orb_gen = 0;  // orb_gen: shells other than Gaussians with n = l + 1, l <= 2
   int4 *orb_chunk = nullptr;
   int inv_nm = 64;
-  // last part (0: k_el_fin): warps per walker, shared memory, radial values of tasks kept there, and
-  // every shell's smallest exponent
+  // last part (0: k_el_fin): warps per walker, shared memory, radial values of tasks kept there
   int fin_wpw = 0, fin_nrow = 0;
   size_t fin_smem = 0;
-  double *shell_zmin = nullptr;
+  int *shell_order = nullptr;  // parameter gradient (pgtile.cuh): shells by l, raw sums [wmax][3][np_raw]
+  double *pg_raw = nullptr;
+  int small = 0;  // small walkers: FP64 kernels with 8 lanes per walker (small.cu), shells by l
+  int *small_order = nullptr;
   int move_batch = 0;  // the Gaussian sweeps run as batched moves
   // device staging for per-call host arrays
   double *d_in = nullptr, *d_out = nullptr;
@@ -234,6 +238,35 @@ int el_tile_fin(champ_ctx *c, const State<double> &st, bool outputs, bool stats,
 // batched Gaussian single-electron moves (movebatch.cu); setup sets champ_ctx::move_batch where they apply
 int move_batch_setup(champ_ctx *c);
 int move_batch_sweep(champ_ctx *c, uint64_t seed, uint64_t isweep, double step);
+
+// parameter gradient of the staged evaluation's contexts (eltile.cu)
+int pg_tile_setup(champ_ctx *c);
+bool pg_tile_fwd_ok(const champ_ctx *c);
+bool pg_tile_bwd_ok(const champ_ctx *c);
+int pg_tile_fwd(champ_ctx *c);
+int pg_tile_bwd(champ_ctx *c);
+// small walkers (small.cu); setup sets champ_ctx::small where they apply
+int small_setup(champ_ctx *c);
+int small_eval(champ_ctx *c, const State<double> &st, bool outputs, bool stats, const ElRot &rot);
+int small_vmc(champ_ctx *c, const State<double> &st, const OpArgs &a);
+int small_dmc(champ_ctx *c, const State<double> &st, bool moves);
+int small_tmove(champ_ctx *c, const State<double> &st, const OpArgs &a);
+
+// Shared-memory carve-out of a kernel: what its resident blocks of this launch shape use and no more, so
+// that the rest of the SM's 256 KB stays L1 cache (with the largest carve-out the shell tables and orbital
+// coefficients that every warp reads over and over came from L2).
+template <class K>
+int fit_carveout(K kern, int threads, size_t smem) {
+  CK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
+  int n = 0;
+  cudaFuncAttributes fa;
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, smem));
+  CK(cudaFuncGetAttributes(&fa, kern));
+  const size_t need = (size_t)std::max(n, 1) * (smem + fa.sharedSizeBytes + 1024);  // 1 KB of each block is the system's
+  const int pct = (int)std::min<size_t>(100, (need * 100 + 228 * 1024 - 1) / (228 * 1024));
+  CK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, pct));
+  return CHAMP_OK;
+}
 
 // kernel launchers per (compute type, e-e-n order), one translation unit each (inst_*.cu)
 #define CHAMP_DECL(TAG, NORD)                                    \

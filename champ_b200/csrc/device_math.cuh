@@ -46,6 +46,11 @@ struct QuadRule {
   double q0[MAXQ][3], wq[MAXQ];
 };
 
+struct ShellRec {
+  int cen, l, b0, p0, np, kind;  // kind: 1 Gaussian with n = l + 1, 0 any other
+  double zmin;                   // smallest exponent among the primitives that weigh in the shell
+};
+
 // System data in device memory (pointers into one allocation).
 template <class T>
 struct Sys {
@@ -60,6 +65,12 @@ struct Sys {
   const int *cshell0;   // [C+1] first shell of each centre (shells grouped by centre)
   int nshc;             // most shells on one centre; 0 when shells are not grouped by centre
   const T *pz, *pc;     // primitive exponent, normalised weight
+  // FP64 Gaussian shells as the tiled kernels read them (shelltab.cuh): a record per shell, exponents and
+  // weights in ascending order of the exponent, and the table of fast_exp
+  const ShellRec *srec;
+  const double2 *sprim;
+  const double *sexp;
+  int nprim;
   // numerical radial tables (shell kind 2): per table (grid type, points, first value, 0) and
   // (r0, h, log h, small-r polynomial c0..c4, large-r a0, ak); per point the value and its
   // spline second derivative

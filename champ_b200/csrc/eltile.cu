@@ -5,27 +5,33 @@
 #include "jastile.cuh"
 #include "orbtile.cuh"
 #include "nlpoints.cuh"
+#include "pgtile.cuh"
 
 template <class K>
-static int big_smem(K kern, size_t bytes) {
-  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  CK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
-  return CHAMP_OK;
+static int big_smem(K kern, int threads, size_t bytes) {
+  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+  return fit_carveout(kern, threads, bytes);
 }
 
 template <int NORD>
-static int fin_attrs_n() {
-  int rc = big_smem(pt::k_fin_points<NORD, false, 1>, 200 * 1024);
-  if (!rc) rc = big_smem(pt::k_fin_points<NORD, false, 4>, 200 * 1024);
-  if (!rc) rc = big_smem(pt::k_fin_points<NORD, true, 1>, 200 * 1024);
-  if (!rc) rc = big_smem(pt::k_fin_points<NORD, true, 4>, 200 * 1024);
+static int fin_attrs_n(size_t b) {
+  int rc = big_smem(pt::k_fin_points<NORD, false, 1>, 128, b);
+  if (!rc) rc = big_smem(pt::k_fin_points<NORD, false, 4>, 128, b);
+  if (!rc) rc = big_smem(pt::k_fin_points<NORD, true, 1>, 128, b);
+  if (!rc) rc = big_smem(pt::k_fin_points<NORD, true, 4>, 128, b);
   return rc;
 }
+static size_t gproj_smem(const champ_ctx *c) { return sizeof(double) * pt::GP_LD * (size_t)((c->nomax + 3) & ~3); }
 static int fin_attrs(champ_ctx *c) {
-  int rc = c->nordc == 4 ? fin_attrs_n<4>() : c->nordc == 5 ? fin_attrs_n<5>() : fin_attrs_n<0>();
-  if (!rc) rc = big_smem(pt::k_gproj<false>, 200 * 1024);
-  if (!rc) rc = big_smem(pt::k_gproj<true>, 200 * 1024);
+  int rc = c->nordc == 4 ? fin_attrs_n<4>(c->fin_smem) : c->nordc == 5 ? fin_attrs_n<5>(c->fin_smem) : fin_attrs_n<0>(c->fin_smem);
+  if (!rc) rc = big_smem(pt::k_gproj<false>, 128, gproj_smem(c));
+  if (!rc) rc = big_smem(pt::k_gproj<true>, 128, gproj_smem(c));
   return rc;
+}
+
+template <int NT>
+static size_t orb_smem(const champ_ctx *c) {
+  return ot::smem_bytes<NT>() + stab::tab_smem(c->sd.nshell, c->sd.nprim);
 }
 
 // Which parts serve the context's system, their shared memory, and the chunks of whole shells that
@@ -49,6 +55,7 @@ int el_tile_setup(champ_ctx *c) {
     CK(cudaMemcpy(b0.data(), c->sd.shb0, sizeof(int) * c->nshell, cudaMemcpyDeviceToHost));
     for (int i = 0; i < c->nshell; i++) {
       const int nb = 2 * sh[i].z + 1;
+      if (sh[i].w != 1 || sh[i].y != sh[i].z + 1 || sh[i].z > 2) c->orb_gen = 1;
       if (ch.empty() || ch.back().w + nb > ot::KB) ch.push_back(make_int4(i, 0, b0[i], 0));
       ch.back().y++;
       ch.back().w += nb;
@@ -62,29 +69,10 @@ int el_tile_setup(champ_ctx *c) {
     c->orb_nt = nomax <= 16 ? 1 : nomax <= 32 ? 2 : 4;
   }
   if (c->nordc <= 1 || c->nct == 1) {
-    // every shell's smallest exponent among the primitives that weigh in it
-    std::vector<int2> pr(c->nshell);
-    CK(cudaMemcpy(pr.data(), c->sd.shprim, sizeof(int2) * c->nshell, cudaMemcpyDeviceToHost));
-    int np = 0;
-    for (const int2 &p : pr) np = std::max(np, p.x + p.y);
-    std::vector<double> z(np), wt(np), zm(c->nshell, 0.0);
-    CK(cudaMemcpy(z.data(), c->sd.pz, sizeof(double) * np, cudaMemcpyDeviceToHost));
-    CK(cudaMemcpy(wt.data(), c->sd.pc, sizeof(double) * np, cudaMemcpyDeviceToHost));
-    for (int i = 0; i < c->nshell; i++) {
-      double wmax = 0, m = 1e300;
-      for (int p = pr[i].x; p < pr[i].x + pr[i].y; p++) wmax = std::max(wmax, std::fabs(wt[p]));
-      for (int p = pr[i].x; p < pr[i].x + pr[i].y; p++)
-        if (std::fabs(wt[p]) >= 1e-8 * wmax) m = std::min(m, z[p]);
-      zm[i] = m < 1e300 ? m : 0.0;
-    }
-    double *d = nullptr;
-    CK(cudaMalloc(&d, sizeof(double) * c->nshell));
-    c->allocs.push_back(d);
-    CK(cudaMemcpy(d, zm.data(), sizeof(double) * c->nshell, cudaMemcpyHostToDevice));
-    c->shell_zmin = d;
     const int wpw = c->N <= 32 ? 1 : 4;
     c->fin_nrow = std::min(c->N * c->C * std::max(c->sd.nshc, 1), wpw == 1 ? 256 : 768);
-    const size_t b = pt::Dims(c->N, c->C, c->nordc, c->fin_nrow).bytes() * (wpw == 1 ? 4 : 1);
+    const size_t b = pt::Dims(c->N, c->C, c->nordc, c->fin_nrow, wpw == 1).bytes() * (wpw == 1 ? 4 : 1) +
+                     stab::tab_smem(c->sd.nshell, c->sd.nprim);
     if (b <= 200 * 1024) {
       c->fin_wpw = wpw;
       c->fin_smem = b;
@@ -94,10 +82,13 @@ int el_tile_setup(champ_ctx *c) {
   for (auto k : {jt::k_jas_tile<4, 1, false>, jt::k_jas_tile<4, 1, true>, jt::k_jas_tile<4, jt::WARPS, false>,
                  jt::k_jas_tile<4, jt::WARPS, true>, jt::k_jas_tile<5, 1, false>, jt::k_jas_tile<5, 1, true>,
                  jt::k_jas_tile<5, jt::WARPS, false>, jt::k_jas_tile<5, jt::WARPS, true>})
-    if (!rc) rc = big_smem(k, 200 * 1024);
-  if (!rc) rc = big_smem(ot::k_orb_tile<1>, ot::smem_bytes<1>());
-  if (!rc) rc = big_smem(ot::k_orb_tile<2>, ot::smem_bytes<2>());
-  if (!rc) rc = big_smem(ot::k_orb_tile<4>, ot::smem_bytes<4>());
+    if (!rc) rc = big_smem(k, 128, c->jas_smem);
+  if (!rc) rc = big_smem(ot::k_orb_tile<1, false, false>, ot::THREADS, orb_smem<1>(c));
+  if (!rc) rc = big_smem(ot::k_orb_tile<1, false, true>, ot::THREADS, orb_smem<1>(c));
+  if (!rc) rc = big_smem(ot::k_orb_tile<2, false, false>, ot::THREADS, orb_smem<2>(c));
+  if (!rc) rc = big_smem(ot::k_orb_tile<2, false, true>, ot::THREADS, orb_smem<2>(c));
+  if (!rc) rc = big_smem(ot::k_orb_tile<4, false, false>, ot::THREADS, orb_smem<4>(c));
+  if (!rc) rc = big_smem(ot::k_orb_tile<4, false, true>, ot::THREADS, orb_smem<4>(c));
   return rc;
 }
 
@@ -119,15 +110,18 @@ int el_tile_jas(champ_ctx *c, const State<double> &st, bool vo) {
   return c->nordc == 4 ? jas<4>(c, st, vo) : jas<5>(c, st, vo);
 }
 
+template <int NT>
+static void orb(champ_ctx *c, const State<double> &st, dim3 g) {
+  if (c->orb_gen) ot::k_orb_tile<NT, false, true><<<g, ot::THREADS, orb_smem<NT>(c), c->stream>>>(c->sd, st, c->orb_chunk, c->orb_nchunk, nullptr, 0);
+  else ot::k_orb_tile<NT, false, false><<<g, ot::THREADS, orb_smem<NT>(c), c->stream>>>(c->sd, st, c->orb_chunk, c->orb_nchunk, nullptr, 0);
+}
 int el_tile_orb(champ_ctx *c, const State<double> &st) {
   const int nmax = std::max(c->nup, c->ndn);
   const long long items = (long long)st.W * nmax;
   const dim3 g((unsigned)((items + ot::EB - 1) / ot::EB), 2);
-  switch (c->orb_nt) {
-  case 1: ot::k_orb_tile<1><<<g, ot::THREADS, ot::smem_bytes<1>(), c->stream>>>(c->sd, st, c->orb_chunk, c->orb_nchunk); break;
-  case 2: ot::k_orb_tile<2><<<g, ot::THREADS, ot::smem_bytes<2>(), c->stream>>>(c->sd, st, c->orb_chunk, c->orb_nchunk); break;
-  default: ot::k_orb_tile<4><<<g, ot::THREADS, ot::smem_bytes<4>(), c->stream>>>(c->sd, st, c->orb_chunk, c->orb_nchunk);
-  }
+  if (c->orb_nt == 1) orb<1>(c, st, g);
+  else if (c->orb_nt == 2) orb<2>(c, st, g);
+  else orb<4>(c, st, g);
   CK(cudaGetLastError());
   return CHAMP_OK;
 }
@@ -141,30 +135,147 @@ int el_tile_inv(champ_ctx *c, const State<double> &st) {
 }
 
 template <int NORD, bool MD>
-static int fin(champ_ctx *c, const State<double> &st, bool outputs, bool stats, const ElRot &rot, bool tables_only) {
+static int fin(champ_ctx *c, const State<double> &st, bool outputs, bool stats, const ElRot &rot, bool tables_only, const pt::Tape &tape) {
   const int W = st.W;
   if (MD) {
     pt::k_md_tables<<<(W + 3) / 4, 128, 0, c->stream>>>(c->sd, st);
     CK(cudaGetLastError());
   }
   if (c->nloc > 0 && !tables_only) {
-    const size_t sm = sizeof(double) * pt::GP_LD * (size_t)((c->nomax + 3) & ~3);
-    pt::k_gproj<MD><<<2 * W, 128, sm, c->stream>>>(c->sd, st);
+    pt::k_gproj<MD><<<2 * W, 128, gproj_smem(c), c->stream>>>(c->sd, st);
     CK(cudaGetLastError());
   }
   if (c->fin_wpw == 1)
-    pt::k_fin_points<NORD, MD, 1><<<(W + 3) / 4, 128, c->fin_smem, c->stream>>>(c->sd, st, c->shell_zmin, c->fin_nrow, outputs, stats, rot, tables_only);
+    pt::k_fin_points<NORD, MD, 1><<<(W + 3) / 4, 128, c->fin_smem, c->stream>>>(c->sd, st, c->fin_nrow, outputs, stats, rot, tables_only, tape);
   else
-    pt::k_fin_points<NORD, MD, 4><<<W, 128, c->fin_smem, c->stream>>>(c->sd, st, c->shell_zmin, c->fin_nrow, outputs, stats, rot, tables_only);
+    pt::k_fin_points<NORD, MD, 4><<<W, 128, c->fin_smem, c->stream>>>(c->sd, st, c->fin_nrow, outputs, stats, rot, tables_only, tape);
   CK(cudaGetLastError());
   return CHAMP_OK;
 }
 template <int NORD>
-static int fin_n(champ_ctx *c, const State<double> &st, bool outputs, bool stats, const ElRot &rot, bool tables_only) {
-  return c->md.multidet ? fin<NORD, true>(c, st, outputs, stats, rot, tables_only)
-                        : fin<NORD, false>(c, st, outputs, stats, rot, tables_only);
+static int fin_n(champ_ctx *c, const State<double> &st, bool outputs, bool stats, const ElRot &rot, bool tables_only, const pt::Tape &tape) {
+  return c->md.multidet ? fin<NORD, true>(c, st, outputs, stats, rot, tables_only, tape)
+                        : fin<NORD, false>(c, st, outputs, stats, rot, tables_only, tape);
 }
 int el_tile_fin(champ_ctx *c, const State<double> &st, bool outputs, bool stats, const ElRot &rot, bool tables_only) {
-  return c->nordc == 4 ? fin_n<4>(c, st, outputs, stats, rot, tables_only)
-       : c->nordc == 5 ? fin_n<5>(c, st, outputs, stats, rot, tables_only) : fin_n<0>(c, st, outputs, stats, rot, tables_only);
+  const pt::Tape t{};
+  return c->nordc == 4 ? fin_n<4>(c, st, outputs, stats, rot, tables_only, t)
+       : c->nordc == 5 ? fin_n<5>(c, st, outputs, stats, rot, tables_only, t) : fin_n<0>(c, st, outputs, stats, rot, tables_only, t);
 }
+
+// ---- parameter gradient (pgtile.cuh) -----------------------------------------------------------
+// The forward pass as the staged evaluation with a tape: e-e-n terms on the tensor cores.
+// (The points' coefficients for the orbital-resolved local energy wait in the place of its orbitals, which
+// are formed after their use.)  One determinant: the orbital and CSF derivatives of a multi-determinant
+// state go through the reference determinant's inverse, which near its nodes amplifies any change of
+// rounding beyond the derivatives themselves.
+bool pg_tile_fwd_ok(const champ_ctx *c) {
+  const bool room = c->ncsfp + c->norbp == 0 || c->C * c->nquad <= 5 * c->norb;
+  return c->el_staged && c->jas_wpw && c->fin_wpw && c->orb_nt && !c->md.multidet && room;
+}
+// The reverse sweep in FP64: one e-e parameter set.
+bool pg_tile_bwd_ok(const champ_ctx *c) {
+  return pg_tile_fwd_ok(c) && c->prec == CHAMP_PREC_FP64 && c->par.nspin2b == 1 && c->pg_raw;
+}
+
+static size_t pgnl_smem(const champ_ctx *c) {
+  return sizeof(double) * 4 * (size_t)c->nbasis + stab::tab_smem(c->sd.nshell, c->sd.nprim);
+}
+
+int pg_tile_setup(champ_ctx *c) {
+  if (!pg_tile_fwd_ok(c)) return CHAMP_OK;
+  std::vector<int4> sh(c->nshell);
+  CK(cudaMemcpy(sh.data(), c->sd.shell, sizeof(int4) * c->nshell, cudaMemcpyDeviceToHost));
+  std::vector<int> order(c->nshell);
+  for (int i = 0; i < c->nshell; i++) order[i] = i;
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return sh[a].z < sh[b].z; });
+  CK(cudaMalloc(&c->shell_order, sizeof(int) * c->nshell));
+  c->allocs.push_back(c->shell_order);
+  CK(cudaMemcpy(c->shell_order, order.data(), sizeof(int) * c->nshell, cudaMemcpyHostToDevice));
+  int rc = big_smem(ot::k_orb_tile<4, true, false>, ot::THREADS, orb_smem<4>(c));
+  if (!rc) rc = big_smem(ot::k_orb_tile<4, true, true>, ot::THREADS, orb_smem<4>(c));
+  if (!rc) rc = big_smem(pg::k_pg_nl, 128, pgnl_smem(c));
+  if (rc || c->prec != CHAMP_PREC_FP64 || c->par.nspin2b != 1) return rc;
+  const size_t pb = pt::Dims(c->N, c->C, c->nordc, 0).bytes() * (c->jas_wpw == 1 ? 4 : 1);
+  for (auto k : {pg::k_pg_points<4, 1>, pg::k_pg_points<4, 4>, pg::k_pg_points<5, 1>, pg::k_pg_points<5, 4>})
+    if (!rc) rc = big_smem(k, 128, pb);
+  for (auto k : {pg::k_pg_pairs<4, 1>, pg::k_pg_pairs<4, 4>, pg::k_pg_pairs<5, 1>, pg::k_pg_pairs<5, 4>})
+    if (!rc) rc = big_smem(k, 128, c->jas_smem);
+  if (rc) return rc;
+  CK(cudaMalloc(&c->pg_raw, sizeof(double) * 3 * (size_t)c->np_raw * c->wmax));
+  c->allocs.push_back(c->pg_raw);
+  return CHAMP_OK;
+}
+
+static ElRot fixed_rotation(const champ_ctx *c) {
+  ElRot r{};
+  for (int i = 0; i < 9; i++) r.R[i] = c->rot[i];
+  return r;
+}
+
+int pg_tile_fwd(champ_ctx *c) {
+  State<double> st = c->std_;
+  st.W = c->W;
+  const int W = c->W;
+  const ElRot rot = fixed_rotation(c);
+  int rc = el_tile_jas(c, st, false);
+  if (!rc) rc = el_tile_orb(c, st);
+  if (!rc) rc = el_tile_inv(c, st);
+  pt::Tape t;
+  t.v = c->pg_tv;
+  t.c = c->pg_tc;
+  t.el = c->pg_el;
+  t.n = c->pg_tn;
+  t.b = c->pg_scr ? c->pg_scr + (size_t)c->N * c->nbasis : nullptr;
+  t.bstride = c->scr_stride;
+  if (!rc) rc = c->nordc == 4 ? fin_n<4>(c, st, false, false, rot, false, t) : fin_n<5>(c, st, false, false, rot, false, t);
+  if (rc) return rc;
+  c->orb5_valid = true;
+  if (c->nloc > 0) {
+    pg::k_pg_nl<<<W, 128, pgnl_smem(c), c->stream>>>(c->sd, st, c->pg_tv, c->pg_tn, c->pg_tc, c->pg_scr,
+                                                                             c->scr_stride, t.b, rot, c->shell_order);
+  } else {
+    CK(cudaMemset2DAsync(c->pg_tv + 3 * c->N, sizeof(double) * 4 * c->N, 0, sizeof(double) * c->N, W, c->stream));
+    if (c->pg_scr)
+      CK(cudaMemset2DAsync(c->pg_scr, sizeof(double) * c->scr_stride, 0, sizeof(double) * (size_t)c->N * c->nbasis, W, c->stream));
+  }
+  CK(cudaGetLastError());
+  if (c->pg_scr) {
+    const long long items = (long long)W * c->N;
+    const dim3 g((unsigned)((items + ot::EB - 1) / ot::EB), (c->norb + 63) / 64);
+    double *all = c->pg_scr + (size_t)c->N * c->nbasis;
+    if (c->orb_gen) ot::k_orb_tile<4, true, true><<<g, ot::THREADS, orb_smem<4>(c), c->stream>>>(c->sd, st, c->orb_chunk, c->orb_nchunk, all, c->scr_stride);
+    else ot::k_orb_tile<4, true, false><<<g, ot::THREADS, orb_smem<4>(c), c->stream>>>(c->sd, st, c->orb_chunk, c->orb_nchunk, all, c->scr_stride);
+    CK(cudaGetLastError());
+    const long long el = items * c->norb;
+    pg::k_pg_blocal<<<(unsigned)std::min<long long>((el + 255) / 256, 148 * 32), 256, 0, c->stream>>>(c->sd, st, c->pg_scr, c->scr_stride);
+    CK(cudaGetLastError());
+  }
+  return CHAMP_OK;
+}
+
+template <int NORD>
+static int bwd(champ_ctx *c) {
+  State<double> st = c->std_;
+  st.W = c->W;
+  const int W = c->W, P = c->np_raw, wpw = c->jas_wpw;
+  CK(cudaMemsetAsync(c->pg_raw, 0, sizeof(double) * 3 * (size_t)P * W, c->stream));
+  const dim3 g(wpw == 1 ? (W + 3) / 4 : W);
+  if (c->nloc > 0) {
+    const size_t b = pt::Dims(c->N, c->C, NORD, 0).bytes() * (wpw == 1 ? 4 : 1);
+    if (wpw == 1) pg::k_pg_points<NORD, 1><<<g, 128, b, c->stream>>>(c->sd, st, c->pg_tn, c->pg_tc, c->pg_raw, P, fixed_rotation(c));
+    else pg::k_pg_points<NORD, 4><<<g, 128, b, c->stream>>>(c->sd, st, c->pg_tn, c->pg_tc, c->pg_raw, P, fixed_rotation(c));
+    CK(cudaGetLastError());
+  }
+  if (wpw == 1) pg::k_pg_pairs<NORD, 1><<<g, 128, c->jas_smem, c->stream>>>(c->sd, st, c->pg_tv, c->pg_raw, P);
+  else pg::k_pg_pairs<NORD, 4><<<g, 128, c->jas_smem, c->stream>>>(c->sd, st, c->pg_tv, c->pg_raw, P);
+  CK(cudaGetLastError());
+  const int nt = make_terms(NORD).n, nab = P - nt, jo = c->nfree - c->nparm_jas;
+  const long long n = (long long)W * c->nparm_jas;
+  if (n > 0)
+    pg::k_pg_out<<<(unsigned)std::min<long long>((n + 127) / 128, 148 * 32), 128, 0, c->stream>>>(c->sd, W, c->pg_raw, P, nab, nt, c->nfree, jo,
+                                                                                               c->pg_dl, c->pg_de);
+  CK(cudaGetLastError());
+  return CHAMP_OK;
+}
+int pg_tile_bwd(champ_ctx *c) { return c->nordc == 4 ? bwd<4>(c) : bwd<5>(c); }

@@ -660,6 +660,37 @@ static int build_sys(champ_ctx *c, const champ_system *d, const std::vector<doub
     s.cshell0 = cs;
     s.nshc = grouped ? nshc : 0;
   }
+  if (std::is_same<T, double>::value) {
+    std::vector<ShellRec> rec(std::max(c->nshell, 1));
+    std::vector<double2> pr(std::max(nprim, 1));
+    for (int i = 0; i < c->nshell; i++) {
+      const int p0 = shpv[i].x, np = shpv[i].y;
+      const int4 sh4 = shv[i];
+      std::vector<int> o(np);
+      double wmax = 0, m = 1e300;
+      for (int p = 0; p < np; p++) {
+        o[p] = p0 + p;
+        wmax = std::max(wmax, std::fabs((double)pcv[p0 + p]));
+      }
+      std::stable_sort(o.begin(), o.end(), [&](int a, int b) { return pzv[a] < pzv[b]; });
+      for (int p = 0; p < np; p++) {
+        pr[p0 + p] = make_double2((double)pzv[o[p]], (double)pcv[o[p]]);
+        if (std::fabs((double)pcv[o[p]]) >= 1e-8 * wmax) m = std::min(m, (double)pzv[o[p]]);
+      }
+      rec[i] = ShellRec{sh4.x, sh4.z, shb0v[i], p0, np, sh4.w == 1 && sh4.y == sh4.z + 1 ? 1 : 0, m < 1e300 ? m : 0.0};
+    }
+    double ex[64];
+    for (int i = 0; i < 64; i++) ex[i] = std::exp2(i / 64.0);
+    ShellRec *dr = dalloc<ShellRec>(c, rec.size());
+    double2 *dp = dalloc<double2>(c, pr.size());
+    double *de = dalloc<double>(c, 64);
+    if (!dr || !dp || !de) return fail(CHAMP_ENOMEM, "device allocation failed");
+    CK(cudaMemcpy(dr, rec.data(), sizeof(ShellRec) * rec.size(), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(dp, pr.data(), sizeof(double2) * pr.size(), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(de, ex, sizeof ex, cudaMemcpyHostToDevice));
+    s.srec = dr; s.sprim = dp; s.sexp = de;
+    s.nprim = nprim;
+  }
   CK(cudaMemcpy(pz, pzv.data(), sizeof(T) * nprim, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(pc, pcv.data(), sizeof(T) * nprim, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(cr0, crv[0].data(), sizeof(T) * crv[0].size(), cudaMemcpyHostToDevice));
@@ -1503,6 +1534,12 @@ int champ_create(const champ_system *d, int32_t w_max, int32_t precision, void *
     // walker state in HBM: the full evaluation as the four kernels of elstage.cuh
     if (!rc && !c->kd.lay.resident) rc = setup_el_staged(c);
     if (!rc && !c->kd.lay.resident && !c->md.multidet) rc = setup_delay(c);
+    // multi-determinant Gaussian moves: the state in shared memory when the moves' part of it fits there
+    if (!rc && !c->kd.lay.resident && c->md.multidet && precision == CHAMP_PREC_FP64) {
+      c->kdm.lay = make_layout<double>(c->N, c->C, c->nbasis, c->nmax, c->nomax, c->std_.astride, c->std_.tvstride,
+                                       c->std_.gstride, c->std_.wstride, false, RESIDENT_LIMIT, true, true);
+      rc = finish_cfg(c->kdm);
+    }
   }
   if (use32 && !rc) {
     rc = build_sys<float>(c, d, pcn, cfull, asa, asb, ecp, pecent, c->sf);
@@ -1653,7 +1690,7 @@ int champ_param_grad_fwd(champ_ctx *c, double *eloc) {
   if (!c->have_walkers) return fail(CHAMP_ESTATE, "no walkers set");
   if (c->smem_pg == 0) return fail(CHAMP_EINVAL, "parameter derivatives: system too large for the kernel's shared memory");
   OpArgs a = pg_args(c, 3);
-  int rc = launch(c, Op::PGrad, a);
+  int rc = pg_tile_fwd_ok(c) ? pg_tile_fwd(c) : launch(c, Op::PGrad, a);
   if (rc) return rc;
   c->have_tape = true;
   c->have_pgrad = false;
@@ -1668,7 +1705,7 @@ int champ_param_grad_bwd(champ_ctx *c, double *dlnpsi, double *deloc) {
   if (!c) return fail(CHAMP_EINVAL, "null context");
   if (!c->have_tape) return fail(CHAMP_ESTATE, "call champ_param_grad_fwd first");
   OpArgs a = pg_args(c, 4);
-  int rc = launch(c, Op::PGradBwd, a);
+  int rc = pg_tile_bwd_ok(c) ? pg_tile_bwd(c) : launch(c, Op::PGradBwd, a);
   if (!rc) rc = pg_orbital_part(c);
   if (rc) return rc;
   c->have_tape = false;
@@ -1684,7 +1721,7 @@ int champ_param_grad(champ_ctx *c, double *dlnpsi, double *deloc, double *eloc) 
   if (!c) return fail(CHAMP_EINVAL, "null context");
   if (!c->have_walkers) return fail(CHAMP_ESTATE, "no walkers set");
   if (c->smem_pg == 0) return fail(CHAMP_EINVAL, "parameter derivatives: system too large for the kernel's shared memory");
-  if (c->pg_mode == 0) {
+  if (c->pg_mode == 0 || pg_tile_bwd_ok(c)) {  // the one-pass kernel only where the tiles do not serve
     int rc = champ_param_grad_fwd(c, nullptr);
     if (!rc) rc = champ_param_grad_bwd(c, nullptr, nullptr);
     if (rc) return rc;
@@ -2051,7 +2088,6 @@ int champ_propose_1e(champ_ctx *c, int32_t iel, const double *xnew, double *rati
   if (!c->have_walkers) return fail(CHAMP_ESTATE, "no walkers set");
   if (iel < 0 || iel >= c->N) return fail(CHAMP_EINVAL, "iel out of range");
   size_t W = c->W;
-  CK(cudaMemcpyAsync(c->d_in, xnew, sizeof(double) * 3 * W, cudaMemcpyHostToDevice, c->stream));
   OpArgs a;
   a.e = iel;
   if (c->h_stage && sizeof(double) * 7 * W <= HSTAGE_BYTES) {
@@ -2084,7 +2120,6 @@ int champ_accept_1e(champ_ctx *c, int32_t iel, const uint8_t *accept) {
   if (!c || !accept) return fail(CHAMP_EINVAL, "null argument");
   if (!c->have_walkers) return fail(CHAMP_ESTATE, "no walkers set");
   if (iel < 0 || iel >= c->N) return fail(CHAMP_EINVAL, "iel out of range");
-  CK(cudaMemcpyAsync(c->d_mask, accept, c->W, cudaMemcpyHostToDevice, c->stream));
   OpArgs a;
   a.e = iel;
   a.mask = c->d_mask;

@@ -68,7 +68,7 @@ struct State {
   // intermediates of the staged evaluation (elstage.cuh) of a state in HBM; null otherwise:
   // per walker grad ln J and div of the Jastrow velocity [4N], scalars [EL_SC] (J, its Laplacian
   // sum, e-e and e-n Coulomb energies, ln|D| and sign(D) of each spin, ln|chi| and sign(chi) of a
-  // multi-determinant state), and the e-n distances as [2][C][N] planes
+  // multi-determinant state, two of the parameter gradient), and the e-n distances as [2][C][N] planes
   double *el_vj, *el_sc;
   T *el_rt;
   // delayed inverse updates of the moves (struct Delay): [W][2][2][dlk_max][nmax] pending terms,
@@ -76,7 +76,7 @@ struct State {
   double *dly;
   int dlk, dlk_max;
 };
-constexpr int EL_SC = 10;        // stride of the staged evaluation's per-walker scalars (el_sc)
+constexpr int EL_SC = 12;        // stride of the staged evaluation's per-walker scalars (el_sc)
 constexpr int NLT = 2 + MAXLCH;  // task record: (e*C+c), r, vps[0..MAXLCH-1]
 constexpr int ZQ = 8;            // stride of the per-electron power sums zq
 constexpr int MAXC_NL = 64;      // centres for the value-only e-e-n fast path
@@ -115,9 +115,10 @@ __host__ __device__ inline int phi_count(int nbasis, int C) { return nbasis * 5 
 
 template <class T>
 static Layout make_layout(int N, int C, int nbasis, int nmax, int nomax, int astride, int tvstride, int gstride,
-                          int wstride, bool nl, size_t resident_limit, bool moves_only = false) {
+                          int wstride, bool nl, size_t resident_limit, bool moves_only = false, bool keep = false) {
   // moves_only: the Gaussian single-electron moves of a state in HBM (one basis channel, no
-  // velocities); vacc and divj then share phi's place and must not be used
+  // velocities); vacc and divj then share phi's place and must not be used.  keep: with the state
+  // itself in shared memory where that fits (an evaluation's scratch not counted)
   Layout L{};
   size_t o = 0;
   auto take = [&](size_t b) { size_t r = o; o += align16(b); return r; };
@@ -137,7 +138,7 @@ static Layout make_layout(int N, int C, int nbasis, int nmax, int nomax, int ast
   L.ren = take(sizeof(T) * N * C * 2);
   L.zq = take(sizeof(T) * N * ZQ);
   L.pf = take(sizeof(T) * N);
-  L.orb5 = take(sizeof(T) * N * 5 * nomax);
+  L.orb5 = keep ? 0 : take(sizeof(T) * N * 5 * nomax);
   L.gproj = nl ? take(sizeof(T) * N * nbasis) : 0;
   L.nlt = nl ? take(sizeof(double) * N * C * NLT) : 0;
   L.tv = take(sizeof(double) * tvstride);
@@ -145,7 +146,7 @@ static Layout make_layout(int N, int C, int nbasis, int nmax, int nomax, int ast
   L.ymd = take(sizeof(double) * tvstride);
   L.wdet = take(sizeof(double) * wstride);
   L.base = base;
-  L.resident = (!moves_only && o <= resident_limit) ? 1 : 0;
+  L.resident = ((!moves_only || keep) && o <= resident_limit) ? 1 : 0;
   L.bytes = L.resident ? o : base;
   return L;
 }

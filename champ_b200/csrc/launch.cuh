@@ -8,10 +8,9 @@
 #define fail champ_fail
 // ---- kernel dispatch over (precision, e-e-n order)
 template <class K>
-static int set_attrs(champ_ctx *c, K kern, size_t smem) {
+static int set_attrs(champ_ctx *c, K kern, size_t smem, int wpb = 4) {
   CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  CK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
-  return CHAMP_OK;
+  return fit_carveout(kern, 32 * wpb, smem);
 }
 template <class T, int NORD, bool MD>
 static int set_smem_attrs(champ_ctx *c) {
@@ -20,7 +19,7 @@ static int set_smem_attrs(champ_ctx *c) {
   if (!rc) rc = set_attrs(c, k_propose<T, NORD, MD>, sm);
   if (!rc) rc = set_attrs(c, k_accept<T, MD>, sm);
   if (!rc) rc = set_attrs(c, k_vmc<T, NORD, MD, 0>, sm);
-  if (!rc) rc = set_attrs(c, k_vmc<T, NORD, MD, 1>, std::is_same<T, float>::value ? std::max(sm, c->kfm.smem) : sm);
+  if (!rc) rc = set_attrs(c, k_vmc<T, NORD, MD, 1>, std::max(sm, std::is_same<T, float>::value ? c->kfm.smem : c->kdm.smem));
   if (!rc) rc = set_attrs(c, k_vmc<T, NORD, MD, 2>, sm);
   if (!rc) rc = set_attrs(c, k_vmc<T, NORD, MD, 3>, sm);
   if (!rc) rc = set_attrs(c, k_vmc<T, NORD, MD, 0, 6>, sm);
@@ -46,7 +45,7 @@ static int set_smem_attrs(champ_ctx *c) {
   if (!rc && c->smem_pg > 0) {
     for (auto kern : {k_pgrad<T, NORD, MD, 1>, k_pgrad<T, NORD, MD, 2>, k_pgrad<T, NORD, MD, 3>, k_pgrad<T, NORD, MD, 4>}) {
       CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->smem_pg));
-      CK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
+      if (int r = fit_carveout(kern, 32 * c->wpb_pg, c->smem_pg)) return r;
     }
   }
   return rc;
@@ -261,6 +260,13 @@ static int launch_t(champ_ctx *c, Op op, const OpArgs &a) {
       if (std::is_same<T, float>::value && a.phase == 1 && !acc6 && c->move_coop && c->kfm.lay.coop) {
         // the block's warps share the proposals' coefficient stream (move-only layout)
         const KCfg &M = c->kfm;
+        kern<<<dim3((st.W + M.wpb - 1) / M.wpb), dim3(32 * M.wpb), M.smem, c->stream>>>(
+            s, st, M.lay, a.nsweep, a.seed, a.sweep0, a.step, c->reinv_every, c->mover);
+        break;
+      }
+      if (std::is_same<T, double>::value && MD && a.phase == 1 && !acc6 && c->kdm.lay.resident) {
+        // the G matrix, T and the determinants are rebuilt with every accepted move: in shared memory, not HBM
+        const KCfg &M = c->kdm;
         kern<<<dim3((st.W + M.wpb - 1) / M.wpb), dim3(32 * M.wpb), M.smem, c->stream>>>(
             s, st, M.lay, a.nsweep, a.seed, a.sweep0, a.step, c->reinv_every, c->mover);
         break;

@@ -7,10 +7,9 @@
 namespace {
 
 template <class K>
-int big_smem(K kern, size_t bytes) {
-  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  CK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
-  return CHAMP_OK;
+int big_smem(K kern, int threads, size_t bytes) {
+  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+  return fit_carveout(kern, threads, bytes);
 }
 
 // up to 32 electrons a warp per walker, else a block per walker
@@ -23,19 +22,23 @@ size_t pairs_smem(const champ_ctx *c) {
   const int wpw = warps_per_walker(c);
   return mv::PairDims<T, NORD>(c->N, c->C).bytes(wpw) * (wpw == 1 ? 4 : 1);
 }
+template <class T, int NT>
+size_t prop_smem(const champ_ctx *c) {
+  return mv::prop_smem<T, NT>() + (sizeof(T) == 8 ? stab::tab_smem(c->sd.nshell, c->sd.nprim) : 0);
+}
 mv::Scr scratch(const champ_ctx *c) { return mv::Scr{c->std_.orb5, 5 * (size_t)c->N * c->nomax, c->N, c->nomax}; }
 
 template <class T, int NORD>
 int setup(champ_ctx *c) {
   const size_t sp = pairs_smem<T, NORD>(c), sw = walk_smem(c);
   if (sp > 200 * 1024 || sw > 200 * 1024) return CHAMP_OK;
-  int rc = big_smem(mv::k_mv_pairs<T, NORD, 1>, sp);
-  if (!rc) rc = big_smem(mv::k_mv_pairs<T, NORD, 4>, sp);
-  if (!rc) rc = big_smem(mv::k_mv_walk<T, 1>, sw);
-  if (!rc) rc = big_smem(mv::k_mv_walk<T, 4>, sw);
-  if (!rc) rc = big_smem(mv::k_mv_prop<T, 1>, mv::prop_smem<T, 1>());
-  if (!rc) rc = big_smem(mv::k_mv_prop<T, 2>, mv::prop_smem<T, 2>());
-  if (!rc) rc = big_smem(mv::k_mv_prop<T, 4>, mv::prop_smem<T, 4>());
+  int rc = big_smem(mv::k_mv_pairs<T, NORD, 1>, 128, sp);
+  if (!rc) rc = big_smem(mv::k_mv_pairs<T, NORD, 4>, 128, sp);
+  if (!rc) rc = big_smem(mv::k_mv_walk<T, 1>, 128, sw);
+  if (!rc) rc = big_smem(mv::k_mv_walk<T, 4>, 128, sw);
+  if (!rc) rc = big_smem(mv::k_mv_prop<T, 1>, 256, prop_smem<T, 1>(c));
+  if (!rc) rc = big_smem(mv::k_mv_prop<T, 2>, 256, prop_smem<T, 2>(c));
+  if (!rc) rc = big_smem(mv::k_mv_prop<T, 4>, 256, prop_smem<T, 4>(c));
   if (!rc) c->move_batch = 1;
   return rc;
 }
@@ -50,9 +53,9 @@ int sweep(champ_ctx *c, const State<T> &st, uint64_t seed, uint64_t isweep, doub
   CK(cudaGetLastError());
   const dim3 g((unsigned)((per + mv::PB - 1) / mv::PB), 2);
   switch (c->orb_nt) {
-  case 1: mv::k_mv_prop<T, 1><<<g, 256, mv::prop_smem<T, 1>(), c->stream>>>(s, W, q, c->orb_chunk, c->orb_nchunk); break;
-  case 2: mv::k_mv_prop<T, 2><<<g, 256, mv::prop_smem<T, 2>(), c->stream>>>(s, W, q, c->orb_chunk, c->orb_nchunk); break;
-  default: mv::k_mv_prop<T, 4><<<g, 256, mv::prop_smem<T, 4>(), c->stream>>>(s, W, q, c->orb_chunk, c->orb_nchunk);
+  case 1: mv::k_mv_prop<T, 1><<<g, 256, prop_smem<T, 1>(c), c->stream>>>(s, W, q, c->orb_chunk, c->orb_nchunk); break;
+  case 2: mv::k_mv_prop<T, 2><<<g, 256, prop_smem<T, 2>(c), c->stream>>>(s, W, q, c->orb_chunk, c->orb_nchunk); break;
+  default: mv::k_mv_prop<T, 4><<<g, 256, prop_smem<T, 4>(c), c->stream>>>(s, W, q, c->orb_chunk, c->orb_nchunk);
   }
   CK(cudaGetLastError());
   const size_t sp = pairs_smem<T, NORD>(c), sw = walk_smem(c);

@@ -27,6 +27,7 @@
 // free between evaluations): corrections [N][N], orbital rows [N][nomax], dJ [N], x' [N][3], uniforms [N].
 #pragma once
 #include "kernels.cuh"
+#include "shelltab.cuh"
 
 namespace mv {
 
@@ -70,30 +71,29 @@ static __device__ __noinline__ void general_shell1(const Sys<double> &s, int ish
   const double pt[3] = {x, y, z};
   shell_eval_put<double, 1>(s, ish, pt, [o](int sl, int, double v) { o[sl * lda<double>()] = v; });
 }
-template <int l>
-__device__ __forceinline__ void gauss_shell1(const Sys<double> &s, int2 pr, double d0, double d1, double d2, double *o) {
-  const double r2 = d0 * d0 + d1 * d1 + d2 * d2;
-  double g = 0;
-  for (int p = pr.x; p < pr.x + pr.y; p++) g += s.pc[p] * exp(-s.pz[p] * r2);
-  double S[9], G[9][3];
-  solid_all<double, false>(l, d0, d1, d2, S, G);
-#pragma unroll
-  for (int sl = 0; sl < 2 * l + 1; sl++) o[sl * lda<double>()] = S[sl] * g;
-}
-__device__ __forceinline__ void put_shell(const Sys<double> &s, int ish, const double *pt, double *o) {
-  const int4 sh = s.shell[ish];
-  if (sh.w == 1 && sh.y == sh.z + 1 && sh.z <= 2) {
-    const double *cc = s.cent + 3 * sh.x;
+__device__ __forceinline__ void put_shell(const Sys<double> &s, const stab::Tab &T, int ish, const double *pt, double *o) {
+  const ShellRec h = T.rec[ish];
+  if (h.kind == 1 && h.l <= 2) {
+    const double *cc = s.cent + 3 * h.cen;
     const double d0 = pt[0] - cc[0], d1 = pt[1] - cc[1], d2 = pt[2] - cc[2];
-    const int2 pr = s.shprim[ish];
-    if (sh.z == 0) gauss_shell1<0>(s, pr, d0, d1, d2, o);
-    else if (sh.z == 1) gauss_shell1<1>(s, pr, d0, d1, d2, o);
-    else gauss_shell1<2>(s, pr, d0, d1, d2, o);
+    const double g = stab::gauss_radial(T, h, d0 * d0 + d1 * d1 + d2 * d2);
+    constexpr int ld = lda<double>();
+    if (h.l == 0) o[0] = g;
+    else if (h.l == 1) {
+      o[0] = d2 * g;
+      o[ld] = d0 * g;
+      o[2 * ld] = d1 * g;
+    } else {
+      double S[9], G[9][3];
+      solid_all<double, false>(2, d0, d1, d2, S, G);
+#pragma unroll
+      for (int i = 0; i < 5; i++) o[i * ld] = S[i] * g;
+    }
   } else {
     general_shell1(s, ish, pt[0], pt[1], pt[2], o);
   }
 }
-__device__ __forceinline__ void put_shell(const Sys<float> &s, int ish, const double *pt, float *o) {
+__device__ __forceinline__ void put_shell(const Sys<float> &s, const stab::Tab &, int ish, const double *pt, float *o) {
   shell_eval_put<float, 1>(s, ish, pt, [o](int sl, int, float v) { o[sl * lda<float>()] = v; });
 }
 
@@ -107,6 +107,8 @@ __global__ void __launch_bounds__(256, 2) k_mv_prop(const __grid_constant__ Sys<
   extern __shared__ __align__(16) char dsm[];
   constexpr int LDA = lda<T>(), LDB = ldb<T, NT>(), NC = 16 * NT;
   T *phi = (T *)dsm, *cf = phi + KB * LDA;
+  stab::Tab Tb{};
+  if constexpr (sizeof(T) == 8) Tb = stab::stage(s, dsm + prop_smem<T, NT>());
   const int sp = blockIdx.y, n = sp ? s.ndn : s.nup, no = s.nocc[sp], e0 = sp ? s.nup : 0;
   const long long items = (long long)W * n, i0 = (long long)blockIdx.x * PB;
   if (i0 >= items) return;
@@ -129,6 +131,7 @@ __global__ void __launch_bounds__(256, 2) k_mv_prop(const __grid_constant__ Sys<
   for (int i = 0; i < 8; i++)
 #pragma unroll
     for (int j = 0; j < NT; j++) acc[i][j] = T(0);
+  __syncthreads();  // the shell tables are in place
   for (int k = 0; k < nchunk; k++) {
     const int4 ch = chunk[k];
     const int nk = sizeof(T) == 4 ? ch.w : (ch.w + 3) & ~3;
@@ -152,7 +155,7 @@ __global__ void __launch_bounds__(256, 2) k_mv_prop(const __grid_constant__ Sys<
     for (int r = ch.w + (wib >> 2); r < nk; r += 2) phi[r * LDA + 32 * grp + lane] = T(0);
     for (int h = wib >> 2; h < ch.y; h += 2) {
       const int ish = ch.x + h;
-      put_shell(s, ish, px, phi + (s.shb0[ish] - ch.z) * LDA + 32 * grp + lane);
+      put_shell(s, Tb, ish, px, phi + (s.shb0[ish] - ch.z) * LDA + 32 * grp + lane);
     }
     cp_async_wait<0>();
     __syncthreads();

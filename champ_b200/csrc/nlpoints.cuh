@@ -18,6 +18,7 @@
 // determinants, 3.8 -> 2.0 ms.  k_el_fin stays for several centre types with e-e-n terms.
 #pragma once
 #include "jastile.cuh"
+#include "shelltab.cuh"
 
 namespace pt {
 
@@ -107,11 +108,13 @@ struct Tab {
 };
 
 // Shared memory of a walker (doubles): scaled distances [Ct][Np], positions, V_k [NORD][N], per-centre
-// sums [NORD - 1][C], rows of the pair table summed [N], the tasks' radial values [nrow], reductions.
+// sums [NORD - 1][C], rows of the pair table summed [N], the tasks' radial values [nrow], reductions,
+// per 32 (electron, centre) pairs the mask of those in range and the number in range before them, and
+// (lane) the distances of lane_jastrow.
 struct Dims {
-  int N, C, Ct, Np, nord, nrow;
-  __host__ __device__ Dims(int N_, int C_, int nord_, int nrow_)
-      : N(N_), C(C_), Ct(nord_ > 1 ? (C_ + 7) & ~7 : 0), Np(0), nord(nord_ > 1 ? nord_ : 0), nrow(nrow_) {
+  int N, C, Ct, Np, nord, nrow, lane;
+  __host__ __device__ Dims(int N_, int C_, int nord_, int nrow_, bool lane_ = false)
+      : N(N_), C(C_), Ct(nord_ > 1 ? (C_ + 7) & ~7 : 0), Np(0), nord(nord_ > 1 ? nord_ : 0), nrow(nrow_), lane(nord_ > 1 && lane_) {
     const int p = (N_ + 3) & ~3;
     Np = p + ((4 - p % 16) + 16) % 16;
   }
@@ -121,7 +124,9 @@ struct Dims {
   __host__ __device__ int f() const { return z() + nord * Ct; }
   __host__ __device__ int row() const { return f() + N; }
   __host__ __device__ int red() const { return row() + nrow; }
-  __host__ __device__ int total() const { return red() + 32; }
+  __host__ __device__ int msk() const { return red() + 32; }
+  __host__ __device__ int lanes() const { return msk() + (N * C + 31) / 32 + 1; }
+  __host__ __device__ int total() const { return lanes() + (lane ? 32 * C : 0); }
   __host__ __device__ size_t bytes() const { return sizeof(double) * (size_t)((total() + 1) & ~1); }
 };
 
@@ -294,34 +299,112 @@ __device__ __forceinline__ double point_jastrow(const Sys<double> &s, const JasP
   return act ? mine - F[e] : 0.0;
 }
 
-// Radial factor of a shell over r^l (so that a basis function is S_lm(d) times it).
-static __device__ __noinline__ double general_radial(const Sys<double> &s, int ish, double r) {
-  double R[3];
-  if (r == 0.0) r = 1e-30;
-  shell_radial<double, false>(s, ish, r, R);
-  return R[0] * ipow(1.0 / r, s.shell[ish].z);
-}
-__device__ __forceinline__ bool is_gauss(int4 sh) { return sh.w == 1 && sh.y == sh.z + 1; }
-__device__ __forceinline__ double gauss_radial(const Sys<double> &s, int2 pr, double zmin, double r2) {
-  double g = 0;
-  for (int p = pr.x; p < pr.x + pr.y; p++) {
-    const double z = s.pz[p];
-    if ((z - zmin) * r2 < 70.0) g += s.pc[p] * exp(-z * r2);
+// The same with a point per lane and no tiles: up to 32 electrons the tiles' rows and their centre part leave
+// most of a warp idle.  pl: [C][32] doubles of the warp.
+template <int NORD>
+__device__ __forceinline__ double lane_jastrow(const Sys<double> &s, const JasPar<double> &J, const Dims &D, const double *sm, double *pl,
+                                            const double *xn, int e, int lane) {
+  using TB = Tab<NORD>;
+  constexpr int NC = jt::make_combos(NORD).n, NT = make_terms(NORD).n, ND = jt::make_combos(NORD).nd;
+  constexpr int QM = NORD > 1 ? NORD - 1 : 1, KM = NORD > 1 ? NORD : 1, NDA = ND > 0 ? ND : 1;
+  const int N = s.N, C = s.C, Np = D.Np;
+  const double *sd = sm, *xs = sm + D.x(), *V = sm + D.v(), *Z = sm + D.z(), *F = sm + D.f();
+  const double sk = J.scalek;
+  double f = -F[e], S[QM], U[KM];
+#pragma unroll
+  for (int q = 0; q < QM; q++) S[q] = 0;
+#pragma unroll
+  for (int k = 0; k < KM; k++) U[k] = 0;
+  for (int c = 0; c < C; c++) {
+    const double a0 = xn[0] - s.cent[3 * c], a1 = xn[1] - s.cent[3 * c + 1], a2 = xn[2] - s.cent[3 * c + 2];
+    const double r = sqrt(a0 * a0 + a1 * a1 + a2 * a2), a = 1.0 / (1.0 + sk * r);
+    double fi, fii;
+    f += jas_en<double, false>(J, s.ctype[c], r, a, fi, fii);
+    if constexpr (NORD > 1) {
+      pl[32 * c + lane] = a;
+      const double re = sd[c * Np + e];
+      double ap[QM + 1], rp[QM + 1];
+      ap[0] = rp[0] = 1;
+#pragma unroll
+      for (int q = 1; q <= QM; q++) {
+        ap[q] = ap[q - 1] * a;
+        rp[q] = rp[q - 1] * re;
+        S[q - 1] += ap[q];
+      }
+      sfor<2 * NC>([&](auto Y) {
+        constexpr int yv = decltype(Y)::v, y = yv / 2, l = TB::cb.l[y], m = TB::cb.m[y], i0 = TB::cb.ll[y][0];
+        constexpr int p = yv % 2 ? m : l + m, q = yv % 2 ? l + m : m;
+        f += J.c[0][i0] * ap[p] * (Z[(q - 1) * C + c] - rp[q]);
+      });
+    }
   }
-  return g;
+  for (int j = 0; j < N; j++) {
+    if (j == e) continue;
+    const double a0 = xn[0] - xs[3 * j], a1 = xn[1] - xs[3 * j + 1], a2 = xn[2] - xs[3 * j + 2];
+    int isb, ipar;
+    double ss, du;
+    pair_class(J, s.nup, e, j, isb, ss, ipar);
+    f += ee_value(J, isb, ss, ipar, sqrt(a0 * a0 + a1 * a1 + a2 * a2), du);
+    if constexpr (NORD > 1) {
+      double X[NDA];
+#pragma unroll
+      for (int y = 0; y < ND; y++) X[y] = 0;
+#pragma unroll 2
+      for (int c = 0; c < C; c++) {
+        const double a = pl[32 * c + lane], b = sd[c * Np + j];
+        double ap[QM + 1], bp[QM + 1];
+        ap[0] = bp[0] = 1;
+#pragma unroll
+        for (int q = 1; q <= QM; q++) { ap[q] = ap[q - 1] * a; bp[q] = bp[q - 1] * b; }
+        sfor<NC>([&](auto Y) {
+          constexpr int y = decltype(Y)::v, l = TB::cb.l[y], m = TB::cb.m[y], dv = TB::cb.dv[y];
+          if constexpr (dv >= 0) {
+            X[dv] += ap[l + m] * bp[m];
+            if constexpr (l > 0) X[dv] += ap[m] * bp[l + m];
+          }
+        });
+      }
+      double u[KM + 1];
+      u[0] = 1;
+#pragma unroll
+      for (int k = 1; k <= KM; k++) {
+        u[k] = u[k - 1] * du;
+        U[k - 1] += u[k];
+        f += u[k] * V[(k - 1) * N + j];
+      }
+      sfor<NC>([&](auto Y) {
+        constexpr int y = decltype(Y)::v, l = TB::cb.l[y], nk = TB::cb.nk[y], dv = TB::cb.dv[y];
+        if constexpr (dv >= 0) {
+          double cu = 0;
+          sfor<nk - 1>([&](auto K) {
+            constexpr int k = decltype(K)::v + 1, ik = TB::cb.ll[y][k];
+            cu += J.c[0][ik] * u[k];
+          });
+          f += (l ? cu : 2 * cu) * X[dv];
+        }
+      });
+    }
+  }
+  if constexpr (NORD > 1)
+    sfor<NT>([&](auto L) {
+      constexpr int ll = decltype(L)::v, k = TB::tl.k[ll], l = TB::tl.l[ll];
+      if constexpr (TB::tl.m[ll] == 0 && l > 0) f += J.c[0][ll] * U[k - 1] * S[l - 1];
+    });
+  return f;
 }
 
 // Determinant ratio at a point: sum_b phi_b(point) g_b.  c0: the centre whose shells' radial
 // factors are tabulated in tab (null: none).
-__device__ __forceinline__ double point_ratio(const Sys<double> &s, const double *zmin, const double *xn, const double *g,
+__device__ __forceinline__ double point_ratio(const Sys<double> &s, const stab::Tab &T, const double *xn, const double *g,
                                              int c0, const double *tab) {
   double dr = 0, d0 = 0, d1 = 0, d2 = 0, r2 = 0;
   int cen = -1;
   const int t0 = tab ? s.cshell0[c0] : 0, t1 = tab ? s.cshell0[c0 + 1] : 0;
+#pragma unroll 1
   for (int ish = 0; ish < s.nshell; ish++) {
-    const int4 sh = s.shell[ish];
-    if (sh.x != cen) {
-      cen = sh.x;
+    const ShellRec h = T.rec[ish];
+    if (h.cen != cen) {
+      cen = h.cen;
       const double *cc = s.cent + 3 * cen;
       d0 = xn[0] - cc[0];
       d1 = xn[1] - cc[1];
@@ -330,11 +413,10 @@ __device__ __forceinline__ double point_ratio(const Sys<double> &s, const double
     }
     double rad;
     if (ish >= t0 && ish < t1) rad = tab[ish - t0];
-    else if (is_gauss(sh)) rad = gauss_radial(s, s.shprim[ish], zmin[ish], r2);
-    else rad = general_radial(s, ish, sqrt(r2));
-    const double *gb = g + s.shb0[ish];
+    else rad = stab::factor(s, T, ish, h, r2);
+    const double *gb = g + h.b0;
     double S[9], G[9][3], acc = 0;
-    switch (sh.z) {
+    switch (h.l) {
     case 0: acc = gb[0]; break;
     case 1: acc = d2 * gb[0] + d0 * gb[1] + d1 * gb[2]; break;
     case 2:
@@ -357,10 +439,20 @@ __device__ __forceinline__ double point_ratio(const Sys<double> &s, const double
   return dr;
 }
 
+// What the forward pass of the parameter gradient keeps (null otherwise): velocities [4N], points'
+// coefficients [N C][nq], E_L and the number of tasks; the task records are the evaluation's.  b (may be
+// null; walkers bstride apart): the coefficients without the determinant ratio, for the nonlocal part of
+// the orbital-resolved local energy.
+struct Tape {
+  double *v = nullptr, *c = nullptr, *el = nullptr, *b = nullptr;
+  int *n = nullptr;
+  size_t bstride = 0;
+};
+
 template <int NORD, bool MD, int WPW>
 __global__ void __launch_bounds__(128, 3) k_fin_points(const __grid_constant__ Sys<double> s,
-                                                       const __grid_constant__ State<double> st, const double *zmin,
-                                                       int nrow, int outputs, int stats, ElRot rot, int tables_only) {
+                                                       const __grid_constant__ State<double> st, int nrow,
+                                                       int outputs, int stats, ElRot rot, int tables_only, Tape tape) {
   using TB = Tab<NORD>;
   __shared__ JasPar<double> J;
   __shared__ EcpPar E;
@@ -369,8 +461,10 @@ __global__ void __launch_bounds__(128, 3) k_fin_points(const __grid_constant__ S
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, wpos = WPW == 1 ? 0 : wib;
   const int tid = WPW == 1 ? lane : (int)threadIdx.x, tpw = 32 * WPW, per = WPW == 1 ? 4 : 1;
   const int N = s.N, C = s.C, nomax = s.nomax;
-  const Dims D(N, C, NORD, nrow);
-  double *sm = (double *)(dsm + (WPW == 1 ? D.bytes() * wib : 0));
+  const Dims D(N, C, NORD, nrow, WPW == 1);
+  const stab::Tab T = stab::stage(s, dsm);
+  __syncthreads();
+  double *sm = (double *)(dsm + stab::tab_smem(s.nshell, s.nprim) + (WPW == 1 ? D.bytes() * wib : 0));
   double *sd = sm, *xs = sm + D.x(), *V = sm + D.v(), *Z = sm + D.z(), *F = sm + D.f(), *row = sm + D.row(), *red = sm + D.red();
   for (int w = blockIdx.x * per + (WPW == 1 ? wib : 0); w < st.W; w += gridDim.x * per) {
     View<double> v{};
@@ -431,6 +525,10 @@ __global__ void __launch_bounds__(128, 3) k_fin_points(const __grid_constant__ S
             ov[0] = vx; ov[1] = vy; ov[2] = vz;
             st.o_divv[(size_t)w * N + e] = v.divj[e] + dvd;
           }
+          if (tape.v) {
+            double *ov = tape.v + (size_t)w * 4 * N + 3 * e;
+            ov[0] = vx; ov[1] = vy; ov[2] = vz;
+          }
         }
       }
     }
@@ -473,35 +571,25 @@ __global__ void __launch_bounds__(128, 3) k_fin_points(const __grid_constant__ S
         a = warp_sum(a);
         if (lane == 0) F[e] = a;
       }
-      // ---- (electron, centre) pairs in range, centre-major; every warp lists its share of the pairs
-      // in its own part of the records
-      const int np = N * C, share = ((np + WPW - 1) / WPW + 31) & ~31, lo = wpos * share, hi = min(np, lo + share);
-      int cnt = 0;
-      for (int base = lo; base < hi; base += 32) {
-        const int j = base + lane;
+      // ---- (electron, centre) pairs in range, centre-major, so that the points of a round mostly share
+      // their centre: first their masks (and the local part), then the records in order
+      const int np = N * C, nch = (np + 31) / 32;
+      unsigned *msk = (unsigned *)(sm + D.msk());
+      int *moff = (int *)(msk + nch);
+      for (int ch = wpos; ch < nch; ch += WPW) {
+        const int j = 32 * ch + lane;
         bool nl = false;
-        double vps[MAXLCH], r = 0;
-        int c = 0, e = 0;
-        if (j < hi) {
-          c = j / N;
-          e = j - c * N;
-          r = rt[j];
-          const int it = s.ctype[c];
-          ecp_vps(E, it, r, vps);
+        if (j < np) {
+          double vps[MAXLCH];
+          const int it = s.ctype[j / N];
+          ecp_vps(E, it, rt[j], vps);
           vloc += vps[E.lpotp1[it] - 1];
           for (int l = 0; l < E.npotd[it]; l++)
             if (l + 1 != E.lpotp1[it] && fabs(vps[l]) > 1e-4) nl = true;
         }
         const unsigned m = __ballot_sync(0xffffffffu, nl);
-        if (nl) {
-          double *rec = v.nlt + (size_t)(lo + cnt + __popc(m & ((1u << lane) - 1u))) * NLT;
-          rec[0] = (double)(e * C + c);
-          rec[1] = r;
-          for (int l = 0; l < MAXLCH; l++) rec[2 + l] = (l < E.npotd[s.ctype[c]]) ? vps[l] : 0.0;
-        }
-        cnt += __popc(m);
+        if (lane == 0) msk[ch] = m;
       }
-      if (lane == 0) red[8 + wpos] = (double)cnt;
       if (tid == 0) {
         double R[9];
         if (rot.random) random_rotation(rot.seed, (uint32_t)w, rot.sweep, R);
@@ -510,29 +598,42 @@ __global__ void __launch_bounds__(128, 3) k_fin_points(const __grid_constant__ S
         for (int i = 0; i < 9; i++) red[16 + i] = R[i];
       }
       jt::walker_sync<WPW>();
-      int off[WPW + 1];  // tasks listed before each warp's
-      off[0] = 0;
+      if (wpos == 0) {
+        int run = 0;
+        for (int base = 0; base < nch; base += 32) {
+          const int n1 = base + lane < nch ? __popc(msk[base + lane]) : 0;
+          int inc = n1;
 #pragma unroll
-      for (int k = 0; k < WPW; k++) off[k + 1] = off[k] + (int)red[8 + k];
-      ntask = off[WPW];
-      auto record = [&](int task) -> const double * {
-        int k = 0;
-#pragma unroll
-        for (int q = 1; q < WPW; q++) k += task >= off[q];
-        int at = task;
-#pragma unroll
-        for (int q = 1; q < WPW; q++)
-          if (k == q) at = task - off[q];
-        return v.nlt + (size_t)(k * share + at) * NLT;
-      };
+          for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += x;
+          }
+          if (base + lane < nch) moff[base + lane] = run + inc - n1;
+          run += __shfl_sync(0xffffffffu, inc, 31);
+        }
+        if (lane == 0) red[25] = (double)run;
+      }
+      jt::walker_sync<WPW>();
+      ntask = (int)red[25];
+      for (int ch = wpos; ch < nch; ch += WPW) {
+        const unsigned m = msk[ch];
+        if ((m >> lane) & 1u) {
+          const int j = 32 * ch + lane, c = j / N, it = s.ctype[c];
+          double vps[MAXLCH], *rec = v.nlt + (size_t)(moff[ch] + __popc(m & ((1u << lane) - 1u))) * NLT;
+          ecp_vps(E, it, rt[j], vps);
+          rec[0] = (double)((j - c * N) * C + c);
+          rec[1] = rt[j];
+          for (int l = 0; l < MAXLCH; l++) rec[2 + l] = (l < E.npotd[it]) ? vps[l] : 0.0;
+        }
+      }
+      jt::walker_sync<WPW>();
       const int nshc = (s.nshc > 0 && ntask * s.nshc <= nrow) ? s.nshc : 0;
       for (int i = tid; i < ntask * nshc; i += tpw) {
         const int tk = i / nshc, k = i - tk * nshc;
-        const double *rc = record(tk);
+        const double *rc = v.nlt + (size_t)tk * NLT;
         const int ish = s.cshell0[(int)rc[0] % C] + k;
         if (ish < s.cshell0[(int)rc[0] % C + 1])
-          row[i] = is_gauss(s.shell[ish]) ? gauss_radial(s, s.shprim[ish], zmin[ish], rc[1] * rc[1])
-                                          : general_radial(s, ish, rc[1]);
+          row[i] = stab::factor(s, T, ish, T.rec[ish], rc[1] * rc[1]);
       }
       jt::walker_sync<WPW>();
       const int nq = E.nquad, npts = ntask * nq;
@@ -540,7 +641,7 @@ __global__ void __launch_bounds__(128, 3) k_fin_points(const __grid_constant__ S
       for (int t0 = 32 * wpos; t0 < npts; t0 += 32 * WPW) {
         const bool act = t0 + lane < npts;
         const int t = act ? t0 + lane : t0, task = t / nq, q = t - task * nq;
-        const double *rec = record(task);
+        const double *rec = v.nlt + (size_t)task * NLT;
         const int idx = (int)rec[0], e = idx / C, c = idx - e * C;
         const double r = rec[1], *cc = s.cent + 3 * c, *xe = xs + 3 * e, *q0 = s.quad->q0[q];
         double qv[3];
@@ -548,14 +649,19 @@ __global__ void __launch_bounds__(128, 3) k_fin_points(const __grid_constant__ S
         for (int k = 0; k < 3; k++) qv[k] = R[3 * k] * q0[0] + R[3 * k + 1] * q0[1] + R[3 * k + 2] * q0[2];
         const double costh = ((xe[0] - cc[0]) * qv[0] + (xe[1] - cc[1]) * qv[1] + (xe[2] - cc[2]) * qv[2]) / r;
         const double xn[3] = {cc[0] + r * qv[0], cc[1] + r * qv[1], cc[2] + r * qv[2]};
-        const double dr = point_ratio(s, zmin, xn, v.gproj + (size_t)e * s.nbasis, c, nshc ? row + task * nshc : nullptr);
-        const double dj = point_jastrow<NORD>(s, J, D, sm, xn, e, act, lane);
+        const double dr = point_ratio(s, T, xn, v.gproj + (size_t)e * s.nbasis, c, nshc ? row + task * nshc : nullptr);
+        double dj;
+        if constexpr (WPW == 1) dj = lane_jastrow<NORD>(s, J, D, sm, sm + D.lanes(), xn, e, lane);
+        else dj = point_jastrow<NORD>(s, J, D, sm, xn, e, act, lane);
         if (!act) continue;
         const int it = s.ctype[c];
         double vp = 0;
         for (int l = 0; l < E.npotd[it]; l++)
           if (l + 1 != E.lpotp1[it]) vp += rec[2 + l] * yl0(l, costh);
-        vnl += s.quad->wq[q] * exp(dj) * vp * dr;
+        const double cb = s.quad->wq[q] * exp(dj) * vp, coeff = cb * dr;
+        vnl += coeff;
+        if (tape.c) tape.c[(size_t)w * N * C * nq + t] = coeff;
+        if (tape.b) tape.b[(size_t)w * tape.bstride + t] = cb;
       }
     }
     d2lnd = warp_sum(d2lnd);
@@ -581,6 +687,13 @@ __global__ void __launch_bounds__(128, 3) k_fin_points(const __grid_constant__ S
         st.s_esum[w] += res.eloc;
         st.s_e2sum[w] += res.eloc * res.eloc;
         st.s_elast[w] = res.eloc;
+      }
+      if (tape.el && lane == 0) {
+        tape.el[w] = res.eloc;
+        tape.n[w] = ntask;
+        double *o = st.el_sc + (size_t)w * EL_SC;  // what the local part of the orbital energies needs
+        o[10] = (res.d2j + res.vj2) / N;
+        o[11] = (res.pe - res.pe_nl) / N;
       }
     }
     if (st.m_fso) {  // FP32 move tables of a mixed-precision state (mirror_store)

@@ -2,6 +2,7 @@
 // staged evaluation, as FP64 tensor-core products, and the Slater-matrix inversion in registers.
 #pragma once
 #include "kernels.cuh"
+#include "shelltab.cuh"
 
 namespace ot {
 
@@ -16,32 +17,20 @@ __host__ __device__ constexpr int ldb() { return 16 * NT + 4; }
 template <int NT>
 __host__ __device__ constexpr size_t smem_bytes() { return sizeof(double) * (size_t)KB * (LDA + ldb<NT>()); }
 
-// A Gaussian shell with n = l + 1, l <= 2: S_lm(d) g(r^2), g = sum_p w e^(-z r^2); no square root or division.
-// grad = grad S g + 2 d S g', lap = S (4 r^2 g'' + (4l + 6) g').
+// A Gaussian shell with n = l + 1, l <= 2: S_lm(d) g(r^2), no square root or division.
 template <int l, class Put>
-__device__ __forceinline__ void gauss_shell5(const Sys<double> &s, int2 pr, double d0, double d1, double d2, Put put) {
-  const double r2 = d0 * d0 + d1 * d1 + d2 * d2;
-  double g = 0, gp = 0, gpp = 0;
-  for (int p = pr.x; p < pr.x + pr.y; p++) {
-    const double z = s.pz[p], e = s.pc[p] * exp(-z * r2);
-    g += e;
-    gp -= z * e;
-    gpp += z * z * e;
-  }
-  const double lp = 4 * r2 * gpp + (4 * l + 6) * gp, t = 2 * gp;
+__device__ __forceinline__ void gauss_shell5(const stab::Rad &R, double d0, double d1, double d2, Put put) {
   double S[9], G[9][3];
   solid_all<double, true>(l, d0, d1, d2, S, G);
-  const int nm = 2 * l + 1;
 #pragma unroll
-  for (int sl = 0; sl < 9; sl++)
-    if (sl < nm) {
-      const double st = S[sl] * t;
-      put(sl, 0, S[sl] * g);
-      put(sl, 1, G[sl][0] * g + st * d0);
-      put(sl, 2, G[sl][1] * g + st * d1);
-      put(sl, 3, G[sl][2] * g + st * d2);
-      put(sl, 4, S[sl] * lp);
-    }
+  for (int sl = 0; sl < 2 * l + 1; sl++) {
+    const double st = S[sl] * R.t;
+    put(sl, 0, S[sl] * R.q);
+    put(sl, 1, G[sl][0] * R.q + st * d0);
+    put(sl, 2, G[sl][1] * R.q + st * d1);
+    put(sl, 3, G[sl][2] * R.q + st * d2);
+    put(sl, 4, S[sl] * R.lap);
+  }
 }
 
 // Any other shell (kept out of line: its registers are not those of the contraction).
@@ -60,17 +49,23 @@ static __device__ __noinline__ void general_shell5(const Sys<double> &s, int ish
 // walkers of 128 electrons, 416 basis functions, 15.6 -> 7.1 ms; 3001 of 20 electrons, 65 functions,
 // 0.32 -> 0.08 ms.  k_el_orb stays for more than 64 orbitals of a spin.
 // chunk[k]: first shell, shells, first basis function, basis functions.
-template <int NT>
-__global__ void __launch_bounds__(THREADS, 2) k_orb_tile(const __grid_constant__ Sys<double> s, State<double> st, const int4 *chunk, int nchunk) {
+// GEN: shells other than those Gaussians occur.
+// ALL: the columns blockIdx.y * 16 NT onwards of all orbitals (s.call), for every electron, into all + w
+// stride as [N][5][norb] instead, without the Slater matrices.
+template <int NT, bool ALL, bool GEN>
+__global__ void __launch_bounds__(THREADS, 2) k_orb_tile(const __grid_constant__ Sys<double> s, State<double> st, const int4 *chunk, int nchunk,
+                                                         double *all, size_t stride) {
   extern __shared__ __align__(16) double sm[];
+  const stab::Tab T = stab::stage(s, sm + KB * (LDA + ldb<NT>()));
   double *phi = sm, *cf = sm + KB * LDA;
   constexpr int LDB = ldb<NT>();
-  const int sp = blockIdx.y, n = sp ? s.ndn : s.nup, no = s.nocc[sp], e0 = sp ? s.nup : 0;
+  const int sp = ALL ? 0 : blockIdx.y, n = ALL ? s.N : (sp ? s.ndn : s.nup), e0 = sp ? s.nup : 0;
+  const int col0 = ALL ? (int)blockIdx.y * 16 * NT : 0, ld = ALL ? s.norb : s.nocc[sp], no = ld - col0;
   const long long items = (long long)st.W * n, i0 = (long long)blockIdx.x * EB;
   if (i0 >= items) return;
   const int tid = threadIdx.x, lane = tid & 31, wib = tid >> 5, rr = lane >> 2, kq = lane & 3;
   const int wm = wib >> 1, wn = wib & 1;
-  const double *coef = s.cocc[sp];
+  const double *coef = ALL ? s.call + col0 : s.cocc[sp];
   double px[3] = {0, 0, 0};
   {
     long long it = i0 + lane;
@@ -79,12 +74,13 @@ __global__ void __launch_bounds__(THREADS, 2) k_orb_tile(const __grid_constant__
     const double *x = st.x + ((size_t)w * s.N + e) * 3;
     px[0] = x[0]; px[1] = x[1]; px[2] = x[2];
   }
-  const bool vec = no % 2 == 0 && (reinterpret_cast<uintptr_t>(coef) & 15) == 0;
+  const bool vec = ld % 2 == 0 && (reinterpret_cast<uintptr_t>(coef) & 15) == 0;
   double acc[5][NT][2];
 #pragma unroll
   for (int i = 0; i < 5; i++)
 #pragma unroll
     for (int j = 0; j < NT; j++) acc[i][j][0] = acc[i][j][1] = 0;
+  __syncthreads();  // the shell tables are in place
   for (int k = 0; k < nchunk; k++) {
     const int4 ch = chunk[k];
     const int nk4 = (ch.w + 3) & ~3;
@@ -94,13 +90,13 @@ __global__ void __launch_bounds__(THREADS, 2) k_orb_tile(const __grid_constant__
       for (int i = tid; i < nk4 * V; i += THREADS) {
         const int r = i / V, c = 2 * (i - r * V);
         double *dst = cf + r * LDB + c;
-        if (r < ch.w && c < no) cp_async16(dst, coef + (size_t)(ch.z + r) * no + c);
+        if (r < ch.w && c < no) cp_async16(dst, coef + (size_t)(ch.z + r) * ld + c);
         else dst[0] = dst[1] = 0.0;
       }
     } else {
       for (int i = tid; i < nk4 * 16 * NT; i += THREADS) {
         const int r = i / (16 * NT), c = i - r * (16 * NT);
-        cf[r * LDB + c] = (r < ch.w && c < no) ? coef[(size_t)(ch.z + r) * no + c] : 0.0;
+        cf[r * LDB + c] = (r < ch.w && c < no) ? coef[(size_t)(ch.z + r) * ld + c] : 0.0;
       }
     }
     cp_async_commit();
@@ -109,21 +105,18 @@ __global__ void __launch_bounds__(THREADS, 2) k_orb_tile(const __grid_constant__
       for (int c = 0; c < 5; c++) phi[r * LDA + c * EB + lane] = 0.0;
     for (int q = wib; q < ch.y; q += 8) {
       const int ish = ch.x + q;
-      const int4 sh = s.shell[ish];
-      double *o = phi + (s.shb0[ish] - ch.z) * LDA + lane;
+      const ShellRec h = T.rec[ish];
+      double *o = phi + (h.b0 - ch.z) * LDA + lane;
       auto put = [o](int sl, int c, double v) { o[sl * LDA + c * EB] = v; };
-      if (sh.w == 1 && sh.y == sh.z + 1) {
-        const double *cc = s.cent + 3 * sh.x;
-        const double d0 = px[0] - cc[0], d1 = px[1] - cc[1], d2 = px[2] - cc[2];
-        const int2 pr = s.shprim[ish];
-        switch (sh.z) {
-        case 0: gauss_shell5<0>(s, pr, d0, d1, d2, put); break;
-        case 1: gauss_shell5<1>(s, pr, d0, d1, d2, put); break;
-        case 2: gauss_shell5<2>(s, pr, d0, d1, d2, put); break;
-        default: general_shell5(s, ish, px[0], px[1], px[2], o);
-        }
-      } else {
+      if (GEN && (h.kind != 1 || h.l > 2)) {
         general_shell5(s, ish, px[0], px[1], px[2], o);
+      } else {
+        const double *cc = s.cent + 3 * h.cen;
+        const double d0 = px[0] - cc[0], d1 = px[1] - cc[1], d2 = px[2] - cc[2];
+        const stab::Rad R = stab::gauss_rad(T, h, d0 * d0 + d1 * d1 + d2 * d2);
+        if (h.l == 0) gauss_shell5<0>(R, d0, d1, d2, put);
+        else if (h.l == 1) gauss_shell5<1>(R, d0, d1, d2, put);
+        else gauss_shell5<2>(R, d0, d1, d2, put);
       }
     }
     cp_async_wait<0>();
@@ -149,7 +142,8 @@ __global__ void __launch_bounds__(THREADS, 2) k_orb_tile(const __grid_constant__
     const long long it = i0 + (row - ch * EB);
     if (it >= items) continue;
     const int w = (int)(it / n), eo = (int)(it - (long long)w * n);
-    double *o = st.orb5 + (((size_t)w * s.N + e0 + eo) * 5 + ch) * nomax;
+    double *o = ALL ? all + (size_t)w * stride + ((size_t)eo * 5 + ch) * ld + col0
+                    : st.orb5 + (((size_t)w * s.N + e0 + eo) * 5 + ch) * nomax;
     double *A = st.ainv + (size_t)w * st.astride + (sp ? s.nup * s.nup : 0) + (size_t)eo * n;
 #pragma unroll
     for (int j = 0; j < NT; j++)
@@ -157,7 +151,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_orb_tile(const __grid_constant__
       for (int h = 0; h < 2; h++) {
         const int c = wn * 8 * NT + 8 * j + 2 * kq + h;
         if (c < no) o[c] = acc[i][j][h];
-        if (ch == 0 && c < n) A[c] = acc[i][j][h];
+        if (!ALL && ch == 0 && c < n) A[c] = acc[i][j][h];
       }
   }
 }
