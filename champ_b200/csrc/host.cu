@@ -1566,6 +1566,8 @@ int champ_create(const champ_system *d, int32_t w_max, int32_t precision, void *
     }
   }
   if (use64 && !rc) rc = move_batch_setup(c);
+  if (use64 && !rc) rc = small_setup(c);
+  if (use64 && !rc) rc = pg_tile_setup(c);
   if (rc) { champ_destroy(c); return rc; }
   c->nfree = c->ncsfp + c->norbp + c->nparm_jas;
   {

@@ -184,6 +184,12 @@ static int launch_t(champ_ctx *c, Op op, const OpArgs &a) {
       return run_el_staged<T, NORD, MD>(c, st, op == Op::EvalOut, false, rot, a.rebuild);
     }
     c->orb5_valid = false;
+    if constexpr (std::is_same<T, double>::value)
+      if (c->small && !a.st_override) {
+        ElRot rot{};
+        for (int i = 0; i < 9; i++) rot.R[i] = R[i];
+        return small_eval(c, st, op == Op::EvalOut, false, rot);
+      }
     if (tc) {
       int rc = run_orb_tc<T>(c, st);
       if (rc) return rc;
@@ -209,6 +215,8 @@ static int launch_t(champ_ctx *c, Op op, const OpArgs &a) {
     break;
   }
   case Op::DmcMove: {
+    if constexpr (std::is_same<T, double>::value)
+      if (c->small && !c->dpar.persist && a.phase != 1) return small_dmc(c, st, a.phase != 2);
     // persistent: as many blocks as the SMs can hold at once (at most 16 per SM; a block that
     // finds the work counter exhausted exits at once), no more than the walkers need
     const int sm = c->num_sms > 0 ? c->num_sms : 148;
@@ -219,6 +227,8 @@ static int launch_t(champ_ctx *c, Op op, const OpArgs &a) {
     break;
   }
   case Op::Tmove: {
+    if constexpr (std::is_same<T, double>::value)
+      if (c->small) return small_tmove(c, st, a);
     const int wl = a.dmc ? c->dpar.wmax : st.W;
     k_dmc_tmove<T, NORD, MD><<<dim3((wl + K.wpb - 1) / K.wpb), block, K.smem, c->stream>>>(
         s, st, K.lay, st.W, a.dmc ? c->dA.nw : nullptr, a.tau, a.variant, a.seed, a.dmc ? c->dA.ctr : nullptr,
@@ -238,6 +248,14 @@ static int launch_t(champ_ctx *c, Op op, const OpArgs &a) {
       rot.sweep = a.sweep0;
       return run_el_staged<T, NORD, MD>(c, st, false, true, rot);
     }
+    if constexpr (std::is_same<T, double>::value)
+      if (c->small && !a.st_override && a.phase == 3) {
+        ElRot rot{};
+        rot.random = 1;
+        rot.seed = a.seed;
+        rot.sweep = a.sweep0;
+        return small_eval(c, st, false, true, rot);
+      }
     if (a.phase >= 0) {
       const bool acc6 = c->mover.kind == 6;
       if (a.phase == 1 && !acc6 && c->move_batch && c->el_staged && !a.st_override)
@@ -274,9 +292,9 @@ static int launch_t(champ_ctx *c, Op op, const OpArgs &a) {
       kern<<<grid, block, K.smem, c->stream>>>(s, st, K.lay, a.nsweep, a.seed, a.sweep0, a.step, c->reinv_every, c->mover);
       break;
     }
-    CK(cudaMemsetAsync(st.s_esum, 0, sizeof(double) * st.W, c->stream));
-    CK(cudaMemsetAsync(st.s_e2sum, 0, sizeof(double) * st.W, c->stream));
-    CK(cudaMemsetAsync(st.s_acc, 0, sizeof(double) * st.W, c->stream));
+    CK(cudaMemsetAsync(st.s_esum, 0, sizeof(double) * 3 * (size_t)c->wmax, c->stream));  // esum, e2sum, acc
+    if constexpr (std::is_same<T, double>::value)
+      if (c->small && !a.st_override) return small_vmc(c, st, a);
     const bool tc = c->tc_on && !a.st_override;  // only FP32 contexts turn it on
     if (!tc) {
       auto kern = c->mover.kind == 6 ? k_vmc<T, NORD, MD, 0, 6> : k_vmc<T, NORD, MD, 0>;

@@ -1,0 +1,111 @@
+// small.cu -- launchers of the small walkers' kernels (small.cuh).
+#include <algorithm>
+
+#include "ctx.h"
+#include "nlpoints.cuh"
+#include "small.cuh"
+
+namespace {
+
+template <class K>
+int big_smem(K kern, size_t bytes) {
+  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+  return fit_carveout(kern, 128, bytes);
+}
+template <int NORD>
+int attrs(const champ_ctx *c) {
+  const size_t b = sizeof(double) * (size_t)sm::Lay(c->N, c->C, c->nordc).total() * 16 + stab::tab_smem(c->sd.nshell, c->sd.nprim);
+  int rc = CHAMP_OK;
+  for (auto k : {sm::k_small<NORD, sm::EVAL>, sm::k_small<NORD, sm::GAUSS>, sm::k_small<NORD, sm::ACCEL>, sm::k_small<NORD, sm::DMC>,
+                 sm::k_small<NORD, sm::DMC_EL>, sm::k_small_tmove<NORD>})
+    if (!rc) rc = big_smem(k, b);
+  return rc;
+}
+
+// Threads of a block: 128 (16 walkers), fewer while the walkers would not reach every SM.
+int threads(const champ_ctx *c, int W) {
+  const int sm = c->num_sms > 0 ? c->num_sms : 148;
+  int t = 128;
+  while (t > 32 && (W * sm::GS + t - 1) / t < sm) t >>= 1;
+  return t;
+}
+
+template <int NORD>
+int run(champ_ctx *c, const State<double> &st, int mode, const sm::Args &A, int W) {
+  const int t = threads(c, W), per = t / sm::GS;
+  const size_t smem = sizeof(double) * (size_t)sm::Lay(c->N, c->C, c->nordc).total() * per + stab::tab_smem(c->sd.nshell, c->sd.nprim);
+  const dim3 g((W + per - 1) / per);
+  switch (mode) {
+  case sm::EVAL: sm::k_small<NORD, sm::EVAL><<<g, t, smem, c->stream>>>(c->sd, st, A); break;
+  case sm::GAUSS: sm::k_small<NORD, sm::GAUSS><<<g, t, smem, c->stream>>>(c->sd, st, A); break;
+  case sm::ACCEL: sm::k_small<NORD, sm::ACCEL><<<g, t, smem, c->stream>>>(c->sd, st, A); break;
+  case sm::DMC: sm::k_small<NORD, sm::DMC><<<g, t, smem, c->stream>>>(c->sd, st, A); break;
+  case sm::DMC_EL: sm::k_small<NORD, sm::DMC_EL><<<g, t, smem, c->stream>>>(c->sd, st, A); break;
+  default: sm::k_small_tmove<NORD><<<g, t, smem, c->stream>>>(c->sd, st, A);
+  }
+  CK(cudaGetLastError());
+  return CHAMP_OK;
+}
+int run(champ_ctx *c, const State<double> &st, int mode, const sm::Args &A, int W) {
+  return c->nordc == 4 ? run<4>(c, st, mode, A, W) : c->nordc == 5 ? run<5>(c, st, mode, A, W) : run<0>(c, st, mode, A, W);
+}
+
+}  // namespace
+
+// Small walkers: state resident in shared memory (kd), one determinant, at most 8 electrons and 4 of a
+// spin, one centre type where there are e-e-n terms.
+int small_setup(champ_ctx *c) {
+  if (!c->kd.lay.resident || c->md.multidet || c->nmax > sm::NO || c->N > sm::NE || (c->nordc > 1 && c->nct != 1)) return CHAMP_OK;
+  if (sizeof(double) * (size_t)sm::Lay(c->N, c->C, c->nordc).total() * 16 + stab::TAB_MAX > 200 * 1024) return CHAMP_OK;
+  std::vector<int4> sh(c->nshell);
+  CK(cudaMemcpy(sh.data(), c->sd.shell, sizeof(int4) * c->nshell, cudaMemcpyDeviceToHost));
+  std::vector<int> order(c->nshell);
+  for (int i = 0; i < c->nshell; i++) order[i] = i;
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return sh[a].z < sh[b].z; });
+  int *d = nullptr;
+  CK(cudaMalloc(&d, sizeof(int) * std::max(c->nshell, 1)));
+  c->allocs.push_back(d);
+  CK(cudaMemcpy(d, order.data(), sizeof(int) * c->nshell, cudaMemcpyHostToDevice));
+  c->small_order = d;
+  const int rc = c->nordc == 4 ? attrs<4>(c) : c->nordc == 5 ? attrs<5>(c) : attrs<0>(c);
+  if (!rc) c->small = 1;
+  return rc;
+}
+
+int small_eval(champ_ctx *c, const State<double> &st, bool outputs, bool stats, const ElRot &rot) {
+  sm::Args A;
+  A.order = c->small_order;
+  A.outputs = outputs;
+  A.stats = stats;
+  A.rot = rot;
+  return run(c, st, sm::EVAL, A, st.W);
+}
+int small_vmc(champ_ctx *c, const State<double> &st, const OpArgs &a) {
+  sm::Args A;
+  A.order = c->small_order;
+  A.nsweep = a.nsweep;
+  A.seed = a.seed;
+  A.sweep0 = a.sweep0;
+  A.step = a.step;
+  A.mv = c->mover;
+  return run(c, st, c->mover.kind == 6 ? sm::ACCEL : sm::GAUSS, A, st.W);
+}
+int small_dmc(champ_ctx *c, const State<double> &st, bool moves) {
+  sm::Args A;
+  A.order = c->small_order;
+  A.P = c->dpar;
+  A.D = c->dA;
+  return run(c, st, moves ? sm::DMC : sm::DMC_EL, A, c->dpar.wmax);
+}
+int small_tmove(champ_ctx *c, const State<double> &st, const OpArgs &a) {
+  sm::Args A;
+  A.order = c->small_order;
+  A.tau = a.tau;
+  A.variant = a.variant;
+  A.seed = a.seed;
+  A.sweep0 = a.sweep0;
+  A.nw = a.dmc ? c->dA.nw : nullptr;
+  A.step_dev = a.dmc ? c->dA.ctr : nullptr;
+  A.moved = a.moved;
+  return run(c, st, 100, A, a.dmc ? c->dpar.wmax : st.W);
+}

@@ -1,0 +1,1137 @@
+// small.cuh -- small walkers (up to 8 electrons, 4 of a spin, one determinant, FP64): moves and E_L with 8
+// lanes per walker, 4 walkers to a warp.
+//
+// A warp per walker leaves most lanes idle on such systems (7 pairs, 2 centres, 4 orbitals, 24
+// shells): the 8-electron dimer's DMC step took 102 thousand warp instructions per walker, at a third of
+// the issue rate.  With 8 lanes a proposal's shells are 3 to a lane and its pairs one to a lane; an
+// evaluation has an electron per lane, a quadrature point per lane.  Orbital values are summed per lane
+// over its shells straight into the (at most 4) orbitals and shared by shuffles, so no basis row is
+// stored, and the determinant ratio at a quadrature point needs no projection on the basis.  The orbital
+// rows of the electrons' positions are kept through the moves: neither the drift at the current
+// position nor the evaluation after the moves forms them again.
+// Everything is FP64; sums differ in order from the warp-per-walker kernels (full_eval, propose).
+// What bounds it: FP64 issue and latency at 12 warps per SM.
+#pragma once
+#include "jastile.cuh"
+
+namespace sm {
+
+using jt::sfor;
+
+constexpr int GS = 8;  // lanes of a walker
+constexpr int NO = 4;  // most electrons (= orbitals) of a spin
+constexpr int NE = 8;  // most electrons
+constexpr int RCAP = 96;  // radial values of the tasks' centres kept per walker
+
+// Doubles of a walker in shared memory.
+struct Lay {
+  int N, C, qm;
+  __host__ __device__ Lay(int N_, int C_, int nord) : N(N_), C(C_), qm(nord > 1 ? nord - 1 : 1) {}
+  __host__ __device__ int ai() const { return 3 * N; }
+  __host__ __device__ int f() const { return ai() + 2 * NO * NO; }
+  __host__ __device__ int a() const { return f() + N * N; }
+  __host__ __device__ int h() const { return a() + N * C; }
+  __host__ __device__ int z() const { return h() + N * C; }
+  __host__ __device__ int pa() const { return z() + N * qm; }
+  __host__ __device__ int ph() const { return pa() + C; }
+  __host__ __device__ int pr() const { return ph() + C; }        // proposed row [5][NO]
+  __host__ __device__ int pl() const { return pr() + 5 * NO; }   // [C][GS] a point's scaled distances per lane
+  __host__ __device__ int row() const { return pl() + C * GS; }  // rows [N][5][NO]; then the tasks
+  __host__ __device__ int rlen() const {
+    const int t = N * C * NLT + RCAP, r = N * 5 * NO, u = 2 * MAXQ;  // u: a T-move's elements and ratios
+    return t > r ? (t > u ? t : u) : (r > u ? r : u);
+  }
+  // odd, so that the walkers of a warp start in different banks
+  __host__ __device__ int total() const { return (row() + rlen()) | 1; }
+};
+
+struct Args {
+  int nsweep = 1, outputs = 0, stats = 0;
+  uint64_t seed = 0, sweep0 = 0;
+  double step = 0;
+  Mover mv{1, 5.0, 1.0, 1.0};
+  ElRot rot{};
+  const int *order = nullptr;  // shells by l, so that the lanes of a round mostly share it
+  DmcPar P{};
+  DmcData D{};
+  double tau = 0;
+  int variant = 0;
+  const int *nw = nullptr;
+  const long long *step_dev = nullptr;
+  int *moved = nullptr;
+};
+
+__device__ __forceinline__ unsigned gmask() { return 0xffu << (threadIdx.x & 24); }
+__device__ __forceinline__ double gsum(double v, unsigned m) {
+  v += __shfl_xor_sync(m, v, 4);
+  v += __shfl_xor_sync(m, v, 2);
+  v += __shfl_xor_sync(m, v, 1);
+  return v;
+}
+
+using stab::Rad;
+
+// Adds a shell's functions times the orbital coefficients cf [2l + 1][no] into o.
+template <int l, int NCH>
+__device__ __forceinline__ void add_shell(const Rad &R, double d0, double d1, double d2, const double *cf, int no, double (&o)[NCH][NO]) {
+  double S[9], G[9][3];
+  solid_all<double, NCH == 5>(l, d0, d1, d2, S, G);
+#pragma unroll
+  for (int i = 0; i < 2 * l + 1; i++) {
+    const double st = S[i] * R.t;
+    const double f0 = S[i] * R.q, f1 = G[i][0] * R.q + st * d0, f2 = G[i][1] * R.q + st * d1, f3 = G[i][2] * R.q + st * d2,
+                 f4 = S[i] * R.lap;
+#pragma unroll
+    for (int k = 0; k < NO; k++) {
+      const double c = k < no ? cf[i * no + k] : 0.0;
+      o[0][k] += c * f0;
+      if constexpr (NCH == 5) {
+        o[1][k] += c * f1;
+        o[2][k] += c * f2;
+        o[3][k] += c * f3;
+        o[4][k] += c * f4;
+      }
+    }
+  }
+}
+
+// Values (NCH 1) or values, gradients and Laplacians (NCH 5) of the spin's orbitals at a point into
+// out[NCH][NO] (shared memory), the walker's lanes over the shells.
+template <int NCH>
+__device__ __noinline__ void orb_row(const Sys<double> &s, const stab::Tab &T, const int *order, int sp, double x, double y, double z,
+                                     double *out) {
+  const int sub = threadIdx.x & 7;
+  const unsigned m = gmask();
+  const int no = s.nocc[sp];
+  const double *cf = s.cocc[sp];
+  double o[NCH][NO];
+#pragma unroll
+  for (int c = 0; c < NCH; c++)
+#pragma unroll
+    for (int k = 0; k < NO; k++) o[c][k] = 0;
+  for (int q = sub; q < s.nshell; q += GS) {
+    const int ish = order[q];
+    const ShellRec h = T.rec[ish];
+    const double *cc = s.cent + 3 * h.cen, *cr = cf + (size_t)h.b0 * no;
+    const double d0 = x - cc[0], d1 = y - cc[1], d2 = z - cc[2], r2 = d0 * d0 + d1 * d1 + d2 * d2;
+    Rad R;
+    if (NCH == 1) R = Rad{stab::factor(s, T, ish, h, r2), 0.0, 0.0};
+    else if (h.kind == 1) R = stab::gauss_rad(T, h, r2);
+    else R = stab::general_rad(s, ish, r2);
+    switch (h.l) {
+    case 0: add_shell<0, NCH>(R, d0, d1, d2, cr, no, o); break;
+    case 1: add_shell<1, NCH>(R, d0, d1, d2, cr, no, o); break;
+    case 2: add_shell<2, NCH>(R, d0, d1, d2, cr, no, o); break;
+    case 3: add_shell<3, NCH>(R, d0, d1, d2, cr, no, o); break;
+    default: add_shell<4, NCH>(R, d0, d1, d2, cr, no, o);
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < NCH; c++)
+#pragma unroll
+    for (int k = 0; k < NO; k++) {
+      const double v = gsum(o[c][k], m);
+      if (((c * NO + k) & 7) == sub) out[c * NO + k] = v;
+    }
+  __syncwarp(m);
+}
+
+template <int NORD>
+struct Tab {
+  static constexpr jt::Combos cb = jt::make_combos(NORD);
+  static constexpr Terms tl = make_terms(NORD);
+};
+
+// Power sums of one electron's scaled distances over the centres, with gradients and Laplacians.
+template <int NORD>
+struct One {
+  static constexpr int QM = NORD > 1 ? NORD - 1 : 1;
+  double S[QM], g[QM][3], L[QM];
+};
+template <int NORD, int LEVEL>
+__device__ __forceinline__ void one_sums(const Sys<double> &s, double sk, const double *xe, const double *pa,
+                                         const double *ph, One<NORD> &o) {
+  constexpr int QM = One<NORD>::QM;
+#pragma unroll
+  for (int q = 0; q < QM; q++) o.S[q] = o.g[q][0] = o.g[q][1] = o.g[q][2] = o.L[q] = 0;
+  if constexpr (NORD > 1)
+    for (int c = 0; c < s.C; c++) {
+      const double a = pa[c];
+      double p = a, pm = 1;
+      double dx = 0, dy = 0, dz = 0, h = 0, s2 = 0;
+      if (LEVEL > 0) {
+        h = ph[c];
+        s2 = sk * sk * a * a;
+        dx = xe[0] - s.cent[3 * c];
+        dy = xe[1] - s.cent[3 * c + 1];
+        dz = xe[2] - s.cent[3 * c + 2];
+      }
+#pragma unroll
+      for (int q = 1; q <= QM; q++) {
+        o.S[q - 1] += p;
+        if (LEVEL > 0) {
+          const double t = q * pm * h;
+          o.g[q - 1][0] += t * dx;
+          o.g[q - 1][1] += t * dy;
+          o.g[q - 1][2] += t * dz;
+          if (LEVEL > 1) o.L[q - 1] += q * p * ((q - 1) * s2 + 2 * h);
+        }
+        pm = p;
+        p *= a;
+      }
+    }
+}
+
+// e-e and e-e-n terms of electron e (position xe, scaled distances pa, ph = -k a^2 / r, sums o) with
+// electron j (xj, aj, power sums zj): value, gradient (LEVEL 1) and Laplacian (2) with respect to e.
+template <int NORD, int LEVEL>
+__device__ __forceinline__ double pair_terms(const Sys<double> &s, const JasPar<double> &J, int e, int j, const double *xe,
+                                             const double *pa, const double *ph, const One<NORD> &o, const double *xj,
+                                             const double *aj, const double *zj, double *g, double &lap, double &rin) {
+  using TB = Tab<NORD>;
+  constexpr int NC = jt::make_combos(NORD).n, NT = make_terms(NORD).n, NCA = NC > 0 ? NC : 1;
+  constexpr int QM = One<NORD>::QM;
+  const double sk = J.scalek;
+  const double r0 = xe[0] - xj[0], r1 = xe[1] - xj[1], r2 = xe[2] - xj[2];
+  const double rij = sqrt(r0 * r0 + r1 * r1 + r2 * r2);
+  const double du = 1.0 / (1.0 + sk * rij);
+  int isb, ipar;
+  double ss;
+  pair_class(J, s.nup, e, j, isb, ss, ipar);
+  double fu = 0, fuu = 0;
+  double f = jas_ee<double, (LEVEL > 0)>(J, isb, ss, ipar, rij, du, fu, fuu);
+  rin = LEVEL > 0 ? 1.0 / rij : 0.0;
+  double w1 = 0, w2 = 0, g0 = 0, g1 = 0, g2 = 0, tt = 0, lp = 0;
+  if constexpr (NORD > 1) {
+    double ax[NCA], ag[NCA][3], al[NCA];
+#pragma unroll
+    for (int y = 0; y < NCA; y++) ax[y] = ag[y][0] = ag[y][1] = ag[y][2] = al[y] = 0;
+    for (int c = 0; c < s.C; c++) {
+      const double a = pa[c], b = aj[c];
+      double ap[QM + 1], bp[QM + 1];
+      ap[0] = bp[0] = 1;
+#pragma unroll
+      for (int q = 1; q <= QM; q++) { ap[q] = ap[q - 1] * a; bp[q] = bp[q - 1] * b; }
+      double h = 0, dx = 0, dy = 0, dz = 0, s2 = 0;
+      if (LEVEL > 0) {
+        h = ph[c];
+        s2 = sk * sk * a * a;
+        dx = xe[0] - s.cent[3 * c];
+        dy = xe[1] - s.cent[3 * c + 1];
+        dz = xe[2] - s.cent[3 * c + 2];
+      }
+      sfor<2 * NC>([&](auto Y) {
+        constexpr int yv = decltype(Y)::v, y = yv / 2, l = TB::cb.l[y], m = TB::cb.m[y];
+        if constexpr (yv % 2 == 0 || l > 0) {
+          constexpr int p = yv % 2 ? m : l + m, q = yv % 2 ? l + m : m;
+          const double wq = (l ? 1.0 : 2.0) * bp[q];
+          ax[y] += ap[p] * wq;
+          if constexpr (LEVEL > 0) {
+            const double t = p * ap[p - 1] * h * wq;
+            ag[y][0] += t * dx;
+            ag[y][1] += t * dy;
+            ag[y][2] += t * dz;
+            if constexpr (LEVEL > 1) al[y] += p * ap[p] * ((p - 1) * s2 + 2 * h) * wq;
+          }
+        }
+      });
+    }
+    double u[NORD + 1];
+    u[0] = 1;
+#pragma unroll
+    for (int q = 1; q <= NORD; q++) u[q] = u[q - 1] * du;
+    sfor<NT>([&](auto LL) {
+      constexpr int ll = decltype(LL)::v, k = TB::tl.k[ll], l = TB::tl.l[ll];
+      if constexpr (TB::tl.m[ll] == 0) {
+        const double c = J.c[0][ll];
+        double Y = 2.0 * s.C;
+        if constexpr (l > 0) Y = o.S[l - 1] + zj[l - 1];
+        f += c * u[k] * Y;
+        if constexpr (LEVEL > 0) {
+          w1 += (c * k) * u[k - 1] * Y;
+          if constexpr (k > 1 && LEVEL > 1) w2 += (c * (k * (k - 1))) * u[k - 2] * Y;
+          if constexpr (l > 0) {
+            const double cu = c * u[k];
+            g0 += cu * o.g[l - 1][0];
+            g1 += cu * o.g[l - 1][1];
+            g2 += cu * o.g[l - 1][2];
+            if constexpr (LEVEL > 1) {
+              tt += (c * k) * u[k - 1] * (r0 * o.g[l - 1][0] + r1 * o.g[l - 1][1] + r2 * o.g[l - 1][2]);
+              lp += cu * o.L[l - 1];
+            }
+          }
+        }
+      }
+    });
+    sfor<NC>([&](auto YY) {
+      constexpr int y = decltype(YY)::v, nk = TB::cb.nk[y];
+      double cu = 0, ct = 0, c2 = 0;
+      sfor<nk>([&](auto K) {
+        constexpr int k = decltype(K)::v, ik = TB::cb.ll[y][k];
+        const double c = J.c[0][ik];
+        cu += c * u[k];
+        if constexpr (k > 0 && LEVEL > 0) ct += (c * k) * u[k - 1];
+        if constexpr (k > 1 && LEVEL > 1) c2 += (c * (k * (k - 1))) * u[k - 2];
+      });
+      f += cu * ax[y];
+      if constexpr (LEVEL > 0) {
+        w1 += ct * ax[y];
+        g0 += cu * ag[y][0];
+        g1 += cu * ag[y][1];
+        g2 += cu * ag[y][2];
+        if constexpr (LEVEL > 1) {
+          w2 += c2 * ax[y];
+          tt += ct * (r0 * ag[y][0] + r1 * ag[y][1] + r2 * ag[y][2]);
+          lp += cu * al[y];
+        }
+      }
+    });
+  }
+  if constexpr (LEVEL > 0) {
+    const double u1 = -sk * du * du;  // du/dr; u'' + 2 u'/r = -2 k du^3 / r
+    const double fr = fu + w1 * u1 * rin;
+    g[0] = fr * r0 + g0;
+    g[1] = fr * r1 + g1;
+    g[2] = fr * r2 + g2;
+    if constexpr (LEVEL > 1) lap = fuu + 2 * fu + w2 * u1 * u1 + 2 * u1 * rin * (w1 * du + tt) + lp;
+  }
+  return f;
+}
+
+// Jastrow of electron e at xe with the others where they are: its scaled distances (v + pa, ph), this
+// lane's pair value pf (lane = other electron; lane e: the e-n term), the sum over all of them minus
+// the pair table's row, and with GRAD the gradient.
+template <int NORD, bool GRAD>
+__device__ __noinline__ void electron_jastrow(const Sys<double> &s, const JasPar<double> &J, double *v, int e, const double *xe,
+                                              double &pf, double &dj, double *g) {
+  const Lay L(s.N, s.C, NORD);
+  const int sub = threadIdx.x & 7, N = s.N, C = s.C;
+  const unsigned m = gmask();
+  double *pa = v + L.pa(), *ph = v + L.ph();
+  const double sk = J.scalek;
+  double en = 0, g0 = 0, g1 = 0, g2 = 0;
+  for (int c = sub; c < C; c += GS) {
+    const double dx = xe[0] - s.cent[3 * c], dy = xe[1] - s.cent[3 * c + 1], dz = xe[2] - s.cent[3 * c + 2];
+    const double r = sqrt(dx * dx + dy * dy + dz * dz), a = 1.0 / (1.0 + sk * r);
+    double fi = 0, fii = 0;
+    en += jas_en<double, GRAD>(J, s.ctype[c], r, a, fi, fii);
+    pa[c] = a;
+    if (GRAD) {
+      ph[c] = -sk * a * a / r;
+      g0 += fi * dx;
+      g1 += fi * dy;
+      g2 += fi * dz;
+    }
+  }
+  __syncwarp(m);
+  One<NORD> o;
+  one_sums<NORD, GRAD ? 1 : 0>(s, sk, xe, pa, ph, o);
+  double d = en, f = 0;
+  if (sub < N && sub != e) {
+    double gp[3], lap, rin;
+    f = pair_terms<NORD, GRAD ? 1 : 0>(s, J, e, sub, xe, pa, ph, o, v + 3 * sub, v + L.a() + sub * C, v + L.z() + sub * L.qm, gp,
+                                       lap, rin);
+    d += f;
+    if (GRAD) {
+      g0 += gp[0];
+      g1 += gp[1];
+      g2 += gp[2];
+    }
+  }
+  if (sub < N) d -= v[L.f() + e * N + sub];
+  dj = gsum(d, m);
+  en = gsum(en, m);
+  pf = sub == e ? en : f;
+  if (GRAD) {
+    g[0] = gsum(g0, m);
+    g[1] = gsum(g1, m);
+    g[2] = gsum(g2, m);
+  }
+}
+
+// Determinant ratio and, with GRAD, gradient of the ratio over it, of electron e with the orbital row
+// r [5][NO] (every lane of the walker).
+template <bool GRAD>
+__device__ __forceinline__ double det_ratio(const Sys<double> &s, const double *v, const Lay &L, int e, const double *r, double *g) {
+  const int sp = e < s.nup ? 0 : 1, n = sp ? s.ndn : s.nup, eo = sp ? e - s.nup : e;
+  const double *A = v + L.ai() + sp * NO * NO + eo;
+  double rho = 0, g0 = 0, g1 = 0, g2 = 0;
+#pragma unroll
+  for (int k = 0; k < NO; k++)
+    if (k < n) {
+      const double a = A[k * NO];
+      rho += a * r[k];
+      if (GRAD) {
+        g0 += a * r[NO + k];
+        g1 += a * r[2 * NO + k];
+        g2 += a * r[3 * NO + k];
+      }
+    }
+  if (GRAD) {
+    const double ri = 1.0 / rho;
+    g[0] += g0 * ri;
+    g[1] += g1 * ri;
+    g[2] += g2 * ri;
+  }
+  return rho;
+}
+
+// Accepts electron e at xn: inverse (Sherman-Morrison), pair table, distances, position and row.
+template <int NORD>
+__device__ __forceinline__ void accept(const Sys<double> &s, double *v, const Lay &L, int e, const double *xn, double pf, double rho,
+                                       int nrow) {
+  const int sub = threadIdx.x & 7, N = s.N, C = s.C;
+  const unsigned m = gmask();
+  const int sp = e < s.nup ? 0 : 1, n = sp ? s.ndn : s.nup, eo = sp ? e - s.nup : e;
+  double *A = v + L.ai() + sp * NO * NO;
+  const double *r = v + L.pr();
+  double nv[2];
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const int i = sub + GS * h, k = i / NO, j = i & (NO - 1);
+    double vb = 0;
+#pragma unroll
+    for (int q = 0; q < NO; q++)
+      if (q < n) vb += r[q] * A[q * NO + j];
+    vb -= j == eo ? 1.0 : 0.0;
+    nv[h] = A[k * NO + j] - A[k * NO + eo] * vb / rho;
+  }
+  __syncwarp(m);
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const int i = sub + GS * h;
+    if (i / NO < n && (i & (NO - 1)) < n) A[i] = nv[h];
+  }
+  if (sub < N) {
+    v[L.f() + e * N + sub] = pf;
+    v[L.f() + sub * N + e] = pf;
+  }
+  for (int c = sub; c < C; c += GS) v[L.a() + e * C + c] = v[L.pa() + c];
+  if (NORD > 1)
+    for (int q = sub; q < L.qm; q += GS) {
+      double z = 0;
+      for (int c = 0; c < C; c++) {
+        double p = 1;
+        for (int k = 0; k <= q; k++) p *= v[L.pa() + c];
+        z += p;
+      }
+      v[L.z() + e * L.qm + q] = z;
+    }
+  if (sub < 3) v[3 * e + sub] = xn[sub];
+  for (int i = sub; i < nrow; i += GS) v[L.row() + e * 5 * NO + i] = r[i];
+  __syncwarp(m);
+}
+
+// Inverses of both spins' Slater matrices from the rows' values: lanes 0-3 the up rows, 4-7 the down
+// rows (k_inv_reg's elimination).  Returns ln|D| and sign(D) (0 when singular).
+__device__ __forceinline__ void invert(const Sys<double> &s, double *v, const Lay &L, double &lnd, double &sgn) {
+  const int sub = threadIdx.x & 7, sp = sub >> 2, r = sub & 3;
+  const unsigned m = gmask(), h4 = 0xfu << (threadIdx.x & 28);
+  const int n = sp ? s.ndn : s.nup, e = (sp ? s.nup : 0) + r, base = threadIdx.x & 28;
+  double a[NO];
+#pragma unroll
+  for (int j = 0; j < NO; j++) a[j] = (r < n && j < n) ? v[L.row() + e * 5 * NO + j] : 0.0;
+  bool used = r >= n, fail = false;
+  double piv = 1.0;
+  int mycol = 0, pv[NO];
+#pragma unroll
+  for (int k = 0; k < NO; k++) {
+    pv[k] = 0;
+    if (k >= n || fail) continue;
+    double best = used ? -1.0 : fabs(a[0]);
+    if (!(best > -1.0)) best = -1.0;
+    int bi = r;
+#pragma unroll
+    for (int o = 2; o > 0; o >>= 1) {
+      const double ob = __shfl_xor_sync(h4, best, o);
+      const int oi = __shfl_xor_sync(h4, bi, o);
+      if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
+    }
+    if (!(best > 0.0)) { fail = true; continue; }
+    pv[k] = bi;
+    if (r == bi) {
+      used = true;
+      piv = a[0];
+      mycol = k;
+      const double pi = 1.0 / a[0];
+#pragma unroll
+      for (int j = 1; j < NO; j++) a[j - 1] = a[j] * pi;
+      a[NO - 1] = pi;
+    }
+    double p[NO];
+#pragma unroll
+    for (int j = 0; j < NO; j++) p[j] = __shfl_sync(h4, a[j], base + bi);
+    if (r != bi) {
+      const double f = a[0];
+#pragma unroll
+      for (int j = 0; j < NO; j++) a[j] = (j + 1 < NO ? a[j + 1] : 0.0) - f * p[j];
+    }
+  }
+  double ln = (r < n && !fail) ? log(fabs(piv)) : 0.0;
+  int neg = (r < n && piv < 0) ? 1 : 0;
+  if (!fail && r < n) {
+#pragma unroll
+    for (int j = 0; j < NO; j++) {
+      const int mm = j - (NO - n);
+      if (mm >= 0) {
+        int p = 0;
+#pragma unroll
+        for (int q = 0; q < NO; q++)
+          if (q == mm) p = pv[q];
+        v[L.ai() + sp * NO * NO + mycol * NO + p] = a[j];
+        if (mm < mycol) neg += p > r;
+      }
+    }
+  }
+  const unsigned bad = __ballot_sync(m, fail) & m;
+  lnd = gsum(ln, m);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) neg += __shfl_xor_sync(m, neg, o);
+  sgn = bad ? 0.0 : ((neg & 1) ? -1.0 : 1.0);
+  __syncwarp(m);
+}
+
+// psi(electron e at xn) / psi for one lane's own point: determinant ratio times the exponential of the
+// Jastrow change.  tab: radial factors of centre tc's shells, or null.
+template <int NORD>
+__device__ __noinline__ double point_psi(const Sys<double> &s, const stab::Tab &T, const JasPar<double> &J, double *v, int e, const double *xn, int tc,
+                                         const double *tab) {
+  const Lay L(s.N, s.C, NORD);
+  const int sub = threadIdx.x & 7, N = s.N, C = s.C;
+  const int sp = e < s.nup ? 0 : 1, n = sp ? s.ndn : s.nup, eo = sp ? e - s.nup : e, no = s.nocc[sp];
+  const double *cf = s.cocc[sp];
+  double o[NO], g[NO];
+#pragma unroll
+  for (int k = 0; k < NO; k++) {
+    o[k] = 0;
+    g[k] = k < n ? v[L.ai() + sp * NO * NO + k * NO + eo] : 0.0;
+  }
+  const int t0 = tab ? s.cshell0[tc] : 0, t1 = tab ? s.cshell0[tc + 1] : 0;
+  double dr = 0, d0 = 0, d1 = 0, d2 = 0, r2 = 0;
+  int cen = -1;
+  for (int ish = 0; ish < s.nshell; ish++) {
+    const ShellRec h = T.rec[ish];
+    if (h.cen != cen) {
+      cen = h.cen;
+      d0 = xn[0] - s.cent[3 * cen];
+      d1 = xn[1] - s.cent[3 * cen + 1];
+      d2 = xn[2] - s.cent[3 * cen + 2];
+      r2 = d0 * d0 + d1 * d1 + d2 * d2;
+    }
+    double rad;
+    if (ish >= t0 && ish < t1) rad = tab[ish - t0];
+    else rad = stab::factor(s, T, ish, h, r2);
+    double S[9], G[9][3];
+    const double *r = cf + (size_t)h.b0 * no;
+    auto add = [&](int sl, double val) {
+#pragma unroll
+      for (int k = 0; k < NO; k++)
+        if (k < no) o[k] += val * r[sl * no + k];
+    };
+    switch (h.l) {
+    case 0: add(0, rad); break;
+    case 1: add(0, d2 * rad); add(1, d0 * rad); add(2, d1 * rad); break;
+    case 2:
+      solid_all<double, false>(2, d0, d1, d2, S, G);
+#pragma unroll
+      for (int i = 0; i < 5; i++) add(i, S[i] * rad);
+      break;
+    case 3:
+      solid_all<double, false>(3, d0, d1, d2, S, G);
+#pragma unroll
+      for (int i = 0; i < 7; i++) add(i, S[i] * rad);
+      break;
+    default:
+      solid_all<double, false>(4, d0, d1, d2, S, G);
+#pragma unroll
+      for (int i = 0; i < 9; i++) add(i, S[i] * rad);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < NO; k++) dr += o[k] * g[k];
+  double *pl = v + L.pl() + sub;
+  double f = 0;
+  One<NORD> os;
+#pragma unroll
+  for (int q = 0; q < One<NORD>::QM; q++) os.S[q] = 0;
+  for (int c = 0; c < C; c++) {
+    const double a0 = xn[0] - s.cent[3 * c], a1 = xn[1] - s.cent[3 * c + 1], a2 = xn[2] - s.cent[3 * c + 2];
+    const double r = sqrt(a0 * a0 + a1 * a1 + a2 * a2), a = 1.0 / (1.0 + J.scalek * r);
+    double fi, fii;
+    f += jas_en<double, false>(J, s.ctype[c], r, a, fi, fii);
+    pl[c * GS] = a;
+    double p = a;
+#pragma unroll
+    for (int q = 0; q < One<NORD>::QM; q++) { os.S[q] += p; p *= a; }
+  }
+  f -= v[L.f() + e * N + e];
+  using TB = Tab<NORD>;
+  constexpr int NC = jt::make_combos(NORD).n, NT = make_terms(NORD).n, NCA = NC > 0 ? NC : 1, QM = One<NORD>::QM;
+  for (int j = 0; j < N; j++) {
+    if (j == e) continue;
+    const double *xj = v + 3 * j, *aj = v + L.a() + j * C, *zj = v + L.z() + j * L.qm;
+    const double r0 = xn[0] - xj[0], r1 = xn[1] - xj[1], q2 = xn[2] - xj[2];
+    const double rij = sqrt(r0 * r0 + r1 * r1 + q2 * q2);
+    int isb, ipar;
+    double ss, du;
+    pair_class(J, s.nup, e, j, isb, ss, ipar);
+    f += pt::ee_value(J, isb, ss, ipar, rij, du) - v[L.f() + e * N + j];
+    if constexpr (NORD > 1) {
+      double ax[NCA];
+#pragma unroll
+      for (int y = 0; y < NCA; y++) ax[y] = 0;
+      for (int c = 0; c < C; c++) {
+        const double a = pl[c * GS], b = aj[c];
+        double ap[QM + 1], bp[QM + 1];
+        ap[0] = bp[0] = 1;
+#pragma unroll
+        for (int q = 1; q <= QM; q++) { ap[q] = ap[q - 1] * a; bp[q] = bp[q - 1] * b; }
+        sfor<NC>([&](auto Y) {
+          constexpr int y = decltype(Y)::v, l = TB::cb.l[y], m = TB::cb.m[y];
+          if constexpr (l > 0) ax[y] += ap[l + m] * bp[m] + ap[m] * bp[l + m];
+          else ax[y] += 2.0 * ap[m] * bp[m];
+        });
+      }
+      double u[NORD + 1];
+      u[0] = 1;
+#pragma unroll
+      for (int q = 1; q <= NORD; q++) u[q] = u[q - 1] * du;
+      sfor<NT>([&](auto LL) {
+        constexpr int ll = decltype(LL)::v, k = TB::tl.k[ll], l = TB::tl.l[ll];
+        if constexpr (TB::tl.m[ll] == 0) {
+          double Y = 2.0 * C;
+          if constexpr (l > 0) Y = os.S[l - 1] + zj[l - 1];
+          f += J.c[0][ll] * u[k] * Y;
+        }
+      });
+      sfor<NC>([&](auto YY) {
+        constexpr int y = decltype(YY)::v, nk = TB::cb.nk[y];
+        double cu = 0;
+        sfor<nk>([&](auto K) {
+          constexpr int k = decltype(K)::v, ik = TB::cb.ll[y][k];
+          cu += J.c[0][ik] * u[k];
+        });
+        f += cu * ax[y];
+      });
+    }
+  }
+  return dr * exp(f);
+}
+
+// E_L and everything it leaves behind (full_eval) from the rows and positions in shared memory.
+struct Res {
+  double eloc, v2;
+};
+template <int NORD>
+__device__ __forceinline__ Res evaluate(const Sys<double> &s, const stab::Tab &T, const JasPar<double> &J, const EcpPar &E, const State<double> &st,
+                                        int w, double *v, const Lay &L, const ElRot &rot, bool outputs) {
+  const int sub = threadIdx.x & 7, N = s.N, C = s.C;
+  const unsigned m = gmask();
+  const double sk = J.scalek;
+  double lnd, sgn;
+  invert(s, v, L, lnd, sgn);
+  const bool ok = sgn != 0.0;
+  // ---- distances and power sums, lane = electron
+  double pe_en = 0, fen = 0, div = 0, vj[3] = {0, 0, 0}, d2j = 0, pe_ee = 0, fsum = 0;
+  const bool act = sub < N;
+  const int i = act ? sub : 0;
+  const double xi[3] = {v[3 * i], v[3 * i + 1], v[3 * i + 2]};
+  double *pa = v + L.a() + i * C, *ph = v + L.h() + i * C;
+  if (act) {
+    double z[ZQ];
+    z[0] = (double)C;
+#pragma unroll
+    for (int q = 1; q < ZQ; q++) z[q] = 0;
+    for (int c = 0; c < C; c++) {
+      const double dx = xi[0] - s.cent[3 * c], dy = xi[1] - s.cent[3 * c + 1], dz = xi[2] - s.cent[3 * c + 2];
+      const double r = sqrt(dx * dx + dy * dy + dz * dz), a = 1.0 / (1.0 + sk * r);
+      double fi, fii;
+      fen += jas_en<double, true>(J, s.ctype[c], r, a, fi, fii);
+      vj[0] += fi * dx;
+      vj[1] += fi * dy;
+      vj[2] += fi * dz;
+      div += fii + 2 * fi;
+      pa[c] = a;
+      ph[c] = -sk * a * a / r;
+      double *ren = st.ren + ((size_t)w * N * C + i * C + c) * 2;
+      ren[0] = r;
+      ren[1] = a;
+      if (s.nloc == 0) pe_en -= s.zc[c] / r;
+      double p = a;
+#pragma unroll
+      for (int q = 1; q < ZQ; q++) { z[q] += p; p *= a; }
+    }
+    if (NORD > 1)
+#pragma unroll
+      for (int q = 1; q < (NORD > 1 ? NORD : 2); q++) v[L.z() + i * L.qm + q - 1] = z[q];
+    double *zg = st.zq + ((size_t)w * N + i) * ZQ;
+#pragma unroll
+    for (int q = 0; q < ZQ; q++) zg[q] = z[q];
+    v[L.f() + i * N + i] = fen;
+    fsum = fen;
+    d2j = div;
+  }
+  __syncwarp(m);
+  double dvd = 0, vx = 0, vy = 0, vz = 0;
+  if (act) {
+    One<NORD> o;
+    one_sums<NORD, 2>(s, sk, xi, pa, ph, o);
+    for (int j = 0; j < N; j++) {
+      if (j == i) continue;
+      double g[3], lap, rin;
+      const double f = pair_terms<NORD, 2>(s, J, i, j, xi, pa, ph, o, v + 3 * j, v + L.a() + j * C, v + L.z() + j * L.qm, g, lap, rin);
+      vj[0] += g[0];
+      vj[1] += g[1];
+      vj[2] += g[2];
+      d2j += lap;
+      div += 0.5 * lap;  // a pair's Laplacian is halved between its electrons; the other half follows
+      v[L.f() + i * N + j] = f;
+      if (outputs) st.o_divv[(size_t)w * N + i] = 0;
+      if (j < i) {
+        fsum += f;
+        pe_ee += rin;
+      }
+    }
+    const int sp = i < s.nup ? 0 : 1, n = sp ? s.ndn : s.nup, eo = sp ? i - s.nup : i;
+    const double *A = v + L.ai() + sp * NO * NO + eo, *r = v + L.row() + i * 5 * NO;
+    double g0 = 0, g1 = 0, g2 = 0, lp = 0;
+#pragma unroll
+    for (int k = 0; k < NO; k++)
+      if (k < n) {
+        const double a = A[k * NO];
+        g0 += a * r[NO + k];
+        g1 += a * r[2 * NO + k];
+        g2 += a * r[3 * NO + k];
+        lp += a * r[4 * NO + k];
+      }
+    dvd = lp - (g0 * g0 + g1 * g1 + g2 * g2);
+    vx = vj[0] + g0;
+    vy = vj[1] + g1;
+    vz = vj[2] + g2;
+    if (outputs) {
+      double *ov = st.o_vel + ((size_t)w * N + i) * 3;
+      ov[0] = vx; ov[1] = vy; ov[2] = vz;
+    }
+  }
+  __syncwarp(m);
+  if (outputs && act) {
+    // the other half of the pair Laplacians, lap_j of every pair (i, j)
+    double other = 0;
+    for (int j = 0; j < N; j++) {
+      if (j == i) continue;
+      const double xj[3] = {v[3 * j], v[3 * j + 1], v[3 * j + 2]};
+      One<NORD> o;
+      one_sums<NORD, 2>(s, sk, xj, v + L.a() + j * C, v + L.h() + j * C, o);
+      double g[3], lap, rin;
+      pair_terms<NORD, 2>(s, J, j, i, xj, v + L.a() + j * C, v + L.h() + j * C, o, v + 3 * i, v + L.a() + i * C,
+                          v + L.z() + i * L.qm, g, lap, rin);
+      other += 0.5 * lap;
+    }
+    st.o_divv[(size_t)w * N + i] = div + other + dvd;
+  }
+  const double v2 = gsum(act ? vx * vx + vy * vy + vz * vz : 0.0, m), d2lnd = gsum(dvd, m);
+  fsum = gsum(fsum, m);
+  d2j = gsum(d2j, m);
+  pe_ee = gsum(pe_ee, m);
+  pe_en = gsum(pe_en, m);
+  // ---- pseudopotential
+  double vloc = 0, vnl = 0;
+  if (s.nloc > 0 && ok) {
+    double *rec = v + L.row(), *tab = rec + N * C * NLT;  // the rows are no longer read
+    double R[9];
+    if (rot.random) random_rotation(rot.seed, (uint32_t)w, rot.sweep, R);
+    else
+#pragma unroll
+      for (int k = 0; k < 9; k++) R[k] = rot.R[k];
+    int ntask = 0;
+    for (int base = 0; base < N * C; base += GS) {
+      const int j = base + sub;
+      bool nl = false;
+      double vps[MAXLCH], r = 0;
+      int c = 0, e = 0;
+      if (j < N * C) {
+        c = j / N;
+        e = j - c * N;
+        const double dx = v[3 * e] - s.cent[3 * c], dy = v[3 * e + 1] - s.cent[3 * c + 1], dz = v[3 * e + 2] - s.cent[3 * c + 2];
+        r = sqrt(dx * dx + dy * dy + dz * dz);
+        const int it = s.ctype[c];
+        ecp_vps(E, it, r, vps);
+        vloc += vps[E.lpotp1[it] - 1];
+        for (int l = 0; l < E.npotd[it]; l++)
+          if (l + 1 != E.lpotp1[it] && fabs(vps[l]) > 1e-4) nl = true;
+      }
+      const unsigned b = (__ballot_sync(m, nl) >> (threadIdx.x & 24)) & 0xffu;
+      if (nl) {
+        double *q = rec + (ntask + __popc(b & ((1u << sub) - 1u))) * NLT;
+        q[0] = (double)(e * C + c);
+        q[1] = r;
+        for (int l = 0; l < MAXLCH; l++) q[2 + l] = l < E.npotd[s.ctype[c]] ? vps[l] : 0.0;
+      }
+      ntask += __popc(b);
+    }
+    __syncwarp(m);
+    const int nsh = (s.nshc > 0 && ntask * s.nshc <= RCAP) ? s.nshc : 0;
+    for (int k = sub; k < ntask * nsh; k += GS) {
+      const int t = k / nsh, q = k - t * nsh, c = (int)rec[t * NLT] % C, ish = s.cshell0[c] + q;
+      if (ish < s.cshell0[c + 1]) tab[k] = stab::factor(s, T, ish, T.rec[ish], rec[t * NLT + 1] * rec[t * NLT + 1]);
+    }
+    __syncwarp(m);
+    const int nq = E.nquad, npts = ntask * nq;
+    for (int t = sub; t < npts; t += GS) {
+      const int task = t / nq, q = t - task * nq;
+      const double *rc = rec + task * NLT;
+      const int idx = (int)rc[0], e = idx / C, c = idx - e * C, it = s.ctype[c];
+      const double r = rc[1], *q0 = s.quad->q0[q];
+      const double qx = R[0] * q0[0] + R[1] * q0[1] + R[2] * q0[2], qy = R[3] * q0[0] + R[4] * q0[1] + R[5] * q0[2],
+                   qz = R[6] * q0[0] + R[7] * q0[1] + R[8] * q0[2];
+      const double *cc = s.cent + 3 * c;
+      const double costh = ((v[3 * e] - cc[0]) * qx + (v[3 * e + 1] - cc[1]) * qy + (v[3 * e + 2] - cc[2]) * qz) / r;
+      const double xn[3] = {cc[0] + r * qx, cc[1] + r * qy, cc[2] + r * qz};
+      const double ratio = point_psi<NORD>(s, T, J, v, e, xn, c, nsh ? tab + task * nsh : nullptr);
+      double vp = 0;
+      for (int l = 0; l < E.npotd[it]; l++)
+        if (l + 1 != E.lpotp1[it]) vp += rc[2 + l] * yl0(l, costh);
+      vnl += s.quad->wq[q] * vp * ratio;
+    }
+    __syncwarp(m);
+    vloc = gsum(vloc, m);
+    vnl = gsum(vnl, m);
+  }
+  const double pe = s.pecent + pe_ee + (s.nloc > 0 ? vloc + vnl : pe_en), d2 = d2lnd + d2j;
+  Res res;
+  res.v2 = v2;
+  res.eloc = ok ? pe - HB * (d2 + v2) : nan("");
+  if (sub == 0) {
+    const double lnpsi = lnd + fsum;
+    st.fsum[w] = fsum;
+    st.lnd[w] = ok ? lnd : -INFINITY;
+    st.sgn[w] = sgn;
+    uint32_t flag = 0;
+    if (!ok) flag |= CHAMP_WS_SINGULAR;
+    if (!isfinite(res.eloc) || !isfinite(lnpsi)) flag |= CHAMP_WS_NONFINITE;
+    st.status[w] = flag;
+    if (outputs) {
+      st.o_lnpsi[w] = lnpsi;
+      st.o_sign[w] = sgn;
+      st.o_psij[w] = fsum;
+      st.o_d2[w] = d2;
+      st.o_pe[w] = pe;
+      st.o_peee[w] = pe_ee;
+      st.o_penl[w] = vnl;
+      st.o_eloc[w] = res.eloc;
+    }
+  }
+  return res;
+}
+
+// What a walker keeps between kernels: positions, inverses and pair table (distances and power sums are
+// written by evaluate); for a mixed-precision state the FP32 move tables.
+__device__ __forceinline__ void store(const Sys<double> &s, const State<double> &st, int w, const double *v, const Lay &L) {
+  const int sub = threadIdx.x & 7, N = s.N, C = s.C;
+  __syncwarp(gmask());
+  for (int i = sub; i < 3 * N; i += GS) st.x[(size_t)w * 3 * N + i] = v[i];
+  for (int sp = 0; sp < 2; sp++) {
+    const int n = sp ? s.ndn : s.nup;
+    double *A = st.ainv + (size_t)w * st.astride + (sp ? s.nup * s.nup : 0);
+    for (int i = sub; i < n * n; i += GS) A[i] = v[L.ai() + sp * NO * NO + (i / n) * NO + i % n];
+  }
+  if (st.m_fso) {
+    const double *rn = st.ren + (size_t)w * N * C * 2, *zz = st.zq + (size_t)w * N * ZQ;
+    for (int i = sub; i < N * N; i += GS) st.m_fso[(size_t)w * N * N + i] = (float)v[L.f() + i];
+    for (int i = sub; i < N * C * 2; i += GS) st.m_ren[(size_t)w * N * C * 2 + i] = (float)rn[i];
+    for (int i = sub; i < N * ZQ; i += GS) st.m_zq[(size_t)w * N * ZQ + i] = (float)zz[i];
+    if (st.m_rtd)
+      for (int i = sub; i < N * C; i += GS) {
+        const int c = i / N, e = i - c * N;
+        st.m_rtd[(size_t)w * N * C + i] = (float)rn[2 * (e * C + c) + 1];
+      }
+  } else {
+    for (int i = sub; i < N * N; i += GS) st.fso[(size_t)w * N * N + i] = v[L.f() + i];
+  }
+}
+
+enum { EVAL = 0, GAUSS = 1, ACCEL = 6, DMC = 7, DMC_EL = 8 };
+
+// EVAL: E_L of the walkers; GAUSS, ACCEL: sweeps of that mover, each followed by E_L; DMC: a
+// drift-diffusion step with E_L, reweighting and copy counts (k_dmc_move); DMC_EL: its second half.
+template <int NORD, int MODE>
+__global__ void __launch_bounds__(128, 3) k_small(const __grid_constant__ Sys<double> s, const __grid_constant__ State<double> st,
+                                                  const __grid_constant__ Args A) {
+  __shared__ JasPar<double> J;
+  __shared__ EcpPar E;
+  extern __shared__ __align__(16) char dsm[];
+  const stab::Tab T = stab::stage(s, dsm);
+  load_params(s, J, E);
+  const Lay L(s.N, s.C, NORD);
+  const int N = s.N, C = s.C, sub = threadIdx.x & 7, grp = threadIdx.x >> 3;
+  const unsigned m = gmask();
+  double *v = (double *)(dsm + stab::tab_smem(s.nshell, s.nprim)) + (size_t)grp * L.total();
+  constexpr bool dmc = MODE == DMC || MODE == DMC_EL, moves = MODE == GAUSS || MODE == ACCEL || MODE == DMC;
+  const int W = dmc ? *A.D.nw : st.W;
+  const uint64_t step0 = dmc ? (uint64_t)A.D.ctr[0] : A.sweep0;
+  const double et = dmc ? *A.D.et : 0, eest = dmc ? *A.D.eest : 0, esigma = dmc ? energy_sigma(A.P, A.D.esg, N) : 0,
+               sqt = dmc ? sqrt(A.P.tau) : 0;
+  const int w = blockIdx.x * (blockDim.x / GS) + grp;
+  double sw = 0, swe = 0;
+  if (w < W) {
+    for (int i = sub; i < 3 * N; i += GS) v[i] = st.x[(size_t)w * 3 * N + i];
+    if (moves) {
+      for (int sp = 0; sp < 2; sp++) {
+        const int n = sp ? s.ndn : s.nup;
+        const double *a = st.ainv + (size_t)w * st.astride + (sp ? s.nup * s.nup : 0);
+        for (int i = sub; i < n * n; i += GS) v[L.ai() + sp * NO * NO + (i / n) * NO + i % n] = a[i];
+      }
+      for (int i = sub; i < N * N; i += GS) v[L.f() + i] = st.fso[(size_t)w * N * N + i];
+      for (int i = sub; i < N * C; i += GS) v[L.a() + i] = st.ren[((size_t)w * N * C + i) * 2 + 1];
+      for (int i = sub; i < N * L.qm; i += GS) v[L.z() + i] = st.zq[((size_t)w * N + i / L.qm) * ZQ + 1 + i % L.qm];
+    }
+    __syncwarp(m);
+    double es = 0, e2 = 0, acc = 0, el = 0;
+    const int nsw = MODE == GAUSS || MODE == ACCEL ? A.nsweep : 1;
+    for (int isw = 0; isw < nsw; isw++) {
+      const uint64_t sweep = step0 + (uint64_t)isw;
+      for (int e = 0; e < N; e++)
+        orb_row<5>(s, T, A.order, e < s.nup ? 0 : 1, v[3 * e], v[3 * e + 1], v[3 * e + 2], v + L.row() + e * 5 * NO);
+      double sdd = 0, spd = 0;
+      for (int e = 0; moves && e < N; e++) {
+        const int sp = e < s.nup ? 0 : 1;
+        const double xo[3] = {v[3 * e], v[3 * e + 1], v[3 * e + 2]};
+        double *pr = v + L.pr();
+        double pf, d0, go[3], gn[3], dj, rho, p, ua, xn[3];
+        if constexpr (MODE == GAUSS) {
+          double g[3];
+          move_randoms(A.seed, (uint32_t)w, sweep, (uint32_t)e, g, &ua);
+          for (int k = 0; k < 3; k++) xn[k] = xo[k] + A.step * g[k];
+          orb_row<5>(s, T, A.order, sp, xn[0], xn[1], xn[2], pr);
+          electron_jastrow<NORD, false>(s, J, v, e, xn, pf, dj, gn);
+          rho = det_ratio<false>(s, v, L, e, pr, gn);
+          p = rho * rho * exp(2.0 * dj);
+        } else {
+          electron_jastrow<NORD, true>(s, J, v, e, xo, pf, d0, go);
+          det_ratio<true>(s, v, L, e, v + L.row() + e * 5 * NO, go);
+          if constexpr (MODE == ACCEL) {
+            MoveRng rng{A.seed, (uint32_t)w, (uint32_t)sweep, (uint32_t)(sweep >> 32), (uint32_t)e, 0u, {0.0, 0.0}, 0};
+            double fxop, areao, rtry;
+            slat_forward(s, A.mv, xo, go, rng, xn, fxop, areao, rtry);
+            SlatBack b;
+            p = rho = dj = pf = 0;
+            if (slat_geometry(s, A.mv, xo, xn, b)) {
+              __syncwarp(m);
+              orb_row<5>(s, T, A.order, sp, xn[0], xn[1], xn[2], pr);
+              electron_jastrow<NORD, true>(s, J, v, e, xn, pf, dj, gn);
+              rho = det_ratio<true>(s, v, L, e, pr, gn);
+              double fxnp, arean;
+              slat_reverse(s, A.mv, b, gn, fxnp, arean);
+              const double rr = rtry / b.rminon;
+              p = rr * rr * rho * rho * exp(2.0 * dj) * fabs((fxnp * areao) / (fxop * arean));
+            }
+            ua = rng.next();
+          } else {
+            double vo[3], vn[3], g[3], db[3];
+            avg_drift(go, A.P.tau, A.P.adrift, vo);
+            move_randoms(A.P.seed, (uint32_t)w, sweep, (uint32_t)e, g, &ua);
+            for (int k = 0; k < 3; k++) xn[k] = xo[k] + A.P.tau * vo[k] + sqt * g[k];
+            orb_row<5>(s, T, A.order, sp, xn[0], xn[1], xn[2], pr);
+            electron_jastrow<NORD, true>(s, J, v, e, xn, pf, dj, gn);
+            rho = det_ratio<true>(s, v, L, e, pr, gn);
+            avg_drift(gn, A.P.tau, A.P.adrift, vn);
+            const double lgf = -0.5 * (g[0] * g[0] + g[1] * g[1] + g[2] * g[2]);
+            for (int k = 0; k < 3; k++) db[k] = xo[k] - xn[k] - A.P.tau * vn[k];
+            const double lgb = -(db[0] * db[0] + db[1] * db[1] + db[2] * db[2]) / (2 * A.P.tau);
+            p = (rho > 0) ? rho * rho * exp(2.0 * dj + lgb - lgf) : 0.0;  // fixed node
+            const double dd = A.P.tau * (g[0] * g[0] + g[1] * g[1] + g[2] * g[2]);
+            sdd += dd;
+            spd += (p < 1.0 ? p : 1.0) * dd;
+          }
+        }
+        if (ua < p) {
+          accept<NORD>(s, v, L, e, xn, pf, rho, 5 * NO);
+          acc += 1;
+        }
+        __syncwarp(m);
+      }
+      ElRot rot = A.rot;
+      if (MODE != EVAL || A.rot.random) {
+        rot.random = 1;
+        rot.seed = dmc ? A.P.seed : (MODE == EVAL ? A.rot.seed : A.seed);
+        rot.sweep = MODE == EVAL ? A.rot.sweep : sweep;
+      }
+      const Res res = evaluate<NORD>(s, T, J, E, st, w, v, L, rot, MODE == EVAL && A.outputs);
+      el = res.eloc;
+      es += el;
+      e2 += el * el;
+      if (dmc && sub == 0) {
+        const double teff = MODE == DMC ? (sdd > 0 ? A.P.tau * spd / sdd : A.P.tau) : A.D.teff[w];
+        const double eint = integrated_energy(A.P, A.D.el[w], A.D.v2[w], el, res.v2, N, eest, et, esigma, teff);
+        double wn = A.D.wt[w] * exp(-eint * teff);
+        if (!isfinite(wn) || !isfinite(el)) wn = 0.0;  // a walker with a non-finite energy dies
+        A.D.wt[w] = wn;
+        A.D.el[w] = el;
+        A.D.v2[w] = res.v2;
+        A.D.ncopy[w] = copy_count(A.P, wn, w, sweep);
+        sw = wn;
+        if (wn > 0) swe = wn * el;
+      }
+    }
+    store(s, st, w, v, L);
+    if (!dmc && sub == 0 && (MODE != EVAL || A.stats)) {
+      st.s_esum[w] += es;
+      st.s_e2sum[w] += e2;
+      st.s_acc[w] += acc;
+      st.s_elast[w] = el;
+    }
+  }
+  if (dmc) {
+    __syncwarp();
+    sw = warp_sum(sw);
+    swe = warp_sum(swe);
+    if ((threadIdx.x & 31) == 0 && sw != 0) {
+      atomicAdd(&A.D.red[0], sw);
+      atomicAdd(&A.D.red[1], swe);
+    }
+    for (int i = W + blockIdx.x * blockDim.x + (int)threadIdx.x; i < A.P.wmax; i += gridDim.x * blockDim.x) A.D.ncopy[i] = 0;
+  }
+}
+
+// T-moves of every electron (tmove_electron): a quadrature point per lane for the ratios, the heat-bath
+// choice in order by every lane.
+template <int NORD>
+__device__ __forceinline__ int tmove(const Sys<double> &s, const stab::Tab &T, const JasPar<double> &J, const EcpPar &E, const State<double> &st, double *v,
+                                     const Lay &L, int w, int e, const Args &A, uint64_t step, double *gp) {
+  const int sub = threadIdx.x & 7, nq = E.nquad, C = s.C;
+  const unsigned m = gmask();
+  MoveRng rng{A.seed, (uint32_t)w, (uint32_t)step, (uint32_t)(step >> 32), 256u + (uint32_t)e, 0u, {0.0, 0.0}, 0};
+  double R[9];
+  rotation_from(rng, R);
+  const double xo[3] = {v[3 * e], v[3 * e + 1], v[3 * e + 2]};
+  auto point = [&](const double *Rm, const double *cc, double r, int q, double *qv, double *xq) {
+    const double *q0 = s.quad->q0[q];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      qv[k] = Rm[3 * k] * q0[0] + Rm[3 * k + 1] * q0[1] + Rm[3 * k + 2] * q0[2];
+      xq[k] = cc[k] + r * qv[k];
+    }
+  };
+  // T elements to the points of centre c about position rv + c, with this lane's points into gp
+  auto elements = [&](const double *Rm, int c, const double *rv, double r, const double *vps, double div, double *rat) {
+    const int it = s.ctype[c];
+    for (int q = sub; q < nq; q += GS) {
+      double qv[3], xq[3];
+      point(Rm, s.cent + 3 * c, r, q, qv, xq);
+      const double costh = (rv[0] * qv[0] + rv[1] * qv[1] + rv[2] * qv[2]) / r;
+      const double psi = point_psi<NORD>(s, T, J, v, e, xq, c, nullptr), ratio = psi / div;
+      double t = 0;
+      for (int l = 0; l < E.npotd[it]; l++)
+        if (l + 1 != E.lpotp1[it]) t += s.quad->wq[q] * (exp(-A.tau * vps[l]) - 1) * yl0(l, costh) * ratio;
+      gp[q] = t;
+      if (rat) rat[q] = psi;
+    }
+    __syncwarp(m);
+  };
+  double *rat = gp + MAXQ;
+  double S = 1.0, pratio = 0.0;
+  int pc = -1, pq = -1;
+  for (int c = 0; c < C; c++) {
+    const double *cc = s.cent + 3 * c;
+    const double rv[3] = {xo[0] - cc[0], xo[1] - cc[1], xo[2] - cc[2]};
+    const double r = sqrt(rv[0] * rv[0] + rv[1] * rv[1] + rv[2] * rv[2]);
+    const int it = s.ctype[c];
+    double vps[MAXLCH];
+    ecp_vps(E, it, r, vps);
+    bool skip = true;
+    for (int l = 0; l < E.npotd[it]; l++)
+      if (l + 1 != E.lpotp1[it] && fabs(vps[l]) > 1e-4) skip = false;
+    if (skip) continue;
+    elements(R, c, rv, r, vps, 1.0, rat);
+    for (int q = 0; q < nq; q++)
+      if (gp[q] > 0) {
+        S += gp[q];
+        if (rng.next() < gp[q] / S) { pc = c; pq = q; pratio = rat[q]; }
+      }
+    __syncwarp(m);
+  }
+  if (pc < 0) return 0;
+  const double *cc = s.cent + 3 * pc;
+  const double r = sqrt((xo[0] - cc[0]) * (xo[0] - cc[0]) + (xo[1] - cc[1]) * (xo[1] - cc[1]) + (xo[2] - cc[2]) * (xo[2] - cc[2]));
+  double qn[3], xn[3];
+  point(R, cc, r, pq, qn, xn);
+  double p = 1.0;
+  if (A.variant == 2) {
+    double vps[MAXLCH], R2[9];
+    ecp_vps(E, s.ctype[pc], r, vps);
+    rotation_from(rng, R2);
+    const double xe[3] = {xn[0] - cc[0], xn[1] - cc[1], xn[2] - cc[2]};
+    elements(R2, pc, xe, r, vps, pratio, nullptr);
+    double Sb = 1.0;
+    for (int q = 0; q < nq; q++)
+      if (gp[q] > 0) Sb += gp[q];
+    p = S / Sb < 1.0 ? S / Sb : 1.0;
+    __syncwarp(m);
+  }
+  if (rng.next() >= p) return 0;
+  double pf, dj, g[3];
+  orb_row<1>(s, T, A.order, e < s.nup ? 0 : 1, xn[0], xn[1], xn[2], v + L.pr());
+  electron_jastrow<NORD, false>(s, J, v, e, xn, pf, dj, g);
+  const double rho = det_ratio<false>(s, v, L, e, v + L.pr(), g);
+  accept<NORD>(s, v, L, e, xn, pf, rho, 0);
+  if (sub == 0) {
+    st.fsum[w] += dj;
+    st.lnd[w] += log(fabs(rho));
+    if (rho < 0) st.sgn[w] = -st.sgn[w];
+  }
+  return 1;
+}
+
+// What a T-move pass leaves besides the positions: log-determinant, sign and Jastrow sum as updated by
+// the accepted moves, pair table, distances and power sums.
+template <int NORD>
+__global__ void __launch_bounds__(128, 3) k_small_tmove(const __grid_constant__ Sys<double> s, const __grid_constant__ State<double> st,
+                                                        const __grid_constant__ Args A) {
+  __shared__ JasPar<double> J;
+  __shared__ EcpPar E;
+  extern __shared__ __align__(16) char dsm[];
+  const stab::Tab T = stab::stage(s, dsm);
+  load_params(s, J, E);
+  const Lay L(s.N, s.C, NORD);
+  const int N = s.N, C = s.C, sub = threadIdx.x & 7, grp = threadIdx.x >> 3;
+  const unsigned m = gmask();
+  double *v = (double *)(dsm + stab::tab_smem(s.nshell, s.nprim)) + (size_t)grp * L.total();
+  const int W = A.nw ? *A.nw : st.W, w = blockIdx.x * (blockDim.x / GS) + grp;
+  const uint64_t step = A.step_dev ? (uint64_t)A.step_dev[0] : A.sweep0;
+  if (w >= W) return;
+  for (int i = sub; i < 3 * N; i += GS) v[i] = st.x[(size_t)w * 3 * N + i];
+  for (int sp = 0; sp < 2; sp++) {
+    const int n = sp ? s.ndn : s.nup;
+    const double *a = st.ainv + (size_t)w * st.astride + (sp ? s.nup * s.nup : 0);
+    for (int i = sub; i < n * n; i += GS) v[L.ai() + sp * NO * NO + (i / n) * NO + i % n] = a[i];
+  }
+  for (int i = sub; i < N * N; i += GS) v[L.f() + i] = st.fso[(size_t)w * N * N + i];
+  for (int i = sub; i < N * C; i += GS) v[L.a() + i] = st.ren[((size_t)w * N * C + i) * 2 + 1];
+  for (int i = sub; i < N * L.qm; i += GS) v[L.z() + i] = st.zq[((size_t)w * N + i / L.qm) * ZQ + 1 + i % L.qm];
+  __syncwarp(m);
+  int n = 0;
+  double *gp = v + L.row();
+  for (int e = 0; e < N; e++) {
+    const int got = tmove<NORD>(s, T, J, E, st, v, L, w, e, A, step, gp);
+    if (got) {
+      // the electron's distances and power sums
+      for (int c = sub; c < C; c += GS) {
+        const double dx = v[3 * e] - s.cent[3 * c], dy = v[3 * e + 1] - s.cent[3 * c + 1], dz = v[3 * e + 2] - s.cent[3 * c + 2];
+        double *ren = st.ren + ((size_t)w * N * C + e * C + c) * 2;
+        ren[0] = sqrt(dx * dx + dy * dy + dz * dz);
+        ren[1] = v[L.a() + e * C + c];
+      }
+      for (int q = 1 + sub; q < ZQ; q += GS) {
+        double z = 0;
+        for (int c = 0; c < C; c++) z += ipow(v[L.a() + e * C + c], q);
+        st.zq[((size_t)w * N + e) * ZQ + q] = z;
+      }
+    }
+    n += got;
+    __syncwarp(m);
+  }
+  store(s, st, w, v, L);
+  if (A.moved && sub == 0) A.moved[w] = n;
+}
+
+}  // namespace sm

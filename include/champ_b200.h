@@ -405,10 +405,13 @@ int champ_set_mover(champ_ctx *ctx, int32_t imetro, double deltar, double deltat
    kernels of every step from the host.
    "phase_timing": 1 records CUDA events around the VMC sweep kernels (champ_phase_times).
    "staged_eval": 1 (default when the walker state of an FP64 or mixed context lives in HBM)
-   runs the FP64 full evaluation as four kernels sized for their own parts (Jastrow and
-   distances; basis and orbitals per electron; Slater-matrix inversion in shared memory;
-   velocities, pseudopotential and E_L), and a VMC sweep of an FP64 context as its moves followed
-   by that evaluation; 0 runs the single-kernel evaluation (and the fused FP64 sweep kernel).
+   runs the FP64 full evaluation as kernels sized for their own parts (Jastrow and
+   distances; basis and orbitals; Slater-matrix inversion; velocities, pseudopotential and E_L), and a
+   VMC sweep of an FP64 context as its moves followed by that evaluation; with it, the Gaussian sweeps of
+   a single-determinant context (one centre type where there are e-e-n terms; more than 16 orbitals
+   per spin in mixed precision) form all proposals' orbitals and pair values before the first
+   decision.  0 runs the single-kernel evaluation (and the fused FP64 sweep kernel) and moves one
+   electron after the other.  The walks are the same.
    "tmoves": 0 (default), 1 or 2 -- T-moves of the variant of champ_tmoves at the start of every
    DMC step (champ_dmc_steps).
    "dmc_ene_int": 1 (default) ene_int_v9 energy integration in the DMC reweighting, 0 none.
@@ -416,10 +419,11 @@ int champ_set_mover(champ_ctx *ctx, int32_t imetro, double deltar, double deltat
    state lives in HBM, 17 to 128 orbitals per spin) runs the FP32 Gaussian moves with the warps of
    a block sharing the proposals' orbital-coefficient stream through shared memory (cp.async), in
    step electron by electron; 0 lets every warp stream the coefficients itself.  The walks are the
-   same.
+   same.  Without effect where the sweeps form all proposals first ("staged_eval").
    "orb_coop": 1 (default where available: the staged evaluation with electrons and up electrons in
    multiples of 4 and more than 16 orbitals per spin) lets the warps of a block of its orbital part
    share the coefficient stream through shared memory; 0 lets every warp stream it.  Same results.
+   Without effect up to 64 orbitals per spin, which are contracted in tiles.
    "mover_cache": 1 (default) lets the accelerated mover of a mixed single-determinant context
    whose walker state lives in HBM take the drift at an electron's current position from the
    orbital rows of the last FP64 evaluation (updated by its accepted moves) instead of evaluating
@@ -430,7 +434,7 @@ int champ_set_mover(champ_ctx *ctx, int32_t imetro, double deltar, double deltat
    context lives in HBM) keeps the accepted moves' Sherman-Morrison terms of a spin aside and
    folds K of them at a time into the inverse as one FP64 tensor-core product (proposals use the
    inverse with the pending terms; all are folded in at the end of a sweep's moves); 0 or 1
-   applies each update at once. */
+   applies each update at once.  Without effect where the sweeps form all proposals first. */
 int champ_set_option(champ_ctx *ctx, const char *name, int64_t value);
 /* Device time of the VMC sweep kernels launched since option "phase_timing" was set to 1 or
    since the previous call (no counterpart in the reference: instrumentation for benchmarks),
@@ -459,7 +463,8 @@ int champ_autotune(champ_ctx *ctx, int32_t nsweep, uint64_t seed, double step, c
    "dmc_persistent", "move_coop", "orb_coop", "mover_cache"); kernel launches per
    champ_vmc_sweeps sweep
    ("launches_per_sweep": 1 for the fused sweep kernel, 2 for moves + single-kernel evaluation,
-   5 for moves + staged evaluation or with the tensor-core orbitals). */
+   5 for moves + staged evaluation, each part counted once however many kernels it takes, or with the
+   tensor-core orbitals). */
 int champ_get_option(const champ_ctx *ctx, const char *name, int64_t *value);
 
 #ifdef __cplusplus

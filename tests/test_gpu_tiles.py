@@ -75,3 +75,60 @@ def test_batched_moves_walk_as_single_moves(n, nup, ncent, nordc, prec):
     assert same.sum() >= 63, same.sum()
     assert np.array_equal(out[0][1][same], out[1][1][same])
     assert 0 < out[0][1].sum() < 64 * 2 * n
+
+
+SMALL = [(1, 1, 1, 0), (2, 1, 1, 0), (3, 2, 2, 4), (4, 4, 1, 4), (5, 3, 2, 5), (7, 4, 3, 4), (8, 4, 2, 5)]
+
+
+@pytest.mark.parametrize("n,nup,ncent,nordc", SMALL)
+def test_small_walkers_match_oracle(oracle_mod, n, nup, ncent, nordc):
+    """The 8-lanes-per-walker kernels at the edges of their range (one electron, one spin only, up to 8
+    electrons and 4 of a spin): evaluation, and two sweeps walked as the oracle walks them."""
+    from champ_b200.engine import Engine
+    s = cluster(n, nup, ncent, nordc)
+    nw = 19  # not a multiple of the walkers of a block
+    x = S.initial_walkers(s, nw, seed=n)
+    orc = oracle_mod.Oracle(s)
+    for prec in ("fp64", "mixed"):
+        eng = Engine(s, nw, prec)
+        eng.set_walkers(x)
+        r = eng.eval_full()
+        for w in range(nw):
+            o = orc.eval(x[w])
+            scale = max(1.0, abs(o["energy"]), abs(o["d2lnpsi"]))
+            assert abs(r["lnpsi"][w] - o["lnpsi"]) <= 1e-9 * max(1.0, abs(o["lnpsi"]))
+            assert r["sign"][w] == o["sign"]
+            assert abs(r["pe_nonloc"][w] - o["pe_nonloc"]) <= 1e-9 * scale
+            assert abs(r["energy"][w] - o["energy"]) <= 1e-9 * scale
+            assert np.abs(r["velocity"][w] - o["vel"]).max() <= 1e-9 * np.abs(o["vel"]).max()
+            assert np.abs(r["div_v"][w] - o["div_v"]).max() <= 1e-9 * max(scale, np.abs(o["div_v"]).max())
+        if prec == "fp64":
+            st = eng.vmc_sweeps(2, seed=11, sweep0=4, step=s.step)
+            ref = orc.vmc(x, 2, seed=11, sweep0=4, step=s.step)
+            assert np.abs(eng.get_walkers() - ref["x"]).max() <= 1e-12
+            scale = np.array([max(1.0, abs(e), abs(orc.eval(y)["d2lnpsi"])) for e, y in zip(ref["elast"], ref["x"])])
+            assert np.all(np.abs(st["elast"] - ref["elast"]) <= 1e-9 * scale)
+            assert np.array_equal(st["accept"], ref["accept"])
+        eng.close()
+
+
+@pytest.mark.parametrize("n,nup,ncent,nordc", [c for c in CASES if c[3] in (4, 5) and c[0] < 70])
+def test_parameter_gradient_matches_single_kernels(n, nup, ncent, nordc):
+    """Tiled forward pass and reverse sweep against the warp-per-walker kernels (staged evaluation off), FP64."""
+    from champ_b200.engine import Engine
+    s = cluster(n, nup, ncent, nordc)
+    x = S.initial_walkers(s, 5, seed=n + 2)
+    out = []
+    for staged in (1, 0):
+        eng = Engine(s, 5, "fp64")
+        if not eng.get_option("staged_eval"):
+            pytest.skip("walker state of this system is resident in shared memory")
+        if not staged:
+            eng.set_option("staged_eval", 0)
+        eng.set_walkers(x)
+        out.append(eng.param_grad())
+        eng.close()
+    for a, b in zip(*out):
+        # per walker: sums of terms as large as the walker's largest derivative
+        scale = np.abs(b).reshape(len(b), -1).max(axis=1).reshape((-1,) + (1,) * (b.ndim - 1))
+        assert np.all(np.abs(a - b) <= 1e-9 * np.maximum(1.0, scale))
