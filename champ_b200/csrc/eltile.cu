@@ -19,6 +19,8 @@ static int fin_attrs_n(size_t b) {
   if (!rc) rc = big_smem(pt::k_fin_points<NORD, false, 4>, 128, b);
   if (!rc) rc = big_smem(pt::k_fin_points<NORD, true, 1>, 128, b);
   if (!rc) rc = big_smem(pt::k_fin_points<NORD, true, 4>, 128, b);
+  if (!rc) rc = big_smem(pt::k_fin_points<NORD, false, 8>, 256, b);
+  if (!rc) rc = big_smem(pt::k_fin_points<NORD, true, 8>, 256, b);
   return rc;
 }
 static size_t gproj_smem(const champ_ctx *c) { return sizeof(double) * pt::GP_LD * (size_t)((c->nomax + 3) & ~3); }
@@ -69,7 +71,7 @@ int el_tile_setup(champ_ctx *c) {
     c->orb_nt = nomax <= 16 ? 1 : nomax <= 32 ? 2 : 4;
   }
   if (c->nordc <= 1 || c->nct == 1) {
-    const int wpw = c->N <= 32 ? 1 : 4;
+    const int wpw = c->N <= 32 ? 1 : c->N <= 64 ? 4 : 8;
     c->fin_nrow = std::min(c->N * c->C * std::max(c->sd.nshc, 1), wpw == 1 ? 256 : 768);
     const size_t b = pt::Dims(c->N, c->C, c->nordc, c->fin_nrow, wpw == 1).bytes() * (wpw == 1 ? 4 : 1) +
                      stab::tab_smem(c->sd.nshell, c->sd.nprim);
@@ -147,6 +149,8 @@ static int fin(champ_ctx *c, const State<double> &st, bool outputs, bool stats, 
   }
   if (c->fin_wpw == 1)
     pt::k_fin_points<NORD, MD, 1><<<(W + 3) / 4, 128, c->fin_smem, c->stream>>>(c->sd, st, c->fin_nrow, outputs, stats, rot, tables_only, tape);
+  else if (c->fin_wpw == 8)
+    pt::k_fin_points<NORD, MD, 8><<<W, 256, c->fin_smem, c->stream>>>(c->sd, st, c->fin_nrow, outputs, stats, rot, tables_only, tape);
   else
     pt::k_fin_points<NORD, MD, 4><<<W, 128, c->fin_smem, c->stream>>>(c->sd, st, c->fin_nrow, outputs, stats, rot, tables_only, tape);
   CK(cudaGetLastError());

@@ -12,10 +12,16 @@
 // and powers once, in place.  The determinant ratio sums the basis functions at the point (lane =
 // point) with the electron's projected G; a primitive whose exponent exceeds the shell's smallest
 // by more than 70 / r^2 is below 1e-30 of the shell and is not formed.
-// What bounds it: the FP64 pipe.  Measured (B200), the part of an evaluation from the inverses on: 4096
-// walkers of 128 electrons and 32 centres, order 4, 46.2 -> 26.2 ms (projection 0.95); 1001 of 51 and
-// 13, order 5, 4.57 -> 1.60 ms; 3001 of 20 and 5, 0.96 -> 0.67 ms; 16384 of 8 and 2 with 200
-// determinants, 3.8 -> 2.0 ms.  k_el_fin stays for several centre types with e-e-n terms.
+// What bounds it: latency between dependent FP64 instructions and mma (an issue in every third cycle; a
+// third of the FP64 pipe), hence the most warps that the registers allow.  Blocks of 8 warps on one walker from 65
+// electrons on put 16 warps on an SM where shared memory holds two such walkers only: 21.0 -> 19.1 ms at 128
+// electrons, against 4 warps and 168 registers.  With 33 to 64 electrons 4 warps at 128 registers, 1.42 -> 1.19 ms; a
+// warp per walker below that keeps 168 registers with one determinant (0.53 against 0.55 ms), and takes 128
+// with several, whose tables add to the wait for memory (1.07 -> 0.91 ms).
+// Measured (B200), the part of an evaluation from the inverses on, projection included, against k_el_fin:
+// 4096 walkers of 128 electrons and 32 centres, order 4, 46.2 -> 20.1 ms (projection 0.95); 1001 of 51
+// and 13, order 5, 4.57 -> 1.23 ms; 3001 of 20 and 5, 0.96 -> 0.56 ms; the multi-determinant dimer (200
+// determinants), 3.8 -> 0.9 ms.  k_el_fin stays for several centre types with e-e-n terms.
 #pragma once
 #include "jastile.cuh"
 #include "shelltab.cuh"
@@ -450,7 +456,7 @@ struct Tape {
 };
 
 template <int NORD, bool MD, int WPW>
-__global__ void __launch_bounds__(128, 3) k_fin_points(const __grid_constant__ Sys<double> s,
+__global__ void __launch_bounds__(WPW == 8 ? 256 : 128, WPW == 8 ? 2 : WPW == 4 || MD ? 4 : 3) k_fin_points(const __grid_constant__ Sys<double> s,
                                                        const __grid_constant__ State<double> st, int nrow,
                                                        int outputs, int stats, ElRot rot, int tables_only, Tape tape) {
   using TB = Tab<NORD>;
@@ -675,10 +681,13 @@ __global__ void __launch_bounds__(128, 3) k_fin_points(const __grid_constant__ S
         o[0] = d2lnd; o[1] = v2; o[2] = vloc; o[3] = vnl;
       }
       __syncthreads();
-      d2lnd = red[0] + red[4] + red[8] + red[12];
-      v2 = red[1] + red[5] + red[9] + red[13];
-      vloc = red[2] + red[6] + red[10] + red[14];
-      vnl = red[3] + red[7] + red[11] + red[15];
+      d2lnd = v2 = vloc = vnl = 0;
+      for (int k = 0; k < WPW; k++) {
+        d2lnd += red[4 * k];
+        v2 += red[4 * k + 1];
+        vloc += red[4 * k + 2];
+        vnl += red[4 * k + 3];
+      }
     }
     if (wpos == 0) {
       EvalRes res;
