@@ -10,7 +10,12 @@
 // rows of the electrons' positions are kept through the moves: neither the drift at the current
 // position nor the evaluation after the moves forms them again.
 // Everything is FP64; sums differ in order from the warp-per-walker kernels (full_eval, propose).
-// What bounds it: FP64 issue and latency at 12 warps per SM.
+// What bounds it: latency between dependent FP64 instructions at 12 warps per SM (168 registers; an issue in
+// every 2.5 cycles).  At 128 registers for 14 to 16 warps the spills cost more than the warps give: 8192 walkers
+// of the dimer 1.00 -> 1.05 ms per evaluation, DMC step 3.44 -> 4.31 ms.
+// Measured (B200) against a warp per walker: dimer of 8 electrons, order 4, 8192 walkers, evaluation
+// 1.04 -> 0.97 ms; DMC step of about the same population 10.0 -> 3.3 ms; C2, order 5, the accelerated
+// moves and their evaluations 9.6 -> 2.2 ms, DMC step 1.33 -> 0.69 ms, T-moves 1.28 -> 0.82 ms.
 #pragma once
 #include "jastile.cuh"
 
@@ -142,55 +147,118 @@ struct Tab {
   static constexpr Terms tl = make_terms(NORD);
 };
 
-// Power sums of one electron's scaled distances over the centres, with gradients and Laplacians.
-template <int NORD>
-struct One {
-  static constexpr int QM = NORD > 1 ? NORD - 1 : 1;
-  double S[QM], g[QM][3], L[QM];
+// e-e-n terms of a pair as a function of its electron e, whose scaled distances are pa (strided by SP) and
+// ph = -k a^2 / r, with the other's aj and power sums zj: value, d/du and d2/du2, and (LEVEL > 0) the gradient
+// over a (w/o the pair's own), its product with d/du along r, and the Laplacian.  The coefficients of
+// u^k are summed first; at each centre they make a polynomial in the electron's own a, so that the gradient
+// is one factor per centre and nothing is kept per power but the three polynomials.
+struct Een {
+  double f = 0, w1 = 0, w2 = 0, g0 = 0, g1 = 0, g2 = 0, tt = 0, lp = 0;
 };
-template <int NORD, int LEVEL>
-__device__ __forceinline__ void one_sums(const Sys<double> &s, double sk, const double *xe, const double *pa,
-                                         const double *ph, One<NORD> &o) {
-  constexpr int QM = One<NORD>::QM;
+template <int NORD, int LEVEL, int SP>
+__device__ __forceinline__ void een_pair(const Sys<double> &s, const JasPar<double> &J, double du, const double *xe, const double *pa,
+                                         const double *ph, const double *aj, const double *zj, double r0, double r1, double r2, Een &o) {
+  using TB = Tab<NORD>;
+  constexpr int NC = jt::make_combos(NORD).n, NT = make_terms(NORD).n, NCA = NC > 0 ? NC : 1, QM = NORD - 1;
+  const double sk = J.scalek;
+  double u[NORD + 1];
+  u[0] = 1;
 #pragma unroll
-  for (int q = 0; q < QM; q++) o.S[q] = o.g[q][0] = o.g[q][1] = o.g[q][2] = o.L[q] = 0;
-  if constexpr (NORD > 1)
-    for (int c = 0; c < s.C; c++) {
-      const double a = pa[c];
-      double p = a, pm = 1;
-      double dx = 0, dy = 0, dz = 0, h = 0, s2 = 0;
-      if (LEVEL > 0) {
-        h = ph[c];
-        s2 = sk * sk * a * a;
-        dx = xe[0] - s.cent[3 * c];
-        dy = xe[1] - s.cent[3 * c + 1];
-        dz = xe[2] - s.cent[3 * c + 2];
+  for (int q = 1; q <= NORD; q++) u[q] = u[q - 1] * du;
+  double b0[QM + 1], b1[QM + 1], b2[QM + 1], cu[NCA], ct[NCA], c2[NCA];
+#pragma unroll
+  for (int q = 0; q <= QM; q++) b0[q] = b1[q] = b2[q] = 0;
+  sfor<NT>([&](auto LL) {
+    constexpr int ll = decltype(LL)::v, k = TB::tl.k[ll], l = TB::tl.l[ll];
+    if constexpr (TB::tl.m[ll] == 0) {
+      const double c = J.c[0][ll];
+      b0[l] += c * u[k];
+      if constexpr (LEVEL > 0 && k > 0) b1[l] += (c * k) * u[k - 1];
+      if constexpr (LEVEL > 1 && k > 1) b2[l] += (c * (k * (k - 1))) * u[k - 2];
+    }
+  });
+  sfor<NC>([&](auto YY) {
+    constexpr int y = decltype(YY)::v, l = TB::cb.l[y], nk = TB::cb.nk[y];
+    double x0 = 0, x1 = 0, x2 = 0;
+    sfor<nk>([&](auto K) {
+      constexpr int k = decltype(K)::v, ik = TB::cb.ll[y][k];
+      const double c = l ? J.c[0][ik] : 2 * J.c[0][ik];
+      x0 += c * u[k];
+      if constexpr (LEVEL > 0 && k > 0) x1 += (c * k) * u[k - 1];
+      if constexpr (LEVEL > 1 && k > 1) x2 += (c * (k * (k - 1))) * u[k - 2];
+    });
+    cu[y] = x0;
+    ct[y] = x1;
+    c2[y] = x2;
+  });
+  o.f = 2.0 * s.C * b0[0];
+  o.w1 = 2.0 * s.C * b1[0];
+  o.w2 = 2.0 * s.C * b2[0];
+#pragma unroll
+  for (int q = 1; q <= QM; q++) {
+    o.f += b0[q] * zj[q - 1];
+    if (LEVEL > 0) o.w1 += b1[q] * zj[q - 1];
+    if (LEVEL > 1) o.w2 += b2[q] * zj[q - 1];
+  }
+  for (int c = 0; c < s.C; c++) {
+    const double a = pa[c * SP], b = aj[c];
+    double bp[QM + 1], P0[QM + 1], P1[QM + 1], P2[QM + 1];
+    bp[0] = 1;
+#pragma unroll
+    for (int q = 1; q <= QM; q++) {
+      bp[q] = bp[q - 1] * b;
+      P0[q] = b0[q];
+      P1[q] = b1[q];
+      P2[q] = b2[q];
+    }
+    sfor<2 * NC>([&](auto Y) {
+      constexpr int yv = decltype(Y)::v, y = yv / 2, l = TB::cb.l[y], m = TB::cb.m[y];
+      if constexpr (yv % 2 == 0 || l > 0) {
+        constexpr int p = yv % 2 ? m : l + m, q = yv % 2 ? l + m : m, nk = TB::cb.nk[y];
+        P0[p] += cu[y] * bp[q];
+        if constexpr (LEVEL > 0 && nk > 1) P1[p] += ct[y] * bp[q];
+        if constexpr (LEVEL > 1 && nk > 2) P2[p] += c2[y] * bp[q];
       }
+    });
+    // the polynomials without their constant term over a, and derivatives with respect to a
+    double p0 = P0[QM], p1 = P1[QM], p2 = P2[QM], d0 = QM * P0[QM], d1 = QM * P1[QM], e0 = QM * (QM - 1) * P0[QM];
 #pragma unroll
-      for (int q = 1; q <= QM; q++) {
-        o.S[q - 1] += p;
-        if (LEVEL > 0) {
-          const double t = q * pm * h;
-          o.g[q - 1][0] += t * dx;
-          o.g[q - 1][1] += t * dy;
-          o.g[q - 1][2] += t * dz;
-          if (LEVEL > 1) o.L[q - 1] += q * p * ((q - 1) * s2 + 2 * h);
-        }
-        pm = p;
-        p *= a;
+    for (int q = QM - 1; q >= 1; q--) {
+      p0 = p0 * a + P0[q];
+      if (LEVEL > 0) {
+        p1 = p1 * a + P1[q];
+        d0 = d0 * a + q * P0[q];
+        d1 = d1 * a + q * P1[q];
+      }
+      if (LEVEL > 1) {
+        p2 = p2 * a + P2[q];
+        if (q > 1) e0 = e0 * a + q * (q - 1) * P0[q];
       }
     }
+    o.f += a * p0;
+    if (LEVEL > 0) {
+      o.w1 += a * p1;
+      const double h = ph[c], dx = xe[0] - s.cent[3 * c], dy = xe[1] - s.cent[3 * c + 1], dz = xe[2] - s.cent[3 * c + 2];
+      const double t = d0 * h;
+      o.g0 += t * dx;
+      o.g1 += t * dy;
+      o.g2 += t * dz;
+      if (LEVEL > 1) {
+        const double s2 = sk * a;
+        o.w2 += a * p2;
+        o.tt += d1 * h * (r0 * dx + r1 * dy + r2 * dz);
+        o.lp += (e0 * a * (s2 * s2) + 2 * h * d0) * a;
+      }
+    }
+  }
 }
 
-// e-e and e-e-n terms of electron e (position xe, scaled distances pa, ph = -k a^2 / r, sums o) with
+// e-e and e-e-n terms of electron e (position xe, scaled distances pa, ph = -k a^2 / r) with
 // electron j (xj, aj, power sums zj): value, gradient (LEVEL 1) and Laplacian (2) with respect to e.
 template <int NORD, int LEVEL>
 __device__ __forceinline__ double pair_terms(const Sys<double> &s, const JasPar<double> &J, int e, int j, const double *xe,
-                                             const double *pa, const double *ph, const One<NORD> &o, const double *xj,
-                                             const double *aj, const double *zj, double *g, double &lap, double &rin) {
-  using TB = Tab<NORD>;
-  constexpr int NC = jt::make_combos(NORD).n, NT = make_terms(NORD).n, NCA = NC > 0 ? NC : 1;
-  constexpr int QM = One<NORD>::QM;
+                                             const double *pa, const double *ph, const double *xj, const double *aj,
+                                             const double *zj, double *g, double &lap, double &rin) {
   const double sk = J.scalek;
   const double r0 = xe[0] - xj[0], r1 = xe[1] - xj[1], r2 = xe[2] - xj[2];
   const double rij = sqrt(r0 * r0 + r1 * r1 + r2 * r2);
@@ -199,103 +267,19 @@ __device__ __forceinline__ double pair_terms(const Sys<double> &s, const JasPar<
   double ss;
   pair_class(J, s.nup, e, j, isb, ss, ipar);
   double fu = 0, fuu = 0;
-  double f = jas_ee<double, (LEVEL > 0)>(J, isb, ss, ipar, rij, du, fu, fuu);
+  const double f = jas_ee<double, (LEVEL > 0)>(J, isb, ss, ipar, rij, du, fu, fuu);
   rin = LEVEL > 0 ? 1.0 / rij : 0.0;
-  double w1 = 0, w2 = 0, g0 = 0, g1 = 0, g2 = 0, tt = 0, lp = 0;
-  if constexpr (NORD > 1) {
-    double ax[NCA], ag[NCA][3], al[NCA];
-#pragma unroll
-    for (int y = 0; y < NCA; y++) ax[y] = ag[y][0] = ag[y][1] = ag[y][2] = al[y] = 0;
-    for (int c = 0; c < s.C; c++) {
-      const double a = pa[c], b = aj[c];
-      double ap[QM + 1], bp[QM + 1];
-      ap[0] = bp[0] = 1;
-#pragma unroll
-      for (int q = 1; q <= QM; q++) { ap[q] = ap[q - 1] * a; bp[q] = bp[q - 1] * b; }
-      double h = 0, dx = 0, dy = 0, dz = 0, s2 = 0;
-      if (LEVEL > 0) {
-        h = ph[c];
-        s2 = sk * sk * a * a;
-        dx = xe[0] - s.cent[3 * c];
-        dy = xe[1] - s.cent[3 * c + 1];
-        dz = xe[2] - s.cent[3 * c + 2];
-      }
-      sfor<2 * NC>([&](auto Y) {
-        constexpr int yv = decltype(Y)::v, y = yv / 2, l = TB::cb.l[y], m = TB::cb.m[y];
-        if constexpr (yv % 2 == 0 || l > 0) {
-          constexpr int p = yv % 2 ? m : l + m, q = yv % 2 ? l + m : m;
-          const double wq = (l ? 1.0 : 2.0) * bp[q];
-          ax[y] += ap[p] * wq;
-          if constexpr (LEVEL > 0) {
-            const double t = p * ap[p - 1] * h * wq;
-            ag[y][0] += t * dx;
-            ag[y][1] += t * dy;
-            ag[y][2] += t * dz;
-            if constexpr (LEVEL > 1) al[y] += p * ap[p] * ((p - 1) * s2 + 2 * h) * wq;
-          }
-        }
-      });
-    }
-    double u[NORD + 1];
-    u[0] = 1;
-#pragma unroll
-    for (int q = 1; q <= NORD; q++) u[q] = u[q - 1] * du;
-    sfor<NT>([&](auto LL) {
-      constexpr int ll = decltype(LL)::v, k = TB::tl.k[ll], l = TB::tl.l[ll];
-      if constexpr (TB::tl.m[ll] == 0) {
-        const double c = J.c[0][ll];
-        double Y = 2.0 * s.C;
-        if constexpr (l > 0) Y = o.S[l - 1] + zj[l - 1];
-        f += c * u[k] * Y;
-        if constexpr (LEVEL > 0) {
-          w1 += (c * k) * u[k - 1] * Y;
-          if constexpr (k > 1 && LEVEL > 1) w2 += (c * (k * (k - 1))) * u[k - 2] * Y;
-          if constexpr (l > 0) {
-            const double cu = c * u[k];
-            g0 += cu * o.g[l - 1][0];
-            g1 += cu * o.g[l - 1][1];
-            g2 += cu * o.g[l - 1][2];
-            if constexpr (LEVEL > 1) {
-              tt += (c * k) * u[k - 1] * (r0 * o.g[l - 1][0] + r1 * o.g[l - 1][1] + r2 * o.g[l - 1][2]);
-              lp += cu * o.L[l - 1];
-            }
-          }
-        }
-      }
-    });
-    sfor<NC>([&](auto YY) {
-      constexpr int y = decltype(YY)::v, nk = TB::cb.nk[y];
-      double cu = 0, ct = 0, c2 = 0;
-      sfor<nk>([&](auto K) {
-        constexpr int k = decltype(K)::v, ik = TB::cb.ll[y][k];
-        const double c = J.c[0][ik];
-        cu += c * u[k];
-        if constexpr (k > 0 && LEVEL > 0) ct += (c * k) * u[k - 1];
-        if constexpr (k > 1 && LEVEL > 1) c2 += (c * (k * (k - 1))) * u[k - 2];
-      });
-      f += cu * ax[y];
-      if constexpr (LEVEL > 0) {
-        w1 += ct * ax[y];
-        g0 += cu * ag[y][0];
-        g1 += cu * ag[y][1];
-        g2 += cu * ag[y][2];
-        if constexpr (LEVEL > 1) {
-          w2 += c2 * ax[y];
-          tt += ct * (r0 * ag[y][0] + r1 * ag[y][1] + r2 * ag[y][2]);
-          lp += cu * al[y];
-        }
-      }
-    });
-  }
+  Een o;
+  if constexpr (NORD > 1) een_pair<NORD, LEVEL, 1>(s, J, du, xe, pa, ph, aj, zj, r0, r1, r2, o);
   if constexpr (LEVEL > 0) {
     const double u1 = -sk * du * du;  // du/dr; u'' + 2 u'/r = -2 k du^3 / r
-    const double fr = fu + w1 * u1 * rin;
-    g[0] = fr * r0 + g0;
-    g[1] = fr * r1 + g1;
-    g[2] = fr * r2 + g2;
-    if constexpr (LEVEL > 1) lap = fuu + 2 * fu + w2 * u1 * u1 + 2 * u1 * rin * (w1 * du + tt) + lp;
+    const double fr = fu + o.w1 * u1 * rin;
+    g[0] = fr * r0 + o.g0;
+    g[1] = fr * r1 + o.g1;
+    g[2] = fr * r2 + o.g2;
+    if constexpr (LEVEL > 1) lap = fuu + 2 * fu + o.w2 * u1 * u1 + 2 * u1 * rin * (o.w1 * du + o.tt) + o.lp;
   }
-  return f;
+  return f + o.f;
 }
 
 // Jastrow of electron e at xe with the others where they are: its scaled distances (v + pa, ph), this
@@ -324,13 +308,10 @@ __device__ __noinline__ void electron_jastrow(const Sys<double> &s, const JasPar
     }
   }
   __syncwarp(m);
-  One<NORD> o;
-  one_sums<NORD, GRAD ? 1 : 0>(s, sk, xe, pa, ph, o);
   double d = en, f = 0;
   if (sub < N && sub != e) {
     double gp[3], lap, rin;
-    f = pair_terms<NORD, GRAD ? 1 : 0>(s, J, e, sub, xe, pa, ph, o, v + 3 * sub, v + L.a() + sub * C, v + L.z() + sub * L.qm, gp,
-                                       lap, rin);
+    f = pair_terms<NORD, GRAD ? 1 : 0>(s, J, e, sub, xe, pa, ph, v + 3 * sub, v + L.a() + sub * C, v + L.z() + sub * L.qm, gp, lap, rin);
     d += f;
     if (GRAD) {
       g0 += gp[0];
@@ -551,25 +532,17 @@ __device__ __noinline__ double point_psi(const Sys<double> &s, const stab::Tab &
   for (int k = 0; k < NO; k++) dr += o[k] * g[k];
   double *pl = v + L.pl() + sub;
   double f = 0;
-  One<NORD> os;
-#pragma unroll
-  for (int q = 0; q < One<NORD>::QM; q++) os.S[q] = 0;
   for (int c = 0; c < C; c++) {
     const double a0 = xn[0] - s.cent[3 * c], a1 = xn[1] - s.cent[3 * c + 1], a2 = xn[2] - s.cent[3 * c + 2];
     const double r = sqrt(a0 * a0 + a1 * a1 + a2 * a2), a = 1.0 / (1.0 + J.scalek * r);
     double fi, fii;
     f += jas_en<double, false>(J, s.ctype[c], r, a, fi, fii);
     pl[c * GS] = a;
-    double p = a;
-#pragma unroll
-    for (int q = 0; q < One<NORD>::QM; q++) { os.S[q] += p; p *= a; }
   }
   f -= v[L.f() + e * N + e];
-  using TB = Tab<NORD>;
-  constexpr int NC = jt::make_combos(NORD).n, NT = make_terms(NORD).n, NCA = NC > 0 ? NC : 1, QM = One<NORD>::QM;
   for (int j = 0; j < N; j++) {
     if (j == e) continue;
-    const double *xj = v + 3 * j, *aj = v + L.a() + j * C, *zj = v + L.z() + j * L.qm;
+    const double *xj = v + 3 * j;
     const double r0 = xn[0] - xj[0], r1 = xn[1] - xj[1], q2 = xn[2] - xj[2];
     const double rij = sqrt(r0 * r0 + r1 * r1 + q2 * q2);
     int isb, ipar;
@@ -577,42 +550,9 @@ __device__ __noinline__ double point_psi(const Sys<double> &s, const stab::Tab &
     pair_class(J, s.nup, e, j, isb, ss, ipar);
     f += pt::ee_value(J, isb, ss, ipar, rij, du) - v[L.f() + e * N + j];
     if constexpr (NORD > 1) {
-      double ax[NCA];
-#pragma unroll
-      for (int y = 0; y < NCA; y++) ax[y] = 0;
-      for (int c = 0; c < C; c++) {
-        const double a = pl[c * GS], b = aj[c];
-        double ap[QM + 1], bp[QM + 1];
-        ap[0] = bp[0] = 1;
-#pragma unroll
-        for (int q = 1; q <= QM; q++) { ap[q] = ap[q - 1] * a; bp[q] = bp[q - 1] * b; }
-        sfor<NC>([&](auto Y) {
-          constexpr int y = decltype(Y)::v, l = TB::cb.l[y], m = TB::cb.m[y];
-          if constexpr (l > 0) ax[y] += ap[l + m] * bp[m] + ap[m] * bp[l + m];
-          else ax[y] += 2.0 * ap[m] * bp[m];
-        });
-      }
-      double u[NORD + 1];
-      u[0] = 1;
-#pragma unroll
-      for (int q = 1; q <= NORD; q++) u[q] = u[q - 1] * du;
-      sfor<NT>([&](auto LL) {
-        constexpr int ll = decltype(LL)::v, k = TB::tl.k[ll], l = TB::tl.l[ll];
-        if constexpr (TB::tl.m[ll] == 0) {
-          double Y = 2.0 * C;
-          if constexpr (l > 0) Y = os.S[l - 1] + zj[l - 1];
-          f += J.c[0][ll] * u[k] * Y;
-        }
-      });
-      sfor<NC>([&](auto YY) {
-        constexpr int y = decltype(YY)::v, nk = TB::cb.nk[y];
-        double cu = 0;
-        sfor<nk>([&](auto K) {
-          constexpr int k = decltype(K)::v, ik = TB::cb.ll[y][k];
-          cu += J.c[0][ik] * u[k];
-        });
-        f += cu * ax[y];
-      });
+      Een o;
+      een_pair<NORD, 0, GS>(s, J, du, xn, pl, pl, v + L.a() + j * C, v + L.z() + j * L.qm, r0, r1, q2, o);
+      f += o.f;
     }
   }
   return dr * exp(f);
@@ -674,12 +614,10 @@ __device__ __forceinline__ Res evaluate(const Sys<double> &s, const stab::Tab &T
   __syncwarp(m);
   double dvd = 0, vx = 0, vy = 0, vz = 0;
   if (act) {
-    One<NORD> o;
-    one_sums<NORD, 2>(s, sk, xi, pa, ph, o);
     for (int j = 0; j < N; j++) {
       if (j == i) continue;
       double g[3], lap, rin;
-      const double f = pair_terms<NORD, 2>(s, J, i, j, xi, pa, ph, o, v + 3 * j, v + L.a() + j * C, v + L.z() + j * L.qm, g, lap, rin);
+      const double f = pair_terms<NORD, 2>(s, J, i, j, xi, pa, ph, v + 3 * j, v + L.a() + j * C, v + L.z() + j * L.qm, g, lap, rin);
       vj[0] += g[0];
       vj[1] += g[1];
       vj[2] += g[2];
@@ -720,10 +658,8 @@ __device__ __forceinline__ Res evaluate(const Sys<double> &s, const stab::Tab &T
     for (int j = 0; j < N; j++) {
       if (j == i) continue;
       const double xj[3] = {v[3 * j], v[3 * j + 1], v[3 * j + 2]};
-      One<NORD> o;
-      one_sums<NORD, 2>(s, sk, xj, v + L.a() + j * C, v + L.h() + j * C, o);
       double g[3], lap, rin;
-      pair_terms<NORD, 2>(s, J, j, i, xj, v + L.a() + j * C, v + L.h() + j * C, o, v + 3 * i, v + L.a() + i * C,
+      pair_terms<NORD, 2>(s, J, j, i, xj, v + L.a() + j * C, v + L.h() + j * C, v + 3 * i, v + L.a() + i * C,
                           v + L.z() + i * L.qm, g, lap, rin);
       other += 0.5 * lap;
     }
