@@ -12,10 +12,11 @@
 // Everything is FP64; sums differ in order from the warp-per-walker kernels (full_eval, propose).
 // What bounds it: latency between dependent FP64 instructions at 12 warps per SM (168 registers; an issue in
 // every 2.5 cycles).  At 128 registers for 14 to 16 warps the spills cost more than the warps give: 8192 walkers
-// of the dimer 1.00 -> 1.05 ms per evaluation, DMC step 3.44 -> 4.31 ms.
+// of the dimer 1.00 -> 1.05 ms per evaluation, DMC step 3.44 -> 4.31 ms.  Two electrons at a time in point_psi
+// filled the evaluation's chains (0.91 -> 0.90 ms) but spilled in the DMC step (3.18 -> 3.33 ms).
 // Measured (B200) against a warp per walker: dimer of 8 electrons, order 4, 8192 walkers, evaluation
-// 1.04 -> 0.97 ms; DMC step of about the same population 10.0 -> 3.3 ms; C2, order 5, the accelerated
-// moves and their evaluations 9.6 -> 2.2 ms, DMC step 1.33 -> 0.69 ms, T-moves 1.28 -> 0.82 ms.
+// 1.04 -> 0.90 ms; DMC step of about the same population 10.0 -> 3.2 ms; C2, order 5, the accelerated
+// moves and their evaluations 9.6 -> 2.1 ms, DMC step 1.33 -> 0.69 ms, T-moves 1.28 -> 0.82 ms.
 #pragma once
 #include "jastile.cuh"
 
@@ -147,7 +148,7 @@ struct Tab {
   static constexpr Terms tl = make_terms(NORD);
 };
 
-// e-e-n terms of a pair as a function of its electron e, whose scaled distances are pa (strided by SP) and
+// e-e-n terms of a pair as a function of its electron e, whose scaled distances are pa and
 // ph = -k a^2 / r, with the other's aj and power sums zj: value, d/du and d2/du2, and (LEVEL > 0) the gradient
 // over a (w/o the pair's own), its product with d/du along r, and the Laplacian.  The coefficients of
 // u^k are summed first; at each centre they make a polynomial in the electron's own a, so that the gradient
@@ -155,7 +156,7 @@ struct Tab {
 struct Een {
   double f = 0, w1 = 0, w2 = 0, g0 = 0, g1 = 0, g2 = 0, tt = 0, lp = 0;
 };
-template <int NORD, int LEVEL, int SP>
+template <int NORD, int LEVEL>
 __device__ __forceinline__ void een_pair(const Sys<double> &s, const JasPar<double> &J, double du, const double *xe, const double *pa,
                                          const double *ph, const double *aj, const double *zj, double r0, double r1, double r2, Een &o) {
   using TB = Tab<NORD>;
@@ -201,7 +202,7 @@ __device__ __forceinline__ void een_pair(const Sys<double> &s, const JasPar<doub
     if (LEVEL > 1) o.w2 += b2[q] * zj[q - 1];
   }
   for (int c = 0; c < s.C; c++) {
-    const double a = pa[c * SP], b = aj[c];
+    const double a = pa[c], b = aj[c];
     double bp[QM + 1], P0[QM + 1], P1[QM + 1], P2[QM + 1];
     bp[0] = 1;
 #pragma unroll
@@ -253,6 +254,58 @@ __device__ __forceinline__ void een_pair(const Sys<double> &s, const JasPar<doub
   }
 }
 
+// The value alone, centre by centre.
+template <int NORD>
+struct EenValue {
+  using TB = Tab<NORD>;
+  static constexpr int NC = jt::make_combos(NORD).n, NT = make_terms(NORD).n, QM = NORD > 1 ? NORD - 1 : 1;
+  double b[QM + 1], cu[NC > 0 ? NC : 1], f;
+  __device__ __forceinline__ void start(const Sys<double> &s, const JasPar<double> &J, double du, const double *zj) {
+    double u[NORD + 1];
+    u[0] = 1;
+#pragma unroll
+    for (int q = 1; q <= NORD; q++) u[q] = u[q - 1] * du;
+#pragma unroll
+    for (int q = 0; q <= QM; q++) b[q] = 0;
+    sfor<NT>([&](auto LL) {
+      constexpr int ll = decltype(LL)::v, k = TB::tl.k[ll], l = TB::tl.l[ll];
+      if constexpr (TB::tl.m[ll] == 0) b[l] += J.c[0][ll] * u[k];
+    });
+    sfor<NC>([&](auto YY) {
+      constexpr int y = decltype(YY)::v, l = TB::cb.l[y], nk = TB::cb.nk[y];
+      double x = 0;
+      sfor<nk>([&](auto K) {
+        constexpr int k = decltype(K)::v, ik = TB::cb.ll[y][k];
+        x += (l ? J.c[0][ik] : 2 * J.c[0][ik]) * u[k];
+      });
+      cu[y] = x;
+    });
+    f = 2.0 * s.C * b[0];
+#pragma unroll
+    for (int q = 1; q <= QM; q++) f += b[q] * zj[q - 1];
+  }
+  __device__ __forceinline__ void add(double a, double r) {
+    double rp[QM + 1], P[QM + 1];
+    rp[0] = 1;
+#pragma unroll
+    for (int q = 1; q <= QM; q++) {
+      rp[q] = rp[q - 1] * r;
+      P[q] = b[q];
+    }
+    sfor<2 * NC>([&](auto Y) {
+      constexpr int yv = decltype(Y)::v, y = yv / 2, l = TB::cb.l[y], m = TB::cb.m[y];
+      if constexpr (yv % 2 == 0 || l > 0) {
+        constexpr int p = yv % 2 ? m : l + m, q = yv % 2 ? l + m : m;
+        P[p] += cu[y] * rp[q];
+      }
+    });
+    double t = P[QM];
+#pragma unroll
+    for (int q = QM - 1; q >= 1; q--) t = t * a + P[q];
+    f += a * t;
+  }
+};
+
 // e-e and e-e-n terms of electron e (position xe, scaled distances pa, ph = -k a^2 / r) with
 // electron j (xj, aj, power sums zj): value, gradient (LEVEL 1) and Laplacian (2) with respect to e.
 template <int NORD, int LEVEL>
@@ -270,7 +323,7 @@ __device__ __forceinline__ double pair_terms(const Sys<double> &s, const JasPar<
   const double f = jas_ee<double, (LEVEL > 0)>(J, isb, ss, ipar, rij, du, fu, fuu);
   rin = LEVEL > 0 ? 1.0 / rij : 0.0;
   Een o;
-  if constexpr (NORD > 1) een_pair<NORD, LEVEL, 1>(s, J, du, xe, pa, ph, aj, zj, r0, r1, r2, o);
+  if constexpr (NORD > 1) een_pair<NORD, LEVEL>(s, J, du, xe, pa, ph, aj, zj, r0, r1, r2, o);
   if constexpr (LEVEL > 0) {
     const double u1 = -sk * du * du;  // du/dr; u'' + 2 u'/r = -2 k du^3 / r
     const double fr = fu + o.w1 * u1 * rin;
@@ -550,8 +603,10 @@ __device__ __noinline__ double point_psi(const Sys<double> &s, const stab::Tab &
     pair_class(J, s.nup, e, j, isb, ss, ipar);
     f += pt::ee_value(J, isb, ss, ipar, rij, du) - v[L.f() + e * N + j];
     if constexpr (NORD > 1) {
-      Een o;
-      een_pair<NORD, 0, GS>(s, J, du, xn, pl, pl, v + L.a() + j * C, v + L.z() + j * L.qm, r0, r1, q2, o);
+      const double *aj = v + L.a() + j * C;
+      EenValue<NORD> o;
+      o.start(s, J, du, v + L.z() + j * L.qm);
+      for (int c = 0; c < C; c++) o.add(pl[c * GS], aj[c]);
       f += o.f;
     }
   }
