@@ -185,7 +185,7 @@ static int launch_t(champ_ctx *c, Op op, const OpArgs &a) {
     }
     c->orb5_valid = false;
     if constexpr (std::is_same<T, double>::value)
-      if (c->small && !a.st_override) {
+      if (!a.st_override && small_serves(c, SmallOp::Eval, st.W)) {
         ElRot rot{};
         for (int i = 0; i < 9; i++) rot.R[i] = R[i];
         return small_eval(c, st, op == Op::EvalOut, false, rot);
@@ -216,7 +216,8 @@ static int launch_t(champ_ctx *c, Op op, const OpArgs &a) {
   }
   case Op::DmcMove: {
     if constexpr (std::is_same<T, double>::value)
-      if (c->small && !c->dpar.persist && a.phase != 1) return small_dmc(c, st, a.phase != 2);
+      if (!c->dpar.persist && a.phase != 1 && small_serves(c, a.phase == 2 ? SmallOp::Eval : SmallOp::Dmc, c->dpar.wtarget))
+        return small_dmc(c, st, a.phase != 2);
     // persistent: as many blocks as the SMs can hold at once (at most 16 per SM; a block that
     // finds the work counter exhausted exits at once), no more than the walkers need
     const int sm = c->num_sms > 0 ? c->num_sms : 148;
@@ -228,7 +229,7 @@ static int launch_t(champ_ctx *c, Op op, const OpArgs &a) {
   }
   case Op::Tmove: {
     if constexpr (std::is_same<T, double>::value)
-      if (c->small) return small_tmove(c, st, a);
+      if (small_serves(c, SmallOp::Dmc, a.dmc ? c->dpar.wtarget : st.W)) return small_tmove(c, st, a);
     const int wl = a.dmc ? c->dpar.wmax : st.W;
     k_dmc_tmove<T, NORD, MD><<<dim3((wl + K.wpb - 1) / K.wpb), block, K.smem, c->stream>>>(
         s, st, K.lay, st.W, a.dmc ? c->dA.nw : nullptr, a.tau, a.variant, a.seed, a.dmc ? c->dA.ctr : nullptr,
@@ -249,7 +250,7 @@ static int launch_t(champ_ctx *c, Op op, const OpArgs &a) {
       return run_el_staged<T, NORD, MD>(c, st, false, true, rot);
     }
     if constexpr (std::is_same<T, double>::value)
-      if (c->small && !a.st_override && a.phase == 3) {
+      if (!a.st_override && a.phase == 3 && small_serves(c, SmallOp::Eval, st.W)) {
         ElRot rot{};
         rot.random = 1;
         rot.seed = a.seed;
@@ -294,7 +295,7 @@ static int launch_t(champ_ctx *c, Op op, const OpArgs &a) {
     }
     CK(cudaMemsetAsync(st.s_esum, 0, sizeof(double) * 3 * (size_t)c->wmax, c->stream));  // esum, e2sum, acc
     if constexpr (std::is_same<T, double>::value)
-      if (c->small && !a.st_override) return small_vmc(c, st, a);
+      if (!a.st_override && small_serves(c, c->mover.kind == 6 ? SmallOp::Accel : SmallOp::Gauss, st.W)) return small_vmc(c, st, a);
     const bool tc = c->tc_on && !a.st_override;  // only FP32 contexts turn it on
     if (!tc) {
       auto kern = c->mover.kind == 6 ? k_vmc<T, NORD, MD, 0, 6> : k_vmc<T, NORD, MD, 0>;

@@ -72,6 +72,25 @@ int small_setup(champ_ctx *c) {
   return rc;
 }
 
+// How many walkers.  A walker on 8 lanes takes longer than on 32 (an evaluation with nonlocal points 440 us
+// against 230), so the kernels pay where a warp per walker fills the SMs more than once: walkers above a number
+// per SM, by what the operation spends on points, which split worst.  Measured (B200, 148 SMs; dimer and C2
+// of 8 electrons, calls of 2 sweeps or 4 steps, us here against a warp per walker):
+//   evaluation      2400 walkers 1325 / 1084, 3600 1492 / 1395, 8192 with mixed-precision sweeps 2790 / 3100;
+//   Gaussian moves  1800 1142 / 1035, 2400 1250 / 1379;
+//   accelerated     250 1439 / 1098, 600 1461 / 1691 and 1539 / 1684;
+//   DMC, T-moves    1800 2776 / 2571 and 2351 / 2294, 2400 2834 / 4399 and 2557 / 3881; T-moves 1800 5758 / 4956 and
+//                   5234 / 6122, 2400 5946 / 7552 and 5448 / 9157 (a warp per walker holds 16 per SM at once).
+// Without a pseudopotential there are no points: Gaussian moves of the Be-like atom 120 / 139 at 60 walkers,
+// 154 / 276 at 2400.
+bool small_serves(const champ_ctx *c, SmallOp op, int W) {
+  if (!c->small) return false;
+  if (c->nloc == 0 && op == SmallOp::Gauss) return true;
+  const int sm = c->num_sms > 0 ? c->num_sms : 148;
+  const int per = op == SmallOp::Eval ? 32 : op == SmallOp::Gauss ? 14 : op == SmallOp::Accel ? 4 : 16;
+  return W > per * sm;
+}
+
 int small_eval(champ_ctx *c, const State<double> &st, bool outputs, bool stats, const ElRot &rot) {
   sm::Args A;
   A.order = c->small_order;

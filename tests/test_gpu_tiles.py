@@ -83,16 +83,20 @@ SMALL = [(1, 1, 1, 0), (2, 1, 1, 0), (3, 2, 2, 4), (4, 4, 1, 4), (5, 3, 2, 5), (
 @pytest.mark.parametrize("n,nup,ncent,nordc", SMALL)
 def test_small_walkers_match_oracle(oracle_mod, n, nup, ncent, nordc):
     """The 8-lanes-per-walker kernels at the edges of their range (one electron, one spin only, up to 8
-    electrons and 4 of a spin): evaluation, and two sweeps walked as the oracle walks them."""
+    electrons and 4 of a spin): evaluation, and two sweeps walked as the oracle walks them.  The kernels serve
+    many walkers only, so the oracle's 19 are the first of 4801 (not a multiple of the walkers of a block) that
+    repeat them; 19 alone take the warp-per-walker kernels, to the same bounds."""
     from champ_b200.engine import Engine
     s = cluster(n, nup, ncent, nordc)
-    nw = 19  # not a multiple of the walkers of a block
+    nw = 19
     x = S.initial_walkers(s, nw, seed=n)
+    many = np.resize(x, (4801,) + x.shape[1:])
     orc = oracle_mod.Oracle(s)
-    for prec in ("fp64", "mixed"):
-        eng = Engine(s, nw, prec)
-        eng.set_walkers(x)
+    for prec, y in (("fp64", many), ("mixed", many), ("fp64", x)):
+        eng = Engine(s, len(y), prec)
+        eng.set_walkers(y)
         r = eng.eval_full()
+        assert np.array_equal(r["energy"], np.resize(r["energy"][:nw], len(y)))
         for w in range(nw):
             o = orc.eval(x[w])
             scale = max(1.0, abs(o["energy"]), abs(o["d2lnpsi"]))
@@ -105,10 +109,10 @@ def test_small_walkers_match_oracle(oracle_mod, n, nup, ncent, nordc):
         if prec == "fp64":
             st = eng.vmc_sweeps(2, seed=11, sweep0=4, step=s.step)
             ref = orc.vmc(x, 2, seed=11, sweep0=4, step=s.step)
-            assert np.abs(eng.get_walkers() - ref["x"]).max() <= 1e-12
+            assert np.abs(eng.get_walkers()[:nw] - ref["x"]).max() <= 1e-12
             scale = np.array([max(1.0, abs(e), abs(orc.eval(y)["d2lnpsi"])) for e, y in zip(ref["elast"], ref["x"])])
-            assert np.all(np.abs(st["elast"] - ref["elast"]) <= 1e-9 * scale)
-            assert np.array_equal(st["accept"], ref["accept"])
+            assert np.all(np.abs(st["elast"][:nw] - ref["elast"]) <= 1e-9 * scale)
+            assert np.array_equal(st["accept"][:nw], ref["accept"])
         eng.close()
 
 
