@@ -43,17 +43,18 @@ FMA_PER_SM_CLK = {"fp64": 64, "fp32": 128}  # FP64 / FP32 fused multiply-adds pe
 # per DMMA m8n8k4 warp instruction), counted by ncu (smsp__sass_thread_inst_executed_op_{d,f}{fma,
 # add,mul}_pred_on.sum, sm__inst_executed_pipe_tensor_subpipe_dmma.sum) on a 256-walker sweep of
 # the same kernels and divided by the walkers (profiles/flops_cluster128.md).  "eval" is the FP64
-# full evaluation (k_el_jas, k_el_orb, k_el_inv, k_el_fin); None until counted: the roofline's
+# full evaluation (k_jas_tile, k_orb_tile, k_inv_reg, k_gproj, k_fin_points), "moves" the batched
+# sweep (k_mv_draw, k_mv_prop, k_mv_pairs, k_mv_walk); None until counted: the roofline's
 # achieved figure is then left out.
 FLOPS_PER_WALKER = {
-    ("cluster128", "eval", "fp64"): 250.86e6,     # CUDA cores 216.31 M + DMMA 34.55 M
-    ("cluster128", "moves", "fp32"): 18.54e6,     # FP32 (plus 2.85 M FP64: the Sherman-Morrison updates)
+    ("cluster128", "eval", "fp64"): 140.56e6,     # CUDA cores 30.05 M + DMMA 110.51 M
+    ("cluster128", "moves", "fp32"): 23.56e6,     # FP32 (plus 2.13 M FP64: the determinant ratios)
     ("cluster128", "sweep", "fp64"): None,
 }
 # DRAM bytes per walker of the same launches (dram__bytes_read.sum + dram__bytes_write.sum).
 DRAM_PER_WALKER = {
-    ("cluster128", "eval", "fp64"): 1555342.0,    # 218.0 MB read + 180.3 MB written / 256
-    ("cluster128", "moves", "fp32"): 162209.0,    # 39.8 MB read + 1.8 MB written / 256
+    ("cluster128", "eval", "fp64"): 1644000.0,    # 289.7 MB read + 131.2 MB written / 256
+    ("cluster128", "moves", "fp32"): 293300.0,    # 74.9 MB read + 0.1 MB written / 256
     ("cluster128", "sweep", "fp64"): None,
 }
 
@@ -335,7 +336,7 @@ def roofline_for(system, nw, arm, clocks, prec):
     peak = 2 * NSM * FMA_PER_SM_CLK[kprec] * mhz * 1e6 / 1e12
     fpw, dpw = FLOPS_PER_WALKER.get(key), DRAM_PER_WALKER.get(key)
     t = ks[kern] * 1e-3
-    name = {"eval": "FP64 full evaluation (k_el_jas, k_el_orb, k_el_inv, k_el_fin)", "moves": "k_vmc<float> move phase",
+    name = {"eval": "FP64 full evaluation (k_jas_tile, k_orb_tile, k_inv_reg, k_gproj, k_fin_points)", "moves": "batched moves (k_mv_*)",
             "sweep": "k_vmc (fused sweep)"}[kern]
     out = {"bound": f"{kprec} FMA rate (CUDA cores; FP64 tensor cores run at the same rate)", "kernel": name,
            "unit": "TFLOP/s", "peak": peak,

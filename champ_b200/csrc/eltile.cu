@@ -42,7 +42,8 @@ int el_tile_setup(champ_ctx *c) {
   const int nmax = std::max(c->nup, c->ndn), nomax = c->nomax;
   c->inv_nm = nmax <= 32 ? 32 : 64;
   if ((c->nordc == 4 || c->nordc == 5) && c->nct == 1) {
-    // one warp per walker up to 32 electrons (4 tiles of rows), else a block per walker
+    // one warp per walker up to 32 electrons (4 tiles of rows, so that a block's warps would have one each
+    // and wait for one another), else a block per walker
     const int wpw = c->N <= 32 ? 1 : jt::WARPS;
     const size_t b = jt::Dims(c->N, c->C, wpw).bytes() * (wpw == 1 ? jt::WARPS : 1);
     if (b <= 200 * 1024) {

@@ -19,8 +19,8 @@
 // the compute type T; ratios and sums are FP64 as there.  The evaluation that follows every sweep
 // rebuilds the inverses and tables from the positions, so nothing but the positions is written back.
 //
-// Measured (B200), one sweep: 4096 walkers of 128 electrons, mixed precision, 19.4 -> 5.4 ms (pairs 2.6,
-// orbital rows 1.8, decisions 1.0); 2048 in FP64, 22.7 -> 4.1 ms; 1001 walkers of 51 electrons,
+// Measured (B200), one sweep: 4096 walkers of 128 electrons, mixed precision, 19.4 -> 5.2 ms (pairs 2.6,
+// orbital rows 1.6, decisions 1.0); 2048 in FP64, 22.7 -> 4.1 ms; 1001 walkers of 51 electrons,
 // order 5, FP64, 1.48 -> 0.39 ms.
 //
 // The scratch is the walker's place in the orbital rows of the FP64 evaluation (5 N nomax doubles,

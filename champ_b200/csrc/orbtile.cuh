@@ -46,8 +46,8 @@ static __device__ __noinline__ void general_shell5(const Sys<double> &s, int ish
 // chunk arrive by cp.async while its basis functions are formed and are shared by the 32
 // electrons (the warp-per-electron contraction streamed them from L2 once per 4 electrons).
 // What bounds it: the FP64 pipe (about a fifth of it the basis functions).  Measured (B200): 4096
-// walkers of 128 electrons, 416 basis functions, 15.6 -> 7.1 ms; 3001 of 20 electrons, 65 functions,
-// 0.32 -> 0.08 ms.  k_el_orb stays for more than 64 orbitals of a spin.
+// walkers of 128 electrons, 416 basis functions, 15.6 -> 6.0 ms; 3001 of 20 electrons, 65 functions,
+// 0.32 -> 0.06 ms.  k_el_orb stays for more than 64 orbitals of a spin.
 // chunk[k]: first shell, shells, first basis function, basis functions.
 // GEN: shells other than those Gaussians occur.
 // ALL: the columns blockIdx.y * 16 NT onwards of all orbitals (s.call), for every electron, into all + w

@@ -8,6 +8,9 @@
 // so a parameter has two sums in registers (value, local energy) and nothing is stored per electron.
 // The e-e-n parameters are the terms of k_jas_tile (pairs) and point_jastrow (points), each with
 // its own sum instead of being weighted by its coefficient.
+// What bounds it: FP64 issue.  Measured (B200), 1024 walkers of 128 electrons, 32 centres, 2064 parameters: the
+// forward pass 122 -> 15 ms (k_pg_nl 3.3, rows of all orbitals 2.9, the evaluation the rest), the reverse sweep
+// 212 -> 4.5 ms (points 3.0, pairs 1.2).
 #pragma once
 #include "nlpoints.cuh"
 #include "orbtile.cuh"

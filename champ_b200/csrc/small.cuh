@@ -14,6 +14,7 @@
 // every 2.5 cycles).  At 128 registers for 14 to 16 warps the spills cost more than the warps give: 8192 walkers
 // of the dimer 1.00 -> 1.05 ms per evaluation, DMC step 3.44 -> 4.31 ms.  Two electrons at a time in point_psi
 // filled the evaluation's chains (0.91 -> 0.90 ms) but spilled in the DMC step (3.18 -> 3.33 ms).
+// A single walker takes longer on 8 lanes than on 32, so few walkers stay with a warp each (small_serves).
 // Measured (B200) against a warp per walker: dimer of 8 electrons, order 4, 8192 walkers, evaluation
 // 1.04 -> 0.90 ms; DMC step of about the same population 10.0 -> 3.2 ms; C2, order 5, the accelerated
 // moves and their evaluations 9.6 -> 2.1 ms, DMC step 1.33 -> 0.69 ms, T-moves 1.28 -> 0.82 ms.

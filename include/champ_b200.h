@@ -240,7 +240,7 @@ int champ_param_grad(champ_ctx *ctx, double *dlnpsi /* [nw][P] */, double *deloc
    all Jastrow parameters from the pair, e-n and point terms recomputed from the positions
    (in FP32 for mixed precision, FP64 otherwise), then contracts the orbital-resolved local
    energy for the CSF and orbital-rotation parameters (FP64).  champ_param_grad runs both (or,
-   with option "param_grad_mode" 1, one fused FP64/FP32 pass).  Outputs as champ_param_grad;
+   with option "param_grad_mode" 1, one fused FP64/FP32 pass where the tiled passes do not serve).  Outputs as champ_param_grad;
    the bwd call consumes the tape (CHAMP_ESTATE without a preceding fwd). */
 int champ_param_grad_fwd(champ_ctx *ctx, double *eloc /* [nw] or NULL */);
 int champ_param_grad_bwd(champ_ctx *ctx, double *dlnpsi /* [nw][P] or NULL */, double *deloc /* [nw][P] or NULL */);
