@@ -98,10 +98,11 @@ struct champ_ctx {
   size_t el_smem[3] = {0, 0, 0};
   int el_nscr = 0;
   // its tensor-core parts (eltile.cu): warps per walker and shared memory of the Jastrow part (0:
-  // k_el_jas), orbital tiles of 16 per block and chunks of shells (0: k_el_orb), rows of the inversion
+  // k_el_jas), orbital tiles of 16 per block of the batched moves and chunks of shells (0: neither these nor
+  // k_orb_tile), whether k_orb_tile serves (else k_el_orb), rows of the inversion
   int jas_wpw = 0;
   size_t jas_smem = 0;
-  int orb_nt = 0, orb_nchunk = 0, orb_gen = 0;  // orb_gen: shells other than Gaussians with n = l + 1, l <= 2
+  int orb_nt = 0, orb_nchunk = 0, orb_tile = 0;
   int4 *orb_chunk = nullptr;
   int inv_nm = 64;
   // last part (0: k_el_fin): warps per walker, shared memory, radial values of tasks kept there

@@ -31,10 +31,6 @@ static int fin_attrs(champ_ctx *c) {
   return rc;
 }
 
-template <int NT>
-static size_t orb_smem(const champ_ctx *c) {
-  return ot::smem_bytes<NT>() + stab::tab_smem(c->sd.nshell, c->sd.nprim);
-}
 
 // Which parts serve the context's system, their shared memory, and the chunks of whole shells that
 // the orbital part forms at a time.
@@ -58,7 +54,6 @@ int el_tile_setup(champ_ctx *c) {
     CK(cudaMemcpy(b0.data(), c->sd.shb0, sizeof(int) * c->nshell, cudaMemcpyDeviceToHost));
     for (int i = 0; i < c->nshell; i++) {
       const int nb = 2 * sh[i].z + 1;
-      if (sh[i].w != 1 || sh[i].y != sh[i].z + 1 || sh[i].z > 2) c->orb_gen = 1;
       if (ch.empty() || ch.back().w + nb > ot::KB) ch.push_back(make_int4(i, 0, b0[i], 0));
       ch.back().y++;
       ch.back().w += nb;
@@ -70,6 +65,9 @@ int el_tile_setup(champ_ctx *c) {
     c->orb_chunk = d;
     c->orb_nchunk = (int)ch.size();
     c->orb_nt = nomax <= 16 ? 1 : nomax <= 32 ? 2 : 4;
+    // one or two orbitals of a spin: 32 or 16 interleaved sums each (k_orb_tile holds up to 8)
+    auto served = [&](int no) { return no == 0 || no > 2; };
+    c->orb_tile = served(c->sd.nocc[0]) && served(c->sd.nocc[1]);
   }
   if (c->nordc <= 1 || c->nct == 1) {
     const int wpw = c->N <= 32 ? 1 : c->N <= 64 ? 4 : 8;
@@ -86,12 +84,11 @@ int el_tile_setup(champ_ctx *c) {
                  jt::k_jas_tile<4, jt::WARPS, true>, jt::k_jas_tile<5, 1, false>, jt::k_jas_tile<5, 1, true>,
                  jt::k_jas_tile<5, jt::WARPS, false>, jt::k_jas_tile<5, jt::WARPS, true>})
     if (!rc) rc = big_smem(k, 128, c->jas_smem);
-  if (!rc) rc = big_smem(ot::k_orb_tile<1, false, false>, ot::THREADS, orb_smem<1>(c));
-  if (!rc) rc = big_smem(ot::k_orb_tile<1, false, true>, ot::THREADS, orb_smem<1>(c));
-  if (!rc) rc = big_smem(ot::k_orb_tile<2, false, false>, ot::THREADS, orb_smem<2>(c));
-  if (!rc) rc = big_smem(ot::k_orb_tile<2, false, true>, ot::THREADS, orb_smem<2>(c));
-  if (!rc) rc = big_smem(ot::k_orb_tile<4, false, false>, ot::THREADS, orb_smem<4>(c));
-  if (!rc) rc = big_smem(ot::k_orb_tile<4, false, true>, ot::THREADS, orb_smem<4>(c));
+  if (!rc) rc = big_smem(ot::k_orb_tile<1, 2, false>, ot::THREADS, ot::smem_bytes<1>());
+  if (!rc) rc = big_smem(ot::k_orb_tile<1, 4, false>, ot::THREADS, ot::smem_bytes<1>());
+  if (!rc) rc = big_smem(ot::k_orb_tile<1, 8, false>, ot::THREADS, ot::smem_bytes<1>());
+  if (!rc) rc = big_smem(ot::k_orb_tile<2, 1, false>, ot::THREADS, ot::smem_bytes<2>());
+  if (!rc) rc = big_smem(ot::k_orb_tile<4, 1, false>, ot::THREADS, ot::smem_bytes<4>());
   return rc;
 }
 
@@ -113,20 +110,28 @@ int el_tile_jas(champ_ctx *c, const State<double> &st, bool vo) {
   return c->nordc == 4 ? jas<4>(c, st, vo) : jas<5>(c, st, vo);
 }
 
-template <int NT>
-static void orb(champ_ctx *c, const State<double> &st, dim3 g) {
-  if (c->orb_gen) ot::k_orb_tile<NT, false, true><<<g, ot::THREADS, orb_smem<NT>(c), c->stream>>>(c->sd, st, c->orb_chunk, c->orb_nchunk, nullptr, 0);
-  else ot::k_orb_tile<NT, false, false><<<g, ot::THREADS, orb_smem<NT>(c), c->stream>>>(c->sd, st, c->orb_chunk, c->orb_nchunk, nullptr, 0);
-}
-int el_tile_orb(champ_ctx *c, const State<double> &st) {
-  const int nmax = std::max(c->nup, c->ndn);
-  const long long items = (long long)st.W * nmax;
-  const dim3 g((unsigned)((items + ot::EB - 1) / ot::EB), 2);
-  if (c->orb_nt == 1) orb<1>(c, st, g);
-  else if (c->orb_nt == 2) orb<2>(c, st, g);
-  else orb<4>(c, st, g);
+// Spins sp0 .. sp0 + ns - 1, which have orbitals of the same class (orb_class).
+template <int NT, int SPLIT>
+static int orb(champ_ctx *c, const State<double> &st, int sp0, int ns) {
+  const int n = std::max(sp0 ? 0 : c->nup, sp0 + ns > 1 ? c->ndn : 0);
+  const long long items = (long long)st.W * n;
+  if (items == 0) return CHAMP_OK;
+  const dim3 g((unsigned)((items + ot::EB - 1) / ot::EB), ns);
+  ot::k_orb_tile<NT, SPLIT, false><<<g, ot::THREADS, ot::smem_bytes<NT>(), c->stream>>>(c->sd, st, c->orb_chunk, c->orb_nchunk, sp0, nullptr, 0);
   CK(cudaGetLastError());
   return CHAMP_OK;
+}
+static int orb_class(int nocc) { return nocc > 32 ? 5 : nocc > 16 ? 4 : nocc > 8 ? 3 : nocc > 4 ? 2 : nocc > 2 ? 1 : 0; }
+static int orb_spins(champ_ctx *c, const State<double> &st, int k, int sp0, int ns) {
+  return k == 5 ? orb<4, 1>(c, st, sp0, ns) : k == 4 ? orb<2, 1>(c, st, sp0, ns) : k == 3 ? orb<1, 2>(c, st, sp0, ns)
+       : k == 2 ? orb<1, 4>(c, st, sp0, ns) : orb<1, 8>(c, st, sp0, ns);
+}
+int el_tile_orb(champ_ctx *c, const State<double> &st) {
+  const int k0 = orb_class(c->sd.nocc[0]), k1 = orb_class(c->sd.nocc[1]);
+  if (k0 == k1) return orb_spins(c, st, k0, 0, 2);
+  int rc = orb_spins(c, st, k0, 0, 1);
+  if (!rc) rc = orb_spins(c, st, k1, 1, 1);
+  return rc;
 }
 
 int el_tile_inv(champ_ctx *c, const State<double> &st) {
@@ -176,7 +181,7 @@ int el_tile_fin(champ_ctx *c, const State<double> &st, bool outputs, bool stats,
 // rounding beyond the derivatives themselves.
 bool pg_tile_fwd_ok(const champ_ctx *c) {
   const bool room = c->ncsfp + c->norbp == 0 || c->C * c->nquad <= 5 * c->norb;
-  return c->el_staged && c->jas_wpw && c->fin_wpw && c->orb_nt && !c->md.multidet && room;
+  return c->el_staged && c->jas_wpw && c->fin_wpw && c->orb_tile && !c->md.multidet && room;
 }
 // The reverse sweep in FP64: one e-e parameter set.
 bool pg_tile_bwd_ok(const champ_ctx *c) {
@@ -197,8 +202,7 @@ int pg_tile_setup(champ_ctx *c) {
   CK(cudaMalloc(&c->shell_order, sizeof(int) * c->nshell));
   c->allocs.push_back(c->shell_order);
   CK(cudaMemcpy(c->shell_order, order.data(), sizeof(int) * c->nshell, cudaMemcpyHostToDevice));
-  int rc = big_smem(ot::k_orb_tile<4, true, false>, ot::THREADS, orb_smem<4>(c));
-  if (!rc) rc = big_smem(ot::k_orb_tile<4, true, true>, ot::THREADS, orb_smem<4>(c));
+  int rc = big_smem(ot::k_orb_tile<4, 1, true>, ot::THREADS, ot::smem_bytes<4>());
   if (!rc) rc = big_smem(pg::k_pg_nl, 128, pgnl_smem(c));
   if (rc || c->prec != CHAMP_PREC_FP64 || c->par.nspin2b != 1) return rc;
   const size_t pb = pt::Dims(c->N, c->C, c->nordc, 0).bytes() * (c->jas_wpw == 1 ? 4 : 1);
@@ -249,8 +253,7 @@ int pg_tile_fwd(champ_ctx *c) {
     const long long items = (long long)W * c->N;
     const dim3 g((unsigned)((items + ot::EB - 1) / ot::EB), (c->norb + 63) / 64);
     double *all = c->pg_scr + (size_t)c->N * c->nbasis;
-    if (c->orb_gen) ot::k_orb_tile<4, true, true><<<g, ot::THREADS, orb_smem<4>(c), c->stream>>>(c->sd, st, c->orb_chunk, c->orb_nchunk, all, c->scr_stride);
-    else ot::k_orb_tile<4, true, false><<<g, ot::THREADS, orb_smem<4>(c), c->stream>>>(c->sd, st, c->orb_chunk, c->orb_nchunk, all, c->scr_stride);
+    ot::k_orb_tile<4, 1, true><<<g, ot::THREADS, ot::smem_bytes<4>(), c->stream>>>(c->sd, st, c->orb_chunk, c->orb_nchunk, 0, all, c->scr_stride);
     CK(cudaGetLastError());
     const long long el = items * c->norb;
     pg::k_pg_blocal<<<(unsigned)std::min<long long>((el + 255) / 256, 148 * 32), 256, 0, c->stream>>>(c->sd, st, c->pg_scr, c->scr_stride);

@@ -142,7 +142,7 @@ static int run_el_staged(champ_ctx *c, const State<T> &st, bool outputs, bool st
     else k_el_jas<T, NORD><<<(W + w0 - 1) / w0, 32 * w0, c->el_smem[0], c->stream>>>(s, st);
     if (rc) return rc;
     CK(cudaGetLastError());
-    if (c->orb_nt) {
+    if (c->orb_tile) {
       rc = el_tile_orb(c, st);
     } else {
       const long long items = (long long)W * c->N;

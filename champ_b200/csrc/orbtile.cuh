@@ -2,7 +2,6 @@
 // staged evaluation, as FP64 tensor-core products, and the Slater-matrix inversion in registers.
 #pragma once
 #include "kernels.cuh"
-#include "shelltab.cuh"
 
 namespace ot {
 
@@ -17,49 +16,43 @@ __host__ __device__ constexpr int ldb() { return 16 * NT + 4; }
 template <int NT>
 __host__ __device__ constexpr size_t smem_bytes() { return sizeof(double) * (size_t)KB * (LDA + ldb<NT>()); }
 
-// A Gaussian shell with n = l + 1, l <= 2: S_lm(d) g(r^2), no square root or division.
-template <int l, class Put>
-__device__ __forceinline__ void gauss_shell5(const stab::Rad &R, double d0, double d1, double d2, Put put) {
-  double S[9], G[9][3];
-  solid_all<double, true>(l, d0, d1, d2, S, G);
-#pragma unroll
-  for (int sl = 0; sl < 2 * l + 1; sl++) {
-    const double st = S[sl] * R.t;
-    put(sl, 0, S[sl] * R.q);
-    put(sl, 1, G[sl][0] * R.q + st * d0);
-    put(sl, 2, G[sl][1] * R.q + st * d1);
-    put(sl, 3, G[sl][2] * R.q + st * d2);
-    put(sl, 4, S[sl] * R.lap);
-  }
-}
-
-// Any other shell (kept out of line: its registers are not those of the contraction).
-static __device__ __noinline__ void general_shell5(const Sys<double> &s, int ish, double x, double y, double z, double *o) {
+// A shell's functions of one electron (out of line: its registers are not those of the contraction, and the
+// compiler fuses the same products with their sums as in warp_basis).
+static __device__ __noinline__ void shell5(const Sys<double> &s, int ish, double x, double y, double z, double *o) {
   const double pt[3] = {x, y, z};
   shell_eval_put<double, 5>(s, ish, pt, [o](int sl, int c, double v) { o[sl * LDA + c * EB] = v; });
 }
 
-// Orbitals of 32 electrons of one spin (grid.y) per block: chunks of basis functions are formed in
+// Orbitals of 32 electrons of one spin (sp0 + blockIdx.y) per block: chunks of basis functions are formed in
 // shared memory (lane = electron, a warp per shell, so that every lane runs the same shell) and
 // contracted with the spin's coefficients by mma m8n8k4: 160 rows (5 channels x 32 electrons) by
 // 16 NT orbitals, 8 warps as 4 (rows) x 2 (orbitals), 5 x NT tiles each.  The coefficients of a
 // chunk arrive by cp.async while its basis functions are formed and are shared by the 32
 // electrons (the warp-per-electron contraction streamed them from L2 once per 4 electrons).
-// What bounds it: the FP64 pipe (about a fifth of it the basis functions).  Measured (B200): 4096
-// walkers of 128 electrons, 416 basis functions, 15.6 -> 6.0 ms; 3001 of 20 electrons, 65 functions,
-// 0.32 -> 0.06 ms.  k_el_orb stays for more than 64 orbitals of a spin.
+// The rows are those of warp_basis and warp_orbitals to the last bit: the same basis functions, and the mma
+// adds its four products in order, each by a fused multiply-add, so an orbital is summed over b as there --
+// in order above 16 orbitals, in LB interleaved sums and their pairwise tree up to 16 (SPLIT = LB).  It has to
+// be so: where psi nearly vanishes the inverse magnifies the last bit of a row by the condition number (ratios
+// of an 80-electron cluster's first moves then differ by 3e-9), and the accelerated mover, whose proposals follow
+// the drift, magnifies it again with every sweep (its walks came apart).
+// What bounds it: the FP64 pipe (about a third of it the basis functions).  Measured (B200): 4096
+// walkers of 128 electrons, 416 basis functions, 15.6 -> 9.2 ms; 1001 of 51 electrons 1.25 -> 0.59; 3001 of 20 electrons, 65
+// functions, 0.32 -> 0.27.  Basis functions by shelltab.cuh's exponential and formulas took 6.0, 0.33 and 0.13 ms,
+// and split the walks; so does shell5 inlined (8.1 ms; other products are then fused with their sums).
+// k_el_orb stays for more than 64 orbitals of a spin, and for one or two (32 or 16 interleaved sums each).
 // chunk[k]: first shell, shells, first basis function, basis functions.
-// GEN: shells other than those Gaussians occur.
 // ALL: the columns blockIdx.y * 16 NT onwards of all orbitals (s.call), for every electron, into all + w
 // stride as [N][5][norb] instead, without the Slater matrices.
-template <int NT, bool ALL, bool GEN>
+template <int NT, int SPLIT, bool ALL>
 __global__ void __launch_bounds__(THREADS, 2) k_orb_tile(const __grid_constant__ Sys<double> s, State<double> st, const int4 *chunk, int nchunk,
-                                                         double *all, size_t stride) {
+                                                         int sp0, double *all, size_t stride) {
+  static_assert(SPLIT == 1 || (NT == 1 && !ALL), "interleaved sums: up to 16 orbitals");
   extern __shared__ __align__(16) double sm[];
-  const stab::Tab T = stab::stage(s, sm + KB * (LDA + ldb<NT>()));
   double *phi = sm, *cf = sm + KB * LDA;
   constexpr int LDB = ldb<NT>();
-  const int sp = ALL ? 0 : blockIdx.y, n = ALL ? s.N : (sp ? s.ndn : s.nup), e0 = sp ? s.nup : 0;
+  // sums of a warp: above 8 orbitals both warps of a row tile hold all of theirs, below they share them
+  constexpr int NS = SPLIT <= 2 ? SPLIT : SPLIT / 2;
+  const int sp = ALL ? 0 : sp0 + blockIdx.y, n = ALL ? s.N : (sp ? s.ndn : s.nup), e0 = sp ? s.nup : 0;
   const int col0 = ALL ? (int)blockIdx.y * 16 * NT : 0, ld = ALL ? s.norb : s.nocc[sp], no = ld - col0;
   const long long items = (long long)st.W * n, i0 = (long long)blockIdx.x * EB;
   if (i0 >= items) return;
@@ -75,12 +68,11 @@ __global__ void __launch_bounds__(THREADS, 2) k_orb_tile(const __grid_constant__
     px[0] = x[0]; px[1] = x[1]; px[2] = x[2];
   }
   const bool vec = ld % 2 == 0 && (reinterpret_cast<uintptr_t>(coef) & 15) == 0;
-  double acc[5][NT][2];
+  double acc[5][NT * NS][2];
 #pragma unroll
   for (int i = 0; i < 5; i++)
 #pragma unroll
-    for (int j = 0; j < NT; j++) acc[i][j][0] = acc[i][j][1] = 0;
-  __syncthreads();  // the shell tables are in place
+    for (int j = 0; j < NT * NS; j++) acc[i][j][0] = acc[i][j][1] = 0;
   for (int k = 0; k < nchunk; k++) {
     const int4 ch = chunk[k];
     const int nk4 = (ch.w + 3) & ~3;
@@ -105,35 +97,67 @@ __global__ void __launch_bounds__(THREADS, 2) k_orb_tile(const __grid_constant__
       for (int c = 0; c < 5; c++) phi[r * LDA + c * EB + lane] = 0.0;
     for (int q = wib; q < ch.y; q += 8) {
       const int ish = ch.x + q;
-      const ShellRec h = T.rec[ish];
-      double *o = phi + (h.b0 - ch.z) * LDA + lane;
-      auto put = [o](int sl, int c, double v) { o[sl * LDA + c * EB] = v; };
-      if (GEN && (h.kind != 1 || h.l > 2)) {
-        general_shell5(s, ish, px[0], px[1], px[2], o);
-      } else {
-        const double *cc = s.cent + 3 * h.cen;
-        const double d0 = px[0] - cc[0], d1 = px[1] - cc[1], d2 = px[2] - cc[2];
-        const stab::Rad R = stab::gauss_rad(T, h, d0 * d0 + d1 * d1 + d2 * d2);
-        if (h.l == 0) gauss_shell5<0>(R, d0, d1, d2, put);
-        else if (h.l == 1) gauss_shell5<1>(R, d0, d1, d2, put);
-        else gauss_shell5<2>(R, d0, d1, d2, put);
-      }
+      shell5(s, ish, px[0], px[1], px[2], phi + (s.shb0[ish] - ch.z) * LDA + lane);
     }
     cp_async_wait<0>();
     __syncthreads();
-    const double *ap = phi + kq * LDA + wm * 40 + rr, *bp = cf + kq * LDB + wn * 8 * NT + rr;
-    for (int ks = 0; ks < nk4; ks += 4) {
-      double a[5], b[NT];
+    if constexpr (SPLIT == 1) {
+      const double *ap = phi + kq * LDA + wm * 40 + rr, *bp = cf + kq * LDB + wn * 8 * NT + rr;
+      for (int ks = 0; ks < nk4; ks += 4) {
+        double a[5], b[NT];
 #pragma unroll
-      for (int i = 0; i < 5; i++) a[i] = ap[ks * LDA + 8 * i];
+        for (int i = 0; i < 5; i++) a[i] = ap[ks * LDA + 8 * i];
 #pragma unroll
-      for (int j = 0; j < NT; j++) b[j] = bp[ks * LDB + 8 * j];
+        for (int j = 0; j < NT; j++) b[j] = bp[ks * LDB + 8 * j];
 #pragma unroll
-      for (int i = 0; i < 5; i++)
+        for (int i = 0; i < 5; i++)
 #pragma unroll
-        for (int j = 0; j < NT; j++) dmma_884(acc[i][j][0], acc[i][j][1], a[i], b[j]);
+          for (int j = 0; j < NT; j++) dmma_884(acc[i][j][0], acc[i][j][1], a[i], b[j]);
+      }
+    } else {
+      // sum q takes the basis functions b = q mod SPLIT, four of them to an mma (zeros past the chunk)
+      const double *ap = phi + wm * 40 + rr, *bp = cf + (SPLIT == 2 ? 8 * wn : 0) + rr;
+      const int q0 = SPLIT == 2 ? 0 : NS * wn;
+#pragma unroll
+      for (int j = 0; j < NS; j++) {
+        const int r0 = (q0 + j - ch.z) & (SPLIT - 1);
+        for (int t = r0; t < ch.w; t += 4 * SPLIT) {
+          const int r = t + SPLIT * kq;
+          const bool in = r < ch.w;
+          const double b = in ? bp[r * LDB] : 0.0;
+#pragma unroll
+          for (int i = 0; i < 5; i++) dmma_884(acc[i][j][0], acc[i][j][1], in ? ap[r * LDA + 8 * i] : 0.0, b);
+        }
+      }
     }
     __syncthreads();
+  }
+  // the interleaved sums by their pairwise tree; the second half of them from the other warp of the row tile
+  if constexpr (SPLIT > 1) {
+#pragma unroll
+    for (int i = 0; i < 5; i++)
+#pragma unroll
+      for (int h = 0; h < 2; h++)
+#pragma unroll
+        for (int d = 1; d < NS; d <<= 1)
+#pragma unroll
+          for (int j = 0; j < NS; j += 2 * d) acc[i][j][h] += acc[i][j + d][h];
+    if constexpr (SPLIT > 2) {
+      double *ex = sm + (size_t)(32 * wm + lane) * 10;
+      if (wn == 1)
+#pragma unroll
+        for (int i = 0; i < 5; i++) {
+          ex[2 * i] = acc[i][0][0];
+          ex[2 * i + 1] = acc[i][0][1];
+        }
+      __syncthreads();
+      if (wn == 1) return;
+#pragma unroll
+      for (int i = 0; i < 5; i++) {
+        acc[i][0][0] += ex[2 * i];
+        acc[i][0][1] += ex[2 * i + 1];
+      }
+    }
   }
   const int nomax = s.nomax;
 #pragma unroll

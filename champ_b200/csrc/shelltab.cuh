@@ -59,7 +59,7 @@ static __device__ __noinline__ double general_radial(const Sys<double> &s, int i
 // the second of a pair).  Two primitives at a time: an exponential is a chain of ten dependent FP64
 // operations, and the callers have too few warps in flight to fill it.  Small walkers' evaluation 0.97 -> 0.91 ms
 // (8192 of 8 electrons), their DMC step 3.28 -> 3.18 ms; the projected points of 3001 walkers of 20 electrons
-// 0.53 -> 0.52 ms.  At 128 electrons, where other warps fill it already: orbital rows 6.09 -> 6.04 ms.
+// 0.53 -> 0.52 ms.
 __device__ __forceinline__ double gauss_radial(const Tab &T, const ShellRec &h, double r2) {
   double g = 0;
   int p = h.p0;

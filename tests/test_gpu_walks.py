@@ -1,0 +1,123 @@
+"""Walks whose every step depends on the last bits of the one before.
+
+Where psi nearly vanishes the inverse Slater matrix magnifies a rounding of the orbital rows by the matrix's
+condition number, and the accelerated mover, whose proposals follow the drift, magnifies it again with every
+sweep: two orders of the same sums walk apart within a few sweeps of a large molecule.  The tiled evaluation
+therefore forms the rows and inverses that the moves start from to the bits of the warp-per-electron
+kernels.  These tests hold it to that: against ratios and walks recorded from those kernels, and against
+the oracle as far as the walk itself allows.  (The recordings are the walks of commit 305d744 on a B200.)"""
+import dataclasses
+import os
+
+import numpy as np
+import pytest
+
+from champ_b200 import system as S
+
+pytestmark = pytest.mark.gpu
+
+GOLDEN = os.path.join(os.path.dirname(__file__), "golden", "accelerated_walks.npz")
+
+
+def cluster(n, nup, ncent, nordc):
+    s = S.cluster128(ncent=ncent, box=14.0 * (max(ncent, 4) / 32) ** (1 / 3), norb=max(nup, n - nup))
+    j = S._jastrow(np.random.default_rng(3), 1, 5, 5, nordc)
+    return dataclasses.replace(s, nelec=n, nup=nup, nordc=nordc, een_cusp=j["een_cusp"], c=j["c"],
+                               det_orb=np.array([list(range(nup)) + list(range(n - nup))], np.int32))
+
+
+# electrons, up electrons, centres, e-e-n order: 3 to 64 orbitals of a spin, in and across the classes of
+# interleaved sums (up to 16) and of tiles of 32 electrons
+SHAPES = [(12, 9, 6, 0), (13, 8, 3, 4), (13, 9, 3, 4), (17, 9, 3, 4), (26, 16, 5, 5), (34, 17, 9, 4), (65, 33, 17, 4),
+          (80, 40, 20, 4), (128, 64, 32, 4)]
+
+
+def ratios(shape, idx=None):
+    """Ratios and gradients of three electrons' moves from 8 unequilibrated walkers (of 400: those of idx, or with
+    the largest drifts, whose psi nearly vanishes)."""
+    from champ_b200.engine import Engine
+    n, nup = shape[:2]
+    s = cluster(*shape)
+    x = S.initial_walkers(s, 400, seed=n + nup)
+    dx = s.step * np.random.default_rng(n).standard_normal((n, 400, 3))
+    if idx is None:
+        eng = Engine(s, 400, "fp64")
+        eng.set_walkers(x)
+        idx = np.argsort(-np.abs(eng.eval_full()["velocity"]).max(axis=(1, 2)))[:8]
+        eng.close()
+    eng = Engine(s, len(idx), "fp64")
+    assert eng.get_option("staged_eval")
+    eng.set_walkers(x[idx])
+    out = [eng.propose_1e(e, np.ascontiguousarray(x[idx, e] + dx[e, idx]), grad=True) for e in (0, nup - 1, n - 1)]
+    eng.close()
+    return idx, np.array([r for r, _ in out]), np.array([g for _, g in out])
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_ratios_as_recorded(shape):
+    """The rows and inverses are those recorded, so a ratio differs by the rounding of its N + C Jastrow terms
+    (2e-14 for the largest molecule), a gradient not even by that."""
+    ref = np.load(GOLDEN)
+    key = "ratio_%d_%d_" % shape[:2]
+    _, r, g = ratios(shape, ref[key + "idx"])
+    assert np.all(np.abs(r - ref[key + "r"]) <= 1e-13 * np.abs(ref[key + "r"]))
+    assert np.all(np.abs(g - ref[key + "g"]) <= 1e-13 * np.abs(ref[key + "g"]).max(axis=2, keepdims=True))
+
+
+RECORDED = [(9, 5, 2, 4, "fp64"), (13, 9, 3, 4, "fp64"), (20, 10, 5, 5, "fp64"), (34, 17, 9, 4, "fp64"), (51, 26, 13, 5, "fp64"),
+            (128, 64, 32, 4, "fp64"), (34, 17, 9, 4, "mixed"), (128, 64, 32, 4, "mixed")]
+
+
+def accelerated_walk(case):
+    from champ_b200.engine import Engine
+    s = cluster(*case[:4])
+    eng = Engine(s, 3, case[4])
+    eng.set_walkers(S.initial_walkers(s, 3, seed=case[0]))
+    eng.set_mover(6)
+    st = eng.vmc_sweeps(4, seed=31, sweep0=2, step=s.step)
+    x = eng.get_walkers()
+    eng.close()
+    return x, st["accept"]
+
+
+@pytest.mark.parametrize("case", RECORDED)
+def test_accelerated_walk_as_recorded(case):
+    """Four accelerated sweeps against the positions recorded from the evaluation by a warp per walker and
+    electron.  Rounding alone takes the largest molecule's electrons 1e-2 bohr apart in as many sweeps."""
+    x, accept = accelerated_walk(case)
+    ref = np.load(GOLDEN)
+    key = "%d_%d_%s" % (case[0], case[3], case[4])
+    assert np.abs(x - ref[key]).max() <= 1e-12
+    assert np.array_equal(accept, ref[key + "_accept"])
+
+
+@pytest.mark.parametrize("n,nup,ncent,nordc", [(24, 13, 6, 5), (40, 20, 10, 4)])
+def test_accelerated_sweep_follows_the_oracle(oracle_mod, n, nup, ncent, nordc):
+    """One accelerated sweep of equilibrated walkers in HBM, electron by electron, against the oracle.  How far
+    the two may come apart is the walk's own: the oracle's sweeps from positions moved by 1e-13 bohr (rounding
+    of a 10-bohr coordinate is 1e-15, of the drift 1e-15 of it) show its magnification, electron by electron."""
+    from champ_b200.engine import Engine
+    s = cluster(n, nup, ncent, nordc)
+    nw = 4
+    eng = Engine(s, nw, "fp64")
+    eng.set_walkers(S.initial_walkers(s, nw, seed=n))
+    eng.vmc_sweeps(20, seed=3, sweep0=0, step=s.step, stats=False)
+    x = eng.get_walkers()
+    eng.set_walkers(x)
+    eng.set_mover(6, deltar=5.0, deltat=1.0, fbias=1.0)
+    st = eng.vmc_sweeps(1, seed=777, sweep0=0, step=0.5)
+    xg = eng.get_walkers()
+    eng.close()
+    orc = oracle_mod.Oracle(s)
+    run = lambda y: orc.vmc_accel(y, 1, seed=777, sweep0=0, deltar=5.0, deltat=1.0, fbias=1.0, nthreads=4)  # noqa: E731
+    ref = run(x)
+    rng = np.random.default_rng(n)
+    grown = np.zeros((nw, n))
+    for _ in range(3):
+        grown = np.maximum(grown, np.abs(run(x + 1e-13 * rng.choice([-1.0, 1.0], x.shape))["x"] - ref["x"]).max(axis=2))
+    # an electron's magnification, with those moved before it
+    bound = 10 * np.maximum.accumulate(grown, axis=1) + 1e-12
+    d = np.abs(xg - ref["x"]).max(axis=2)
+    print(f"{n} electrons: first {d[:, 0].max():.1e}, all {d.max():.1e} bohr; allowed {bound[:, 0].max():.1e} {bound.max():.1e}")
+    assert np.all(d <= bound)
+    assert np.array_equal(st["accept"], ref["accept"])
