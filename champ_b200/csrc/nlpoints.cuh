@@ -116,7 +116,7 @@ struct Tab {
 // Shared memory of a walker (doubles): scaled distances [Ct][Np], positions, V_k [NORD][N], per-centre
 // sums [NORD - 1][C], rows of the pair table summed [N], the tasks' radial values [nrow], reductions,
 // per 32 (electron, centre) pairs the mask of those in range and the number in range before them, and
-// (lane) the distances of lane_jastrow.
+// (lane) the distances of lane_jastrow; and per electron what the velocities add to the energy [2][N].
 struct Dims {
   int N, C, Ct, Np, nord, nrow, lane;
   __host__ __device__ Dims(int N_, int C_, int nord_, int nrow_, bool lane_ = false)
@@ -132,7 +132,8 @@ struct Dims {
   __host__ __device__ int red() const { return row() + nrow; }
   __host__ __device__ int msk() const { return red() + 32; }
   __host__ __device__ int lanes() const { return msk() + (N * C + 31) / 32 + 1; }
-  __host__ __device__ int total() const { return lanes() + (lane ? 32 * C : 0); }
+  __host__ __device__ int vel() const { return lanes() + (lane ? 32 * C : 0); }
+  __host__ __device__ int total() const { return vel() + 2 * N; }
   __host__ __device__ size_t bytes() const { return sizeof(double) * (size_t)((total() + 1) & ~1); }
 };
 
@@ -471,7 +472,7 @@ __global__ void __launch_bounds__(WPW == 8 ? 256 : 128, WPW == 8 ? 2 : WPW == 4 
   const stab::Tab T = stab::stage(s, dsm);
   __syncthreads();
   double *sm = (double *)(dsm + stab::tab_smem(s.nshell, s.nprim) + (WPW == 1 ? D.bytes() * wib : 0));
-  double *sd = sm, *xs = sm + D.x(), *V = sm + D.v(), *Z = sm + D.z(), *F = sm + D.f(), *row = sm + D.row(), *red = sm + D.red();
+  double *sd = sm, *xs = sm + D.x(), *V = sm + D.v(), *Z = sm + D.z(), *F = sm + D.f(), *row = sm + D.row(), *red = sm + D.red(), *vel = sm + D.vel();
   for (int w = blockIdx.x * per + (WPW == 1 ? wib : 0); w < st.W; w += gridDim.x * per) {
     View<double> v{};
     v.xs = xs;
@@ -499,33 +500,43 @@ __global__ void __launch_bounds__(WPW == 8 ? 256 : 128, WPW == 8 ? 2 : WPW == 4 
     const bool points = s.nloc > 0 && ok && !tables_only;
     double d2lnd = 0, v2 = 0, vloc = 0, vnl = 0;
     if (!tables_only) {
-      // velocities: 8 lanes per electron (det_velocities)
+      // velocities: 8 lanes per electron, the sums in the order of det_velocities (a lane's orbitals are those of
+      // 4 lanes there).  Near a node grad psi / psi and lap psi / psi grow as 1 / d and their squares cancel in
+      // E_L, which keeps the last bits of these sums: in another order the energies of a few thousand
+      // unequilibrated walkers differed by 1e-8.
       for (int e4 = 4 * wpos; e4 < N; e4 += 4 * WPW) {
         const int e = e4 + (lane >> 3), l8 = lane & 7;
-        double g0 = 0, g1 = 0, g2 = 0, lp = 0;
-        if (e < N) {
-          const int sp = e < s.nup ? 0 : 1, n = sp ? s.ndn : s.nup, eo = sp ? e - s.nup : e;
-          const double *G = gam_ptr<double, MD>(s, v, sp), *oe = v.orb5 + (size_t)e * 5 * nomax;
-          for (int k = l8; k < s.nocc[sp]; k += 8) {
-            const double a = G[k * n + eo];
-            g0 += a * oe[nomax + k];
-            g1 += a * oe[2 * nomax + k];
-            g2 += a * oe[3 * nomax + k];
-            lp += a * oe[4 * nomax + k];
-          }
-        }
+        double q[4][4];
 #pragma unroll
-        for (int o = 1; o <= 4; o <<= 1) {
-          g0 += __shfl_xor_sync(0xffffffffu, g0, o);
-          g1 += __shfl_xor_sync(0xffffffffu, g1, o);
-          g2 += __shfl_xor_sync(0xffffffffu, g2, o);
-          lp += __shfl_xor_sync(0xffffffffu, lp, o);
+        for (int c = 0; c < 4; c++)
+#pragma unroll
+          for (int i = 0; i < 4; i++) q[c][i] = 0;
+        if (e < N) {
+          const int sp = e < s.nup ? 0 : 1, n = sp ? s.ndn : s.nup, eo = sp ? e - s.nup : e, no = s.nocc[sp];
+          const double *G = gam_ptr<double, MD>(s, v, sp), *oe = v.orb5 + (size_t)e * 5 * nomax;
+          for (int k0 = l8; k0 < no; k0 += 32)
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+              const int k = k0 + 8 * i;
+              if (k < no) {
+                const double a = G[k * n + eo];
+#pragma unroll
+                for (int c = 0; c < 4; c++) q[c][i] += a * oe[(c + 1) * nomax + k];
+              }
+            }
+        }
+        double g[4];
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+          g[c] = (q[c][0] + q[c][2]) + (q[c][1] + q[c][3]);
+#pragma unroll
+          for (int o = 4; o >= 1; o >>= 1) g[c] += __shfl_xor_sync(0xffffffffu, g[c], o);
         }
         if (e < N && l8 == 0) {
-          const double dvd = lp - (g0 * g0 + g1 * g1 + g2 * g2);
-          const double vx = v.vacc[3 * e] + g0, vy = v.vacc[3 * e + 1] + g1, vz = v.vacc[3 * e + 2] + g2;
-          d2lnd += dvd;
-          v2 += vx * vx + vy * vy + vz * vz;
+          const double dvd = g[3] - (g[0] * g[0] + g[1] * g[1] + g[2] * g[2]);
+          const double vx = v.vacc[3 * e] + g[0], vy = v.vacc[3 * e + 1] + g[1], vz = v.vacc[3 * e + 2] + g[2];
+          vel[e] = dvd;
+          vel[N + e] = vx * vx + vy * vy + vz * vz;
           if (outputs) {
             double *ov = st.o_vel + ((size_t)w * N + e) * 3;
             ov[0] = vx; ov[1] = vy; ov[2] = vz;
@@ -670,26 +681,28 @@ __global__ void __launch_bounds__(WPW == 8 ? 256 : 128, WPW == 8 ? 2 : WPW == 4 
         if (tape.b) tape.b[(size_t)w * tape.bstride + t] = cb;
       }
     }
-    d2lnd = warp_sum(d2lnd);
-    v2 = warp_sum(v2);
     vloc = warp_sum(vloc);
     vnl = warp_sum(vnl);
     if (WPW > 1) {
       __syncthreads();
       if (lane == 0) {
-        double *o = red + 4 * wpos;  // the task counts and the rotation are no longer read
-        o[0] = d2lnd; o[1] = v2; o[2] = vloc; o[3] = vnl;
+        double *o = red + 2 * wpos;  // the task counts and the rotation are no longer read
+        o[0] = vloc; o[1] = vnl;
       }
       __syncthreads();
-      d2lnd = v2 = vloc = vnl = 0;
+      vloc = vnl = 0;
       for (int k = 0; k < WPW; k++) {
-        d2lnd += red[4 * k];
-        v2 += red[4 * k + 1];
-        vloc += red[4 * k + 2];
-        vnl += red[4 * k + 3];
+        vloc += red[2 * k];
+        vnl += red[2 * k + 1];
       }
+    } else {
+      __syncwarp();
     }
     if (wpos == 0) {
+      for (int e = 0; e < N && !tables_only; e++) {  // in det_velocities' order, too
+        d2lnd += vel[e];
+        v2 += vel[N + e];
+      }
       EvalRes res;
       finish_eval(s, st, w, v, lane, outputs != 0, ok, lnd, sgn, sc[0], sc[1], sc[2], sc[3], d2lnd, v2, vloc, vnl, ntask, res);
       if (stats && lane == 0) {
