@@ -248,10 +248,10 @@ int pg_tile_fwd(champ_ctx *c);
 int pg_tile_bwd(champ_ctx *c);
 // small walkers (small.cu); setup sets champ_ctx::small where they apply, small_serves adds the rule on the
 // number of walkers
-enum class SmallOp { Eval, Gauss, Accel, Dmc };
+enum class SmallOp { Eval, Gauss, Dmc };
 int small_setup(champ_ctx *c);
 bool small_serves(const champ_ctx *c, SmallOp op, int W);
-int small_eval(champ_ctx *c, const State<double> &st, bool outputs, bool stats, const ElRot &rot);
+int small_eval(champ_ctx *c, const State<double> &st, const ElRot &rot);
 int small_vmc(champ_ctx *c, const State<double> &st, const OpArgs &a);
 int small_dmc(champ_ctx *c, const State<double> &st, bool moves);
 int small_tmove(champ_ctx *c, const State<double> &st, const OpArgs &a);

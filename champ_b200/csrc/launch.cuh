@@ -184,12 +184,6 @@ static int launch_t(champ_ctx *c, Op op, const OpArgs &a) {
       return run_el_staged<T, NORD, MD>(c, st, op == Op::EvalOut, false, rot, a.rebuild);
     }
     c->orb5_valid = false;
-    if constexpr (std::is_same<T, double>::value)
-      if (!a.st_override && small_serves(c, SmallOp::Eval, st.W)) {
-        ElRot rot{};
-        for (int i = 0; i < 9; i++) rot.R[i] = R[i];
-        return small_eval(c, st, op == Op::EvalOut, false, rot);
-      }
     if (tc) {
       int rc = run_orb_tc<T>(c, st);
       if (rc) return rc;
@@ -250,12 +244,12 @@ static int launch_t(champ_ctx *c, Op op, const OpArgs &a) {
       return run_el_staged<T, NORD, MD>(c, st, false, true, rot);
     }
     if constexpr (std::is_same<T, double>::value)
-      if (!a.st_override && a.phase == 3 && small_serves(c, SmallOp::Eval, st.W)) {
+      if (!a.st_override && a.phase == 3 && c->mover.kind != 6 && small_serves(c, SmallOp::Eval, st.W)) {
         ElRot rot{};
         rot.random = 1;
         rot.seed = a.seed;
         rot.sweep = a.sweep0;
-        return small_eval(c, st, false, true, rot);
+        return small_eval(c, st, rot);
       }
     if (a.phase >= 0) {
       const bool acc6 = c->mover.kind == 6;
@@ -295,7 +289,7 @@ static int launch_t(champ_ctx *c, Op op, const OpArgs &a) {
     }
     CK(cudaMemsetAsync(st.s_esum, 0, sizeof(double) * 3 * (size_t)c->wmax, c->stream));  // esum, e2sum, acc
     if constexpr (std::is_same<T, double>::value)
-      if (!a.st_override && small_serves(c, c->mover.kind == 6 ? SmallOp::Accel : SmallOp::Gauss, st.W)) return small_vmc(c, st, a);
+      if (!a.st_override && c->mover.kind != 6 && small_serves(c, SmallOp::Gauss, st.W)) return small_vmc(c, st, a);
     const bool tc = c->tc_on && !a.st_override;  // only FP32 contexts turn it on
     if (!tc) {
       auto kern = c->mover.kind == 6 ? k_vmc<T, NORD, MD, 0, 6> : k_vmc<T, NORD, MD, 0>;

@@ -16,8 +16,8 @@ template <int NORD>
 int attrs(const champ_ctx *c) {
   const size_t b = sizeof(double) * (size_t)sm::Lay(c->N, c->C, c->nordc).total() * 16 + stab::tab_smem(c->sd.nshell, c->sd.nprim);
   int rc = CHAMP_OK;
-  for (auto k : {sm::k_small<NORD, sm::EVAL>, sm::k_small<NORD, sm::GAUSS>, sm::k_small<NORD, sm::ACCEL>, sm::k_small<NORD, sm::DMC>,
-                 sm::k_small<NORD, sm::DMC_EL>, sm::k_small_tmove<NORD>})
+  for (auto k : {sm::k_small<NORD, sm::EVAL>, sm::k_small<NORD, sm::GAUSS>, sm::k_small<NORD, sm::DMC>, sm::k_small<NORD, sm::DMC_EL>,
+                 sm::k_small_tmove<NORD>})
     if (!rc) rc = big_smem(k, b);
   return rc;
 }
@@ -38,7 +38,6 @@ int run(champ_ctx *c, const State<double> &st, int mode, const sm::Args &A, int 
   switch (mode) {
   case sm::EVAL: sm::k_small<NORD, sm::EVAL><<<g, t, smem, c->stream>>>(c->sd, st, A); break;
   case sm::GAUSS: sm::k_small<NORD, sm::GAUSS><<<g, t, smem, c->stream>>>(c->sd, st, A); break;
-  case sm::ACCEL: sm::k_small<NORD, sm::ACCEL><<<g, t, smem, c->stream>>>(c->sd, st, A); break;
   case sm::DMC: sm::k_small<NORD, sm::DMC><<<g, t, smem, c->stream>>>(c->sd, st, A); break;
   case sm::DMC_EL: sm::k_small<NORD, sm::DMC_EL><<<g, t, smem, c->stream>>>(c->sd, st, A); break;
   default: sm::k_small_tmove<NORD><<<g, t, smem, c->stream>>>(c->sd, st, A);
@@ -78,24 +77,27 @@ int small_setup(champ_ctx *c) {
 // of 8 electrons, calls of 2 sweeps or 4 steps, us here against a warp per walker):
 //   evaluation      2400 walkers 1325 / 1084, 3600 1492 / 1395, 8192 with mixed-precision sweeps 2790 / 3100;
 //   Gaussian moves  1800 1142 / 1035, 2400 1250 / 1379;
-//   accelerated     250 1439 / 1098, 600 1461 / 1691 and 1539 / 1684;
 //   DMC, T-moves    1800 2776 / 2571 and 2351 / 2294, 2400 2834 / 4399 and 2557 / 3881; T-moves 1800 5758 / 4956 and
 //                   5234 / 6122, 2400 5946 / 7552 and 5448 / 9157 (a warp per walker holds 16 per SM at once).
 // Without a pseudopotential there are no points: Gaussian moves of the Be-like atom 120 / 139 at 60 walkers,
 // 154 / 276 at 2400.
+// Two uses stay with a warp per walker for their bits, not for their time.  Accelerated sweeps, and the E_L after
+// them: a proposal follows the drift, so a walk magnifies the rounding of its sums -- of 8192 walkers of the dimer,
+// after four sweeps, the worst electron by up to 6e-3 bohr between the two kernels (C2: 4e-10); 8.0 against
+// 2.6 ms for a sweep of 8192 of C2.  And evaluations of walkers that a caller supplies: near a node the inverse magnifies
+// the rounding of its rows (drifts of 8192 unequilibrated walkers to 5e-11), and the moves start from it.
 bool small_serves(const champ_ctx *c, SmallOp op, int W) {
   if (!c->small) return false;
   if (c->nloc == 0 && op == SmallOp::Gauss) return true;
   const int sm = c->num_sms > 0 ? c->num_sms : 148;
-  const int per = op == SmallOp::Eval ? 32 : op == SmallOp::Gauss ? 14 : op == SmallOp::Accel ? 4 : 16;
+  const int per = op == SmallOp::Eval ? 32 : op == SmallOp::Gauss ? 14 : 16;
   return W > per * sm;
 }
 
-int small_eval(champ_ctx *c, const State<double> &st, bool outputs, bool stats, const ElRot &rot) {
+// the E_L after a sweep of Gaussian moves, and its statistics
+int small_eval(champ_ctx *c, const State<double> &st, const ElRot &rot) {
   sm::Args A;
   A.order = c->small_order;
-  A.outputs = outputs;
-  A.stats = stats;
   A.rot = rot;
   return run(c, st, sm::EVAL, A, st.W);
 }
@@ -106,8 +108,7 @@ int small_vmc(champ_ctx *c, const State<double> &st, const OpArgs &a) {
   A.seed = a.seed;
   A.sweep0 = a.sweep0;
   A.step = a.step;
-  A.mv = c->mover;
-  return run(c, st, c->mover.kind == 6 ? sm::ACCEL : sm::GAUSS, A, st.W);
+  return run(c, st, sm::GAUSS, A, st.W);
 }
 int small_dmc(champ_ctx *c, const State<double> &st, bool moves) {
   sm::Args A;

@@ -16,8 +16,9 @@
 // filled the evaluation's chains (0.91 -> 0.90 ms) but spilled in the DMC step (3.18 -> 3.33 ms).
 // A single walker takes longer on 8 lanes than on 32, so few walkers stay with a warp each (small_serves).
 // Measured (B200) against a warp per walker: dimer of 8 electrons, order 4, 8192 walkers, evaluation
-// 1.04 -> 0.90 ms; DMC step of about the same population 10.0 -> 3.2 ms; C2, order 5, the accelerated
-// moves and their evaluations 9.6 -> 2.1 ms, DMC step 1.33 -> 0.69 ms, T-moves 1.28 -> 0.82 ms.
+// 1.04 -> 0.90 ms; DMC step of about the same population 10.0 -> 3.2 ms; C2, order 5, DMC step 1.33 -> 0.69 ms,
+// T-moves 1.28 -> 0.82 ms.  Accelerated sweeps, which follow the last bit of the drift, and evaluations of walkers
+// that a caller supplies stay with a warp per walker (small_serves).
 #pragma once
 #include "jastile.cuh"
 
@@ -53,10 +54,9 @@ struct Lay {
 };
 
 struct Args {
-  int nsweep = 1, outputs = 0, stats = 0;
+  int nsweep = 1;
   uint64_t seed = 0, sweep0 = 0;
   double step = 0;
-  Mover mv{1, 5.0, 1.0, 1.0};
   ElRot rot{};
   const int *order = nullptr;  // shells by l, so that the lanes of a round mostly share it
   DmcPar P{};
@@ -620,7 +620,7 @@ struct Res {
 };
 template <int NORD>
 __device__ __forceinline__ Res evaluate(const Sys<double> &s, const stab::Tab &T, const JasPar<double> &J, const EcpPar &E, const State<double> &st,
-                                        int w, double *v, const Lay &L, const ElRot &rot, bool outputs) {
+                                        int w, double *v, const Lay &L, const ElRot &rot) {
   const int sub = threadIdx.x & 7, N = s.N, C = s.C;
   const unsigned m = gmask();
   const double sk = J.scalek;
@@ -628,7 +628,7 @@ __device__ __forceinline__ Res evaluate(const Sys<double> &s, const stab::Tab &T
   invert(s, v, L, lnd, sgn);
   const bool ok = sgn != 0.0;
   // ---- distances and power sums, lane = electron
-  double pe_en = 0, fen = 0, div = 0, vj[3] = {0, 0, 0}, d2j = 0, pe_ee = 0, fsum = 0;
+  double pe_en = 0, fen = 0, vj[3] = {0, 0, 0}, d2j = 0, pe_ee = 0, fsum = 0;
   const bool act = sub < N;
   const int i = act ? sub : 0;
   const double xi[3] = {v[3 * i], v[3 * i + 1], v[3 * i + 2]};
@@ -646,7 +646,7 @@ __device__ __forceinline__ Res evaluate(const Sys<double> &s, const stab::Tab &T
       vj[0] += fi * dx;
       vj[1] += fi * dy;
       vj[2] += fi * dz;
-      div += fii + 2 * fi;
+      d2j += fii + 2 * fi;
       pa[c] = a;
       ph[c] = -sk * a * a / r;
       double *ren = st.ren + ((size_t)w * N * C + i * C + c) * 2;
@@ -665,7 +665,6 @@ __device__ __forceinline__ Res evaluate(const Sys<double> &s, const stab::Tab &T
     for (int q = 0; q < ZQ; q++) zg[q] = z[q];
     v[L.f() + i * N + i] = fen;
     fsum = fen;
-    d2j = div;
   }
   __syncwarp(m);
   double dvd = 0, vx = 0, vy = 0, vz = 0;
@@ -678,9 +677,7 @@ __device__ __forceinline__ Res evaluate(const Sys<double> &s, const stab::Tab &T
       vj[1] += g[1];
       vj[2] += g[2];
       d2j += lap;
-      div += 0.5 * lap;  // a pair's Laplacian is halved between its electrons; the other half follows
       v[L.f() + i * N + j] = f;
-      if (outputs) st.o_divv[(size_t)w * N + i] = 0;
       if (j < i) {
         fsum += f;
         pe_ee += rin;
@@ -702,25 +699,8 @@ __device__ __forceinline__ Res evaluate(const Sys<double> &s, const stab::Tab &T
     vx = vj[0] + g0;
     vy = vj[1] + g1;
     vz = vj[2] + g2;
-    if (outputs) {
-      double *ov = st.o_vel + ((size_t)w * N + i) * 3;
-      ov[0] = vx; ov[1] = vy; ov[2] = vz;
-    }
   }
   __syncwarp(m);
-  if (outputs && act) {
-    // the other half of the pair Laplacians, lap_j of every pair (i, j)
-    double other = 0;
-    for (int j = 0; j < N; j++) {
-      if (j == i) continue;
-      const double xj[3] = {v[3 * j], v[3 * j + 1], v[3 * j + 2]};
-      double g[3], lap, rin;
-      pair_terms<NORD, 2>(s, J, j, i, xj, v + L.a() + j * C, v + L.h() + j * C, v + 3 * i, v + L.a() + i * C,
-                          v + L.z() + i * L.qm, g, lap, rin);
-      other += 0.5 * lap;
-    }
-    st.o_divv[(size_t)w * N + i] = div + other + dvd;
-  }
   const double v2 = gsum(act ? vx * vx + vy * vy + vz * vz : 0.0, m), d2lnd = gsum(dvd, m);
   fsum = gsum(fsum, m);
   d2j = gsum(d2j, m);
@@ -802,16 +782,6 @@ __device__ __forceinline__ Res evaluate(const Sys<double> &s, const stab::Tab &T
     if (!ok) flag |= CHAMP_WS_SINGULAR;
     if (!isfinite(res.eloc) || !isfinite(lnpsi)) flag |= CHAMP_WS_NONFINITE;
     st.status[w] = flag;
-    if (outputs) {
-      st.o_lnpsi[w] = lnpsi;
-      st.o_sign[w] = sgn;
-      st.o_psij[w] = fsum;
-      st.o_d2[w] = d2;
-      st.o_pe[w] = pe;
-      st.o_peee[w] = pe_ee;
-      st.o_penl[w] = vnl;
-      st.o_eloc[w] = res.eloc;
-    }
   }
   return res;
 }
@@ -842,9 +812,9 @@ __device__ __forceinline__ void store(const Sys<double> &s, const State<double> 
   }
 }
 
-enum { EVAL = 0, GAUSS = 1, ACCEL = 6, DMC = 7, DMC_EL = 8 };
+enum { EVAL = 0, GAUSS = 1, DMC = 7, DMC_EL = 8 };
 
-// EVAL: E_L of the walkers; GAUSS, ACCEL: sweeps of that mover, each followed by E_L; DMC: a
+// EVAL: E_L of the walkers after a sweep; GAUSS: sweeps of Gaussian moves, each followed by E_L; DMC: a
 // drift-diffusion step with E_L, reweighting and copy counts (k_dmc_move); DMC_EL: its second half.
 template <int NORD, int MODE>
 __global__ void __launch_bounds__(128, 3) k_small(const __grid_constant__ Sys<double> s, const __grid_constant__ State<double> st,
@@ -858,7 +828,7 @@ __global__ void __launch_bounds__(128, 3) k_small(const __grid_constant__ Sys<do
   const int N = s.N, C = s.C, sub = threadIdx.x & 7, grp = threadIdx.x >> 3;
   const unsigned m = gmask();
   double *v = (double *)(dsm + stab::tab_smem(s.nshell, s.nprim)) + (size_t)grp * L.total();
-  constexpr bool dmc = MODE == DMC || MODE == DMC_EL, moves = MODE == GAUSS || MODE == ACCEL || MODE == DMC;
+  constexpr bool dmc = MODE == DMC || MODE == DMC_EL, moves = MODE == GAUSS || MODE == DMC;
   const int W = dmc ? *A.D.nw : st.W;
   const uint64_t step0 = dmc ? (uint64_t)A.D.ctr[0] : A.sweep0;
   const double et = dmc ? *A.D.et : 0, eest = dmc ? *A.D.eest : 0, esigma = dmc ? energy_sigma(A.P, A.D.esg, N) : 0,
@@ -879,7 +849,7 @@ __global__ void __launch_bounds__(128, 3) k_small(const __grid_constant__ Sys<do
     }
     __syncwarp(m);
     double es = 0, e2 = 0, acc = 0, el = 0;
-    const int nsw = MODE == GAUSS || MODE == ACCEL ? A.nsweep : 1;
+    const int nsw = MODE == GAUSS ? A.nsweep : 1;
     for (int isw = 0; isw < nsw; isw++) {
       const uint64_t sweep = step0 + (uint64_t)isw;
       for (int e = 0; e < N; e++)
@@ -901,40 +871,21 @@ __global__ void __launch_bounds__(128, 3) k_small(const __grid_constant__ Sys<do
         } else {
           electron_jastrow<NORD, true>(s, J, v, e, xo, pf, d0, go);
           det_ratio<true>(s, v, L, e, v + L.row() + e * 5 * NO, go);
-          if constexpr (MODE == ACCEL) {
-            MoveRng rng{A.seed, (uint32_t)w, (uint32_t)sweep, (uint32_t)(sweep >> 32), (uint32_t)e, 0u, {0.0, 0.0}, 0};
-            double fxop, areao, rtry;
-            slat_forward(s, A.mv, xo, go, rng, xn, fxop, areao, rtry);
-            SlatBack b;
-            p = rho = dj = pf = 0;
-            if (slat_geometry(s, A.mv, xo, xn, b)) {
-              __syncwarp(m);
-              orb_row<5>(s, T, A.order, sp, xn[0], xn[1], xn[2], pr);
-              electron_jastrow<NORD, true>(s, J, v, e, xn, pf, dj, gn);
-              rho = det_ratio<true>(s, v, L, e, pr, gn);
-              double fxnp, arean;
-              slat_reverse(s, A.mv, b, gn, fxnp, arean);
-              const double rr = rtry / b.rminon;
-              p = rr * rr * rho * rho * exp(2.0 * dj) * fabs((fxnp * areao) / (fxop * arean));
-            }
-            ua = rng.next();
-          } else {
-            double vo[3], vn[3], g[3], db[3];
-            avg_drift(go, A.P.tau, A.P.adrift, vo);
-            move_randoms(A.P.seed, (uint32_t)w, sweep, (uint32_t)e, g, &ua);
-            for (int k = 0; k < 3; k++) xn[k] = xo[k] + A.P.tau * vo[k] + sqt * g[k];
-            orb_row<5>(s, T, A.order, sp, xn[0], xn[1], xn[2], pr);
-            electron_jastrow<NORD, true>(s, J, v, e, xn, pf, dj, gn);
-            rho = det_ratio<true>(s, v, L, e, pr, gn);
-            avg_drift(gn, A.P.tau, A.P.adrift, vn);
-            const double lgf = -0.5 * (g[0] * g[0] + g[1] * g[1] + g[2] * g[2]);
-            for (int k = 0; k < 3; k++) db[k] = xo[k] - xn[k] - A.P.tau * vn[k];
-            const double lgb = -(db[0] * db[0] + db[1] * db[1] + db[2] * db[2]) / (2 * A.P.tau);
-            p = (rho > 0) ? rho * rho * exp(2.0 * dj + lgb - lgf) : 0.0;  // fixed node
-            const double dd = A.P.tau * (g[0] * g[0] + g[1] * g[1] + g[2] * g[2]);
-            sdd += dd;
-            spd += (p < 1.0 ? p : 1.0) * dd;
-          }
+          double vo[3], vn[3], g[3], db[3];
+          avg_drift(go, A.P.tau, A.P.adrift, vo);
+          move_randoms(A.P.seed, (uint32_t)w, sweep, (uint32_t)e, g, &ua);
+          for (int k = 0; k < 3; k++) xn[k] = xo[k] + A.P.tau * vo[k] + sqt * g[k];
+          orb_row<5>(s, T, A.order, sp, xn[0], xn[1], xn[2], pr);
+          electron_jastrow<NORD, true>(s, J, v, e, xn, pf, dj, gn);
+          rho = det_ratio<true>(s, v, L, e, pr, gn);
+          avg_drift(gn, A.P.tau, A.P.adrift, vn);
+          const double lgf = -0.5 * (g[0] * g[0] + g[1] * g[1] + g[2] * g[2]);
+          for (int k = 0; k < 3; k++) db[k] = xo[k] - xn[k] - A.P.tau * vn[k];
+          const double lgb = -(db[0] * db[0] + db[1] * db[1] + db[2] * db[2]) / (2 * A.P.tau);
+          p = (rho > 0) ? rho * rho * exp(2.0 * dj + lgb - lgf) : 0.0;  // fixed node
+          const double dd = A.P.tau * (g[0] * g[0] + g[1] * g[1] + g[2] * g[2]);
+          sdd += dd;
+          spd += (p < 1.0 ? p : 1.0) * dd;
         }
         if (ua < p) {
           accept<NORD>(s, v, L, e, xn, pf, rho, 5 * NO);
@@ -942,13 +893,13 @@ __global__ void __launch_bounds__(128, 3) k_small(const __grid_constant__ Sys<do
         }
         __syncwarp(m);
       }
-      ElRot rot = A.rot;
-      if (MODE != EVAL || A.rot.random) {
+      ElRot rot = A.rot;  // EVAL: the sweep's
+      if (MODE != EVAL) {
         rot.random = 1;
-        rot.seed = dmc ? A.P.seed : (MODE == EVAL ? A.rot.seed : A.seed);
-        rot.sweep = MODE == EVAL ? A.rot.sweep : sweep;
+        rot.seed = dmc ? A.P.seed : A.seed;
+        rot.sweep = sweep;
       }
-      const Res res = evaluate<NORD>(s, T, J, E, st, w, v, L, rot, MODE == EVAL && A.outputs);
+      const Res res = evaluate<NORD>(s, T, J, E, st, w, v, L, rot);
       el = res.eloc;
       es += el;
       e2 += el * el;
@@ -966,7 +917,7 @@ __global__ void __launch_bounds__(128, 3) k_small(const __grid_constant__ Sys<do
       }
     }
     store(s, st, w, v, L);
-    if (!dmc && sub == 0 && (MODE != EVAL || A.stats)) {
+    if (!dmc && sub == 0) {
       st.s_esum[w] += es;
       st.s_e2sum[w] += e2;
       st.s_acc[w] += acc;

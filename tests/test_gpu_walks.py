@@ -140,3 +140,23 @@ def test_accelerated_sweep_follows_the_oracle(oracle_mod, n, nup, ncent, nordc):
     print(f"{n} electrons: first {d[:, 0].max():.1e}, all {d.max():.1e} bohr; allowed {bound[:, 0].max():.1e} {bound.max():.1e}")
     assert np.all(d <= bound)
     assert np.array_equal(st["accept"], ref["accept"])
+
+
+@pytest.mark.parametrize("case", ["dimer", "c2bfd", "mixed"])
+def test_accelerated_walk_of_few_among_many(case):
+    """A small walker's evaluation and accelerated walk, bit for bit, do not depend on how many walk beside it."""
+    from champ_b200.engine import Engine
+    s = S.c2_bfd_example(10) if case == "c2bfd" else S.c2_dimer()
+    prec = "mixed" if case == "mixed" else "fp64"
+    x = S.initial_walkers(s, 40, seed=11)
+    out = []
+    for y in (x, np.resize(x, (5003,) + x.shape[1:])):
+        eng = Engine(s, len(y), prec)
+        eng.set_walkers(y)
+        r = eng.eval_full()
+        eng.set_mover(6)
+        st = eng.vmc_sweeps(3, seed=19, sweep0=1, step=s.step)
+        out.append((r["energy"][:40], r["velocity"][:40], eng.get_walkers()[:40], st["elast"][:40], st["accept"][:40]))
+        eng.close()
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
