@@ -139,6 +139,7 @@ struct champ_ctx {
   double *pg_tv = nullptr, *pg_tc = nullptr;
   int *pg_tn = nullptr;
   bool have_tape = false;
+  bool tape_tiled = false;  // by the tiled forward pass, which also leaves the distances that the tiled reverse sweep reads
   int pg_mode = 0;  // 0: forward pass + reverse sweep; 1: one fused pass
   int nquad = 12;   // points of the nonlocal quadrature rule in use
   QuadRule quad{};  // its points and weights (host copy)

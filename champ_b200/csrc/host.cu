@@ -1692,8 +1692,10 @@ int champ_param_grad_fwd(champ_ctx *c, double *eloc) {
   if (!c->have_walkers) return fail(CHAMP_ESTATE, "no walkers set");
   if (c->smem_pg == 0) return fail(CHAMP_EINVAL, "parameter derivatives: system too large for the kernel's shared memory");
   OpArgs a = pg_args(c, 3);
-  int rc = pg_tile_fwd_ok(c) ? pg_tile_fwd(c) : launch(c, Op::PGrad, a);
+  const bool tiled = pg_tile_fwd_ok(c);
+  int rc = tiled ? pg_tile_fwd(c) : launch(c, Op::PGrad, a);
   if (rc) return rc;
+  c->tape_tiled = tiled;
   c->have_tape = true;
   c->have_pgrad = false;
   if (eloc) {
@@ -1707,7 +1709,7 @@ int champ_param_grad_bwd(champ_ctx *c, double *dlnpsi, double *deloc) {
   if (!c) return fail(CHAMP_EINVAL, "null context");
   if (!c->have_tape) return fail(CHAMP_ESTATE, "call champ_param_grad_fwd first");
   OpArgs a = pg_args(c, 4);
-  int rc = pg_tile_bwd_ok(c) ? pg_tile_bwd(c) : launch(c, Op::PGradBwd, a);
+  int rc = c->tape_tiled && pg_tile_bwd_ok(c) ? pg_tile_bwd(c) : launch(c, Op::PGradBwd, a);
   if (!rc) rc = pg_orbital_part(c);
   if (rc) return rc;
   c->have_tape = false;

@@ -136,3 +136,47 @@ def test_parameter_gradient_matches_single_kernels(n, nup, ncent, nordc):
         # per walker: sums of terms as large as the walker's largest derivative
         scale = np.abs(b).reshape(len(b), -1).max(axis=1).reshape((-1,) + (1,) * (b.ndim - 1))
         assert np.all(np.abs(a - b) <= 1e-9 * np.maximum(1.0, scale))
+
+
+@pytest.mark.parametrize("first", [0, 1])
+def test_gradient_passes_with_the_option_changed_between(first):
+    """A tape of the single kernels swept in reverse after the staged evaluation is switched on (its distances were
+    never formed), and a tiled tape after it is switched off: the derivatives of either pair of passes."""
+    from champ_b200.engine import Engine
+    s = cluster(40, 24, 7, 5)
+    x = S.initial_walkers(s, 5, seed=42)
+    ref = Engine(s, 5, "fp64")
+    ref.set_option("staged_eval", 0)
+    ref.set_walkers(x)
+    dl0, de0, _ = ref.param_grad()
+    ref.close()
+    eng = Engine(s, 5, "fp64")
+    eng.set_option("staged_eval", first)
+    eng.set_walkers(x)
+    eng.param_grad_fwd()
+    eng.set_option("staged_eval", 1 - first)
+    dl, de = eng.param_grad_bwd()
+    eng.close()
+    for a, b in ((dl, dl0), (de, de0)):
+        assert np.all(np.abs(a - b) <= 1e-9 * np.maximum(1.0, np.abs(b).max(axis=1, keepdims=True)))
+
+
+@pytest.mark.parametrize("n,nup,ncent,nordc", [(33, 17, 9, 4), (51, 26, 13, 5), (65, 33, 17, 4), (72, 40, 33, 4)])
+def test_parameter_gradient_with_virtual_orbitals(n, nup, ncent, nordc):
+    """As above with three orbitals to a centre, so that the points' coefficients have room and the tiles serve
+    beyond 32 and 64 electrons and 32 centres, and orbital rotations into virtual orbitals are among the parameters."""
+    from champ_b200.engine import Engine
+    s = cluster(n, nup, ncent, nordc)
+    s = dataclasses.replace(s, coef=S.cluster128(ncent=ncent, box=14.0 * (max(ncent, 4) / 32) ** (1 / 3), norb=3 * ncent).coef)
+    x = S.initial_walkers(s, 3, seed=n + 2)
+    out = []
+    for staged in (1, 0):
+        eng = Engine(s, 3, "fp64")
+        eng.set_option("staged_eval", staged)
+        eng.set_walkers(x)
+        out.append(eng.param_grad())
+        eng.close()
+    assert not all(np.array_equal(a, b) for a, b in zip(*out))  # two kernels
+    for a, b in zip(*out):
+        scale = np.abs(b).reshape(len(b), -1).max(axis=1).reshape((-1,) + (1,) * (b.ndim - 1))
+        assert np.all(np.abs(a - b) <= 1e-9 * np.maximum(1.0, scale))
