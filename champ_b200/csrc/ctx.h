@@ -257,21 +257,14 @@ int small_vmc(champ_ctx *c, const State<double> &st, const OpArgs &a);
 int small_dmc(champ_ctx *c, const State<double> &st, bool moves);
 int small_tmove(champ_ctx *c, const State<double> &st, const OpArgs &a);
 
-// Shared-memory carve-out of a kernel: what its resident blocks of this launch shape use and no more, so
-// that the rest of the SM's 256 KB stays L1 cache (with the largest carve-out the shell tables and orbital
-// coefficients that every warp reads over and over came from L2).
+// Allows a kernel smem bytes of dynamic shared memory and fits its shared-memory carve-out to what its resident
+// blocks of that shape use and no more, so that the rest of the SM's 256 KB stays L1 cache (with the largest
+// carve-out the shell tables and orbital coefficients that every warp reads over and over came from L2).
+// Both are attributes of the kernel, not of the context: they only ever grow, so that a context made later, for a
+// smaller system, takes nothing from those that are there.  threads 0: the default carve-out.
+int champ_kernel_smem(const void *kern, int threads, size_t smem);
 template <class K>
-int fit_carveout(K kern, int threads, size_t smem) {
-  CK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
-  int n = 0;
-  cudaFuncAttributes fa;
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, smem));
-  CK(cudaFuncGetAttributes(&fa, kern));
-  const size_t need = (size_t)std::max(n, 1) * (smem + fa.sharedSizeBytes + 1024);  // 1 KB of each block is the system's
-  const int pct = (int)std::min<size_t>(100, (need * 100 + 228 * 1024 - 1) / (228 * 1024));
-  CK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, pct));
-  return CHAMP_OK;
-}
+int kernel_smem(K kern, int threads, size_t smem) { return champ_kernel_smem((const void *)kern, threads, smem); }
 
 // kernel launchers per (compute type, e-e-n order), one translation unit each (inst_*.cu)
 #define CHAMP_DECL(TAG, NORD)                                    \

@@ -7,30 +7,41 @@
 #include "nlpoints.cuh"
 #include "pgtile.cuh"
 
-template <class K>
-static int big_smem(K kern, int threads, size_t bytes) {
-  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-  return fit_carveout(kern, threads, bytes);
-}
-
-template <int NORD>
-static int fin_attrs_n(size_t b) {
-  int rc = big_smem(pt::k_fin_points<NORD, false, 1>, 128, b);
-  if (!rc) rc = big_smem(pt::k_fin_points<NORD, false, 4>, 128, b);
-  if (!rc) rc = big_smem(pt::k_fin_points<NORD, true, 1>, 128, b);
-  if (!rc) rc = big_smem(pt::k_fin_points<NORD, true, 4>, 128, b);
-  if (!rc) rc = big_smem(pt::k_fin_points<NORD, false, 8>, 256, b);
-  if (!rc) rc = big_smem(pt::k_fin_points<NORD, true, 8>, 256, b);
-  return rc;
-}
 static size_t gproj_smem(const champ_ctx *c) { return sizeof(double) * pt::GP_LD * (size_t)((c->nomax + 3) & ~3); }
-static int fin_attrs(champ_ctx *c) {
-  int rc = c->nordc == 4 ? fin_attrs_n<4>(c->fin_smem) : c->nordc == 5 ? fin_attrs_n<5>(c->fin_smem) : fin_attrs_n<0>(c->fin_smem);
-  if (!rc) rc = big_smem(pt::k_gproj<false>, 128, gproj_smem(c));
-  if (!rc) rc = big_smem(pt::k_gproj<true>, 128, gproj_smem(c));
+
+// The attributes of the kernels that the context launches.
+template <int NORD, bool MD>
+static int fin_attrs(const champ_ctx *c) {
+  int rc = c->fin_wpw == 1   ? kernel_smem(pt::k_fin_points<NORD, MD, 1>, 128, c->fin_smem)
+           : c->fin_wpw == 8 ? kernel_smem(pt::k_fin_points<NORD, MD, 8>, 256, c->fin_smem)
+           : c->fin_wpw      ? kernel_smem(pt::k_fin_points<NORD, MD, 4>, 128, c->fin_smem)
+                             : CHAMP_OK;
+  if (!rc && c->fin_wpw && c->nloc > 0) rc = kernel_smem(pt::k_gproj<MD>, 128, gproj_smem(c));
   return rc;
 }
-
+template <int NORD>
+static int el_attrs(const champ_ctx *c) {
+  int rc = c->md.multidet ? fin_attrs<NORD, true>(c) : fin_attrs<NORD, false>(c);
+  if constexpr (NORD > 1) {
+    if (c->jas_wpw == 1) {
+      if (!rc) rc = kernel_smem(jt::k_jas_tile<NORD, 1, false>, 128, c->jas_smem);
+      if (!rc) rc = kernel_smem(jt::k_jas_tile<NORD, 1, true>, 128, c->jas_smem);
+    } else if (c->jas_wpw) {
+      if (!rc) rc = kernel_smem(jt::k_jas_tile<NORD, jt::WARPS, false>, 128, c->jas_smem);
+      if (!rc) rc = kernel_smem(jt::k_jas_tile<NORD, jt::WARPS, true>, 128, c->jas_smem);
+    }
+  }
+  return rc;
+}
+static int orb_class(int nocc) { return nocc > 32 ? 5 : nocc > 16 ? 4 : nocc > 8 ? 3 : nocc > 4 ? 2 : nocc > 2 ? 1 : 0; }
+static int orb_attrs(int k) {
+  return k == 5   ? kernel_smem(ot::k_orb_tile<4, 1, false>, ot::THREADS, ot::smem_bytes<4>())
+         : k == 4 ? kernel_smem(ot::k_orb_tile<2, 1, false>, ot::THREADS, ot::smem_bytes<2>())
+         : k == 3 ? kernel_smem(ot::k_orb_tile<1, 2, false>, ot::THREADS, ot::smem_bytes<1>())
+         : k == 2 ? kernel_smem(ot::k_orb_tile<1, 4, false>, ot::THREADS, ot::smem_bytes<1>())
+         : k == 1 ? kernel_smem(ot::k_orb_tile<1, 8, false>, ot::THREADS, ot::smem_bytes<1>())
+                  : CHAMP_OK;
+}
 
 // Which parts serve the context's system, their shared memory, and the chunks of whole shells that
 // the orbital part forms at a time.
@@ -79,16 +90,9 @@ int el_tile_setup(champ_ctx *c) {
       c->fin_smem = b;
     }
   }
-  int rc = fin_attrs(c);
-  for (auto k : {jt::k_jas_tile<4, 1, false>, jt::k_jas_tile<4, 1, true>, jt::k_jas_tile<4, jt::WARPS, false>,
-                 jt::k_jas_tile<4, jt::WARPS, true>, jt::k_jas_tile<5, 1, false>, jt::k_jas_tile<5, 1, true>,
-                 jt::k_jas_tile<5, jt::WARPS, false>, jt::k_jas_tile<5, jt::WARPS, true>})
-    if (!rc) rc = big_smem(k, 128, c->jas_smem);
-  if (!rc) rc = big_smem(ot::k_orb_tile<1, 2, false>, ot::THREADS, ot::smem_bytes<1>());
-  if (!rc) rc = big_smem(ot::k_orb_tile<1, 4, false>, ot::THREADS, ot::smem_bytes<1>());
-  if (!rc) rc = big_smem(ot::k_orb_tile<1, 8, false>, ot::THREADS, ot::smem_bytes<1>());
-  if (!rc) rc = big_smem(ot::k_orb_tile<2, 1, false>, ot::THREADS, ot::smem_bytes<2>());
-  if (!rc) rc = big_smem(ot::k_orb_tile<4, 1, false>, ot::THREADS, ot::smem_bytes<4>());
+  int rc = c->nordc == 4 ? el_attrs<4>(c) : c->nordc == 5 ? el_attrs<5>(c) : el_attrs<0>(c);
+  for (int sp = 0; sp < 2; sp++)
+    if (!rc && c->orb_tile) rc = orb_attrs(orb_class(c->sd.nocc[sp]));
   return rc;
 }
 
@@ -121,7 +125,6 @@ static int orb(champ_ctx *c, const State<double> &st, int sp0, int ns) {
   CK(cudaGetLastError());
   return CHAMP_OK;
 }
-static int orb_class(int nocc) { return nocc > 32 ? 5 : nocc > 16 ? 4 : nocc > 8 ? 3 : nocc > 4 ? 2 : nocc > 2 ? 1 : 0; }
 static int orb_spins(champ_ctx *c, const State<double> &st, int k, int sp0, int ns) {
   return k == 5 ? orb<4, 1>(c, st, sp0, ns) : k == 4 ? orb<2, 1>(c, st, sp0, ns) : k == 3 ? orb<1, 2>(c, st, sp0, ns)
        : k == 2 ? orb<1, 4>(c, st, sp0, ns) : orb<1, 8>(c, st, sp0, ns);
@@ -192,6 +195,15 @@ static size_t pgnl_smem(const champ_ctx *c) {
   return sizeof(double) * 4 * (size_t)c->nbasis + stab::tab_smem(c->sd.nshell, c->sd.nprim);
 }
 
+template <int NORD>
+static int bwd_attrs(const champ_ctx *c) {
+  const bool one = c->jas_wpw == 1;
+  const size_t b = pt::Dims(c->N, c->C, NORD, 0).bytes() * (one ? 4 : 1);
+  int rc = one ? kernel_smem(pg::k_pg_points<NORD, 1>, 128, b) : kernel_smem(pg::k_pg_points<NORD, 4>, 128, b);
+  if (!rc) rc = one ? kernel_smem(pg::k_pg_pairs<NORD, 1>, 128, c->jas_smem) : kernel_smem(pg::k_pg_pairs<NORD, 4>, 128, c->jas_smem);
+  return rc;
+}
+
 int pg_tile_setup(champ_ctx *c) {
   if (!pg_tile_fwd_ok(c)) return CHAMP_OK;
   std::vector<int4> sh(c->nshell);
@@ -202,14 +214,10 @@ int pg_tile_setup(champ_ctx *c) {
   CK(cudaMalloc(&c->shell_order, sizeof(int) * c->nshell));
   c->allocs.push_back(c->shell_order);
   CK(cudaMemcpy(c->shell_order, order.data(), sizeof(int) * c->nshell, cudaMemcpyHostToDevice));
-  int rc = big_smem(ot::k_orb_tile<4, 1, true>, ot::THREADS, ot::smem_bytes<4>());
-  if (!rc) rc = big_smem(pg::k_pg_nl, 128, pgnl_smem(c));
+  int rc = kernel_smem(ot::k_orb_tile<4, 1, true>, ot::THREADS, ot::smem_bytes<4>());
+  if (!rc) rc = kernel_smem(pg::k_pg_nl, 128, pgnl_smem(c));
   if (rc || c->prec != CHAMP_PREC_FP64 || c->par.nspin2b != 1) return rc;
-  const size_t pb = pt::Dims(c->N, c->C, c->nordc, 0).bytes() * (c->jas_wpw == 1 ? 4 : 1);
-  for (auto k : {pg::k_pg_points<4, 1>, pg::k_pg_points<4, 4>, pg::k_pg_points<5, 1>, pg::k_pg_points<5, 4>})
-    if (!rc) rc = big_smem(k, 128, pb);
-  for (auto k : {pg::k_pg_pairs<4, 1>, pg::k_pg_pairs<4, 4>, pg::k_pg_pairs<5, 1>, pg::k_pg_pairs<5, 4>})
-    if (!rc) rc = big_smem(k, 128, c->jas_smem);
+  rc = c->nordc == 4 ? bwd_attrs<4>(c) : bwd_attrs<5>(c);
   if (rc) return rc;
   CK(cudaMalloc(&c->pg_raw, sizeof(double) * 3 * (size_t)c->np_raw * c->wmax));
   c->allocs.push_back(c->pg_raw);

@@ -13,6 +13,7 @@
 #include <cstdio>
 #include <cstring>
 #include <algorithm>
+#include <map>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -1020,6 +1021,33 @@ static int alloc_state_copy(champ_ctx *c, const State<T> &a, State<T> &b) {
 }
 
 static const int DMC_STAT_CAP = 1 << 16;
+
+int champ_kernel_smem(const void *kern, int threads, size_t smem) {
+  struct Attr {
+    size_t limit = 0;
+    int pct = 0;
+  };
+  static std::mutex mu;
+  static std::map<std::pair<int, const void *>, Attr> attrs;
+  int dev = 0;
+  CK(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lk(mu);
+  Attr &a = attrs[{dev, kern}];
+  if (smem > a.limit) {
+    CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    a.limit = smem;
+  }
+  if (threads == 0 || a.pct == 100) return CHAMP_OK;
+  CK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
+  int n = 0;
+  cudaFuncAttributes fa;
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, smem));
+  CK(cudaFuncGetAttributes(&fa, kern));
+  const size_t need = (size_t)std::max(n, 1) * (smem + fa.sharedSizeBytes + 1024);  // 1 KB of each block is the system's
+  a.pct = std::max(a.pct, (int)std::min<size_t>(100, (need * 100 + 228 * 1024 - 1) / (228 * 1024)));
+  CK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, a.pct));
+  return CHAMP_OK;
+}
 
 // ---------------------------------------------------------------------------------------
 // Evaluation without allocation.  Some callers cannot call cudaMalloc: host codes whose

@@ -9,8 +9,7 @@
 // ---- kernel dispatch over (precision, e-e-n order)
 template <class K>
 static int set_attrs(champ_ctx *c, K kern, size_t smem, int wpb = 4) {
-  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  return fit_carveout(kern, 32 * wpb, smem);
+  return kernel_smem(kern, 32 * wpb, smem);
 }
 template <class T, int NORD, bool MD>
 static int set_smem_attrs(champ_ctx *c) {
@@ -27,14 +26,11 @@ static int set_smem_attrs(champ_ctx *c) {
   if (!rc) rc = set_attrs(c, k_dmc_move<T, NORD, MD>, sm);
   if (!rc) rc = set_attrs(c, k_dmc_tmove<T, NORD, MD>, sm);
   if (!rc && std::is_same<T, float>::value && c->prec == CHAMP_PREC_FP32) {
-    CK(cudaFuncSetAttribute(orbtc::k_orb_tc<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024 + 128));
-    CK(cudaFuncSetAttribute(orbtc::k_orb_tc<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024 + 128));
-    CK(cudaFuncSetAttribute(orbtc::k_orb_tc<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)orbtc::smem_bytes(256, 2)));
-    CK(cudaFuncSetAttribute(orbf::k_orb_fused, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)orbf::fsmem_bytes(96)));
-    CK(cudaFuncSetAttribute(k_basis_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)std::min<size_t>(4 * (size_t)c->nbasis * 5 * sizeof(float), 227 * 1024)));
+    rc = kernel_smem(orbtc::k_orb_tc<4>, 0, 200 * 1024 + 128);
+    if (!rc) rc = kernel_smem(orbtc::k_orb_tc<3>, 0, 200 * 1024 + 128);
+    if (!rc) rc = kernel_smem(orbtc::k_orb_tc<2>, 0, orbtc::smem_bytes(256, 2));
+    if (!rc) rc = kernel_smem(orbf::k_orb_fused, 0, orbf::fsmem_bytes(96));
+    if (!rc) rc = kernel_smem(k_basis_rows, 0, std::min<size_t>(4 * (size_t)c->nbasis * 5 * sizeof(float), 227 * 1024));
   }
   if (!rc && c->el_staged && std::is_same<T, double>::value) {
     rc = set_attrs(c, k_el_jas<T, NORD>, c->el_smem[0]);
@@ -43,10 +39,8 @@ static int set_smem_attrs(champ_ctx *c) {
     if (!rc) rc = set_attrs(c, k_el_fin<T, NORD, MD>, c->el_smem[2]);
   }
   if (!rc && c->smem_pg > 0) {
-    for (auto kern : {k_pgrad<T, NORD, MD, 1>, k_pgrad<T, NORD, MD, 2>, k_pgrad<T, NORD, MD, 3>, k_pgrad<T, NORD, MD, 4>}) {
-      CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->smem_pg));
-      if (int r = fit_carveout(kern, 32 * c->wpb_pg, c->smem_pg)) return r;
-    }
+    for (auto kern : {k_pgrad<T, NORD, MD, 1>, k_pgrad<T, NORD, MD, 2>, k_pgrad<T, NORD, MD, 3>, k_pgrad<T, NORD, MD, 4>})
+      if (!rc) rc = kernel_smem(kern, 32 * c->wpb_pg, c->smem_pg);
   }
   return rc;
 }

@@ -6,12 +6,6 @@
 
 namespace {
 
-template <class K>
-int big_smem(K kern, int threads, size_t bytes) {
-  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-  return fit_carveout(kern, threads, bytes);
-}
-
 // up to 32 electrons a warp per walker, else a block per walker
 int warps_per_walker(const champ_ctx *c) { return c->N <= 32 ? 1 : 4; }
 size_t walk_smem(const champ_ctx *c) {
@@ -32,13 +26,13 @@ template <class T, int NORD>
 int setup(champ_ctx *c) {
   const size_t sp = pairs_smem<T, NORD>(c), sw = walk_smem(c);
   if (sp > 200 * 1024 || sw > 200 * 1024) return CHAMP_OK;
-  int rc = big_smem(mv::k_mv_pairs<T, NORD, 1>, 128, sp);
-  if (!rc) rc = big_smem(mv::k_mv_pairs<T, NORD, 4>, 128, sp);
-  if (!rc) rc = big_smem(mv::k_mv_walk<T, 1>, 128, sw);
-  if (!rc) rc = big_smem(mv::k_mv_walk<T, 4>, 128, sw);
-  if (!rc) rc = big_smem(mv::k_mv_prop<T, 1>, 256, prop_smem<T, 1>(c));
-  if (!rc) rc = big_smem(mv::k_mv_prop<T, 2>, 256, prop_smem<T, 2>(c));
-  if (!rc) rc = big_smem(mv::k_mv_prop<T, 4>, 256, prop_smem<T, 4>(c));
+  const bool one = warps_per_walker(c) == 1;
+  int rc = one ? kernel_smem(mv::k_mv_pairs<T, NORD, 1>, 128, sp) : kernel_smem(mv::k_mv_pairs<T, NORD, 4>, 128, sp);
+  if (!rc) rc = one ? kernel_smem(mv::k_mv_walk<T, 1>, 128, sw) : kernel_smem(mv::k_mv_walk<T, 4>, 128, sw);
+  if (!rc)
+    rc = c->orb_nt == 1   ? kernel_smem(mv::k_mv_prop<T, 1>, 256, prop_smem<T, 1>(c))
+         : c->orb_nt == 2 ? kernel_smem(mv::k_mv_prop<T, 2>, 256, prop_smem<T, 2>(c))
+                          : kernel_smem(mv::k_mv_prop<T, 4>, 256, prop_smem<T, 4>(c));
   if (!rc) c->move_batch = 1;
   return rc;
 }

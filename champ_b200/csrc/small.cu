@@ -7,18 +7,13 @@
 
 namespace {
 
-template <class K>
-int big_smem(K kern, size_t bytes) {
-  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-  return fit_carveout(kern, 128, bytes);
-}
 template <int NORD>
 int attrs(const champ_ctx *c) {
   const size_t b = sizeof(double) * (size_t)sm::Lay(c->N, c->C, c->nordc).total() * 16 + stab::tab_smem(c->sd.nshell, c->sd.nprim);
   int rc = CHAMP_OK;
   for (auto k : {sm::k_small<NORD, sm::EVAL>, sm::k_small<NORD, sm::GAUSS>, sm::k_small<NORD, sm::DMC>, sm::k_small<NORD, sm::DMC_EL>,
                  sm::k_small_tmove<NORD>})
-    if (!rc) rc = big_smem(k, b);
+    if (!rc) rc = kernel_smem(k, 128, b);
   return rc;
 }
 
