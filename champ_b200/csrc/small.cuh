@@ -502,6 +502,10 @@ __device__ __forceinline__ void invert(const Sys<double> &s, double *v, const La
       for (int j = 0; j < NO; j++) a[j] = (j + 1 < NO ? a[j + 1] : 0.0) - f * p[j];
     }
   }
+  if (fail && r < n)  // a singular matrix stays as it is, as in k_inv_reg
+#pragma unroll
+    for (int j = 0; j < NO; j++)
+      if (j < n) v[L.ai() + sp * NO * NO + r * NO + j] = v[L.row() + e * 5 * NO + j];
   double ln = (r < n && !fail) ? log(fabs(piv)) : 0.0;
   int neg = (r < n && piv < 0) ? 1 : 0;
   if (!fail && r < n) {

@@ -100,3 +100,28 @@ def test_mixed_sweeps_of_few_among_many():
     assert same.sum() >= 59
     assert np.array_equal(out[0][1][same], out[1][1][same])
     assert np.allclose(out[0][2][same], out[1][2][same], rtol=1e-9, atol=1e-9)
+
+
+def test_singular_walkers_leave_their_matrix():
+    """Up electrons so far out that every orbital is zero there: the walker is flagged, its energy NaN, and the evaluation
+    leaves the zero matrix in the inverse's place, so that the ratio of a move back is zero whatever the
+    walkers beside it are; the others are as without it."""
+    from champ_b200.engine import Engine
+    s = system("dimer")
+    nw, bad = 4801, [0, 7, 13, 16, 100, 2000, 4800]
+    x = S.initial_walkers(s, nw, seed=15)
+    y = x.copy()
+    y[bad, :s.nup] += 1e4 * np.arange(1, s.nup + 1)[:, None]
+    out = []
+    for z in (x, y):
+        eng = Engine(s, nw, "mixed")
+        eng.set_walkers(z)
+        st = eng.vmc_sweeps(1, seed=21, sweep0=0, step=s.step)  # FP32 moves, then the small kernel's E_L
+        r = eng.propose_1e(0, np.broadcast_to(s.cent[0] + 0.4, (nw, 3)).copy())
+        out.append((st["elast"], eng.get_walkers(), eng.walker_status(), r))
+        eng.close()
+    good = np.setdiff1d(np.arange(nw), bad)
+    for a, b in zip(*out):
+        assert np.array_equal(a[good], b[good])
+    assert np.all(np.isnan(out[1][0][bad])) and np.all(out[1][2][bad] & 1) and not out[1][2][good].any()
+    assert np.array_equal(out[1][3][bad], np.zeros(len(bad)))
