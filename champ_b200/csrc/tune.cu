@@ -3,7 +3,8 @@
 // The options that change only the speed of a VMC sweep, never its results beyond rounding --
 // "delay_rank", "staged_eval", "move_coop", "orb_coop", and for the tensor-core orbitals of FP32 contexts
 // "orbital_tc" and "orbital_tc_chunk" -- are timed one at a time over a few sweeps of the context's own walkers
-// (device time from CUDA events on the context's stream), and each keeps its fastest value.  The
+// (device time from CUDA events on the context's stream), and each keeps its fastest value; one that the sweeps do
+// not read keeps the value it has.  The
 // result can be stored in a text file under a key of the system's shape and reused.
 #include <cuda_runtime.h>
 
@@ -71,6 +72,17 @@ bool read_cache(const char *path, const std::string &key, std::string &val) {
   return found;
 }
 
+// Options that the context's sweeps do not read with its present mover and evaluation: the batched Gaussian moves take
+// no updates and no proposals one by one, and k_orb_tile has its own stream of coefficients.  They keep their value,
+// which other sweeps of the context may read: timing them would choose by noise.
+bool idle(const champ_ctx *c, const char *name) {
+  const bool gauss = c->mover.kind != 6, batched = gauss && c->move_batch && c->el_staged;
+  if (!strcmp(name, "delay_rank")) return batched;
+  if (!strcmp(name, "move_coop")) return batched || !gauss;
+  if (!strcmp(name, "orb_coop")) return c->orb_tile != 0;
+  return false;
+}
+
 }  // namespace
 
 extern "C" {
@@ -80,7 +92,7 @@ int champ_autotune(champ_ctx *c, int32_t nsweep, uint64_t seed, double step, con
   if (!c) return champ_fail(CHAMP_EINVAL, "null context");
   if (!c->have_walkers) return champ_fail(CHAMP_ESTATE, "no walkers set");
   if (nsweep < 1) return champ_fail(CHAMP_EINVAL, "nsweep < 1");
-  const std::vector<Knob> knobs = {{"delay_rank", {0, 4, 8, 16}}, {"staged_eval", {1, 0}}, {"move_coop", {1, 0}}, {"orb_coop", {1, 0}},
+  const std::vector<Knob> knobs = {{"staged_eval", {1, 0}}, {"delay_rank", {0, 4, 8, 16}}, {"move_coop", {1, 0}}, {"orb_coop", {1, 0}},
                                    {"orbital_tc", {1, 2}}, {"orbital_tc_chunk", {2, 4, 8}}};
   const std::string key = shape_key(c);
   std::string out, cached;
@@ -114,6 +126,11 @@ int champ_autotune(champ_ctx *c, int32_t nsweep, uint64_t seed, double step, con
       int64_t best = cur;
       float best_ms = 1e30f;
       char line[160];
+      if (idle(c, k.name)) {
+        snprintf(line, sizeof line, "%s%s=%lld", chosen.empty() ? "" : " ", k.name, (long long)cur);
+        chosen += line;
+        continue;
+      }
       std::string times;
       for (int64_t v : k.values) {
         if (champ_set_option(c, k.name, v)) continue;

@@ -138,3 +138,26 @@ def test_evaluation_and_sweep_follow_the_oracle(oracle_mod, name, prec):
         assert np.array_equal(st["accept"], ref["accept"])
     assert 0 < st["accept"].sum() < 3 * s.nelec
     eng.close()
+
+
+def test_autotune_times_what_the_sweeps_read(tmp_path):
+    """Options without effect on the batched Gaussian sweeps keep their values, also in the cache; the accelerated
+    mover's delayed updates are timed."""
+    from champ_b200.engine import Engine
+    s = S.cluster128(ncent=8)
+    eng = Engine(s, 64, "mixed")
+    eng.set_walkers(S.initial_walkers(s, 64, seed=3))
+    eng.set_option("delay_rank", 8)
+    eng.set_option("orb_coop", 0)
+    cache = tmp_path / "tune.txt"
+    rep = eng.autotune(nsweep=1, cache=str(cache))
+    assert "staged_eval ms/sweep" in rep
+    assert eng.get_option("staged_eval") == 1  # several times faster
+    for name in ("delay_rank", "move_coop", "orb_coop"):
+        assert name + " ms/sweep" not in rep, rep
+    assert (eng.get_option("delay_rank"), eng.get_option("move_coop"), eng.get_option("orb_coop")) == (8, 1, 0)
+    assert "delay_rank=8 move_coop=1 orb_coop=0" in cache.read_text()
+    eng.set_mover(6)
+    rep = eng.autotune(nsweep=1)
+    assert "delay_rank ms/sweep" in rep and "move_coop ms/sweep" not in rep, rep
+    eng.close()
