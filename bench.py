@@ -42,7 +42,7 @@ FMA_PER_SM_CLK = {"fp64": 64, "fp32": 128}  # FP64 / FP32 fused multiply-adds pe
 # Executed floating-point operations per walker of one sweep phase (2 per FMA, 1 per add/mul, 512
 # per DMMA m8n8k4 warp instruction), counted by ncu (smsp__sass_thread_inst_executed_op_{d,f}{fma,
 # add,mul}_pred_on.sum, sm__inst_executed_pipe_tensor_subpipe_dmma.sum) on a 256-walker sweep of
-# the same kernels and divided by the walkers (profiles/flops_cluster128.md).  "eval" is the FP64
+# the same kernels and divided by the walkers (tables in profiles/).  "eval" is the FP64
 # full evaluation (k_jas_tile, k_orb_tile, k_inv_reg, k_gproj, k_fin_points), "moves" the batched
 # sweep (k_mv_draw, k_mv_prop, k_mv_pairs, k_mv_walk); None until counted: the roofline's
 # achieved figure is then left out.

@@ -1559,7 +1559,7 @@ int champ_create(const champ_system *d, int32_t w_max, int32_t precision, void *
     c->kd.lay = make_layout<double>(c->N, c->C, c->nbasis, c->nmax, c->nomax, c->std_.astride, c->std_.tvstride,
                                     c->std_.gstride, c->std_.wstride, c->nloc > 0, RESIDENT_LIMIT);
     if (!rc) rc = finish_cfg(c->kd);
-    // walker state in HBM: the full evaluation as the four kernels of elstage.cuh
+    // walker state in HBM: the full evaluation as the parts of elstage.cuh
     if (!rc && !c->kd.lay.resident) rc = setup_el_staged(c);
     if (!rc && !c->kd.lay.resident && !c->md.multidet) rc = setup_delay(c);
     // multi-determinant Gaussian moves: the state in shared memory when the moves' part of it fits there

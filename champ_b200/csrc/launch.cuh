@@ -119,7 +119,7 @@ static int run_orb_tc(champ_ctx *c, const State<T> &st) {
   }
 }
 
-// The full evaluation of every walker as the four parts of elstage.cuh (FP64 state in HBM).
+// The full evaluation of every walker as the parts of elstage.cuh (FP64 state in HBM).
 template <class T, int NORD, bool MD>
 static int run_el_staged(champ_ctx *c, const State<T> &st, bool outputs, bool stats, const ElRot &rot,
                          bool rebuild = false) {
@@ -152,7 +152,7 @@ static int run_el_staged(champ_ctx *c, const State<T> &st, bool outputs, bool st
         s, st, c->el_nscr, outputs ? 1 : 0, stats ? 1 : 0, rot, vo ? 1 : 0);
     if (rc) return rc;
     CK(cudaGetLastError());
-    c->orb5_valid = st.orb5 == c->std_.orb5;  // k_el_orb wrote every electron's row
+    c->orb5_valid = st.orb5 == c->std_.orb5;  // the orbital part wrote every electron's row
     return CHAMP_OK;
   }
 }

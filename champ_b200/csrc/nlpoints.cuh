@@ -10,8 +10,8 @@
 //   X_pq(p, j) of the same terms took 6 (10).
 // A lane's fragment element is one (point, electron) pair, so each lane forms its pair's distance
 // and powers once, in place.  The determinant ratio sums the basis functions at the point (lane =
-// point) with the electron's projected G; a primitive whose exponent exceeds the shell's smallest
-// by more than 70 / r^2 is below 1e-30 of the shell and is not formed.
+// point) with the electron's projected G; a primitive whose exponent exceeds the shell's smallest weighing one
+// by more than 70 / r^2 is not formed (gauss_radial).
 // What bounds it: latency between dependent FP64 instructions and mma (an issue in every third cycle; a
 // third of the FP64 pipe), hence the most warps that the registers allow.  Blocks of 8 warps on one walker from 65
 // electrons on put 16 warps on an SM where shared memory holds two such walkers only: 21.0 -> 19.1 ms at 128
@@ -19,7 +19,7 @@
 // warp per walker below that keeps 168 registers with one determinant (0.53 against 0.55 ms), and takes 128
 // with several, whose tables add to the wait for memory (1.07 -> 0.91 ms).
 // Measured (B200), the part of an evaluation from the inverses on, projection included, against k_el_fin:
-// 4096 walkers of 128 electrons and 32 centres, order 4, 46.2 -> 20.1 ms (projection 0.95); 1001 of 51
+// 4096 walkers of 128 electrons and 32 centres, order 4, 46.2 -> 20.2 ms (projection 0.95); 1001 of 51
 // and 13, order 5, 4.57 -> 1.23 ms; 3001 of 20 and 5, 0.96 -> 0.56 ms; the multi-determinant dimer (200
 // determinants), 3.8 -> 0.9 ms.  k_el_fin stays for several centre types with e-e-n terms.
 #pragma once

@@ -324,8 +324,6 @@ __global__ void __launch_bounds__(128, 2) k_pg_pairs(const __grid_constant__ Sys
   const int wpos = WPW == 1 ? 0 : wib;
   double *sm = (double *)(dsm + (WPW == 1 ? D.bytes() * wib : 0));
   double *sd = sm + D.d(), *sh = sm + D.h() + wpos * D.KS * 32, *xs = sm + D.x(), *ss = sm + D.s(), *cen = sm + D.cen(), *zs = sm + D.z();
-  double *lz = zs + jt::SP * 4 * D.KS;
-  (void)lz;
   const int Np = D.Np, Cp = 4 * D.KS, KS = D.KS;
   const double sk = J.scalek, ar = 1.0 / sk, b1 = J.b[0][0], b2 = J.b[0][1], ba = 1.0 + b2 * ar, r1c = ar * ar / (ba * ba);
   const int tpw = 32 * WPW, tid = WPW == 1 ? lane : (int)threadIdx.x;

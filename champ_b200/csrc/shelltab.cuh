@@ -12,7 +12,7 @@ namespace stab {
 // exp(x) for x <= 0 by table and polynomial (P. T. P. Tang, Table-driven implementation of the exponential
 // function in IEEE floating-point arithmetic, ACM TOMS 15, 1989): x = (64 m + j) ln2 / 64 + r, |r| <= ln2 / 128,
 // exp(x) = 2^m t[j] (1 + r + r^2/2 + ... + r^5/120); the omitted term is below 4e-17.  Below -700 it
-// returns 0 (where the result would leave the normal range).
+// returns 0: 1e-304 there, short of the -708 where the result would leave the normal range.
 __device__ __forceinline__ double fast_exp(double x, const double *t) {
   const double magic = 6755399441055744.0;  // 1.5 * 2^52: adding it rounds to an integer in the low word
   const double f = fma(x, 92.332482616893656877, magic);  // 64 / ln 2
@@ -55,8 +55,9 @@ static __device__ __noinline__ double general_radial(const Sys<double> &s, int i
   shell_radial<double, false>(s, ish, r, R);
   return R[0] * ipow(1.0 / r, s.shell[ish].z);
 }
-// Gaussian shells (exponents ascending): primitives below 1e-30 of the shell's widest are not formed (but for
-// the second of a pair).  Two primitives at a time: an exponential is a chain of ten dependent FP64
+// Gaussian shells (exponents ascending): a primitive is not formed (but for the second of a pair) where its
+// exponential is below e^-70 = 4e-31 of that of the widest primitive that weighs -- at least 1e-8 of the shell's
+// largest weight -- hence below 4e-23 of that primitive's value.  Two primitives at a time: an exponential is a chain of ten dependent FP64
 // operations, and the callers have too few warps in flight to fill it.  Small walkers' evaluation 0.97 -> 0.91 ms
 // (8192 of 8 electrons), their DMC step 3.28 -> 3.18 ms; the projected points of 3001 walkers of 20 electrons
 // 0.53 -> 0.52 ms.

@@ -1,6 +1,8 @@
 """The 8-lanes-per-walker kernels at the numbers of walkers that they serve (on 148 SMs more than 2368 for DMC and
 T-moves, 2072 for Gaussian moves, 4736 for the E_L of a mixed-precision sweep), walker by walker against the oracle
 and against the kernels with a warp per walker."""
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -125,3 +127,34 @@ def test_singular_walkers_leave_their_matrix():
         assert np.array_equal(a[good], b[good])
     assert np.all(np.isnan(out[1][0][bad])) and np.all(out[1][2][bad] & 1) and not out[1][2][good].any()
     assert np.array_equal(out[1][3][bad], np.zeros(len(bad)))
+
+
+def test_exponential_of_the_shell_tables(oracle_mod):
+    """Local energies of one electron in three contracted s shells about a bare nucleus, from 1e-3 bohr to where the
+    tightest primitives are not formed and on: a ratio of sums of the tables' exponentials.  A primitive's relative
+    error is 2 ulp of its argument z r^2 (below 70 where it counts) and 2 of its own, 4e-14 at most; a term of the
+    Laplacian is up to 6 z + 4 z^2 r^2 times the function."""
+    from champ_b200.engine import Engine
+    base = S.cluster128(ncent=1, box=3.5, norb=1)
+    z = np.array([0.05, 0.9, 12.0, 0.08, 2.0, 0.3, 6.0, 40.0])
+    one = np.zeros(3, np.int32)
+    s = dataclasses.replace(
+        base, nelec=1, nup=1, cent=np.zeros((1, 3)), shell_cent=one, shell_n=one + 1, shell_l=one, shell_kind=one + 1,
+        shell_nprim=np.array([3, 2, 3], np.int32), prim_zeta=z, prim_coef=np.array([0.4, 0.7, 0.3, 0.8, -0.2, 0.5, 0.4, 0.6]),
+        basis_shell=np.arange(3, dtype=np.int32), basis_m=one, coef=np.array([[0.6, 0.5, 0.7]]), det_orb=np.zeros((1, 1), np.int32),
+        nloc=0, nordc=0, een_cusp=0, c=np.zeros((1, 0)), a4=np.zeros_like(base.a4), b=np.zeros_like(base.b))
+    rng = np.random.default_rng(6)
+    r = np.exp(np.linspace(np.log(1e-3), np.log(25.0), 3000))
+    u = rng.standard_normal((3000, 3))
+    x = (r[:, None] * u / np.linalg.norm(u, axis=1, keepdims=True))[:, None, :]
+    eng = Engine(s, 3000, "fp64")
+    eng.set_walkers(x)
+    st = eng.vmc_sweeps(1, seed=3, sweep0=0, step=1e-6)
+    y = eng.get_walkers()
+    eng.close()
+    orc = oracle_mod.Oracle(s)
+    e = np.array([orc.eval(p)["energy"] for p in y])
+    rr = np.linalg.norm(y[:, 0], axis=1)
+    zmax = np.minimum(40.0, 70.0 / rr ** 2 + 0.05)  # the tightest exponent that counts
+    bound = 1e-13 * (6 * zmax + 4 * zmax ** 2 * rr ** 2 + s.znuc[0] / rr)
+    assert np.all(np.abs(st["elast"] - e) <= bound)
