@@ -16,9 +16,63 @@ __host__ __device__ constexpr int ldb() { return 16 * NT + 4; }
 template <int NT>
 __host__ __device__ constexpr size_t smem_bytes() { return sizeof(double) * (size_t)KB * (LDA + ldb<NT>()); }
 
-// A shell's functions of one electron (out of line: its registers are not those of the contraction, and the
-// compiler fuses the same products with their sums as in warp_basis).
-static __device__ __noinline__ void shell5(const Sys<double> &s, int ish, double x, double y, double z, double *o) {
+// A Gaussian shell with n = l + 1, l <= 2, of one electron: the operations of shell_eval_put with the products fused
+// with their sums as the compiler fuses them in warp_basis, written out, so that the bits are the same
+// wherever it is inlined and l is a constant.
+template <int l>
+__device__ __forceinline__ void gauss_shell5(const Sys<double> &s, int2 pr, double d0, double d1, double d2, double *o) {
+  double r = sqrt(__dadd_rn(__fma_rn(d0, d0, __dmul_rn(d1, d1)), __dmul_rn(d2, d2)));
+  if (r == 0.0) { r = 1e-30; d0 = r; }
+  const double ri = 1.0 / r, rm1 = l == 0 ? 1.0 : l == 1 ? r : __dmul_rn(r, r), rm2 = __dmul_rn(rm1, ri), rm3 = __dmul_rn(rm2, ri);
+  double R0 = 0, R1 = 0, R2 = 0;
+#pragma unroll 2
+  for (int p = pr.x; p < pr.x + pr.y; p++) {
+    const double zr = __dmul_rn(__dmul_rn(2 * s.pz[p], r), r), ex = __dmul_rn(s.pc[p], exp(-0.5 * zr));
+    R0 = __fma_rn(rm1, ex, R0);
+    R1 = __dadd_rn(R1, __dmul_rn(__dmul_rn(rm2, __dadd_rn(l, -zr)), ex));
+    R2 = __dadd_rn(R2, __dmul_rn(__dmul_rn(rm3, __fma_rn(__dadd_rn(zr, -(2 * l + 1)), zr, l * (l - 1))), ex));
+  }
+  const double ril = l == 0 ? 1.0 : l == 1 ? ri : __dmul_rn(ri, ri), d[3] = {d0, d1, d2};
+  const double lap = __fma_rn(-__dmul_rn(__dmul_rn(l * (l + 1), ri), ri), R0, __fma_rn(2 * ri, R1, R2));
+  // function S, its gradient G (zero where Z says so)
+  auto put = [&](int sl, double S, const double *G, const int *Z) {
+    const double Y = __dmul_rn(S, ril), lr = __dmul_rn(__dmul_rn(__dmul_rn(l * S, ril), ri), ri);
+    o[sl * LDA] = __dmul_rn(Y, R0);
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      const double a = __dmul_rn(__dmul_rn(Y, d[k]), ri);
+      double v = __dmul_rn(a, R1);
+      if (l > 0) {
+        const double q = -__dmul_rn(lr, d[k]);
+        v = __fma_rn(a, R1, __dmul_rn(Z[k] ? __fma_rn(G[k], ril, q) : q, R0));
+      }
+      o[sl * LDA + (k + 1) * EB] = v;
+    }
+    o[sl * LDA + 4 * EB] = __dmul_rn(Y, lap);
+  };
+  if constexpr (l == 0) {
+    put(0, 1.0, nullptr, nullptr);
+  } else if constexpr (l == 1) {
+    const double G[3] = {1.0, 1.0, 1.0};
+    const int Z[3][3] = {{0, 0, 1}, {1, 0, 0}, {0, 1, 0}};
+    put(0, d2, G, Z[0]);
+    put(1, d0, G, Z[1]);
+    put(2, d1, G, Z[2]);
+  } else {
+    const double s3 = 1.7320508075688772, x2 = __dmul_rn(d0, d0), y2 = __dmul_rn(d1, d1);
+    const double sx = __dmul_rn(s3, d0), sy = __dmul_rn(s3, d1), sz = __dmul_rn(s3, d2);
+    const double G[5][3] = {{-d0, -d1, 2 * d2}, {sz, 0.0, sx}, {0.0, sz, sy}, {sx, -sy, 0.0}, {sy, sx, 0.0}};
+    const int Z[5][3] = {{1, 1, 1}, {1, 0, 1}, {0, 1, 1}, {1, 1, 0}, {1, 1, 0}};
+    put(0, 0.5 * __dadd_rn(2 * __dmul_rn(d2, d2), -__dadd_rn(x2, y2)), G[0], Z[0]);
+    put(1, __dmul_rn(sx, d2), G[1], Z[1]);
+    put(2, __dmul_rn(sy, d2), G[2], Z[2]);
+    put(3, __dmul_rn(0.5 * s3, __dadd_rn(x2, -y2)), G[3], Z[3]);
+    put(4, __dmul_rn(sx, d1), G[4], Z[4]);
+  }
+}
+// Any other shell (out of line: its registers are not those of the contraction, and the compiler fuses there
+// what it fuses in warp_basis).
+static __device__ __noinline__ void general_shell5(const Sys<double> &s, int ish, double x, double y, double z, double *o) {
   const double pt[3] = {x, y, z};
   shell_eval_put<double, 5>(s, ish, pt, [o](int sl, int c, double v) { o[sl * LDA + c * EB] = v; });
 }
@@ -35,10 +89,10 @@ static __device__ __noinline__ void shell5(const Sys<double> &s, int ish, double
 // be so: where psi nearly vanishes the inverse magnifies the last bit of a row by the condition number (ratios
 // of an 80-electron cluster's first moves then differ by 3e-9), and the accelerated mover, whose proposals follow
 // the drift, magnifies it again with every sweep (its walks came apart).
-// What bounds it: the FP64 pipe (about a third of it the basis functions).  Measured (B200): 4096
-// walkers of 128 electrons, 416 basis functions, 15.6 -> 9.2 ms; 1001 of 51 electrons 1.25 -> 0.59; 3001 of 20 electrons, 65
-// functions, 0.32 -> 0.27.  Basis functions by shelltab.cuh's exponential and formulas took 6.0, 0.33 and 0.13 ms,
-// and split the walks; so does shell5 inlined (8.1 ms; other products are then fused with their sums).
+// What bounds it: the FP64 pipe (about a fourth of it the basis functions).  Measured (B200): 4096
+// walkers of 128 electrons, 416 basis functions, 15.6 -> 7.2 ms; two sweeps of 1001 of 51 electrons 1.25 -> 0.42; 3001 of 20
+// electrons, 65 functions, 0.32 -> 0.18.  Basis functions by shelltab.cuh's exponential and formulas took 6.0, 0.33 and
+// 0.13 ms, and split the walks; shell_eval_put out of line 9.2 ms (indexed arrays in local memory).
 // k_el_orb stays for more than 64 orbitals of a spin, and for one or two (32 or 16 interleaved sums each).
 // chunk[k]: first shell, shells, first basis function, basis functions.
 // ALL: the columns blockIdx.y * 16 NT onwards of all orbitals (s.call), for every electron, into all + w
@@ -97,7 +151,18 @@ __global__ void __launch_bounds__(THREADS, 2) k_orb_tile(const __grid_constant__
       for (int c = 0; c < 5; c++) phi[r * LDA + c * EB + lane] = 0.0;
     for (int q = wib; q < ch.y; q += 8) {
       const int ish = ch.x + q;
-      shell5(s, ish, px[0], px[1], px[2], phi + (s.shb0[ish] - ch.z) * LDA + lane);
+      const int4 sh = s.shell[ish];
+      double *o = phi + (s.shb0[ish] - ch.z) * LDA + lane;
+      if (sh.w != 1 || sh.y != sh.z + 1 || sh.z > 2) {
+        general_shell5(s, ish, px[0], px[1], px[2], o);
+        continue;
+      }
+      const int2 pr = s.shprim[ish];
+      const double *cc = s.cent + 3 * sh.x;
+      const double d0 = px[0] - cc[0], d1 = px[1] - cc[1], d2 = px[2] - cc[2];
+      if (sh.z == 0) gauss_shell5<0>(s, pr, d0, d1, d2, o);
+      else if (sh.z == 1) gauss_shell5<1>(s, pr, d0, d1, d2, o);
+      else gauss_shell5<2>(s, pr, d0, d1, d2, o);
     }
     cp_async_wait<0>();
     __syncthreads();
