@@ -112,6 +112,8 @@ struct champ_ctx {
   double *pg_raw = nullptr;
   int small = 0;  // small walkers: FP64 kernels with 8 lanes per walker (small.cu), shells by l
   int *small_order = nullptr;
+  int4 *small_chunk = nullptr;  // and in chunks for the accelerated moves
+  int small_nchunk = 0;
   int move_batch = 0;  // the Gaussian sweeps run as batched moves
   // device staging for per-call host arrays
   double *d_in = nullptr, *d_out = nullptr;
@@ -249,7 +251,7 @@ int pg_tile_fwd(champ_ctx *c);
 int pg_tile_bwd(champ_ctx *c);
 // small walkers (small.cu); setup sets champ_ctx::small where they apply, small_serves adds the rule on the
 // number of walkers
-enum class SmallOp { Eval, Gauss, Dmc };
+enum class SmallOp { Eval, Gauss, Accel, Dmc };
 int small_setup(champ_ctx *c);
 bool small_serves(const champ_ctx *c, SmallOp op, int W);
 int small_eval(champ_ctx *c, const State<double> &st, const ElRot &rot);

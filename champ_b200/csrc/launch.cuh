@@ -283,7 +283,7 @@ static int launch_t(champ_ctx *c, Op op, const OpArgs &a) {
     }
     CK(cudaMemsetAsync(st.s_esum, 0, sizeof(double) * 3 * (size_t)c->wmax, c->stream));  // esum, e2sum, acc
     if constexpr (std::is_same<T, double>::value)
-      if (!a.st_override && c->mover.kind != 6 && small_serves(c, SmallOp::Gauss, st.W)) return small_vmc(c, st, a);
+      if (!a.st_override && small_serves(c, c->mover.kind == 6 ? SmallOp::Accel : SmallOp::Gauss, st.W)) return small_vmc(c, st, a);
     const bool tc = c->tc_on && !a.st_override;  // only FP32 contexts turn it on
     if (!tc) {
       auto kern = c->mover.kind == 6 ? k_vmc<T, NORD, MD, 0, 6> : k_vmc<T, NORD, MD, 0>;

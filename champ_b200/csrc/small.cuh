@@ -17,8 +17,8 @@
 // A single walker takes longer on 8 lanes than on 32, so few walkers stay with a warp each (small_serves).
 // Measured (B200) against a warp per walker: dimer of 8 electrons, order 4, 8192 walkers, evaluation
 // 1.04 -> 0.90 ms; DMC step of about the same population 10.0 -> 3.2 ms; C2, order 5, DMC step 1.33 -> 0.69 ms,
-// T-moves 1.28 -> 0.82 ms.  Accelerated sweeps, which follow the last bit of the drift, and evaluations of walkers
-// that a caller supplies stay with a warp per walker (small_serves).
+// T-moves 1.28 -> 0.82 ms; its accelerated sweep of 8192 walkers 8.0 -> 5.1 ms (k_small_accel, whose sums are those
+// of a warp per walker).
 #pragma once
 #include "jastile.cuh"
 
@@ -30,11 +30,12 @@ constexpr int GS = 8;  // lanes of a walker
 constexpr int NO = 4;  // most electrons (= orbitals) of a spin
 constexpr int NE = 8;  // most electrons
 constexpr int RCAP = 96;  // radial values of the tasks' centres kept per walker
+constexpr int ACH = 24;   // basis functions formed at a time by k_small_accel
 
 // Doubles of a walker in shared memory.
 struct Lay {
-  int N, C, qm;
-  __host__ __device__ Lay(int N_, int C_, int nord) : N(N_), C(C_), qm(nord > 1 ? nord - 1 : 1) {}
+  int N, C, qm, ext;  // ext: basis functions beside the rows (k_small_accel)
+  __host__ __device__ Lay(int N_, int C_, int nord, int ext_ = 0) : N(N_), C(C_), qm(nord > 1 ? nord - 1 : 1), ext(ext_) {}
   __host__ __device__ int ai() const { return 3 * N; }
   __host__ __device__ int f() const { return ai() + 2 * NO * NO; }
   __host__ __device__ int a() const { return f() + N * N; }
@@ -46,7 +47,7 @@ struct Lay {
   __host__ __device__ int pl() const { return pr() + 5 * NO; }   // [C][GS] a point's scaled distances per lane
   __host__ __device__ int row() const { return pl() + C * GS; }  // rows [N][5][NO]; then the tasks
   __host__ __device__ int rlen() const {
-    const int t = N * C * NLT + RCAP, r = N * 5 * NO, u = 2 * MAXQ;  // u: a T-move's elements and ratios
+    const int t = N * C * NLT + RCAP, r = N * 5 * NO + ext, u = 2 * MAXQ;  // u: a T-move's elements and ratios
     return t > r ? (t > u ? t : u) : (r > u ? r : u);
   }
   // odd, so that the walkers of a warp start in different banks
@@ -59,6 +60,11 @@ struct Args {
   double step = 0;
   ElRot rot{};
   const int *order = nullptr;  // shells by l, so that the lanes of a round mostly share it
+  // accelerated moves: whole shells of up to ACH functions (first shell, shells, first function, functions), and
+  // every how many sweeps the inverses are formed anew
+  const int4 *chunk = nullptr;
+  int nchunk = 0, reinv = 1;
+  Mover mv{1, 5.0, 1.0, 1.0};
   DmcPar P{};
   DmcData D{};
   double tau = 0;
@@ -620,17 +626,18 @@ __device__ __noinline__ double point_psi(const Sys<double> &s, const stab::Tab &
 
 // E_L and everything it leaves behind (full_eval) from the rows and positions in shared memory.
 struct Res {
-  double eloc, v2;
+  double eloc, v2, lnd, sgn;
 };
 template <int NORD>
 __device__ __forceinline__ Res evaluate(const Sys<double> &s, const stab::Tab &T, const JasPar<double> &J, const EcpPar &E, const State<double> &st,
-                                        int w, double *v, const Lay &L, const ElRot &rot) {
+                                        int w, double *v, const Lay &L, const ElRot &rot, bool anew = true, double lnd = 0,
+                                        double sgn = 1) {
   const int sub = threadIdx.x & 7, N = s.N, C = s.C;
   const unsigned m = gmask();
   const double sk = J.scalek;
-  double lnd, sgn;
-  invert(s, v, L, lnd, sgn);
-  const bool ok = sgn != 0.0;
+  if (anew) invert(s, v, L, lnd, sgn);  // else the inverses, ln|D| and sign as the moves left them
+  const bool ok = sgn != 0.0 && (anew || isfinite(lnd));
+  if (!ok) sgn = 0.0;
   // ---- distances and power sums, lane = electron
   double pe_en = 0, fen = 0, vj[3] = {0, 0, 0}, d2j = 0, pe_ee = 0, fsum = 0;
   const bool act = sub < N;
@@ -776,11 +783,13 @@ __device__ __forceinline__ Res evaluate(const Sys<double> &s, const stab::Tab &T
   const double pe = s.pecent + pe_ee + (s.nloc > 0 ? vloc + vnl : pe_en), d2 = d2lnd + d2j;
   Res res;
   res.v2 = v2;
+  res.lnd = ok ? lnd : -INFINITY;
+  res.sgn = sgn;
   res.eloc = ok ? pe - HB * (d2 + v2) : nan("");
   if (sub == 0) {
     const double lnpsi = lnd + fsum;
     st.fsum[w] = fsum;
-    st.lnd[w] = ok ? lnd : -INFINITY;
+    st.lnd[w] = res.lnd;
     st.sgn[w] = sgn;
     uint32_t flag = 0;
     if (!ok) flag |= CHAMP_WS_SINGULAR;
@@ -937,6 +946,309 @@ __global__ void __launch_bounds__(128, 3) k_small(const __grid_constant__ Sys<do
       atomicAdd(&A.D.red[1], swe);
     }
     for (int i = W + blockIdx.x * blockDim.x + (int)threadIdx.x; i < A.P.wmax; i += gridDim.x * blockDim.x) A.D.ncopy[i] = 0;
+  }
+}
+
+// ---- accelerated Metropolis moves (metrop_slat_mov1.f90:82-546).  A proposal follows the drift, and each move
+// changes the next electron's drift: a walk magnifies the last bit of whatever it is formed from, 1e-16 to 6e-3 bohr
+// within four sweeps for the worst of 8192 walkers of the dimer.  So everything a proposal depends on is formed
+// here by the operations, in the order, of a warp per walker (propose, accept_move, k_vmc): basis functions
+// and their interleaved sums, the drift and its sums over lanes, the inverse's updates and when it is formed anew.
+// With Gaussian shells up to d the walks are the same to the bit; with others (shell_eval_put as compiled here) to
+// rounding, which their examples magnify little: positions of C2 3e-10 bohr after 15 sweeps, of Be 1e-12.
+// k_small's cheaper sums took 2.6 ms for a sweep of 8192 walkers of C2, a warp per walker takes 8.0, this 5.1.
+
+// A Gaussian shell with n = l + 1, l <= 2, [slot][channel]: the operations of shell_eval_put with those products
+// fused with their sums that the compiler fuses in k_vmc.
+template <int l>
+__device__ __forceinline__ void gauss_shell5(const Sys<double> &s, int2 pr, double d0, double d1, double d2, double *o) {
+  double r = sqrt(__fma_rn(d2, d2, __fma_rn(d0, d0, __dmul_rn(d1, d1))));
+  if (r == 0.0) { r = 1e-30; d0 = r; }
+  const double ri = 1.0 / r, rm1 = l == 0 ? 1.0 : l == 1 ? r : __dmul_rn(r, r), rm2 = __dmul_rn(rm1, ri), rm3 = __dmul_rn(rm2, ri);
+  double R0 = 0, R1 = 0, R2 = 0;
+#pragma unroll 2
+  for (int p = pr.x; p < pr.x + pr.y; p++) {
+    const double zr = __dmul_rn(__dmul_rn(2 * s.pz[p], r), r), ex = __dmul_rn(s.pc[p], exp(-0.5 * zr));
+    R0 = __fma_rn(rm1, ex, R0);
+    R1 = __dadd_rn(R1, __dmul_rn(__dmul_rn(rm2, __dadd_rn(l, -zr)), ex));
+    R2 = __dadd_rn(R2, __dmul_rn(__dmul_rn(rm3, __dadd_rn(l * (l - 1), -__dmul_rn(__dadd_rn(2 * l + 1, -zr), zr))), ex));
+  }
+  const double ril = l == 0 ? 1.0 : l == 1 ? ri : __dmul_rn(ri, ri), d[3] = {d0, d1, d2};
+  const double lap = __fma_rn(-__dmul_rn(__dmul_rn(l * (l + 1), ri), ri), R0, __fma_rn(2 * ri, R1, R2));
+  // function S, its gradient G (zero where Z says so)
+  auto put = [&](int sl, double S, const double *G, const int *Z) {
+    const double Y = __dmul_rn(S, ril), lr = __dmul_rn(__dmul_rn(__dmul_rn(l * S, ril), ri), ri);
+    o[sl * 5] = __dmul_rn(Y, R0);
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      const double a = __dmul_rn(__dmul_rn(Y, d[k]), ri);
+      double v = __dmul_rn(a, R1);
+      if (l > 0) {
+        const double q = -__dmul_rn(lr, d[k]);
+        v = __fma_rn(a, R1, __dmul_rn(Z[k] ? __fma_rn(G[k], ril, q) : q, R0));
+      }
+      o[sl * 5 + k + 1] = v;
+    }
+    o[sl * 5 + 4] = __dmul_rn(Y, lap);
+  };
+  if constexpr (l == 0) {
+    put(0, 1.0, nullptr, nullptr);
+  } else if constexpr (l == 1) {
+    const double G[3] = {1.0, 1.0, 1.0};
+    const int Z[3][3] = {{0, 0, 1}, {1, 0, 0}, {0, 1, 0}};
+    put(0, d2, G, Z[0]);
+    put(1, d0, G, Z[1]);
+    put(2, d1, G, Z[2]);
+  } else {
+    const double s3 = 1.7320508075688772, x2 = __dmul_rn(d0, d0);
+    const double sx = __dmul_rn(s3, d0), sy = __dmul_rn(s3, d1), sz = __dmul_rn(s3, d2);
+    const double G[5][3] = {{-d0, -d1, 2 * d2}, {sz, 0.0, sx}, {0.0, sz, sy}, {sx, -sy, 0.0}, {sy, sx, 0.0}};
+    const int Z[5][3] = {{1, 1, 1}, {1, 0, 1}, {0, 1, 1}, {1, 1, 0}, {1, 1, 0}};
+    put(0, 0.5 * __dadd_rn(2 * __dmul_rn(d2, d2), -__fma_rn(d1, d1, x2)), G[0], Z[0]);
+    put(1, __dmul_rn(sx, d2), G[1], Z[1]);
+    put(2, __dmul_rn(sy, d2), G[2], Z[2]);
+    put(3, __dmul_rn(0.5 * s3, __fma_rn(-d1, d1, x2)), G[3], Z[3]);
+    put(4, __dmul_rn(sx, d1), G[4], Z[4]);
+  }
+}
+static __device__ __noinline__ void general_shell5(const Sys<double> &s, int ish, double x, double y, double z, double *o) {
+  const double pt[3] = {x, y, z};
+  shell_eval_put<double, 5>(s, ish, pt, [o](int sl, int c, double v) { o[sl * 5 + c] = v; });
+}
+
+// The orbital row at a point into out [5][NO]: warp_orbitals' sums of up to LM orbitals, 32 / LM interleaved ones
+// per orbital -- G = 4 / LM of them in each lane -- and their tree.  phi: ACH basis functions.
+template <int LM>
+__device__ __noinline__ void accel_row(const Sys<double> &s, const int4 *chunk, int nchunk, int sp, double x, double y, double z, double *phi,
+                                       double *out) {
+  constexpr int G = 4 / LM;
+  const int sub = threadIdx.x & 7, no = s.nocc[sp];
+  const unsigned m = gmask();
+  const double *cf = s.cocc[sp];
+  double o[5][4];
+#pragma unroll
+  for (int c = 0; c < 5; c++)
+#pragma unroll
+    for (int k = 0; k < 4; k++) o[c][k] = 0;
+  for (int q = 0; q < nchunk; q++) {
+    const int4 ch = chunk[q];
+    for (int h = sub; h < ch.y; h += GS) {
+      const int ish = ch.x + h;
+      const int4 sh = s.shell[ish];
+      double *f = phi + (s.shb0[ish] - ch.z) * 5;
+      if (sh.w != 1 || sh.y != sh.z + 1 || sh.z > 2) {
+        general_shell5(s, ish, x, y, z, f);
+        continue;
+      }
+      const int2 pr = s.shprim[ish];
+      const double *cc = s.cent + 3 * sh.x;
+      if (sh.z == 0) gauss_shell5<0>(s, pr, x - cc[0], y - cc[1], z - cc[2], f);
+      else if (sh.z == 1) gauss_shell5<1>(s, pr, x - cc[0], y - cc[1], z - cc[2], f);
+      else gauss_shell5<2>(s, pr, x - cc[0], y - cc[1], z - cc[2], f);
+    }
+    __syncwarp(m);
+    for (int b = ch.z + ((sub - ch.z) & 7); b < ch.z + ch.w; b += GS) {
+      const double *p = phi + (b - ch.z) * 5;
+#pragma unroll
+      for (int g = 0; g < G; g++)
+        if (((b >> 3) & (G - 1)) == g)
+#pragma unroll
+          for (int k = 0; k < LM; k++)
+            if (k < no) {
+              const double c = cf[(size_t)b * no + k];
+#pragma unroll
+              for (int i = 0; i < 5; i++) o[i][g * LM + k] += c * p[i];
+            }
+    }
+    __syncwarp(m);
+  }
+#pragma unroll
+  for (int c = 0; c < 5; c++) {
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+#pragma unroll
+      for (int d = 1; d < 8; d <<= 1) o[c][k] += __shfl_xor_sync(m, o[c][k], d);
+#pragma unroll
+    for (int d = 1; d < G; d <<= 1)
+#pragma unroll
+      for (int g = 0; g < G; g += 2 * d)
+#pragma unroll
+        for (int k = 0; k < LM; k++) o[c][g * LM + k] += o[c][(g + d) * LM + k];
+#pragma unroll
+    for (int k = 0; k < NO; k++)
+      if (((c * NO + k) & 7) == sub) out[c * NO + k] = k < LM ? o[c][k < LM ? k : 0] : 0.0;
+  }
+  __syncwarp(m);
+}
+__device__ __forceinline__ void accel_orbitals(const Sys<double> &s, const Args &A, int e, const double *x, double *phi, double *out) {
+  const int sp = e < s.nup ? 0 : 1, no = s.nocc[sp];
+  if (no > 2) accel_row<4>(s, A.chunk, A.nchunk, sp, x[0], x[1], x[2], phi, out);
+  else if (no > 1) accel_row<2>(s, A.chunk, A.nchunk, sp, x[0], x[1], x[2], phi, out);
+  else accel_row<1>(s, A.chunk, A.nchunk, sp, x[0], x[1], x[2], phi, out);
+}
+
+// propose() of electron e at xn with the orbital row r: determinant ratio, Jastrow change and drift; this lane's
+// pair value in pf (lane e: the e-n term).  Distances: ren [N][C][2] in the place of a and h, rnew [C][2] of pa and ph.
+template <int NORD>
+__device__ __noinline__ void accel_propose(const Sys<double> &s, const JasPar<double> &J, double *v, int e, const double *xn, const double *r,
+                                           double &rho, double &dj, double &pf, double *grad) {
+  const Lay L(s.N, s.C, NORD);
+  const int sub = threadIdx.x & 7, N = s.N, C = s.C;
+  const unsigned m = gmask();
+  double *rnew = v + L.pa();
+  const double *ren = v + L.a(), *fso = v + L.f();
+  for (int c = sub; c < C; c += GS) {
+    double q, d;
+    cen_dist(s, J.scalek, xn, c, q, d);
+    rnew[2 * c] = q;
+    rnew[2 * c + 1] = d;
+  }
+  __syncwarp(m);
+  const int sp = e < s.nup ? 0 : 1, n = sp ? s.ndn : s.nup, eo = sp ? e - s.nup : e;
+  const double *Ai = v + L.ai() + sp * NO * NO + eo;
+  double t[4];  // lanes k = 0 .. 3 of the warp's sums, which add k and k + 2 first
+#pragma unroll
+  for (int c = 0; c < 4; c++) {
+    double q[NO];
+#pragma unroll
+    for (int k = 0; k < NO; k++) q[k] = k < n ? __dmul_rn(Ai[k * NO], r[c * NO + k]) : 0.0;
+    t[c] = (q[0] + q[2]) + (q[1] + q[3]);
+  }
+  rho = t[0];
+  double d = 0, g[4][3], fen[4];  // of this lane and those 8, 16 and 24 above it
+#pragma unroll
+  for (int i = 0; i < 4; i++) fen[i] = g[i][0] = g[i][1] = g[i][2] = 0;
+  double f = 0;
+  if (sub < N && sub != e) {
+    f = pair_value<double, NORD, true>(s, J, e, sub, xn, rnew, v + 3 * sub, ren + 2 * C * sub, g[0]);
+    d = f - fso[e * N + sub];
+  }
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+    for (int c = sub + 8 * i; c < C; c += 32) {
+      double fi = 0, fii = 0;
+      fen[i] += jas_en<double, true>(J, s.ctype[c], rnew[2 * c], rnew[2 * c + 1], fi, fii);
+      const double *cc = s.cent + 3 * c;
+      g[i][0] += fi * (xn[0] - cc[0]);
+      g[i][1] += fi * (xn[1] - cc[1]);
+      g[i][2] += fi * (xn[2] - cc[2]);
+    }
+  const double fent = gsum((fen[0] + fen[2]) + (fen[1] + fen[3]), m);
+  if (sub == 0) d += fent - fso[e * N + e];
+  dj = gsum(d, m);
+  pf = sub == e ? fent : f;
+#pragma unroll
+  for (int k = 0; k < 3; k++) grad[k] = gsum((g[0][k] + g[2][k]) + (g[1][k] + g[3][k]), m) + t[1 + k] / rho;
+}
+
+// accept_move() of electron e at xn.
+__device__ __forceinline__ void accel_accept(const Sys<double> &s, double *v, const Lay &L, int e, const double *xn, double pf) {
+  const int sub = threadIdx.x & 7, N = s.N, C = s.C;
+  const unsigned m = gmask();
+  const int sp = e < s.nup ? 0 : 1, n = sp ? s.ndn : s.nup, eo = sp ? e - s.nup : e;
+  double *A = v + L.ai() + sp * NO * NO;
+  const double *r = v + L.pr();
+  auto vb = [&](int j) {
+    double a = 0;
+#pragma unroll
+    for (int k = 0; k < NO; k++)
+      if (k < n) a += r[k] * A[k * NO + j];
+    return a - (j == eo ? 1.0 : 0.0);
+  };
+  const double rinv = 1.0 / (vb(eo) + 1.0);
+  double nv[2];
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const int i = sub + GS * h, k = i / NO, j = i & (NO - 1);
+    nv[h] = A[i] - A[k * NO + eo] * vb(j) * rinv;
+  }
+  __syncwarp(m);
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const int i = sub + GS * h;
+    if (i / NO < n && (i & (NO - 1)) < n) A[i] = nv[h];
+  }
+  if (sub < N) {
+    v[L.f() + e * N + sub] = pf;
+    v[L.f() + sub * N + e] = pf;
+  }
+  for (int i = sub; i < 2 * C; i += GS) v[L.a() + 2 * C * e + i] = v[L.pa() + i];
+  if (sub < 3) v[3 * e + sub] = xn[sub];
+  for (int i = sub; i < 5 * NO; i += GS) v[L.row() + e * 5 * NO + i] = r[i];
+  __syncwarp(m);
+}
+
+template <int NORD>
+__global__ void __launch_bounds__(128, 3) k_small_accel(const __grid_constant__ Sys<double> s, const __grid_constant__ State<double> st,
+                                                        const __grid_constant__ Args A) {
+  __shared__ JasPar<double> J;
+  __shared__ EcpPar E;
+  extern __shared__ __align__(16) char dsm[];
+  const stab::Tab T = stab::stage(s, dsm);
+  load_params(s, J, E);
+  const Lay L(s.N, s.C, NORD, 5 * ACH);
+  const int N = s.N, C = s.C, sub = threadIdx.x & 7, grp = threadIdx.x >> 3;
+  const unsigned m = gmask();
+  double *v = (double *)(dsm + stab::tab_smem(s.nshell, s.nprim)) + (size_t)grp * L.total();
+  double *phi = v + L.row() + N * 5 * NO, *pr = v + L.pr();
+  const int w = blockIdx.x * (blockDim.x / GS) + grp;
+  if (w >= st.W) return;
+  for (int i = sub; i < 3 * N; i += GS) v[i] = st.x[(size_t)w * 3 * N + i];
+  for (int sp = 0; sp < 2; sp++) {
+    const int n = sp ? s.ndn : s.nup;
+    const double *a = st.ainv + (size_t)w * st.astride + (sp ? s.nup * s.nup : 0);
+    for (int i = sub; i < n * n; i += GS) v[L.ai() + sp * NO * NO + (i / n) * NO + i % n] = a[i];
+  }
+  for (int i = sub; i < N * N; i += GS) v[L.f() + i] = st.fso[(size_t)w * N * N + i];
+  double lnd = st.lnd[w], sgn = st.sgn[w], es = 0, e2 = 0, acc = 0, el = 0;
+  __syncwarp(m);
+  for (int isw = 0; isw < A.nsweep; isw++) {
+    const uint64_t sweep = A.sweep0 + (uint64_t)isw;
+    for (int i = sub; i < N * C; i += GS) cen_dist(s, J.scalek, v + 3 * (i / C), i % C, v[L.a() + 2 * i], v[L.a() + 2 * i + 1]);
+    for (int e = 0; e < N; e++) accel_orbitals(s, A, e, v + 3 * e, phi, v + L.row() + e * 5 * NO);
+    for (int e = 0; e < N; e++) {
+      const double xo[3] = {v[3 * e], v[3 * e + 1], v[3 * e + 2]};
+      double rho, dj, pf, go[3], gn[3], xn[3], fxop, areao, rtry, p = 0;
+      accel_propose<NORD>(s, J, v, e, xo, v + L.row() + e * 5 * NO, rho, dj, pf, go);
+      MoveRng rng{A.seed, (uint32_t)w, (uint32_t)sweep, (uint32_t)(sweep >> 32), (uint32_t)e, 0u, {0.0, 0.0}, 0};
+      slat_forward(s, A.mv, xo, go, rng, xn, fxop, areao, rtry);
+      SlatBack b;
+      if (slat_geometry(s, A.mv, xo, xn, b)) {
+        double fxnp, arean;
+        __syncwarp(m);
+        accel_orbitals(s, A, e, xn, phi, pr);
+        accel_propose<NORD>(s, J, v, e, xn, pr, rho, dj, pf, gn);
+        slat_reverse(s, A.mv, b, gn, fxnp, arean);
+        const double rr = rtry / b.rminon;
+        p = rr * rr * rho * rho * exp(2.0 * dj) * fabs((fxnp * areao) / (fxop * arean));
+      }
+      if (rng.next() < p) {
+        accel_accept(s, v, L, e, xn, pf);
+        lnd += log(fabs(rho));
+        if (rho < 0) sgn = -sgn;
+        acc += 1;
+      }
+      __syncwarp(m);
+    }
+    ElRot rot{};
+    rot.random = 1;
+    rot.seed = A.seed;
+    rot.sweep = sweep;
+    const bool anew = A.reinv <= 1 || sweep % (uint64_t)A.reinv == 0;
+    const Res res = evaluate<NORD>(s, T, J, E, st, w, v, L, rot, anew, lnd, sgn);
+    lnd = res.lnd;
+    sgn = res.sgn;
+    el = res.eloc;
+    es += el;
+    e2 += el * el;
+    __syncwarp(m);
+  }
+  store(s, st, w, v, L);
+  if (sub == 0) {
+    st.s_esum[w] += es;
+    st.s_e2sum[w] += e2;
+    st.s_acc[w] += acc;
+    st.s_elast[w] = el;
   }
 }
 
