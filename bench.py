@@ -47,13 +47,13 @@ FMA_PER_SM_CLK = {"fp64": 64, "fp32": 128}  # FP64 / FP32 fused multiply-adds pe
 # sweep (k_mv_draw, k_mv_prop, k_mv_pairs, k_mv_walk); None until counted: the roofline's
 # achieved figure is then left out.
 FLOPS_PER_WALKER = {
-    ("cluster128", "eval", "fp64"): 140.56e6,     # CUDA cores 30.05 M + DMMA 110.51 M
+    ("cluster128", "eval", "fp64"): 113.66e6,     # CUDA cores 33.14 M + DMMA 80.51 M
     ("cluster128", "moves", "fp32"): 23.56e6,     # FP32 (plus 2.13 M FP64: the determinant ratios)
     ("cluster128", "sweep", "fp64"): None,
 }
 # DRAM bytes per walker of the same launches (dram__bytes_read.sum + dram__bytes_write.sum).
 DRAM_PER_WALKER = {
-    ("cluster128", "eval", "fp64"): 1644000.0,    # 289.7 MB read + 131.2 MB written / 256
+    ("cluster128", "eval", "fp64"): 1658700.0,    # 287.9 MB read + 136.7 MB written / 256
     ("cluster128", "moves", "fp32"): 293300.0,    # 74.9 MB read + 0.1 MB written / 256
     ("cluster128", "sweep", "fp64"): None,
 }

@@ -411,7 +411,11 @@ int champ_set_mover(champ_ctx *ctx, int32_t imetro, double deltar, double deltat
    a single-determinant context (one centre type where there are e-e-n terms; more than 16 orbitals
    per spin in mixed precision) form all proposals' orbitals and pair values before the first
    decision.  0 runs the single-kernel evaluation (and the fused FP64 sweep kernel) and moves one
-   electron after the other.  The walks are the same.
+   electron after the other.  Gaussian walks are the same; accelerated walks follow the drift and
+   magnify rounding, so those of the two evaluations come apart.  For the same reason a walker's last
+   bits are part of its walk: FP64 walkers of up to 8 electrons are served by other kernels from some
+   hundreds to thousands of walkers on, which keep the bits of the accelerated walks with Gaussian
+   shells up to d and agree to rounding elsewhere.
    "tmoves": 0 (default), 1 or 2 -- T-moves of the variant of champ_tmoves at the start of every
    DMC step (champ_dmc_steps).
    "dmc_ene_int": 1 (default) ene_int_v9 energy integration in the DMC reweighting, 0 none.
@@ -423,7 +427,7 @@ int champ_set_mover(champ_ctx *ctx, int32_t imetro, double deltar, double deltat
    "orb_coop": 1 (default where available: the staged evaluation with electrons and up electrons in
    multiples of 4 and more than 16 orbitals per spin) lets the warps of a block of its orbital part
    share the coefficient stream through shared memory; 0 lets every warp stream it.  Same results.
-   Without effect up to 64 orbitals per spin, which are contracted in tiles.
+   Without effect from 3 to 64 orbitals per spin, which are contracted in tiles.
    "mover_cache": 1 (default) lets the accelerated mover of a mixed single-determinant context
    whose walker state lives in HBM take the drift at an electron's current position from the
    orbital rows of the last FP64 evaluation (updated by its accepted moves) instead of evaluating
@@ -445,12 +449,13 @@ int champ_set_option(champ_ctx *ctx, const char *name, int64_t value);
    Synchronises the stream and resets the sums. */
 int champ_phase_times(champ_ctx *ctx, double *ms /* [4] */, int32_t *launches /* [4] or NULL */);
 /* Autotuning of the launch shapes (no counterpart in the reference): for the options that change
-   only the speed of a VMC sweep -- "delay_rank" (0, 4, 8, 16), "staged_eval" (1, 0), "move_coop"
+   only the speed of a VMC sweep -- "staged_eval" (1, 0), "delay_rank" (0, 4, 8, 16), "move_coop"
    (1, 0), "orb_coop" (1, 0), and with the
    tensor-core orbitals of an FP32 context "orbital_tc" (1, 2) and "orbital_tc_chunk" (2, 4, 8) --
    one option at a time, in that order, times nsweep sweeps of the context's walkers (step size
    step, after one untimed sweep; device time from CUDA events) for each value it accepts, and
-   keeps the fastest.  The probe sweeps move the walkers as equilibration sweeps would.  With
+   keeps the fastest; an option that the sweeps do not read with the present mover and evaluation
+   keeps the value it has.  The probe sweeps move the walkers as equilibration sweeps would.  With
    cache_path (may be NULL) the choice is appended to that text file under a key of the system's
    shape (electrons, centres, basis functions, orbitals, determinants, e-e-n order, pseudopotential,
    precision, walkers), and a later call with the same key applies it without timing.  report
