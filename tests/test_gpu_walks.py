@@ -171,3 +171,30 @@ def test_accelerated_walk_of_few_among_many(case):
     else:
         assert np.array_equal(x0, x1)
         assert np.allclose(l0, l1, rtol=1e-10, atol=1e-10)  # E_L in another order of sums
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1, 0), (2, 1, 1, 0), (3, 2, 2, 4), (4, 4, 1, 4), (5, 3, 2, 5), (7, 4, 3, 4), (3, 2, 12, 4), (2, 1, 20, 5)])
+def test_accelerated_sweeps_at_the_edges_of_the_small_kernel(oracle_mod, shape):
+    """One electron to a spin, one spin, 1 to 4 orbitals (32 to 8 interleaved sums), more centres than lanes: the
+    first of many against the same walkers alone, to the bit, and one sweep against the oracle."""
+    from champ_b200.engine import Engine
+    s = cluster(*shape)
+    x = S.initial_walkers(s, 24, seed=sum(shape))
+    out = []
+    for y in (x, np.resize(x, (1200,) + x.shape[1:])):
+        eng = Engine(s, len(y), "fp64")
+        eng.set_walkers(y)
+        eng.set_mover(6, deltar=5.0, deltat=1.0, fbias=1.0)
+        walk = []
+        for k in range(6):
+            st = eng.vmc_sweeps(1, seed=5, sweep0=k, step=s.step)
+            walk.append((eng.get_walkers()[:24], st["accept"][:24], st["elast"][:24]))
+        out.append(walk)
+        eng.close()
+    for (xa, aa, ea), (xb, ab, eb) in zip(*out):
+        assert np.array_equal(xa, xb) and np.array_equal(aa, ab)
+        assert np.allclose(ea, eb, rtol=1e-9, atol=1e-9)
+    ref = oracle_mod.Oracle(s).vmc_accel(x, 1, seed=5, sweep0=0, deltar=5.0, deltat=1.0, fbias=1.0)
+    same = np.abs(out[1][0][0] - ref["x"]).max(axis=(1, 2)) <= 1e-9
+    assert same.sum() >= 23  # a draw may tie at the last bit
+    assert np.array_equal(out[1][0][1][same], ref["accept"][same])
