@@ -8,6 +8,7 @@
 // shared memory; larger per-walker scratch (orbitals of all electrons, projected
 // coefficients, pseudopotential task lists) in HBM.
 #include <cuda_runtime.h>
+#include <sys/mman.h>
 
 #include <cmath>
 #include <cstdio>
@@ -975,6 +976,13 @@ static int copy_eval_out(champ_ctx *c, const champ_eval_out *o) {
   return CHAMP_OK;
 }
 
+static void release_stage(champ_ctx *c) {
+  if (!c->h_stage) return;
+  cudaHostUnregister(c->h_stage);
+  munmap(c->h_stage, HSTAGE_BYTES);
+  c->h_stage = nullptr;
+}
+
 template <class T>
 static int copy_stats(champ_ctx *c, const champ_vmc_stats *s) {
   State<T> &st = stof<T>(c);
@@ -1620,12 +1628,17 @@ int champ_create(const champ_system *d, int32_t w_max, int32_t precision, void *
   c->d_in = dalloc<double>(c, (size_t)w_max * 3 * c->N);
   c->d_out = dalloc<double>(c, (size_t)w_max * 4 * c->N);
   c->d_mask = dalloc<uint8_t>(c, w_max);
-  // without it (no page-locked memory to be had) the calls copy their arrays directly
-  if (cudaHostAlloc((void **)&c->h_stage, HSTAGE_BYTES, cudaHostAllocMapped) != cudaSuccess ||
-      cudaHostGetDevicePointer((void **)&c->h_stage_dev, c->h_stage, 0) != cudaSuccess) {
-    if (c->h_stage) cudaFreeHost(c->h_stage);
-    c->h_stage = nullptr;
-    cudaGetLastError();
+  // without it (no page-locked memory to be had) the calls copy their arrays directly; registered, not allocated by
+  // CUDA: 0.34 ms against 1.2 to 2.5
+  // (left out of forked children: a copy on write would part the host's pages from the device's)
+  void *m = mmap(nullptr, HSTAGE_BYTES, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+  if (m != MAP_FAILED) {
+    c->h_stage = (char *)m;
+    if (madvise(m, HSTAGE_BYTES, MADV_DONTFORK) != 0 || cudaHostRegister(m, HSTAGE_BYTES, cudaHostRegisterMapped) != cudaSuccess ||
+        cudaHostGetDevicePointer((void **)&c->h_stage_dev, m, 0) != cudaSuccess) {
+      release_stage(c);
+      cudaGetLastError();
+    }
   }
   if (!c->d_in || !c->d_out || !c->d_mask) { champ_destroy(c); return fail(CHAMP_ENOMEM, "staging allocation failed"); }
   {
@@ -1673,7 +1686,7 @@ int champ_destroy(champ_ctx *c) {
   for (void *e : c->ev_pool) cudaEventDestroy((cudaEvent_t)e);
   if (c->cap_stream) cudaStreamDestroy(c->cap_stream);
   for (void *p : c->allocs) cudaFree(p);
-  if (c->h_stage) cudaFreeHost(c->h_stage);
+  release_stage(c);
   if (c->cublas) cublasDestroy((cublasHandle_t)c->cublas);
   delete c;
   return CHAMP_OK;
